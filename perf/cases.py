@@ -376,6 +376,153 @@ def run(state):
     return {n: state.t[n] for n in state.outputs}
 
 
+# ---- the same in 64 bits, in plain torch -----------------------------------------------------------------------------
+class _Plain(_State):
+    """The inputs of a case without the package: no context, dispatches are dropped, caches are filled in torch."""
+
+    class _Hint:
+        @staticmethod
+        def decode_splits_hint(kv, ctx):
+            return 1
+
+    def __init__(self, seed):
+        self.gen = torch.Generator(device="cuda")
+        self.gen.manual_seed(seed)
+        self.rng = np.random.default_rng(seed)
+        self.t, self.b, self.outputs = {}, {}, []
+        self.s = type("NoSession", (), {"ctx": self._Hint})
+        self.cached = {}
+
+    def put(self, name, tensor):
+        self.t[name] = self.b[name] = tensor
+        return tensor
+
+    def call(self, kernel, names, push, groups):
+        pass
+
+    def once(self, kernel, names, push, groups):
+        self.cached[names.split()[1][:-1]] = _q8(self.t["src"])  # "ks" -> k, "gks" -> gk
+
+
+def _q8(x):
+    """The values that Q8_0 keeps of f16 `x` (blocks of 32 along the last dim), as f64: f16 scale times whole number."""
+    b = x.float().reshape(-1, 32)
+    d = b.abs().amax(1, keepdim=True) * torch.tensor(1.0 / 127.0, dtype=torch.float32, device=x.device)
+    whole = torch.round(b * torch.where(d > 0, 1.0 / d, torch.zeros_like(d)))
+    return (d.half().double() * whole.double()).reshape(x.shape)
+
+
+def _norm64(x, w, plus_one=False):
+    x = x.double()
+    y = x * torch.rsqrt((x * x).mean(-1, keepdim=True) + 1e-6)
+    return y if w is None else y * (w.double() + (1.0 if plus_one else 0.0))
+
+
+def _rope64(x, cs):
+    """x [tokens, heads, n]: pair i couples dims (i, i + n / 2); as many pairs turn as the table holds."""
+    half, live = x.shape[-1] // 2, cs.shape[1]
+    c, s = cs[:, None, :, 0].double(), cs[:, None, :, 1].double()
+    lo, hi, y = x[..., :live], x[..., half:half + live], x.clone()
+    y[..., :live], y[..., half:half + live] = lo * c - hi * s, hi * c + lo * s
+    return y
+
+
+def _f16(x):
+    return x.half().double()
+
+
+def _attention64(q, k, v, at, key_at, window=0):
+    """q [m, heads, n] at positions `at`, k and v [keys, kv, n] at `key_at`: causal softmax attention in f64, scale 1 / sqrt(n)
+    except head_dim 256 and 512, whose callers pass 1 / 16 and 512 ** -0.5 (the same values)."""
+    m, heads, n = q.shape
+    kv, out = k.shape[1], torch.empty(q.shape, dtype=torch.float64, device=q.device)
+    rows = max(1, min(m, int(2e8) // k.shape[0]))
+    for h in range(heads):
+        kh, vh = k[:, h * kv // heads].double(), v[:, h * kv // heads].double()
+        for i in range(0, m, rows):
+            s = (q[i:i + rows, h].double() @ kh.T) / math.sqrt(n)
+            back = at[i:i + rows, None] - key_at[None, :]
+            s.masked_fill_((back < 0) | (back >= window) if window else back < 0, -math.inf)
+            out[i:i + rows, h] = torch.softmax(s, -1) @ vh
+    return out
+
+
+def _range(a, b):
+    return torch.arange(a, b, device="cuda")
+
+
+def _over_ring(st, q, kn, vn, q0, n, ring=("k_ring", "v_ring")):
+    """Sliding attention of a chunk from position q0: the ring holds what came before it."""
+    m, first = q.shape[0], max(0, q0 - RING)
+    slots, at = _range(first, q0) % RING, _range(first, q0 + m)
+    k, v = (torch.cat([st.t[r][slots], new.reshape(m, -1)]).reshape(len(at), -1, n) for r, new in zip(ring, (kn, vn)))
+    return _attention64(q, k, v, _range(q0, q0 + m), at, RING)
+
+
+def _after_append(ring, new, q0):
+    last = min(new.shape[0], RING)
+    r = ring.double()
+    r[_range(q0 + new.shape[0] - last, q0 + new.shape[0]) % RING] = new[new.shape[0] - last:].double().reshape(last, -1)
+    return r
+
+
+def exact(case, seed):
+    """What `run` returns, from the same inputs, in f64.  Values that the path stores as f16 or Q8_0 between its steps (normed
+    and rotated heads, caches) are stored so here too; quantised bytes and scales have no 64-bit value (None)."""
+    st = _Plain(seed)
+    c, kind = _arguments(case), case["kind"]
+    _KINDS[kind](st, **c)
+    t, out = st.t, {n: None for n in st.outputs}
+    if kind in ("token", "append"):
+        m, kv, pos = c.get("m", 1), c["kv"], c.get("pos", c.get("ctx", 1) - 1)
+        q = _norm64(t["q_raw"].reshape(m, -1, D), t["q_w"], c["plus_one"])
+        if kind == "append":
+            out["q"] = _rope64(q, t["cs"])
+            return out
+        k = _f16(_rope64(_f16(_norm64(t["k_raw"].reshape(1, kv, D), t["k_w"], c["plus_one"])), t["cs"]))
+        v = _f16(_norm64(t["v_raw"].reshape(1, kv, D), None))
+        out["q"] = _rope64(_f16(q), t["cs"]).reshape(-1, D)
+        keys, values = (torch.cat([st.cached[n][:pos], _q8(x.reshape(1, -1).half())]).reshape(-1, kv, D) for n, x in (("k", k), ("v", v)))
+        out["out"] = _attention64(_f16(out["q"])[None], keys, values, _range(pos, pos + 1), _range(0, pos + 1))[0]
+        return out
+    if kind in ("decode", "paged"):
+        kv, total = c["kv"], c["ctx"] if kind == "decode" else c["q0"] + c["m"]
+        m = t["q"].shape[0]
+        k, v = (st.cached[n].reshape(total, kv, D) for n in "kv")
+        out["out"] = _attention64(t["q"], k, v, _range(total - m, total), _range(0, total))
+        if kind == "decode":
+            out["out"] = out["out"].reshape(-1, D)
+            if m > 1:
+                out["out_sl"] = _over_ring(st, t["q_sl"], t["k_new"], t["v_new"], total - m, D)
+        return out
+    if kind == "linear":
+        out["out"] = _attention64(t["q"], t["k"], t["v"], _range(c["q0"], c["q0"] + c["m"]), _range(0, c["q0"] + c["m"]), c["window"])
+        return out
+    if kind in ("ring", "model_sliding"):
+        out["out"] = _over_ring(st, t["q"], t["k"], t["v"], c["q0"], D if kind == "ring" else 256)
+        out["k_ring"], out["v_ring"] = _after_append(t["k_ring"], t["k"], c["q0"]), _after_append(t["v_ring"], t["v"], c["q0"])
+        return out
+    if kind == "model_global":
+        m, q0 = c["m"], c["q0"]
+        k = torch.cat([st.cached["gk"][:q0], _q8(t["k"])]).reshape(-1, 4, 512)
+        out["gv"] = t["gv"].double()
+        out["gv"][q0:q0 + m] = t["v"].double()
+        out["out"] = _attention64(_q8(t["q"]), k, out["gv"][:q0 + m].reshape(-1, 4, 512), _range(q0, q0 + m), _range(0, q0 + m))
+        return out
+    # model_token
+    pos = c["ctx"] - 1
+    n = {x: _f16(_norm64(t[x + "_raw"], t[x + "_w"] if x[1] in "qk" else None)) for x in ("sq", "sk", "sv", "gq", "gk", "gx")}
+    for x in ("sq", "sk", "gq", "gk"):
+        n[x] = _f16(_rope64(n[x][None], t[x[0] + "_cs"]))[0]
+    out["s_out"] = _over_ring(st, n["sq"][None], n["sk"], n["sv"], pos, 256)[0]
+    out["k_ring"], out["v_ring"] = _after_append(t["k_ring"], n["sk"].reshape(1, -1), pos), _after_append(t["v_ring"], n["sv"].reshape(1, -1), pos)
+    out["gv"] = t["gv"].double()
+    out["gv"][pos] = n["gx"].reshape(-1)
+    keys = torch.cat([st.cached["gk"][:pos], _q8(n["gk"].reshape(1, -1).half())]).reshape(-1, 4, 512)
+    out["g_out"] = _attention64(n["gq"][None], keys, out["gv"].reshape(-1, 4, 512), _range(pos, pos + 1), _range(0, pos + 1))[0]
+    return out
+
+
 # ---- what a pass cannot do without -----------------------------------------------------------------------------------
 def _pairs(m, q0, window=0):
     """Visible (query, key) pairs of m queries from q0 under the causal mask and the window."""
