@@ -1,6 +1,7 @@
 // Internal: what a registry entry is and the launchers each .cu file provides.
 #pragma once
 
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stddef.h>
 #include <stdint.h>
@@ -95,6 +96,14 @@ int launch_combine_ranks_d128(const LaunchArgs&);
 template <int HD, int G, int WINDOW, int RING, int TWO_RANGE, int OUT_F32> int launch_prefill_generic(const LaunchArgs&);
 int launch_prefill_paged_q8kv_scalar_d128(const LaunchArgs&);
 template <int VARIANT> int launch_prefill_global_flash_ref(const LaunchArgs&);
+
+// attn_prefill_wide.cu: the tensor-core form of the reference-shaped prefill kernels (head_dim 256 f16, head_dim 512 int8 Q/K)
+struct KvOperand;
+template <int HD, int G, bool QI8, bool TWO_SRC>
+bool prefill_wide_takes(const LaunchArgs&, const KvOperand& k0, const KvOperand& v0, const KvOperand& k1, const KvOperand& v1, const void* q, float scale);
+template <int HD, int G, bool QI8, bool TWO_SRC>
+int launch_prefill_wide(const LaunchArgs&, const void* q, const __half* q_scales, const KvOperand& k0, const KvOperand& v0, const KvOperand& k1,
+                        const KvOperand& v1, void* out, const void* step, uint32_t n_kv, uint32_t m, uint32_t window, uint32_t ring, float scale);
 
 // attn_exchange.cu
 int launch_reduce_exchange_d128(const LaunchArgs&);

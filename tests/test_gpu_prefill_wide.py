@@ -1,0 +1,162 @@
+"""The tensor-core prefill of the reference-shaped heads (head_dim 256 f16 with a 1024-token window, head_dim 512 with int8
+Q and K) where its tiles can go wrong: query counts around the 32- and 8-token tiles, histories around the 128-key tiles
+and the ring's wrap, rows past the end that hold NaN, values that are not finite, and the calls it leaves to the streaming
+kernel.
+
+Tolerance against the f64 oracle: the output is f16 (relative 2^-11), P keeps 22 bits, sums and exponentials are f32:
+1e-5 of the largest |v| (below 5 for these normals)."""
+import numpy as np
+import pytest
+
+from cases import assert_close, bind
+from oracle import sg_oracle as O
+
+pytestmark = pytest.mark.gpu
+RTOL, ATOL, R, W = 2.0**-11, 5e-5, 1024, 1024
+NAN16 = 0x7E00
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    import super_gemma_b200 as sg
+
+    return sg.GpuContext(0)
+
+
+def _step(ctx, q0):
+    import super_gemma_b200 as sg
+
+    s = ctx.new_step_buffer()
+    sg.StepState(pos=q0, q0=q0).write_to(s)
+    return s
+
+
+def _bits(x):
+    return O.f32_to_f16_bits(np.ascontiguousarray(x, np.float32).ravel()).astype(np.uint16)
+
+
+def _normal(seed, *shape):
+    return np.random.default_rng(seed).standard_normal(shape, dtype=np.float32).astype(np.float16).astype(np.float32)
+
+
+def _sliding(ctx, q, k, v, q0, m, n_kv, ring, scale=0.0625, poison=True):
+    """k, v: rows of positions [first, q0 + m) with first = max(0, q0 - R); linear caches start at position 0 (q0 <= R)."""
+    n_q, row = 2 * n_kv, n_kv * 256
+    up = lambda b: ctx.buffer_from_iter(np.ascontiguousarray(b))
+    out = ctx.new_buffer(m * n_q * 256, np.uint16)
+    kb, vb = _bits(k).reshape(-1, row), _bits(v).reshape(-1, row)
+    junk = np.full((70, row), NAN16, np.uint16) if poison else np.zeros((70, row), np.uint16)
+    if ring:
+        hist = len(kb) - m
+        kr, vr = np.zeros((R, row), np.uint16), np.zeros((R, row), np.uint16)
+        if poison and hist < R:
+            kr[:], vr[:] = NAN16, NAN16
+        for i in range(hist):
+            kr[(q0 - hist + i) % R], vr[(q0 - hist + i) % R] = kb[i], vb[i]
+        bufs = [up(kr), up(vr), up(np.vstack([kb[hist:], junk])), up(np.vstack([vb[hist:], junk]))]
+        name = "attn_prefill_sliding_ring"
+    else:
+        bufs, name = [up(np.vstack([kb, junk])), up(np.vstack([vb, junk]))], "attn_prefill_sliding"
+    ctx.dispatch_blocking(ctx.load_kernel(name), bind(up(_bits(q)), *bufs, out, _step(ctx, q0)), scale, [n_kv, m, 1])
+    return O.f16_bits_to_f32(out.read()).reshape(m, n_q, 256)
+
+
+def _sliding_case(seed, q0, m, n_kv):
+    hist = min(q0, R)
+    return _normal(seed, m, 2 * n_kv, 256), _normal(seed + 1, hist + m, n_kv, 256), _normal(seed + 2, hist + m, n_kv, 256), hist
+
+
+@pytest.mark.parametrize("m", [1, 31, 33, 128, 200])
+@pytest.mark.parametrize("q0", [0, 1, 127, 128, 1000, 1023, 1024])
+@pytest.mark.parametrize("ring", [False, True])
+def test_sliding_edges(ctx, m, q0, ring):
+    q, k, v, hist = _sliding_case(m * 7 + q0, q0, m, 2)
+    got = _sliding(ctx, q, k, v, q0, m, 2, ring)
+    want = O.attention_f64(q, k, v, m, hist, 4, 2, 256, 0.0625, window=W)
+    assert_close(got, want, ATOL, RTOL, f"m={m} q0={q0} ring={ring}")
+
+
+@pytest.mark.parametrize("q0,m", [(1025, 5), (1531, 1300), (70001, 160)])
+def test_sliding_ring_wrapped(ctx, q0, m):
+    q, k, v, hist = _sliding_case(q0, q0, m, 16)
+    got = _sliding(ctx, q, k, v, q0, m, 16, True)
+    toks = np.unique([0, 1, m // 2, m - 1]).astype(np.uint32)
+    want = O.attention_f64(q, k, v, m, hist, 32, 16, 256, 0.0625, window=W, tokens=toks)
+    assert_close(got[toks], want, ATOL, RTOL, f"wrapped q0={q0} m={m}")
+
+
+def _iq(ctx, q, k, v, q0, m, scale=0.044194174, pad=80, v_bits=None):
+    qs, qq, qd = O.q8_quant_div(q.ravel())
+    ks, kq, kd = O.q8_quant_div(k.ravel())
+    up = lambda b: ctx.buffer_from_iter(np.ascontiguousarray(b))
+    tail = np.full(pad * 2048, NAN16, np.uint16)
+    bufs = [up(qq), up(qs), up(np.concatenate([kq, np.full(pad * 2048, 77, np.int8)])),
+            up(np.concatenate([ks.view(np.uint16), np.full(pad * 64, NAN16, np.uint16)])),
+            up(np.concatenate([_bits(v) if v_bits is None else v_bits, tail]))]
+    out = ctx.new_buffer(m * 32 * 512, np.uint16)
+    ctx.dispatch_blocking(ctx.load_kernel("attn_prefill_global_flash_sp_iq"), bind(*bufs, out, _step(ctx, q0)), scale, [32, m // 16, 1])
+    return O.f16_bits_to_f32(out.read()).reshape(m, 32, 512), qd.reshape(q.shape), kd.reshape(k.shape)
+
+
+@pytest.mark.parametrize("m,q0", [(16, 0), (16, 111), (16, 112), (48, 1), (64, 2000), (144, 640)])
+def test_global_int8_edges(ctx, m, q0):
+    q, k, v = _normal(m + q0, m, 32, 512), _normal(m + q0 + 1, q0 + m, 4, 512), _normal(m + q0 + 2, q0 + m, 4, 512)
+    got, qd, kd = _iq(ctx, q, k, v, q0, m)
+    toks = np.unique([0, 1, 7, 8, m - 1]).astype(np.uint32)
+    want = O.attention_f64(qd, kd, v, m, q0, 32, 4, 512, 0.044194174, tokens=toks)
+    assert_close(got[toks], want, ATOL, RTOL, f"iq m={m} q0={q0}")
+    assert np.all(np.isfinite(got))
+
+
+def test_global_int8_peaked_scores(ctx):
+    """Scores that grow along the keys by far more than 2^8: every tile raises the running maximum."""
+    m, q0 = 16, 700
+    q, k, v = _normal(5, m, 32, 512), _normal(6, q0 + m, 4, 512), _normal(7, q0 + m, 4, 512)
+    q = np.repeat(q[:, ::8], 8, axis=1)
+    k += (np.arange(q0 + m)[:, None, None] * 1e-3 * q.mean(0)[::8][None]).astype(np.float16).astype(np.float32)
+    got, qd, kd = _iq(ctx, q, k.astype(np.float16).astype(np.float32), v, q0, m, scale=0.5)
+    want = O.attention_f64(qd, kd, v, m, q0, 32, 4, 512, 0.5)
+    assert_close(got, want, 2 * ATOL, RTOL, "peaked")  # scores of some 60: their rounding moves the exponent by 60 * 2^-24
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+def test_values_that_are_not_finite_reach_only_who_sees_them(ctx, value):
+    m, q0, n_kv, at = 64, 300, 2, 330  # the key at position 330 is seen by queries 30 and later
+    q, k, v, hist = _sliding_case(9, q0, m, n_kv)
+    clean = _sliding(ctx, q, k, v, q0, m, n_kv, True)
+    v2 = v.copy()
+    v2[at, 1, 17] = value
+    got = _sliding(ctx, q, k, v2, q0, m, n_kv, True)
+    # both sides are rounded to f16, and the tile that sees the value is computed by another statement: one f16 step
+    assert_close(got[:30], clean[:30], ATOL, 2 * RTOL, "queries before it")
+    assert_close(got[30:, :2], clean[30:, :2], ATOL, 2 * RTOL, "the other kv head")
+    hit = got[30:, 2:]
+    assert np.all(np.isnan(hit[..., 17]) if np.isnan(value) else hit[..., 17] == value)
+    rest = np.delete(np.arange(256), 17)
+    assert_close(hit[..., rest], clean[30:, 2:][..., rest], ATOL, 2 * RTOL, "its other dims")
+
+
+@pytest.mark.parametrize("scale", [-0.0625, 0.0])
+def test_scales_the_tiles_do_not_take(ctx, scale):
+    q, k, v, hist = _sliding_case(11, 200, 40, 2)
+    got = _sliding(ctx, q, k, v, 200, 40, 2, True, scale=scale, poison=False)
+    want = O.attention_f64(q, k, v, 40, hist, 4, 2, 256, scale, window=W)
+    assert_close(got, want, ATOL, RTOL, f"scale {scale}")
+
+
+def test_keys_past_the_end_of_the_cache_are_reported(ctx):
+    import super_gemma_b200 as sg
+
+    q, k, v, _ = _sliding_case(13, 100, 40, 2)
+    up = lambda b: ctx.buffer_from_iter(np.ascontiguousarray(b))
+    out = ctx.new_buffer(40 * 4 * 256, np.uint16)
+    with pytest.raises(sg.GpuError):
+        ctx.dispatch_blocking(ctx.load_kernel("attn_prefill_sliding"),
+                              bind(up(_bits(q)), up(_bits(k[:120])), up(_bits(v[:120])), out, _step(ctx, 100)), 0.0625, [2, 40, 1])
+    assert np.all(np.isfinite(O.f16_bits_to_f32(out.read())))
+
+
+def test_reruns_give_the_same_bits(ctx):
+    q, k, v, _ = _sliding_case(15, 1500, 96, 16)
+    a, b = (_sliding(ctx, q, k, v, 1500, 96, 16, True) for _ in range(2))
+    assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
