@@ -1,0 +1,573 @@
+// Decode over f16 values: the reference-shaped split-K kernels (head_dim 256 over the ring, head_dim 512 over f16 or Q8_0 keys,
+// head_dim 128 over the ring) and the verify step of up to four drafted tokens over the ring, head_dim 128.
+//
+// All of them are a few query rows (<= 8: the query heads of a kv head, times the drafted tokens) against many keys, bound by
+// the bytes of K and V.  A warp takes 16 keys at a time: their rows arrive by one bulk copy each in the warp's own slots
+// (K and V apart, so that the next K is on its way while this V is used; row pitch + 16 bytes keeps ldmatrix free of bank
+// conflicts), S = K Q^T and O^T += V^T P^T are mma.sync m16n8k16 with the keys or 16 dims as M and the rows as N: tcgen05 has
+// no tile this small.  Warps never wait for one another before the end, where their states merge in warp order.
+// Precision is that of the f32 statement (attn_decode_sliding.wgsl:84-107): Q8_0 keys enter as whole numbers and every block's
+// sum is multiplied by its f32 scale; P = (hi + lo) * 2^-14 with both halves f16 (22 bits, the factor keeps lo out of f16's
+// subnormals); running maximum and sums in f32.
+// Measured (us a call, streaming kernel before -> this one): head_dim 512, Q8_0 keys, 32768 tokens, 32 splits 427 -> 41.8
+// (206 MB, 4.9 TB/s); head_dim 256, 1024 slots, 16 splits 12.3 -> 6.1; verify of 4 tokens over the ring, 16 kv heads about
+// 205 -> 8.
+// Rows that hold no visible key are not copied but zeroed, and a CTA whose result is not finite computes it again by the
+// streaming statement: a tile multiplies by p = 0 what that statement skips.
+#include <mutex>
+#include <string>
+
+#include "attn_stream.cuh"
+#include "sgb_common.cuh"
+#include "sgb_kernels.h"
+
+namespace sgb {
+
+namespace {
+
+constexpr int TILE = 16;
+constexpr float P_SCALE = 16384.0f;
+
+__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
+{
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a)
+{
+    uint32_t d;
+    asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
+    return d;
+}
+__device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t (&r)[4])
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm_x4_trans(uint32_t addr, uint32_t (&r)[4])
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+__device__ __forceinline__ float key_max(float v)
+{
+    v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 4));
+    v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 8));
+    return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 16));
+}
+__device__ __forceinline__ float key_sum(float v)
+{
+    v += __shfl_xor_sync(0xffffffffu, v, 4);
+    v += __shfl_xor_sync(0xffffffffu, v, 8);
+    return v + __shfl_xor_sync(0xffffffffu, v, 16);
+}
+// Four signed bytes as two f16 pairs, exactly: 0x6400 | (q + 128) = q + 1152 as f16.
+__device__ __forceinline__ void bytes_to_f16(uint32_t x, uint32_t& p01, uint32_t& p23)
+{
+    const uint32_t u = x ^ 0x80808080u;
+    uint32_t a = __byte_perm(u, 0x64646464u, 0x4140), b = __byte_perm(u, 0x64646464u, 0x4342);
+    const __half2 off = __float2half2_rn(1152.0f);
+    __half2 ha = __hsub2(*reinterpret_cast<__half2*>(&a), off), hb = __hsub2(*reinterpret_cast<__half2*>(&b), off);
+    p01 = *reinterpret_cast<uint32_t*>(&ha);
+    p23 = *reinterpret_cast<uint32_t*>(&hb);
+}
+
+// Keys of one 16-key tile that are copied: [from, to), row `row0 + i` of the operands; i is also its position minus pos0.
+struct KeyTile {
+    size_t row0;
+    int from, to;
+    int64_t pos0;
+    const KvOperand *k, *v;
+};
+
+template <int HD, bool KQ8, int ROWS>
+struct RowsWarp {
+    static constexpr int K_ROW = HD * (KQ8 ? 1 : 2), K_PITCH = K_ROW + 16, V_PITCH = HD * 2 + 16;
+    static constexpr int SC_ROW = KQ8 ? HD / 16 : 0, SC_PITCH = SC_ROW + (KQ8 ? 16 : 0);
+    struct __align__(16) Slots {
+        uint8_t k[TILE * K_PITCH];
+        uint8_t v[TILE * V_PITCH];  // afterwards the warp's output [ROWS][HD] f32
+        uint8_t sc[TILE * SC_PITCH + 16];
+        uint64_t k_full, v_full;
+        float m[8], l[8];
+    };
+    static_assert(sizeof(Slots::v) >= ROWS * HD * 4, "the V slot doubles as the merge buffer");
+
+    float o[HD / 16][4];  // dims 16c + g, 16c + g + 8 x rows 2*t4, 2*t4 + 1
+    float m[2], l[2];
+
+    // All tiles of this warp.  n tiles; tile(i, KeyTile&) describes the i-th.  row_lo/row_hi: positions rows 2*t4 + e may see.
+    // q_sm: [8][q_pitch] f16 query rows.
+    template <typename TileFn>
+    __device__ __forceinline__ void run(Slots& sl, int n, TileFn tile, const uint8_t* q_sm, int kvh, int n_kv, float scale, const int64_t (&row_lo)[2],
+                                        const int64_t (&row_hi)[2], uint32_t* status)
+    {
+        constexpr int Q_PITCH = HD * 2 + (KQ8 ? 32 : 16);
+        const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+        const uint32_t kb = smem_u32(sl.k), vb = smem_u32(sl.v), sb = smem_u32(sl.sc), kbar = smem_u32(&sl.k_full), vbar = smem_u32(&sl.v_full);
+        const int i16 = lane & 15;
+        auto issue_k = [&](int i) {
+            KeyTile t;
+            tile(i, t);
+            fence_proxy_async_smem();  // the slot was read through the generic proxy
+            if (lane == 0) mbar_arrive_expect_tx(&sl.k_full, (uint32_t)(t.to - t.from) * (K_ROW + SC_ROW));
+            __syncwarp();
+            if (i16 >= t.from && i16 < t.to) {
+                const size_t r = (t.row0 + i16) * n_kv + kvh;
+                if (lane < 16)
+                    bulk_copy(kb + i16 * K_PITCH, (const uint8_t*)t.k->data + r * K_ROW, K_ROW, kbar);
+                else if (KQ8)
+                    bulk_copy(sb + i16 * SC_PITCH, (const uint8_t*)t.k->scales + r * SC_ROW, SC_ROW, kbar);
+            }
+        };
+        auto issue_v = [&](int i) {
+            KeyTile t;
+            tile(i, t);
+            if (lane < 16 && !(i16 >= t.from && i16 < t.to)) {  // p = 0 there, and 0 times a stale Inf or NaN would not be
+                for (int c = 0; c < HD * 2; c += 16) *reinterpret_cast<uint4*>(sl.v + i16 * V_PITCH + c) = make_uint4(0u, 0u, 0u, 0u);
+            }
+            fence_proxy_async_smem();
+            if (lane == 0) mbar_arrive_expect_tx(&sl.v_full, (uint32_t)(t.to - t.from) * HD * 2);
+            __syncwarp();
+            if (lane < 16 && i16 >= t.from && i16 < t.to)
+                bulk_copy(vb + i16 * V_PITCH, (const uint8_t*)t.v->data + ((t.row0 + i16) * n_kv + kvh) * HD * 2, HD * 2, vbar);
+        };
+#pragma unroll
+        for (int c = 0; c < HD / 16; c++) o[c][0] = o[c][1] = o[c][2] = o[c][3] = 0.0f;
+        m[0] = m[1] = NEG_SENTINEL;
+        l[0] = l[1] = 0.0f;
+        bool failed = false;
+        if (n > 0) {
+            issue_k(0);
+            issue_v(0);
+        }
+        const uint32_t k_addr = kb + ((lane & 7) + 8 * ((lane >> 3) & 1)) * K_PITCH + (lane >> 4) * 16;
+        const uint32_t v_addr = vb + ((lane & 7) + 8 * (lane >> 4)) * V_PITCH + ((lane >> 3) & 1) * 16;
+        const uint8_t* q_row = q_sm + g * Q_PITCH + t4 * (KQ8 ? 8 : 4);
+        for (int i = 0; i < n; ++i) {
+            KeyTile t;
+            tile(i, t);
+            mbar_wait(&sl.k_full, i & 1, status, 601, failed);
+            float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // keys g (0, 1) and g + 8 (2, 3) x rows 2*t4, 2*t4 + 1
+            if constexpr (KQ8) {
+                uint4 sa[2], sc[2];  // 16 block scales of keys g and g + 8
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    sa[h] = *reinterpret_cast<const uint4*>(sl.sc + g * SC_PITCH + 16 * h);
+                    sc[h] = *reinterpret_cast<const uint4*>(sl.sc + (g + 8) * SC_PITCH + 16 * h);
+                }
+                const __half* ha = reinterpret_cast<const __half*>(sa);
+                const __half* hc = reinterpret_cast<const __half*>(sc);
+#pragma unroll
+                for (int b = 0; b < HD / 32; b++) {
+                    uint32_t x[4];
+                    ldsm_x4(k_addr + 32 * b, x);
+                    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                    for (int cc = 0; cc < 2; cc++) {
+                        uint32_t a[4];
+                        bytes_to_f16(x[2 * cc], a[0], a[2]);
+                        bytes_to_f16(x[2 * cc + 1], a[1], a[3]);
+                        const uint2 q = *reinterpret_cast<const uint2*>(q_row + (2 * b + cc) * 32);
+                        mma16816(acc, a, q.x, q.y);
+                    }
+                    const float fa = __half2float(ha[b]), fc = __half2float(hc[b]);
+                    s[0] = fmaf(fa, acc[0], s[0]);
+                    s[1] = fmaf(fa, acc[1], s[1]);
+                    s[2] = fmaf(fc, acc[2], s[2]);
+                    s[3] = fmaf(fc, acc[3], s[3]);
+                }
+            } else {
+                float s1[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                for (int c = 0; c < HD / 16; c++) {
+                    uint32_t a[4];
+                    ldsm_x4(k_addr + 32 * c, a);
+                    const uint32_t b0 = *reinterpret_cast<const uint32_t*>(q_row + 32 * c), b1 = *reinterpret_cast<const uint32_t*>(q_row + 32 * c + 16);
+                    mma16816((c & 1) ? s1 : s, a, b0, b1);
+                }
+#pragma unroll
+                for (int e = 0; e < 4; e++) s[e] += s1[e];
+            }
+            __syncwarp();
+            if (i + 1 < n) issue_k(i + 1);
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                s[e] *= scale;
+                const int key = g + 8 * (e >> 1);
+                const int64_t pos = t.pos0 + key;
+                if (key < t.from || key >= t.to || pos < row_lo[e & 1] || pos > row_hi[e & 1]) s[e] = -INFINITY;
+            }
+            float p[4];
+            const float n0 = fmaxf(m[0], key_max(fmaxf(s[0], s[2]))), n1 = fmaxf(m[1], key_max(fmaxf(s[1], s[3])));
+            if (__any_sync(0xffffffffu, n0 != m[0] || n1 != m[1])) {
+                const float c0 = __expf(m[0] - n0), c1 = __expf(m[1] - n1);
+                l[0] *= c0;
+                l[1] *= c1;
+#pragma unroll
+                for (int c = 0; c < HD / 16; c++) {
+                    o[c][0] *= c0;
+                    o[c][1] *= c1;
+                    o[c][2] *= c0;
+                    o[c][3] *= c1;
+                }
+                m[0] = n0;
+                m[1] = n1;
+            }
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                p[e] = __expf(s[e] - m[e & 1]);
+                l[e & 1] += p[e];
+                p[e] *= P_SCALE;
+            }
+            uint32_t hi[2], lo[2];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const uint32_t w = pack_half2(p[2 * h], p[2 * h + 1]);
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
+                hi[h] = movmatrix_trans(w);
+                lo[h] = movmatrix_trans(pack_half2(p[2 * h] - f.x, p[2 * h + 1] - f.y));
+            }
+            mbar_wait(&sl.v_full, i & 1, status, 602, failed);
+#pragma unroll
+            for (int c = 0; c < HD / 16; c++) {
+                uint32_t a[4];
+                ldsm_x4_trans(v_addr + 32 * c, a);
+                mma16816(o[c], a, hi[0], hi[1]);
+                mma16816(o[c], a, lo[0], lo[1]);
+            }
+            __syncwarp();
+            if (i + 1 < n) issue_v(i + 1);
+        }
+        // the state for the merge: [row][HD], m, l
+        l[0] = key_sum(l[0]);
+        l[1] = key_sum(l[1]);
+        float* dst = reinterpret_cast<float*>(sl.v);
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int r = 2 * t4 + e;
+            if (r < ROWS) {
+#pragma unroll
+                for (int c = 0; c < HD / 16; c++) {
+                    dst[r * HD + 16 * c + g] = o[c][e] * (1.0f / P_SCALE);
+                    dst[r * HD + 16 * c + g + 8] = o[c][2 + e] * (1.0f / P_SCALE);
+                }
+                if (g == 0) {
+                    sl.m[r] = m[e];
+                    sl.l[r] = l[e];
+                }
+            }
+        }
+    }
+};
+
+// Query rows -> shared memory, [8][HD] f16 with the pitch the MMAs want; rows >= live are zero.
+template <int HD, bool KQ8, typename RowPtr>
+__device__ __forceinline__ void stage_queries(uint8_t* q_sm, int live, RowPtr row_ptr)
+{
+    constexpr int Q_PITCH = HD * 2 + (KQ8 ? 32 : 16);
+    for (int i = threadIdx.x; i < 8 * HD / 8; i += blockDim.x) {
+        const int r = i / (HD / 8), c = i % (HD / 8);
+        uint4 u = make_uint4(0u, 0u, 0u, 0u);
+        if (r < live) u = __ldg(reinterpret_cast<const uint4*>(row_ptr(r)) + c);
+        *reinterpret_cast<uint4*>(q_sm + r * Q_PITCH + 16 * c) = u;
+    }
+}
+
+template <int HD, int G, bool KQ8, int WARPS>
+struct DecodeRowsSmem {
+    uint8_t q[8 * (HD * 2 + (KQ8 ? 32 : 16))];
+    typename RowsWarp<HD, KQ8, G>::Slots w[WARPS];
+};
+
+// Split-K partials.  Grid, split ranges and partials as decode_generic_kernel.
+template <int HD, int G, bool KQ8, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) decode_rows_kernel(const __half* __restrict__ q, const __grid_constant__ KvOperand kop,
+                                                                 const __grid_constant__ KvOperand vop, float* __restrict__ part,
+                                                                 const uint32_t* __restrict__ step, int step_slot, uint32_t n_splits, float scale,
+                                                                 uint32_t* status)
+{
+    using W = RowsWarp<HD, KQ8, G>;
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    DecodeRowsSmem<HD, G, KQ8, WARPS>& sm = *reinterpret_cast<DecodeRowsSmem<HD, G, KQ8, WARPS>*>(smem_raw);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int kvh = blockIdx.x, n_kv = gridDim.x, split = blockIdx.y, n_q = n_kv * G;
+    const uint32_t i = blockIdx.z, m_q = gridDim.z;
+    if (lane == 0) {
+        mbar_init(&sm.w[warp].k_full, 1);
+        mbar_init(&sm.w[warp].v_full, 1);
+        mbar_fence_init();
+    }
+    pdl_wait();
+    pdl_launch_dependents();
+    const uint32_t kv_len = __ldg(step + step_slot);
+    const uint32_t chunk = (kv_len + n_splits - 1) / n_splits;
+    const uint32_t t_begin = min((uint32_t)split * chunk, kv_len);
+    uint32_t t_end = min(t_begin + chunk, kv_len);
+    const uint32_t vis_end = kv_len + i >= m_q ? kv_len + i - m_q + 1 : 0;  // query i of m_q sees t <= kv_len - m_q + i
+    t_end = min(t_end, vis_end);
+    const size_t have = min(kop.rows, vop.rows);
+    if (t_end > t_begin && t_end > have) {
+        if (threadIdx.x == 0) report_error(status, DEV_ERR_BOUNDS, kop.rows <= vop.rows ? 202 : 204, (uint32_t)have, (uint32_t)have);
+        t_end = max((uint32_t)have, t_begin);
+    }
+    const int tiles = t_end > t_begin ? (int)((t_end - t_begin + TILE - 1) / TILE) : 0;
+    auto q_row = [&](int r) { return q + ((size_t)i * n_q + kvh * G + r) * HD; };
+    stage_queries<HD, KQ8>(sm.q, G, q_row);
+    __syncthreads();
+    W w;
+    const int64_t lo[2] = {0, 0}, hi[2] = {INT64_MAX, INT64_MAX};
+    w.run(sm.w[warp], tiles > warp ? (tiles - warp + WARPS - 1) / WARPS : 0,
+          [&](int n, KeyTile& t) {
+              t.row0 = t_begin + (size_t)(warp + n * WARPS) * TILE;
+              t.from = 0;
+              t.to = (int)min((size_t)TILE, t_end - t.row0);
+              t.pos0 = 0;
+              t.k = &kop;
+              t.v = &vop;
+          },
+          sm.q, kvh, n_kv, scale, lo, hi, status);
+    __syncthreads();
+    bool odd = false;
+    for (int idx = threadIdx.x; idx < G * HD; idx += WARPS * 32) {
+        const int r = idx / HD, d = idx % HD;
+        float big = sm.w[0].m[r];
+#pragma unroll
+        for (int k = 1; k < WARPS; k++) big = fmaxf(big, sm.w[k].m[r]);
+        float acc = 0.0f, l = 0.0f;
+#pragma unroll
+        for (int k = 0; k < WARPS; k++) {
+            const float f = __expf(sm.w[k].m[r] - big);
+            acc = fmaf(f, reinterpret_cast<const float*>(sm.w[k].v)[idx], acc);
+            l = fmaf(f, sm.w[k].l[r], l);
+        }
+        odd |= !(fabsf(acc) <= 3.4e38f) || !(fabsf(l) <= 3.4e38f);
+        float* row = part + (((size_t)i * n_q + kvh * G + r) * n_splits + split) * (HD + 2);
+        row[d] = acc;
+        if (d == 0) {
+            row[HD] = big;
+            row[HD + 1] = l;
+        }
+    }
+    if (__syncthreads_or(odd)) {  // again by the streaming statement, a warp per row
+        constexpr int DPL = HD / 32;
+        for (int r = warp; r < G; r += WARPS) {
+            float qr[DPL], kk[DPL], vv[DPL];
+            load_f16<DPL>(q_row(r) + lane * DPL, qr);
+            Stream<1, DPL> st;
+            st.init();
+            for (size_t t = t_begin; t < t_end; t++) {
+                load_row<HD, KQ8 ? FMT_Q8 : FMT_F16, DPL>(kop, t, kvh, n_kv, lane * DPL, kk);
+                load_row<HD, FMT_F16, DPL>(vop, t, kvh, n_kv, lane * DPL, vv);
+                st.step(0, qr, kk, vv, scale);
+            }
+            float* row = part + (((size_t)i * n_q + kvh * G + r) * n_splits + split) * (HD + 2);
+#pragma unroll
+            for (int d = 0; d < DPL; d++) row[lane * DPL + d] = st.acc[0][d];
+            if (lane == 0) {
+                row[HD] = st.m[0];
+                row[HD + 1] = st.l[0];
+            }
+        }
+    }
+}
+
+// ---- verify over the ring: m <= 4 tokens x 2 heads = 8 rows, a cluster of 8 CTAs per kv head ------------------------------
+constexpr int V_HD = 128, V_G = 2, V_WARPS = 4, V_CTAS = 8, V_DPL = V_HD / 32;
+
+struct VerifySmem {
+    uint8_t q[8 * (V_HD * 2 + 16)];
+    RowsWarp<V_HD, false, 8>::Slots w[V_WARPS];
+    float acc[8][V_HD], m[8], l[8];  // this CTA's merged rows, read by the cluster
+};
+
+__device__ __forceinline__ const float* map_to_rank(const float* p, uint32_t rank)
+{
+    uint64_t out;
+    asm("mapa.u64 %0, %1, %2;" : "=l"(out) : "l"(reinterpret_cast<uint64_t>(p)), "r"(rank));
+    return reinterpret_cast<const float*>(out);
+}
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__global__ void __cluster_dims__(V_CTAS, 1, 1) __launch_bounds__(V_WARPS * 32)
+    verify_ring_kernel(const __half* __restrict__ q, const __grid_constant__ KvOperand k_ring, const __grid_constant__ KvOperand v_ring,
+                       const __grid_constant__ KvOperand k_new, const __grid_constant__ KvOperand v_new, float* __restrict__ out,
+                       const uint32_t* __restrict__ step, uint32_t n_kv, uint32_t m_q, uint32_t window, uint32_t ring, float scale, uint32_t* status)
+{
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    VerifySmem& sm = *reinterpret_cast<VerifySmem*>(smem_raw);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t4 = lane & 3;
+    const int kvh = blockIdx.x / V_CTAS, rank = blockIdx.x % V_CTAS, n_q = (int)n_kv * V_G, rows = (int)m_q * V_G;
+    if (lane == 0) {
+        mbar_init(&sm.w[warp].k_full, 1);
+        mbar_init(&sm.w[warp].v_full, 1);
+        mbar_fence_init();
+    }
+    pdl_wait();
+    pdl_launch_dependents();
+    const int64_t q0 = __ldg(step + STEP_Q0);
+    const int64_t band_lo = q0 + 1 > window ? q0 + 1 - window : 0;  // the first query's
+    const int64_t first = band_lo / TILE * TILE;
+    const int n_hist = q0 > band_lo ? (int)((q0 - 1) / TILE - first / TILE + 1) : 0, tiles = n_hist + 1;  // the draft is one tile
+    auto q_row = [&](int r) { return q + ((size_t)(r / V_G) * n_q + kvh * V_G + r % V_G) * V_HD; };
+    stage_queries<V_HD, false>(sm.q, rows, q_row);
+    __syncthreads();
+    int64_t lo[2], hi[2];
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+        const int64_t qpos = q0 + min(2 * t4 + e, rows - 1) / V_G;
+        lo[e] = qpos + 1 > window ? qpos + 1 - window : 0;
+        hi[e] = qpos;
+    }
+    const int me = rank * V_WARPS + warp;
+    RowsWarp<V_HD, false, 8> w;
+    w.run(sm.w[warp], tiles > me ? (tiles - me + V_CTAS * V_WARPS - 1) / (V_CTAS * V_WARPS) : 0,
+          [&](int n, KeyTile& t) {
+              const int it = me + n * V_CTAS * V_WARPS;
+              if (it < n_hist) {
+                  t.pos0 = first + (int64_t)it * TILE;
+                  t.row0 = (size_t)(t.pos0 % ring);
+                  t.from = (int)max((int64_t)0, band_lo - t.pos0);
+                  t.to = (int)min((int64_t)TILE, q0 - t.pos0);
+                  t.k = &k_ring;
+                  t.v = &v_ring;
+              } else {
+                  t.pos0 = q0;
+                  t.row0 = 0;
+                  t.from = 0;
+                  t.to = (int)m_q;
+                  t.k = &k_new;
+                  t.v = &v_new;
+              }
+          },
+          sm.q, kvh, (int)n_kv, scale, lo, hi, status);
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < 8 * V_HD; idx += V_WARPS * 32) {
+        const int r = idx / V_HD, d = idx % V_HD;
+        float big = sm.w[0].m[r];
+#pragma unroll
+        for (int k = 1; k < V_WARPS; k++) big = fmaxf(big, sm.w[k].m[r]);
+        float acc = 0.0f, l = 0.0f;
+#pragma unroll
+        for (int k = 0; k < V_WARPS; k++) {
+            const float f = __expf(sm.w[k].m[r] - big);
+            acc = fmaf(f, reinterpret_cast<const float*>(sm.w[k].v)[idx], acc);
+            l = fmaf(f, sm.w[k].l[r], l);
+        }
+        sm.acc[r][d] = acc;
+        if (d == 0) {
+            sm.m[r] = big;
+            sm.l[r] = l;
+        }
+    }
+    cluster_sync();
+    bool odd = false;
+    if (rank < rows) {  // CTA `rank` owns row `rank`: merge the cluster's states in rank order
+        const int d = threadIdx.x;  // V_WARPS * 32 == V_HD
+        float mk[V_CTAS], big = NEG_SENTINEL;
+#pragma unroll
+        for (int k = 0; k < V_CTAS; k++) {
+            mk[k] = *map_to_rank(&sm.m[rank], k);
+            big = fmaxf(big, mk[k]);
+        }
+        float acc = 0.0f, l = 0.0f;
+#pragma unroll
+        for (int k = 0; k < V_CTAS; k++) {
+            const float f = __expf(mk[k] - big);
+            acc = fmaf(f, *map_to_rank(&sm.acc[rank][d], k), acc);
+            l = fmaf(f, *map_to_rank(&sm.l[rank], k), l);
+        }
+        const float y = acc / l;
+        odd = !(fabsf(y) <= 3.4e38f);
+        out[((size_t)(rank / V_G) * n_q + kvh * V_G + rank % V_G) * V_HD + d] = y;
+    }
+    cluster_sync();  // nobody leaves while its shared memory is read
+    if (__syncthreads_or(odd) && warp == 0) {  // this CTA's row again, by the streaming statement
+        const uint32_t i = rank / V_G, qpos = (uint32_t)q0 + i, begin = qpos + 1 > window ? qpos + 1 - window : 0;
+        float qr[V_DPL], kk[V_DPL], vv[V_DPL];
+        load_f16<V_DPL>(q_row(rank) + lane * V_DPL, qr);
+        Stream<1, V_DPL> st;
+        st.init();
+        for (uint32_t t = begin; t <= qpos; t++) {
+            const bool old = t < (uint32_t)q0;
+            const size_t row = old ? t % ring : t - (uint32_t)q0;
+            load_row<V_HD, FMT_F16, V_DPL>(old ? k_ring : k_new, row, kvh, (int)n_kv, lane * V_DPL, kk);
+            load_row<V_HD, FMT_F16, V_DPL>(old ? v_ring : v_new, row, kvh, (int)n_kv, lane * V_DPL, vv);
+            st.step(0, qr, kk, vv, scale);
+        }
+#pragma unroll
+        for (int d = 0; d < V_DPL; d++) out[((size_t)i * n_q + kvh * V_G + rank % V_G) * V_HD + lane * V_DPL + d] = st.acc[0][d] / st.l[0];
+    }
+}
+
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+template <typename Kern>
+int allow_smem(const LaunchArgs& a, Kern kern, size_t smem)
+{
+    static std::mutex attr_mutex;
+    static bool attr_set[64] = {};
+    std::lock_guard<std::mutex> lock(attr_mutex);
+    if (a.device < 64 && attr_set[a.device]) return 0;
+    if (int r = check_cuda(a, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "cudaFuncSetAttribute(decode_rows)")) return r;
+    if (a.device < 64) attr_set[a.device] = true;
+    return 0;
+}
+
+}  // namespace
+
+// The bulk copies need 16-byte aligned bases; anything else stays on the streaming kernel.
+bool decode_rows_takes(const KvOperand& k, const KvOperand& v, const void* q)
+{
+    return aligned16(k.data) && aligned16(v.data) && aligned16(q) && (k.scales == nullptr || aligned16(k.scales));
+}
+
+template <int HD, int G, bool KQ8>
+int launch_decode_rows(const LaunchArgs& a, const void* q, const KvOperand& k, const KvOperand& v, void* part, const void* step, int step_slot,
+                       uint32_t n_kv, uint32_t n_splits, uint32_t m_q, float scale)
+{
+    // warps per CTA: what fits the shared memory at head_dim 512 (one CTA per SM), four elsewhere (three or more CTAs per SM)
+    constexpr int WARPS = HD == 512 ? (KQ8 ? 8 : 6) : 4;
+    constexpr size_t smem = sizeof(DecodeRowsSmem<HD, G, KQ8, WARPS>);
+    static_assert(smem <= 227 * 1024, "one CTA per SM");
+    auto kern = decode_rows_kernel<HD, G, KQ8, WARPS>;
+    {
+        static std::mutex attr_mutex;
+        static bool attr_set[64] = {};
+        std::lock_guard<std::mutex> lock(attr_mutex);
+        if (a.device >= 64 || !attr_set[a.device]) {
+            if (int r = check_cuda(a, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "cudaFuncSetAttribute(decode_rows)")) return r;
+            if (a.device < 64) attr_set[a.device] = true;
+        }
+    }
+    const cudaError_t e = launch_dependent(kern, dim3(n_kv, n_splits, m_q), dim3(WARPS * 32), smem, a.stream, (const __half*)q, k, v, (float*)part,
+                                           (const uint32_t*)step, step_slot, n_splits, scale, a.status);
+    ++*a.launches;
+    return check_cuda(a, e, "attn_decode");
+}
+template int launch_decode_rows<256, 2, false>(const LaunchArgs&, const void*, const KvOperand&, const KvOperand&, void*, const void*, int, uint32_t, uint32_t, uint32_t, float);
+template int launch_decode_rows<512, 8, false>(const LaunchArgs&, const void*, const KvOperand&, const KvOperand&, void*, const void*, int, uint32_t, uint32_t, uint32_t, float);
+template int launch_decode_rows<512, 8, true>(const LaunchArgs&, const void*, const KvOperand&, const KvOperand&, void*, const void*, int, uint32_t, uint32_t, uint32_t, float);
+template int launch_decode_rows<128, 2, false>(const LaunchArgs&, const void*, const KvOperand&, const KvOperand&, void*, const void*, int, uint32_t, uint32_t, uint32_t, float);
+
+int launch_verify_ring_d128(const LaunchArgs& a, const void* q, const KvOperand& k_ring, const KvOperand& v_ring, const KvOperand& k_new,
+                            const KvOperand& v_new, void* out, const void* step, uint32_t n_kv, uint32_t m, uint32_t window, uint32_t ring, float scale)
+{
+    constexpr size_t smem = sizeof(VerifySmem);
+    static_assert(smem <= 100 * 1024, "two or more CTAs per SM");
+    if (int r = allow_smem(a, verify_ring_kernel, smem)) return r;
+    const cudaError_t e = launch_dependent(verify_ring_kernel, dim3(n_kv * V_CTAS), dim3(V_WARPS * 32), smem, a.stream, (const __half*)q, k_ring, v_ring,
+                                           k_new, v_new, (float*)out, (const uint32_t*)step, n_kv, m, window, ring, scale, a.status);
+    ++*a.launches;
+    return check_cuda(a, e, "attn_verify_sliding_ring");
+}
+
+}  // namespace sgb

@@ -249,6 +249,8 @@ int launch_decode_generic(const LaunchArgs& a)
     if (q.bytes < m_q * n_q * HD * 2) return fail_validation(a, "decode: q buffer too small");
     if (int r = need_bytes(a, part_i, m_q * n_q * p.n_splits * (HD + 2) * 4, "part")) return r;
     if (int r = need_bytes(a, step_i, 16, "step")) return r;
+    if (decode_rows_takes(kop, vop, q.ptr))
+        return launch_decode_rows<HD, G, KFMT == FMT_Q8>(a, q.ptr, kop, vop, a.b[part_i].ptr, a.b[step_i].ptr, STEP_SLOT, n_kv, p.n_splits, m_q, p.scale);
     decode_generic_kernel<HD, G, KFMT, VFMT><<<dim3(n_kv, p.n_splits, m_q), GEN_THREADS, 0, a.stream>>>(
         (const __half*)q.ptr, kop, vop, (float*)a.b[part_i].ptr, (const uint32_t*)a.b[step_i].ptr, STEP_SLOT, p.n_splits,
         p.scale, a.status);
@@ -353,6 +355,11 @@ int launch_prefill_generic(const LaunchArgs& a)
     if (a.b[0].bytes < m * n_q * HD * 2) return fail_validation(a, "attn_prefill: q buffer too small");
     if (int r = need_bytes(a, bi, m * n_q * HD * (OUT_F32 ? 4 : 2), "out")) return r;
     if (int r = need_bytes(a, bi + 1, 16, "step")) return r;
+    if constexpr (HD == 128 && TWO_RANGE) {
+        // up to four queries are the eight rows of one MMA column; more queries are the streaming kernel's (or the flash kernel's)
+        if (m <= 4 && decode_rows_takes(kh, vh, a.b[0].ptr) && decode_rows_takes(kc, vc, a.b[0].ptr))
+            return launch_verify_ring_d128(a, a.b[0].ptr, kh, vh, kc, vc, a.b[bi].ptr, a.b[bi + 1].ptr, n_kv, (uint32_t)m, WINDOW, RING, scale);
+    }
     if constexpr (HD == 256 && !OUT_F32) {
         if (prefill_wide_takes<HD, G, false, TWO_RANGE != 0>(a, kh, vh, kc, vc, a.b[0].ptr, scale))
             return launch_prefill_wide<HD, G, false, TWO_RANGE != 0>(a, a.b[0].ptr, nullptr, kh, vh, kc, vc, a.b[bi].ptr, a.b[bi + 1].ptr, n_kv,

@@ -97,8 +97,16 @@ template <int HD, int G, int WINDOW, int RING, int TWO_RANGE, int OUT_F32> int l
 int launch_prefill_paged_q8kv_scalar_d128(const LaunchArgs&);
 template <int VARIANT> int launch_prefill_global_flash_ref(const LaunchArgs&);
 
-// attn_prefill_wide.cu: the tensor-core form of the reference-shaped prefill kernels (head_dim 256 f16, head_dim 512 int8 Q/K)
+// attn_decode_rows.cu: split-K decode over f16 values and the draft's verify over the ring, on warp-level MMAs
 struct KvOperand;
+bool decode_rows_takes(const KvOperand& k, const KvOperand& v, const void* q);
+template <int HD, int G, bool KQ8>
+int launch_decode_rows(const LaunchArgs&, const void* q, const KvOperand& k, const KvOperand& v, void* part, const void* step, int step_slot,
+                       uint32_t n_kv, uint32_t n_splits, uint32_t m_q, float scale);
+int launch_verify_ring_d128(const LaunchArgs&, const void* q, const KvOperand& k_ring, const KvOperand& v_ring, const KvOperand& k_new,
+                            const KvOperand& v_new, void* out, const void* step, uint32_t n_kv, uint32_t m, uint32_t window, uint32_t ring, float scale);
+
+// attn_prefill_wide.cu: the tensor-core form of the reference-shaped prefill kernels (head_dim 256 f16, head_dim 512 int8 Q/K)
 template <int HD, int G, bool QI8, bool TWO_SRC>
 bool prefill_wide_takes(const LaunchArgs&, const KvOperand& k0, const KvOperand& v0, const KvOperand& k1, const KvOperand& v1, const void* q, float scale);
 template <int HD, int G, bool QI8, bool TWO_SRC>
