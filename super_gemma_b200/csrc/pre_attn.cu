@@ -227,59 +227,143 @@ __device__ __forceinline__ void quant_oct_f32(const float (&x)[8], __half& scale
     packed = make_uint2(p[0], p[1]);
 }
 
-// kv_norm_rope_append_paged_q8_d128: three warp-aligned segments of 16 threads per row: K rows (norm with k_w, rope),
-// V rows (weightless norm), both landing Q8_0-quantised at row page_table[t / page] * page + t % page with
-// t = step[0] + token; and, for qkv_norm_rope_append_paged_q8_d128, Q rows (norm with q_w, rope, f16 out): the
-// whole pre-attention step of a layer in one launch.
+// kv_norm_rope_append_paged_q8_d128: K rows (norm with k_w, rope) and V rows (weightless norm), both landing Q8_0-quantised at
+// row page_table[t / page] * page + t % page with t = step[0] + token; and, for qkv_norm_rope_append_paged_q8_d128, Q rows
+// (norm with q_w, rope, f16 out): the whole pre-attention step of a layer in one launch.
+//
+// A block works on one token (blockIdx.x) and, of that token's rows (q heads, k heads, v heads in this order), on every
+// gridDim.y-th group of ROWS_PER_PASS: a thread keeps its octet of dims for all of them, so the token's cos/sin values and the
+// page lookup are read once and stay in registers instead of once per row (they were four times the bytes of a row's own
+// octet, and made the kernel issue-bound).  The launcher gives a long chunk one block per token and a short one as
+// many blocks per token as there are groups, where latency counts.
+constexpr int ROWS_PER_PASS = PRE_THREADS / 16;
+
 template <bool PLUS_ONE>
 __global__ void __launch_bounds__(PRE_THREADS)
     kv_norm_rope_append_kernel(const __half* __restrict__ q_raw, const float* __restrict__ q_w, __half* __restrict__ q_out,
-                               uint32_t n_q, uint32_t q_rows,
-                               const __half* __restrict__ k_raw, const __half* __restrict__ v_raw, const float* __restrict__ k_w,
+                               uint32_t n_q, const __half* __restrict__ k_raw, const __half* __restrict__ v_raw, const float* __restrict__ k_w,
                                const float2* __restrict__ cos_sin, __half* __restrict__ k_scales, int8_t* __restrict__ k_quants,
                                __half* __restrict__ v_scales, int8_t* __restrict__ v_quants, const uint32_t* __restrict__ page_table,
                                uint32_t table_len, uint32_t page, const uint32_t* __restrict__ step, uint32_t n_kv, uint32_t half_rot,
-                               uint32_t kv_rows, size_t dst_rows, uint32_t* status)
+                               size_t dst_rows, uint32_t* status)
 {
     pdl_wait();  // the raw q, k, v rows come from earlier kernels of the stream
     pdl_launch_dependents();
-    // 32-bit index arithmetic (the host checks the thread count < 2^32): 64-bit divisions would cost more than the rest
-    const uint32_t g = blockIdx.x * PRE_THREADS + threadIdx.x;
-    const uint32_t seg = (kv_rows * 16 + 31) / 32 * 32;  // threads per K or V segment: whole warps
-    float v[8];
-    if (g >= 2 * seg) {
-        const uint32_t row = (g - 2 * seg) >> 4;
-        const int o = (int)(g & 15);
-        const bool live = row < q_rows;
-        norm_rope_oct_d128<PLUS_ONE>(q_raw + (size_t)row * 128, q_w, cos_sin + (size_t)(row / n_q) * half_rot, half_rot, o, live, v);
-        if (live) *reinterpret_cast<uint4*>(q_out + (size_t)row * 128 + 8 * o) = pack_f16x8(v);
-        return;
+    const uint32_t token = blockIdx.x, rows = n_q + 2 * n_kv;
+    const int o = threadIdx.x & 15, slot = threadIdx.x >> 4;
+    // rotation: dims [8 o, 8 o + 8) pair with +-64; half_rot is a multiple of 8 (checked on the host), so a whole octet turns or none
+    const uint32_t pair0 = (uint32_t)(o & 7) * 8;
+    const bool turns = pair0 < half_rot;
+    float c[8], sn[8];
+    if (turns) {
+        const float4* cp = reinterpret_cast<const float4*>(cos_sin + (size_t)token * half_rot + pair0);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float4 cs = __ldg(cp + j);
+            c[2 * j] = cs.x;
+            c[2 * j + 1] = cs.z;
+            // low half: lo*c - hi*s with lo = own; high half: hi*c + lo*s with hi = own (x - y is x + (-y), bit for bit)
+            sn[2 * j] = o < 8 ? -cs.y : cs.y;
+            sn[2 * j + 1] = o < 8 ? -cs.w : cs.w;
+        }
     }
-    const bool is_v = g >= seg;
-    const uint32_t row = (is_v ? g - seg : g) >> 4;  // (token, kv head)
-    const int o = (int)(g & 15);
-    const bool live = row < kv_rows;
-    const uint32_t token = row / n_kv, head = row - token * n_kv;
-    norm_rope_oct_d128<PLUS_ONE>((is_v ? v_raw : k_raw) + (size_t)row * 128, is_v ? nullptr : k_w, cos_sin + (size_t)token * half_rot,
-                                 is_v ? 0u : half_rot, o, live, v);
-    __half s;
-    uint2 packed;
-    quant_oct_f32(v, s, packed);
-    if (!live) return;
-    const uint32_t t = __ldg(step + STEP_POS) + token;
-    const uint32_t p = t / page;
-    if (p >= table_len) {
-        report_error(status, DEV_ERR_BOUNDS, 104, p, table_len);
-        return;
+    size_t dst_row = 0;
+    bool placed = true;
+    {
+        const uint32_t t = __ldg(step + STEP_POS) + token, p = t / page;
+        if (p < table_len) dst_row = (size_t)__ldg(page_table + p) * page + (t - p * page);
+        placed = p < table_len && dst_row < dst_rows;
+        if (!placed && threadIdx.x == 0 && blockIdx.y == 0) {
+            if (p >= table_len)
+                report_error(status, DEV_ERR_BOUNDS, 104, p, table_len);
+            else
+                report_error(status, DEV_ERR_BOUNDS, 105, (uint32_t)dst_row, (uint32_t)dst_rows);
+        }
     }
-    const size_t dst_row = (size_t)__ldg(page_table + p) * page + (t - p * page);
-    if (dst_row >= dst_rows) {
-        report_error(status, DEV_ERR_BOUNDS, 105, (uint32_t)dst_row, (uint32_t)dst_rows);
-        return;
+    auto octet = [&](uint32_t r) {
+        if (r >= rows) return make_uint4(0u, 0u, 0u, 0u);
+        const __half* src = r < n_q           ? q_raw + ((size_t)token * n_q + r) * 128
+                            : r < n_q + n_kv ? k_raw + ((size_t)token * n_kv + (r - n_q)) * 128
+                                             : v_raw + ((size_t)token * n_kv + (r - n_q - n_kv)) * 128;
+        return __ldg(reinterpret_cast<const uint4*>(src + 8 * o));
+    };
+    uint4 next = octet(blockIdx.y * ROWS_PER_PASS + slot);
+    for (uint32_t r0 = blockIdx.y * ROWS_PER_PASS; r0 < rows; r0 += gridDim.y * ROWS_PER_PASS) {
+        const uint32_t r = r0 + slot;
+        const bool live = r < rows, is_q = r < n_q, is_v = r >= n_q + n_kv;
+        const uint32_t head = is_q ? r : is_v ? r - n_q - n_kv : r - n_q;
+        float v[8];
+        const uint4 u = next;
+        next = octet(r + gridDim.y * ROWS_PER_PASS);  // on its way while this row is worked on
+        float wv[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) wv[i] = 1.0f;
+        if (live && !is_v) {
+            const float* w = (is_q ? q_w : k_w) + 8 * o;
+            const float4 w0 = __ldg(reinterpret_cast<const float4*>(w)), w1 = __ldg(reinterpret_cast<const float4*>(w) + 1);
+            const float x[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+            for (int i = 0; i < 8; i++) wv[i] = PLUS_ONE ? 1.0f + x[i] : x[i];
+        }
+        {
+            const __half2* h = reinterpret_cast<const __half2*>(&u);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const float2 f = __half22float2(h[j]);
+                v[2 * j] = f.x;
+                v[2 * j + 1] = f.y;
+            }
+        }
+        float ss = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 8; i++) ss = fmaf(v[i], v[i], ss);
+#pragma unroll
+        for (int d = 1; d < 16; d <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);  // fixed tree: every lane gets the same bits
+        const float inv = rsqrtf(ss / 128.0f + RMS_EPS);
+        uint32_t own[4];  // the normed octet as f16 pairs: what the chain of kernels stores between norm and rotation
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            own[j] = pack_half2(v[2 * j] * inv * wv[2 * j], v[2 * j + 1] * inv * wv[2 * j + 1]);
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&own[j]));
+            v[2 * j] = f.x;
+            v[2 * j + 1] = f.y;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const uint32_t other = __shfl_xor_sync(0xffffffffu, own[j], 8);  // the partner octet, dims +-64
+            if (turns && !is_v) {
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&other));
+                const float a = __fadd_rn(__fmul_rn(v[2 * j], c[2 * j]), __fmul_rn(f.x, sn[2 * j]));
+                const float b = __fadd_rn(__fmul_rn(v[2 * j + 1], c[2 * j + 1]), __fmul_rn(f.y, sn[2 * j + 1]));
+                own[j] = pack_half2(a, b);
+                const float2 y = __half22float2(*reinterpret_cast<const __half2*>(&own[j]));
+                v[2 * j] = y.x;
+                v[2 * j + 1] = y.y;
+            }
+        }
+        if (r0 + ROWS_PER_PASS <= n_q) {  // only q rows in this pass (uniform over the block)
+            *reinterpret_cast<uint4*>(q_out + ((size_t)token * n_q + head) * 128 + 8 * o) = make_uint4(own[0], own[1], own[2], own[3]);
+            continue;
+        }
+        __half s;
+        uint2 packed;
+        quant_oct_f32(v, s, packed);
+        if (!live) continue;
+        if (is_q) {
+            *reinterpret_cast<uint4*>(q_out + ((size_t)token * n_q + head) * 128 + 8 * o) = make_uint4(own[0], own[1], own[2], own[3]);
+        } else if (placed) {
+            const size_t drow = dst_row * n_kv + head;  // row of [128] quants / [4] scales
+            if ((o & 3) == 0) (is_v ? v_scales : k_scales)[drow * 4 + (o >> 2)] = s;
+            *reinterpret_cast<uint2*>((is_v ? v_quants : k_quants) + drow * 128 + 8 * o) = packed;
+        }
     }
-    const size_t drow = dst_row * n_kv + head;  // row of [128] quants / [4] scales
-    if ((o & 3) == 0) (is_v ? v_scales : k_scales)[drow * 4 + (o >> 2)] = s;
-    *reinterpret_cast<uint2*>((is_v ? v_quants : k_quants) + drow * 128 + 8 * o) = packed;
+}
+
+// Blocks per token: one for chunks that fill the GPU by themselves (two 256-thread blocks per SM and more), else one per group of rows.
+inline dim3 append_grid(const LaunchArgs& a, size_t tokens, uint32_t rows)
+{
+    const uint32_t groups = min(1024u, (rows + ROWS_PER_PASS - 1) / ROWS_PER_PASS);
+    return dim3((uint32_t)tokens, tokens >= 2 * (size_t)a.sm_count ? 1 : groups);
 }
 
 inline uint32_t grid_for(size_t n) { return (uint32_t)((n + PRE_THREADS - 1) / PRE_THREADS); }
@@ -374,13 +458,12 @@ int launch_kv_norm_rope_append_paged_q8_d128(const LaunchArgs& a)
     if (kv_rows == 0) return 0;
     if (kv_rows >= (1u << 26)) return fail_validation(a, "kv_norm_rope_append_paged_q8_d128: at most 2^26 (token, head) rows per launch");
     if (reinterpret_cast<uintptr_t>(a.b[3].ptr) & 15) return fail_validation(a, "kv_norm_rope_append_paged_q8_d128: cos_sin must be 16-byte aligned");
-    const size_t seg = (kv_rows * 16 + 31) / 32 * 32;
     auto kern = p.plus_one ? kv_norm_rope_append_kernel<true> : kv_norm_rope_append_kernel<false>;
-    const cudaError_t e = launch_dependent(kern, dim3(grid_for(2 * seg)), dim3(PRE_THREADS), 0, a.stream,
-        nullptr, nullptr, nullptr, 1u, 0u,
+    const cudaError_t e = launch_dependent(kern, append_grid(a, tokens, 2 * (p.row_len / 128)), dim3(PRE_THREADS), 0, a.stream,
+        nullptr, nullptr, nullptr, 0u,
         (const __half*)a.b[0].ptr, (const __half*)a.b[1].ptr, (const float*)a.b[2].ptr, (const float2*)a.b[3].ptr, (__half*)a.b[4].ptr,
         (int8_t*)a.b[5].ptr, (__half*)a.b[6].ptr, (int8_t*)a.b[7].ptr, (const uint32_t*)a.b[8].ptr, (uint32_t)(a.b[8].bytes / 4), p.page,
-        (const uint32_t*)a.b[9].ptr, p.row_len / 128, p.rot_dims / 2, (uint32_t)kv_rows, dst_rows, a.status);
+        (const uint32_t*)a.b[9].ptr, p.row_len / 128, p.rot_dims / 2, dst_rows, a.status);
     ++*a.launches;
     return check_cuda(a, e, "kv_norm_rope_append_paged_q8_d128");
 }
@@ -411,13 +494,12 @@ int launch_qkv_norm_rope_append_paged_q8_d128(const LaunchArgs& a)
     if (kv_rows >= (1u << 26) || q_rows >= (1u << 26))
         return fail_validation(a, "qkv_norm_rope_append_paged_q8_d128: at most 2^26 (token, head) rows of q and of k per launch");
     if (reinterpret_cast<uintptr_t>(kv[3].ptr) & 15) return fail_validation(a, "qkv_norm_rope_append_paged_q8_d128: cos_sin must be 16-byte aligned");
-    const size_t seg = (kv_rows * 16 + 31) / 32 * 32;
     auto kern = p.plus_one ? kv_norm_rope_append_kernel<true> : kv_norm_rope_append_kernel<false>;
-    const cudaError_t e = launch_dependent(kern, dim3(grid_for(2 * seg + q_rows * 16)), dim3(PRE_THREADS), 0, a.stream,
-        (const __half*)a.b[0].ptr, (const float*)a.b[1].ptr, (__half*)a.b[2].ptr, p.n_q_heads, (uint32_t)q_rows, (const __half*)kv[0].ptr,
+    const cudaError_t e = launch_dependent(kern, append_grid(a, tokens, p.n_q_heads + 2 * (p.row_len / 128)), dim3(PRE_THREADS), 0, a.stream,
+        (const __half*)a.b[0].ptr, (const float*)a.b[1].ptr, (__half*)a.b[2].ptr, p.n_q_heads, (const __half*)kv[0].ptr,
         (const __half*)kv[1].ptr, (const float*)kv[2].ptr, (const float2*)kv[3].ptr, (__half*)kv[4].ptr, (int8_t*)kv[5].ptr,
         (__half*)kv[6].ptr, (int8_t*)kv[7].ptr, (const uint32_t*)kv[8].ptr, (uint32_t)(kv[8].bytes / 4), p.page,
-        (const uint32_t*)kv[9].ptr, p.row_len / 128, p.rot_dims / 2, (uint32_t)kv_rows, dst_rows, a.status);
+        (const uint32_t*)kv[9].ptr, p.row_len / 128, p.rot_dims / 2, dst_rows, a.status);
     ++*a.launches;
     return check_cuda(a, e, "qkv_norm_rope_append_paged_q8_d128");
 }
