@@ -120,7 +120,26 @@ __device__ __forceinline__ float quad_sum(float v)
     return v + __shfl_xor_sync(0xffffffffu, v, 2);
 }
 
-template <int NSTAGES, int MIN_CTAS, int SUB>
+constexpr int MAX_CLUSTER = 8;
+__device__ __forceinline__ uint32_t cluster_ctas()
+{
+    uint32_t n;
+    asm("mov.u32 %0, %cluster_nctaid.x;" : "=r"(n));
+    return n;
+}
+__device__ __forceinline__ const float* map_to_rank(const float* p, uint32_t rank)
+{
+    uint64_t out;
+    asm("mapa.u64 %0, %1, %2;" : "=l"(out) : "l"(reinterpret_cast<uint64_t>(p)), "r"(rank));
+    return reinterpret_cast<const float*>(out);
+}
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// CLUSTERED: the sub-splits of a (kv head, split) spread over a cluster of CTAs as well, SUB = 4 in each.
+template <int NSTAGES, int MIN_CTAS, int SUB, bool CLUSTERED>
 __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
     decode_paged_kernel(const __grid_constant__ CUtensorMap tm_kq, const __grid_constant__ CUtensorMap tm_ks,
                         const __grid_constant__ CUtensorMap tm_vq, const __grid_constant__ CUtensorMap tm_vs,
@@ -135,7 +154,9 @@ __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int HEADS_PER_CTA = WPC / SUB;
-    const int kvh = blockIdx.x * HEADS_PER_CTA + warp / SUB, sub = warp % SUB, split = blockIdx.y;
+    const int n_cta = CLUSTERED ? (int)cluster_ctas() : 1, rank = CLUSTERED ? (int)blockIdx.x % n_cta : 0;
+    const int kvh = ((int)blockIdx.x / n_cta) * HEADS_PER_CTA + warp / SUB, sub = warp % SUB, split = blockIdx.y;
+    const uint32_t n_sub = SUB * n_cta, first_sub = rank * SUB + sub;  // sub-splits of a split; this warp's
     const int n_q = (int)n_kv * G;
     const bool active = kvh < (int)n_kv;  // idle warps of the last CTA when n_kv * SUB is not a multiple of 4
     const int g = lane >> 2, t4 = lane & 3;
@@ -153,9 +174,9 @@ __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
     const uint32_t chunk = (kv_len + n_splits - 1) / n_splits;
     const uint32_t t_begin = min((uint32_t)split * chunk, kv_len);
     const uint32_t t_end = min(t_begin + chunk, kv_len);
-    const uint32_t s_begin = t_begin / STAGE_TOK + sub;  // this warp's first stage; it then strides by SUB
+    const uint32_t s_begin = t_begin / STAGE_TOK + first_sub;  // this warp's first stage; it then strides by n_sub
     const uint32_t n_stages = t_begin < t_end ? (t_end + STAGE_TOK - 1) / STAGE_TOK - t_begin / STAGE_TOK : 0;
-    const uint32_t n_iter = active && n_stages > (uint32_t)sub ? (n_stages - sub + SUB - 1) / SUB : 0;
+    const uint32_t n_iter = active && n_stages > first_sub ? (n_stages - first_sub + n_sub - 1) / n_sub : 0;
     __syncwarp();
 
     const uint32_t page_shift = 31 - __clz(page);
@@ -184,7 +205,7 @@ __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
     const uint32_t bar0 = smem_u32(&sm.full[warp][0]);
     auto issue = [&](uint32_t it, uint32_t pp) {
         const uint32_t st = it % NSTAGES;
-        const uint32_t tok0 = (s_begin + it * SUB) * STAGE_TOK;
+        const uint32_t tok0 = (s_begin + it * n_sub) * STAGE_TOK;
         const int row = (int)((pp << page_shift) + (tok0 & (page - 1)));
         const uint32_t bar = bar0 + st * 8;
         if (lane == 0) {
@@ -201,7 +222,7 @@ __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
     {
         const uint32_t n_pre = min(n_iter, (uint32_t)NSTAGES);
         uint32_t my_pp = 0;
-        if ((uint32_t)lane < n_pre) my_pp = lookup(s_begin + lane * SUB);
+        if ((uint32_t)lane < n_pre) my_pp = lookup(s_begin + lane * n_sub);
         for (uint32_t it = 0; it < n_pre; ++it) {
             const uint32_t pp = __shfl_sync(0xffffffffu, my_pp, it);
             if (lane < 4) issue(it, pp);
@@ -210,7 +231,7 @@ __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
     // The page of the next stage to be issued is looked up one iteration early, so the load's
     // latency is covered by a tile of work.
     uint32_t next_pp = 0;
-    if (n_iter > (uint32_t)NSTAGES && lane < 4) next_pp = lookup(s_begin + NSTAGES * SUB);
+    if (n_iter > (uint32_t)NSTAGES && lane < 4) next_pp = lookup(s_begin + NSTAGES * n_sub);
 
     // MMA roles.  QK^T: A = K (16 tokens x 16 dims of chunk c), B = Q^T (16 dims x 8 query rows).
     //            PV  : A = V^T (16 dims of chunk c x 16 tokens), B = P'^T (16 tokens x 8 query rows).
@@ -274,7 +295,7 @@ __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
     for (uint32_t it = 0; it < n_iter; ++it) {
         const int st = it % NSTAGES;
         mbar_wait(&sm.full[warp][st], (it / NSTAGES) & 1, status, 305, failed);
-        const int tok0 = (int)((s_begin + it * SUB) * STAGE_TOK);
+        const int tok0 = (int)((s_begin + it * n_sub) * STAGE_TOK);
         const uint32_t kq_base = smem_u32(sm.kq[warp][st]), vq_base = smem_u32(sm.vq[warp][st]);
 
         // ---- S = K Q^T per 32-wide block, then the block scales: s[th][e] = score of token g + 8*th
@@ -389,7 +410,7 @@ __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
         __syncwarp();
         if (lane < 4 && it + NSTAGES < n_iter) {
             issue(it + NSTAGES, next_pp);
-            if (it + NSTAGES + 1 < n_iter) next_pp = lookup(s_begin + (it + NSTAGES + 1) * SUB);
+            if (it + NSTAGES + 1 < n_iter) next_pp = lookup(s_begin + (it + NSTAGES + 1) * n_sub);
         }
     }
 
@@ -441,6 +462,60 @@ __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
         }
     }
 
+    // ---- merge the CTAs of a cluster in rank order ------------------------------------------------------
+    // Each leaves its state where warp 0's K ring was; rank r then owns every n_cta-th stretch of 16 dims of all rows.
+    if constexpr (CLUSTERED) {
+        float* mine = reinterpret_cast<float*>(sm.kq[0][0]);
+        __syncthreads();  // the merge above has read what the other warps left
+        if (warp == 0) {
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                float* dst = mine + (2 * t4 + e) * (HD + 2);
+#pragma unroll
+                for (int c = 0; c < 8; c++) *reinterpret_cast<float2*>(dst + 16 * c + 2 * g) = make_float2(o[c][e], o[c][2 + e]);
+                if (g == 0) {
+                    dst[HD] = m_run[e];
+                    dst[HD + 1] = l_row[e];
+                }
+            }
+        }
+        __syncwarp();
+        cluster_sync();
+        const uint32_t r = threadIdx.x >> 4, in_stretch = threadIdx.x & 15;  // 8 rows x 16 dims = the CTA's 128 threads
+        if (r < rows) {
+            float mk[MAX_CLUSTER], lk[MAX_CLUSTER], big = NEG_SENTINEL, l = 0.0f;
+            const float* row[MAX_CLUSTER];
+#pragma unroll
+            for (int k = 0; k < MAX_CLUSTER; k++) {
+                row[k] = map_to_rank(mine + r * (HD + 2), min(k, n_cta - 1));
+                mk[k] = k < n_cta ? row[k][HD] : NEG_SENTINEL;
+                lk[k] = k < n_cta ? row[k][HD + 1] : 0.0f;
+                big = fmaxf(big, mk[k]);
+            }
+#pragma unroll
+            for (int k = 0; k < MAX_CLUSTER; k++) {
+                mk[k] = k < n_cta ? ex2(mk[k] - big) : 0.0f;
+                l = fmaf(mk[k], lk[k], l);
+            }
+            float* dst = part + (((size_t)(r / G) * n_q + kvh * G + r % G) * n_splits + split) * (HD + 2);
+            for (uint32_t d = rank * 16 + in_stretch; d < HD; d += 16 * n_cta) {
+                float v[MAX_CLUSTER], acc = 0.0f;
+#pragma unroll
+                for (int k = 0; k < MAX_CLUSTER; k++) v[k] = k < n_cta ? row[k][d] : 0.0f;
+#pragma unroll
+                for (int k = 0; k < MAX_CLUSTER; k++) acc = fmaf(mk[k], v[k], acc);
+                dst[d] = acc;
+            }
+            if (rank == 0 && in_stretch == 0) {
+                dst[HD] = big == NEG_SENTINEL ? NEG_SENTINEL : big * 0.6931471805599453f;  // back to natural log
+                dst[HD + 1] = l;
+            }
+        }
+        __syncwarp();
+        cluster_sync();  // nobody leaves while its shared memory is read
+        return;
+    }
+
     // ---- the split's partial, straight from registers ------------------------------------------------
     if (active && sub == 0) {
 #pragma unroll
@@ -484,33 +559,36 @@ int encode_pool_maps(const LaunchArgs& a, CUtensorMap (&tm)[4], const void* cons
     return 0;
 }
 
-template <int NSTAGES, int MIN_CTAS, int SUB>
+template <int NSTAGES, int MIN_CTAS, int SUB, bool CLUSTERED>
 cudaError_t launch_decode_variant(cudaStream_t stream, int device, const CUtensorMap (&tm)[4], const __half* q,
                                   const uint32_t* page_table, uint32_t table_len, uint32_t page, uint32_t pool_pages, float* part,
-                                  const uint32_t* step, uint32_t n_kv, uint32_t n_splits, float scale, uint32_t m_q, uint32_t* status)
+                                  const uint32_t* step, uint32_t n_kv, uint32_t n_splits, float scale, uint32_t m_q, uint32_t* status,
+                                  uint32_t cluster)
 {
     using Smem = DecodeSmem<NSTAGES>;
     const size_t smem = sizeof(Smem) + 1024;
+    auto kern = decode_paged_kernel<NSTAGES, MIN_CTAS, SUB, CLUSTERED>;
     static std::mutex attr_mutex;
     static bool attr_set[64] = {};
     {
         std::lock_guard<std::mutex> lock(attr_mutex);
         if (device >= 0 && device < 64 && !attr_set[device]) {
-            cudaError_t e = cudaFuncSetAttribute(decode_paged_kernel<NSTAGES, MIN_CTAS, SUB>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (e != cudaSuccess) return e;
             attr_set[device] = true;
         }
     }
-    const uint32_t ctas_x = (n_kv * SUB + WPC - 1) / WPC;
-    return launch_dependent(decode_paged_kernel<NSTAGES, MIN_CTAS, SUB>, dim3(ctas_x, n_splits), dim3(WPC * 32), smem, stream, tm[0],
-                            tm[1], tm[2], tm[3], q, page_table, table_len, page, pool_pages, part, step, n_kv, n_splits, scale, m_q, status);
+    const uint32_t ctas_x = (n_kv * SUB + WPC - 1) / WPC * cluster;
+    return launch_dependent_clusters(kern, cluster, dim3(ctas_x, n_splits), dim3(WPC * 32), smem, stream, tm[0], tm[1], tm[2], tm[3], q, page_table,
+                                     table_len, page, pool_pages, part, step, n_kv, n_splits, scale, m_q, status);
 }
 
 // Shape of the launch.  Three 4.5 KB stages per warp = 54 KB per CTA and 128 registers per thread let
 // four CTAs = 16 warps live on an SM.  The number of sub-splits per (kv head, split) is the largest
-// of 4, 2, 1 for which all warps still fit on the GPU at once (one wave): extra waves cost more
-// than the parallelism buys.  SGB_DECODE_SUB=1|2|4 overrides the choice (tuning aid; results agree
+// of 32, 16, 8 (clusters of 8, 4, 2 CTAs), 4, 2, 1 for which all warps still fit on the GPU at once (one wave): extra waves
+// cost more than the parallelism buys, while few splits (a short sequence) leave most of the chip idle and every warp a long
+// chain of stages: 1000 tokens, one split, 16 kv heads took 18.2 us a launch with 4 sub-splits per split, 7.1 with 32.
+// SGB_DECODE_SUB=1|2|4|8|16|32 overrides the choice (tuning aid; results agree
 // within rounding, each choice is bit-reproducible).
 cudaError_t launch_decode(cudaStream_t stream, int device, int sm_count, const CUtensorMap (&tm)[4], const __half* q,
                           const uint32_t* page_table, uint32_t table_len, uint32_t page, uint32_t pool_pages, float* part,
@@ -522,12 +600,14 @@ cudaError_t launch_decode(cudaStream_t stream, int device, int sm_count, const C
     }();
     const uint64_t slots = (uint64_t)(sm_count > 0 ? sm_count : 148) * 16;
     const uint64_t tasks = (uint64_t)n_kv * n_splits;
-    int sub = tasks * 4 <= slots ? 4 : tasks * 2 <= slots ? 2 : 1;
-    if (forced == 1 || forced == 2 || forced == 4) sub = forced;
+    int sub = 32;
+    while (sub > 1 && tasks * sub > slots) sub /= 2;
+    if (forced >= 1 && forced <= 4 * MAX_CLUSTER && (forced & (forced - 1)) == 0) sub = forced;
 #define SGB_DECODE_ARGS stream, device, tm, q, page_table, table_len, page, pool_pages, part, step, n_kv, n_splits, scale, m_q, status
-    if (sub == 4) return launch_decode_variant<3, 4, 4>(SGB_DECODE_ARGS);
-    if (sub == 2) return launch_decode_variant<3, 4, 2>(SGB_DECODE_ARGS);
-    return launch_decode_variant<3, 4, 1>(SGB_DECODE_ARGS);
+    if (sub > 4) return launch_decode_variant<3, 4, 4, true>(SGB_DECODE_ARGS, sub / 4);
+    if (sub == 4) return launch_decode_variant<3, 4, 4, false>(SGB_DECODE_ARGS, 1);
+    if (sub == 2) return launch_decode_variant<3, 4, 2, false>(SGB_DECODE_ARGS, 1);
+    return launch_decode_variant<3, 4, 1, false>(SGB_DECODE_ARGS, 1);
 #undef SGB_DECODE_ARGS
 }
 

@@ -54,19 +54,27 @@ int encode_tensor_map(const LaunchArgs& a, void* out_map /*CUtensorMap*/, int el
 // launch); the kernel calls pdl_wait() before reading.  SGB_PDL=0 in the environment turns the attribute off.
 bool pdl_enabled();
 template <typename... KArgs, typename... Args>
-cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args)
+cudaError_t launch_dependent_clusters(void (*kern)(KArgs...), uint32_t cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeClusterDimension;  // `cluster` CTAs along x
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args)
+{
+    return launch_dependent_clusters(kern, 1, grid, block, smem, stream, args...);
 }
 
 // The registry (sgb_registry.cu).
