@@ -118,6 +118,8 @@ __global__ void __launch_bounds__(FLASH_THREADS, 2) flash_prefill_kernel(const _
     }
 
     const int tid = threadIdx.x, warp = tid >> 5;
+    pdl_wait();  // the step words, q, K and V come from earlier kernels of the stream
+    pdl_launch_dependents();
     // Launch order (blockIdx.x, then pieces): groups of `head_group` kv heads one after the other; inside a group the latest
     // query tile (the one with the most keys) of every head first, then the one before it, and so on.  The CTAs that run
     // together then read the K/V of one group, which the launcher sizes to stay in L2, and within the group the short
@@ -450,6 +452,8 @@ constexpr int MAX_PIECES = 16;
 __global__ void __launch_bounds__(256) combine_pieces_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
                                                              float* __restrict__ out, uint32_t rows, uint32_t pieces)
 {
+    pdl_wait();  // the partials come from the kernel before this one
+    pdl_launch_dependents();
     const uint32_t row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= rows) return;
     float m[MAX_PIECES], l[MAX_PIECES];
@@ -625,14 +629,14 @@ int run_flash(const LaunchArgs& a, const BufView& q, const BufView& k0, const Bu
     }
     FlashParams prm{(const uint32_t*)step.ptr, (float*)out.ptr, part_acc, part_ml, a.status, m_tokens, n_kv, window, ring, scale, head_group};
     const dim3 grid(q_tiles * n_kv, 1, pieces);
-    flash_prefill_kernel<TWO_SRC><<<grid, FLASH_THREADS, smem, a.stream>>>(tq, tk0, tv0, tk1, tv1, prm);
+    const cudaError_t e = launch_dependent(flash_prefill_kernel<TWO_SRC>, grid, dim3(FLASH_THREADS), smem, a.stream, tq, tk0, tv0, tk1, tv1, prm);
     ++*a.launches;
-    if (int r = check_cuda(a, cudaGetLastError(), "attn_prefill_flash")) return r;
+    if (int r = check_cuda(a, e, "attn_prefill_flash")) return r;
     if (pieces > 1) {
-        combine_pieces_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, a.stream>>>(part_acc, part_ml, (float*)out.ptr, (uint32_t)rows,
-                                                                              (uint32_t)pieces);
+        const cudaError_t e2 = launch_dependent(combine_pieces_kernel, dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, a.stream, part_acc, part_ml,
+                                                (float*)out.ptr, (uint32_t)rows, (uint32_t)pieces);
         ++*a.launches;
-        return check_cuda(a, cudaGetLastError(), "attn_prefill_flash combine");
+        return check_cuda(a, e2, "attn_prefill_flash combine");
     }
     return 0;
 }

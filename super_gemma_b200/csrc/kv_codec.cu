@@ -6,6 +6,8 @@
 //   scale = RTNE f16(d);  id = d > 0 ? 1/d : 0;  q = round_half_even(x * id)
 //   dequant: f16(f32(scale) * f32(q))            (kv_dequant_q8.wgsl:26)
 // All of them are HBM-bound byte shuffles: 16-byte accesses, one block of 32 values per thread.
+// A warp per row in the paged gather, with the page looked up once per row, four loads under way per lane and f16 multiplies,
+// was slower (131072 tokens, 16 heads: 200 us a side against 175; 8192: 14.2 against 12.6): left as it is.
 #include "sgb_common.cuh"
 #include "sgb_kernels.h"
 
@@ -66,6 +68,8 @@ __global__ void __launch_bounds__(CODEC_THREADS) kv_quant_q8_kernel(const __half
                                                                     __half* __restrict__ scales,
                                                                     int8_t* __restrict__ quants, size_t n_blocks)
 {
+    pdl_wait();
+    pdl_launch_dependents();
     const size_t blk = (size_t)blockIdx.x * CODEC_THREADS + threadIdx.x;
     if (blk >= n_blocks) return;
     uint4 in[4];
@@ -82,6 +86,8 @@ __global__ void __launch_bounds__(CODEC_THREADS) kv_dequant_q8_kernel(const __ha
                                                                       const int8_t* __restrict__ quants,
                                                                       __half* __restrict__ dst, size_t n_halfblocks)
 {
+    pdl_wait();
+    pdl_launch_dependents();
     const size_t hb = (size_t)blockIdx.x * CODEC_THREADS + threadIdx.x;
     if (hb >= n_halfblocks) return;
     const float d = __half2float(scales[hb >> 1]);
@@ -109,6 +115,8 @@ __global__ void __launch_bounds__(CODEC_THREADS) kv_append_kernel(const uint4* _
                                                                   size_t dst_rows, uint32_t* status)
 {
     constexpr int VEC_PER_ROW = ROW_LEN / 8;
+    pdl_wait();
+    pdl_launch_dependents();
     const size_t i = (size_t)blockIdx.x * CODEC_THREADS + threadIdx.x;
     if (i >= n_vec) return;
     const size_t token = i / VEC_PER_ROW, j = i % VEC_PER_ROW;
@@ -132,6 +140,8 @@ __global__ void __launch_bounds__(CODEC_THREADS) kv_append_q8_kernel(const __hal
                                                                      uint32_t blocks_per_row, size_t n_blocks,
                                                                      size_t dst_rows, uint32_t* status)
 {
+    pdl_wait();
+    pdl_launch_dependents();
     const size_t blk = (size_t)blockIdx.x * CODEC_THREADS + threadIdx.x;
     if (blk >= n_blocks) return;
     const size_t token = blk / blocks_per_row, local = blk % blocks_per_row;
@@ -172,6 +182,8 @@ __global__ void __launch_bounds__(CODEC_THREADS) kv_dequant_paged_kernel(const _
                                                                          uint32_t row_len, size_t dst_rows,
                                                                          size_t src_rows, uint32_t* status)
 {
+    pdl_wait();
+    pdl_launch_dependents();
     const uint32_t hb_per_row = row_len / 16;
     const size_t kv_len = step[STEP_KV_LEN_GLOBAL];
     // The flash kernel reads whole 64-key tiles and masks what lies past kv_len; a masked key weighs 0, but
@@ -227,10 +239,10 @@ int launch_kv_quant_q8(const LaunchArgs& a)
     if (int r = need_bytes(a, 1, n_blocks * 2, "scales")) return r;
     if (int r = need_bytes(a, 2, n_blocks * 32, "quants")) return r;
     if (n_blocks == 0) return 0;
-    kv_quant_q8_kernel<<<blocks_for(n_blocks, CODEC_THREADS), CODEC_THREADS, 0, a.stream>>>(
+    const cudaError_t e = launch_dependent(kv_quant_q8_kernel, dim3(blocks_for(n_blocks, CODEC_THREADS)), dim3(CODEC_THREADS), 0, a.stream,
         (const __half*)a.b[0].ptr, (__half*)a.b[1].ptr, (int8_t*)a.b[2].ptr, n_blocks);
     ++*a.launches;
-    return check_cuda(a, cudaGetLastError(), "kv_quant_q8");
+    return check_cuda(a, e, "kv_quant_q8");
 }
 
 // bindings: scales f16, quants i8, dst f16.  Covers dst.len / 32 blocks.
@@ -241,10 +253,10 @@ int launch_kv_dequant_q8(const LaunchArgs& a)
     if (int r = need_bytes(a, 0, n_blocks * 2, "scales")) return r;
     if (int r = need_bytes(a, 1, n_blocks * 32, "quants")) return r;
     if (n_blocks == 0) return 0;
-    kv_dequant_q8_kernel<<<blocks_for(n_blocks * 2, CODEC_THREADS), CODEC_THREADS, 0, a.stream>>>(
+    const cudaError_t e = launch_dependent(kv_dequant_q8_kernel, dim3(blocks_for(n_blocks * 2, CODEC_THREADS)), dim3(CODEC_THREADS), 0, a.stream,
         (const __half*)a.b[0].ptr, (const int8_t*)a.b[1].ptr, (__half*)a.b[2].ptr, n_blocks * 2);
     ++*a.launches;
-    return check_cuda(a, cudaGetLastError(), "kv_dequant_q8");
+    return check_cuda(a, e, "kv_dequant_q8");
 }
 
 // bindings: src f16 [n x ROW_LEN], dst f16 [slots x ROW_LEN], step.
@@ -258,10 +270,10 @@ int launch_kv_append(const LaunchArgs& a)
     const size_t dst_rows = a.b[1].bytes / (ROW_LEN * 2);
     if (RING > 0 && dst_rows < (size_t)RING) return fail_validation(a, "kv_append: ring buffer smaller than the ring");
     if (n_vec == 0) return 0;
-    kv_append_kernel<ROW_LEN, RING><<<blocks_for(n_vec, CODEC_THREADS), CODEC_THREADS, 0, a.stream>>>(
+    const cudaError_t e = launch_dependent(kv_append_kernel<ROW_LEN, RING>, dim3(blocks_for(n_vec, CODEC_THREADS)), dim3(CODEC_THREADS), 0, a.stream,
         (const uint4*)a.b[0].ptr, (uint4*)a.b[1].ptr, (const uint32_t*)a.b[2].ptr, n_vec, dst_rows, a.status);
     ++*a.launches;
-    return check_cuda(a, cudaGetLastError(), "kv_append");
+    return check_cuda(a, e, "kv_append");
 }
 template int launch_kv_append<4096, 1024>(const LaunchArgs&);  // kv_append_sliding (16 kv heads x 256)
 template int launch_kv_append<2048, 0>(const LaunchArgs&);     // kv_append_global  (4 kv heads x 512)
@@ -278,11 +290,11 @@ int launch_kv_append_global_q8(const LaunchArgs& a)
     if (a.b[1].bytes / 2 < dst_rows * (ROW_LEN / 32))
         return fail_validation(a, "kv_append_global_q8: scales buffer shorter than the quants buffer implies");
     if (n_blocks == 0) return 0;
-    kv_append_q8_kernel<<<blocks_for(n_blocks, CODEC_THREADS), CODEC_THREADS, 0, a.stream>>>(
-        (const __half*)a.b[0].ptr, (__half*)a.b[1].ptr, (int8_t*)a.b[2].ptr, nullptr, 0, 1, (const uint32_t*)a.b[3].ptr,
-        ROW_LEN / 32, n_blocks, dst_rows, a.status);
+    const cudaError_t e = launch_dependent(kv_append_q8_kernel, dim3(blocks_for(n_blocks, CODEC_THREADS)), dim3(CODEC_THREADS), 0, a.stream,
+        (const __half*)a.b[0].ptr, (__half*)a.b[1].ptr, (int8_t*)a.b[2].ptr, nullptr, 0, 1, (const uint32_t*)a.b[3].ptr, ROW_LEN / 32,
+        n_blocks, dst_rows, a.status);
     ++*a.launches;
-    return check_cuda(a, cudaGetLastError(), "kv_append_global_q8");
+    return check_cuda(a, e, "kv_append_global_q8");
 }
 template int launch_kv_append_global_q8<2048>(const LaunchArgs&);
 
@@ -304,11 +316,11 @@ int launch_kv_append_paged_q8_d128(const LaunchArgs& a)
     if (a.b[1].bytes / 2 < dst_rows * (p.row_len / 32))
         return fail_validation(a, "kv_append_paged_q8_d128: scales buffer too short for the quants buffer");
     if (n_blocks == 0) return 0;
-    kv_append_q8_kernel<<<blocks_for(n_blocks, CODEC_THREADS), CODEC_THREADS, 0, a.stream>>>(
-        (const __half*)a.b[0].ptr, (__half*)a.b[1].ptr, (int8_t*)a.b[2].ptr, (const uint32_t*)a.b[3].ptr,
-        (uint32_t)(a.b[3].bytes / 4), p.page, (const uint32_t*)a.b[4].ptr, p.row_len / 32, n_blocks, dst_rows, a.status);
+    const cudaError_t e = launch_dependent(kv_append_q8_kernel, dim3(blocks_for(n_blocks, CODEC_THREADS)), dim3(CODEC_THREADS), 0, a.stream,
+        (const __half*)a.b[0].ptr, (__half*)a.b[1].ptr, (int8_t*)a.b[2].ptr, (const uint32_t*)a.b[3].ptr, (uint32_t)(a.b[3].bytes / 4),
+        p.page, (const uint32_t*)a.b[4].ptr, p.row_len / 32, n_blocks, dst_rows, a.status);
     ++*a.launches;
-    return check_cuda(a, cudaGetLastError(), "kv_append_paged_q8_d128");
+    return check_cuda(a, e, "kv_append_paged_q8_d128");
 }
 
 // Shared with the paged flash prefill launcher.
@@ -322,11 +334,11 @@ int run_kv_dequant_paged(const LaunchArgs& a, const BufView& scales, const BufVi
     if (dst_rows == 0) return 0;
     size_t want = (dst_rows * (row_len / 16) + CODEC_THREADS - 1) / CODEC_THREADS;
     const uint32_t grid = (uint32_t)(want < (size_t)a.sm_count * 16 ? want : (size_t)a.sm_count * 16);
-    kv_dequant_paged_kernel<<<grid, CODEC_THREADS, 0, a.stream>>>(
+    const cudaError_t e = launch_dependent(kv_dequant_paged_kernel, dim3(grid), dim3(CODEC_THREADS), 0, a.stream,
         (const __half*)scales.ptr, (const int8_t*)quants.ptr, (const uint32_t*)table.ptr, (uint32_t)(table.bytes / 4), page,
         (__half*)dst.ptr, (const uint32_t*)step.ptr, row_len, dst_rows, src_rows, a.status);
     ++*a.launches;
-    return check_cuda(a, cudaGetLastError(), "kv_dequant_paged");
+    return check_cuda(a, e, "kv_dequant_paged");
 }
 
 // bindings: scales f16, quants i8, page_table u32, dst f16 [rows x row_len], step.  push {row_len, page}.

@@ -86,6 +86,8 @@ template <int BPR, bool PLUS_ONE>
 __global__ void __launch_bounds__(PRE_THREADS) rmsnorm_kernel(const __half* __restrict__ x, const float* __restrict__ w,
                                                               __half* __restrict__ y, size_t n_blocks)
 {
+    pdl_wait();
+    pdl_launch_dependents();
     const size_t blk = (size_t)blockIdx.x * PRE_THREADS + threadIdx.x;
     const bool live = blk < n_blocks;  // whole rows only, and BPR divides 32: a row never straddles a warp
     float v[32];
@@ -109,6 +111,8 @@ __global__ void __launch_bounds__(PRE_THREADS) rmsnorm_kernel(const __half* __re
 __global__ void __launch_bounds__(PRE_THREADS) rope_kernel(__half* __restrict__ xs, const float2* __restrict__ cos_sin,
                                                            uint32_t head_dim, uint32_t half_rot, uint32_t n_heads, size_t pairs_total)
 {
+    pdl_wait();
+    pdl_launch_dependents();
     const size_t g = (size_t)blockIdx.x * PRE_THREADS + threadIdx.x;
     if (g >= pairs_total) return;
     const size_t row = g / half_rot;
@@ -199,6 +203,8 @@ __global__ void __launch_bounds__(PRE_THREADS) norm_rope_d128_kernel(const __hal
                                                                      const float2* __restrict__ cos_sin, __half* __restrict__ y,
                                                                      uint32_t n_heads, uint32_t half_rot, uint32_t rows)
 {
+    pdl_wait();
+    pdl_launch_dependents();
     // 32-bit index arithmetic (the host checks rows * 16 < 2^32): 64-bit divisions would cost more than the rest
     const uint32_t g = blockIdx.x * PRE_THREADS + threadIdx.x;
     const uint32_t row = g >> 4;
@@ -237,6 +243,7 @@ __device__ __forceinline__ void quant_oct_f32(const float (&x)[8], __half& scale
 // octet, and made the kernel issue-bound).  The launcher gives a long chunk one block per token and a short one as
 // many blocks per token as there are groups, where latency counts.
 constexpr int ROWS_PER_PASS = PRE_THREADS / 16;
+constexpr int ROWS_AHEAD = 4;  // loads of a thread under way at a time
 
 template <bool PLUS_ONE>
 __global__ void __launch_bounds__(PRE_THREADS)
@@ -287,14 +294,11 @@ __global__ void __launch_bounds__(PRE_THREADS)
                                              : v_raw + ((size_t)token * n_kv + (r - n_q - n_kv)) * 128;
         return __ldg(reinterpret_cast<const uint4*>(src + 8 * o));
     };
-    uint4 next = octet(blockIdx.y * ROWS_PER_PASS + slot);
-    for (uint32_t r0 = blockIdx.y * ROWS_PER_PASS; r0 < rows; r0 += gridDim.y * ROWS_PER_PASS) {
+    auto work = [&](uint32_t r0, const uint4& u) {
         const uint32_t r = r0 + slot;
         const bool live = r < rows, is_q = r < n_q, is_v = r >= n_q + n_kv;
         const uint32_t head = is_q ? r : is_v ? r - n_q - n_kv : r - n_q;
         float v[8];
-        const uint4 u = next;
-        next = octet(r + gridDim.y * ROWS_PER_PASS);  // on its way while this row is worked on
         float wv[8];
 #pragma unroll
         for (int i = 0; i < 8; i++) wv[i] = 1.0f;
@@ -343,18 +347,29 @@ __global__ void __launch_bounds__(PRE_THREADS)
         }
         if (r0 + ROWS_PER_PASS <= n_q) {  // only q rows in this pass (uniform over the block)
             *reinterpret_cast<uint4*>(q_out + ((size_t)token * n_q + head) * 128 + 8 * o) = make_uint4(own[0], own[1], own[2], own[3]);
-            continue;
+            return;
         }
         __half s;
         uint2 packed;
         quant_oct_f32(v, s, packed);
-        if (!live) continue;
+        if (!live) return;
         if (is_q) {
             *reinterpret_cast<uint4*>(q_out + ((size_t)token * n_q + head) * 128 + 8 * o) = make_uint4(own[0], own[1], own[2], own[3]);
         } else if (placed) {
             const size_t drow = dst_row * n_kv + head;  // row of [128] quants / [4] scales
             if ((o & 3) == 0) (is_v ? v_scales : k_scales)[drow * 4 + (o >> 2)] = s;
             *reinterpret_cast<uint2*>((is_v ? v_quants : k_quants) + drow * 128 + 8 * o) = packed;
+        }
+    };
+    const uint32_t stride = gridDim.y * ROWS_PER_PASS;
+    for (uint32_t base = blockIdx.y * ROWS_PER_PASS; base < rows; base += ROWS_AHEAD * stride) {
+        uint4 u[ROWS_AHEAD];
+#pragma unroll
+        for (int k = 0; k < ROWS_AHEAD; k++) u[k] = octet(base + k * stride + slot);
+#pragma unroll
+        for (int k = 0; k < ROWS_AHEAD; k++) {
+            if (base + k * stride >= rows) break;  // uniform over the block
+            work(base + k * stride, u[k]);
         }
     }
 }
@@ -389,10 +404,9 @@ int launch_rmsnorm(const LaunchArgs& a)
     if (int r = need_bytes(a, 2, a.b[0].bytes, "y")) return r;
     const size_t n_blocks = a.b[0].bytes / 64;
     if (n_blocks == 0) return 0;
-    rmsnorm_kernel<ROW_LEN / 32, PLUS_ONE != 0><<<grid_for(n_blocks), PRE_THREADS, 0, a.stream>>>(
-        (const __half*)a.b[0].ptr, (const float*)a.b[1].ptr, (__half*)a.b[2].ptr, n_blocks);
+    const cudaError_t e = launch_dependent(rmsnorm_kernel<ROW_LEN / 32, PLUS_ONE != 0>, dim3(grid_for(n_blocks)), dim3(PRE_THREADS), 0, a.stream, (const __half*)a.b[0].ptr, (const float*)a.b[1].ptr, (__half*)a.b[2].ptr, n_blocks);
     ++*a.launches;
-    return check_cuda(a, cudaGetLastError(), "rmsnorm");
+    return check_cuda(a, e, "rmsnorm");
 }
 template int launch_rmsnorm<256, 0>(const LaunchArgs&);
 template int launch_rmsnorm<256, 1>(const LaunchArgs&);
@@ -407,10 +421,9 @@ int launch_rope(const LaunchArgs& a)
     const size_t pairs = rows * (ROT_DIMS / 2);
     if (int r = need_bytes(a, 1, rows / N_HEADS * (ROT_DIMS / 2) * 8, "cos_sin")) return r;
     if (pairs == 0) return 0;
-    rope_kernel<<<grid_for(pairs), PRE_THREADS, 0, a.stream>>>((__half*)a.b[0].ptr, (const float2*)a.b[1].ptr, HEAD_DIM, ROT_DIMS / 2,
-                                                                 N_HEADS, pairs);
+    const cudaError_t e = launch_dependent(rope_kernel, dim3(grid_for(pairs)), dim3(PRE_THREADS), 0, a.stream, (__half*)a.b[0].ptr, (const float2*)a.b[1].ptr, HEAD_DIM, ROT_DIMS / 2, N_HEADS, pairs);
     ++*a.launches;
-    return check_cuda(a, cudaGetLastError(), "rope");
+    return check_cuda(a, e, "rope");
 }
 template int launch_rope<256, 256, 32>(const LaunchArgs&);
 template int launch_rope<256, 256, 16>(const LaunchArgs&);
@@ -431,10 +444,9 @@ int launch_norm_rope_d128(const LaunchArgs& a)
     if (rows >= (1u << 27)) return fail_validation(a, "attn_norm_rope_d128: at most 2^27 rows per launch");
     if (reinterpret_cast<uintptr_t>(a.b[2].ptr) & 15) return fail_validation(a, "attn_norm_rope_d128: cos_sin must be 16-byte aligned");
     auto kern = p.plus_one ? norm_rope_d128_kernel<true> : norm_rope_d128_kernel<false>;
-    kern<<<grid_for(rows * 16), PRE_THREADS, 0, a.stream>>>((const __half*)a.b[0].ptr, (const float*)a.b[1].ptr, (const float2*)a.b[2].ptr,
-                                                           (__half*)a.b[3].ptr, p.n_heads, p.rot_dims / 2, (uint32_t)rows);
+    const cudaError_t e = launch_dependent(kern, dim3(grid_for(rows * 16)), dim3(PRE_THREADS), 0, a.stream, (const __half*)a.b[0].ptr, (const float*)a.b[1].ptr, (const float2*)a.b[2].ptr, (__half*)a.b[3].ptr, p.n_heads, p.rot_dims / 2, (uint32_t)rows);
     ++*a.launches;
-    return check_cuda(a, cudaGetLastError(), "attn_norm_rope_d128");
+    return check_cuda(a, e, "attn_norm_rope_d128");
 }
 
 // kv_norm_rope_append_paged_q8_d128: k_raw, v_raw f16[n x row_len], k_w f32[128], cos_sin, k_scales, k_quants,
