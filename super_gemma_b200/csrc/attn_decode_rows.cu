@@ -2,17 +2,17 @@
 // head_dim 128 over the ring) and the verify step of up to four drafted tokens over the ring, head_dim 128.
 //
 // All of them are a few query rows (<= 8: the query heads of a kv head, times the drafted tokens) against many keys, bound by
-// the bytes of K and V.  A warp takes 16 keys at a time: their rows arrive by one bulk copy each in the warp's own slots
-// (K and V apart, so that the next K is on its way while this V is used; row pitch + 16 bytes keeps ldmatrix free of bank
-// conflicts), S = K Q^T and O^T += V^T P^T are mma.sync m16n8k16 with the keys or 16 dims as M and the rows as N: tcgen05 has
+// the bytes of K and V.  A warp takes 16 keys at a time: they arrive by TMA, 128 bytes of all 16 rows to a copy (128-byte
+// swizzle), in the warp's own slots (K and V apart, so that the next K is on its way while this V is used).  S = K Q^T and O^T += V^T P^T are mma.sync m16n8k16 with the keys or 16 dims as M and the rows as N: tcgen05 has
 // no tile this small.  Warps never wait for one another before the end, where their states merge in warp order.
 // Precision is that of the f32 statement (attn_decode_sliding.wgsl:84-107): Q8_0 keys enter as whole numbers and every block's
 // sum is multiplied by its f32 scale; P = (hi + lo) * 2^-14 with both halves f16 (22 bits, the factor keeps lo out of f16's
 // subnormals); running maximum and sums in f32.
-// Measured (us a call, streaming kernel before -> this one): head_dim 512, Q8_0 keys, 32768 tokens, 32 splits 427 -> 41.8
-// (206 MB, 4.9 TB/s); head_dim 256, 1024 slots, 16 splits 12.3 -> 6.1; verify of 4 tokens over the ring, 16 kv heads about
-// 205 -> 8.
-// Rows that hold no visible key are not copied but zeroed, and a CTA whose result is not finite computes it again by the
+// Measured (us a call, streaming kernel before -> this one): head_dim 512, Q8_0 keys, 32768 tokens, 32 splits 427 -> 40.6
+// (206 MB, 5.1 TB/s on the 128 SMs that 4 x 32 CTAs occupy); head_dim 256, 1024 slots, 16 splits 12.3 -> 5.7; verify of 4 tokens over
+// the ring, 16 kv heads 148 -> 8.4.
+// A copy per row instead (48 a tile at head_dim 512) was bound by the rate at which an SM's copy unit takes them: 41.8 us.
+// V rows that hold no visible key are zeroed once they have arrived, and a CTA whose result is not finite computes it again by the
 // streaming statement: a tile multiplies by p = 0 what that statement skips.
 #include <mutex>
 #include <string>
@@ -49,11 +49,6 @@ __device__ __forceinline__ void ldsm_x4_trans(uint32_t addr, uint32_t (&r)[4])
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
-__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar)
-{
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
 __device__ __forceinline__ float key_max(float v)
 {
     v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 4));
@@ -77,22 +72,21 @@ __device__ __forceinline__ void bytes_to_f16(uint32_t x, uint32_t& p01, uint32_t
     p23 = *reinterpret_cast<uint32_t*>(&hb);
 }
 
-// Keys of one 16-key tile that are copied: [from, to), row `row0 + i` of the operands; i is also its position minus pos0.
+// One 16-key tile: its tensor maps and first row, which of its rows are keys, [from, to), and the position of row 0.
 struct KeyTile {
-    size_t row0;
-    int from, to;
+    const CUtensorMap *k, *sc, *v;
+    int row0, from, to;
     int64_t pos0;
-    const KvOperand *k, *v;
 };
 
 template <int HD, bool KQ8, int ROWS>
 struct RowsWarp {
-    static constexpr int K_ROW = HD * (KQ8 ? 1 : 2), K_PITCH = K_ROW + 16, V_PITCH = HD * 2 + 16;
-    static constexpr int SC_ROW = KQ8 ? HD / 16 : 0, SC_PITCH = SC_ROW + (KQ8 ? 16 : 0);
-    struct __align__(16) Slots {
-        uint8_t k[TILE * K_PITCH];
-        uint8_t v[TILE * V_PITCH];  // afterwards the warp's output [ROWS][HD] f32
-        uint8_t sc[TILE * SC_PITCH + 16];
+    static constexpr int K_PIECES = HD * (KQ8 ? 1 : 2) / 128, V_PIECES = HD * 2 / 128;  // copies of [16 rows][128 bytes]
+    static constexpr uint32_t PIECE = TILE * 128, SC_ROW = KQ8 ? HD / 16 : 0;           // bytes
+    struct __align__(1024) Slots {
+        uint8_t k[K_PIECES][PIECE];
+        uint8_t v[V_PIECES][PIECE];  // afterwards the warp's output [ROWS][HD] f32
+        __align__(128) uint8_t sc[TILE * SC_ROW + 128];
         uint64_t k_full, v_full;
         float m[8], l[8];
     };
@@ -104,38 +98,27 @@ struct RowsWarp {
     // All tiles of this warp.  n tiles; tile(i, KeyTile&) describes the i-th.  row_lo/row_hi: positions rows 2*t4 + e may see.
     // q_sm: [8][q_pitch] f16 query rows.
     template <typename TileFn>
-    __device__ __forceinline__ void run(Slots& sl, int n, TileFn tile, const uint8_t* q_sm, int kvh, int n_kv, float scale, const int64_t (&row_lo)[2],
+    __device__ __forceinline__ void run(Slots& sl, int n, TileFn tile, const uint8_t* q_sm, int kvh, float scale, const int64_t (&row_lo)[2],
                                         const int64_t (&row_hi)[2], uint32_t* status)
     {
         constexpr int Q_PITCH = HD * 2 + (KQ8 ? 32 : 16);
         const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
-        const uint32_t kb = smem_u32(sl.k), vb = smem_u32(sl.v), sb = smem_u32(sl.sc), kbar = smem_u32(&sl.k_full), vbar = smem_u32(&sl.v_full);
-        const int i16 = lane & 15;
         auto issue_k = [&](int i) {
             KeyTile t;
             tile(i, t);
             fence_proxy_async_smem();  // the slot was read through the generic proxy
-            if (lane == 0) mbar_arrive_expect_tx(&sl.k_full, (uint32_t)(t.to - t.from) * (K_ROW + SC_ROW));
+            if (lane == 0) mbar_arrive_expect_tx(&sl.k_full, K_PIECES * PIECE + TILE * SC_ROW);
             __syncwarp();
-            if (i16 >= t.from && i16 < t.to) {
-                const size_t r = (t.row0 + i16) * n_kv + kvh;
-                if (lane < 16)
-                    bulk_copy(kb + i16 * K_PITCH, (const uint8_t*)t.k->data + r * K_ROW, K_ROW, kbar);
-                else if (KQ8)
-                    bulk_copy(sb + i16 * SC_PITCH, (const uint8_t*)t.k->scales + r * SC_ROW, SC_ROW, kbar);
-            }
+            if (lane < K_PIECES) tma_load_3d(sl.k[lane], t.k, &sl.k_full, lane * (KQ8 ? 128 : 64), kvh, t.row0);
+            if (KQ8 && lane == K_PIECES) tma_load_3d(sl.sc, t.sc, &sl.k_full, 0, kvh, t.row0);
         };
         auto issue_v = [&](int i) {
             KeyTile t;
             tile(i, t);
-            if (lane < 16 && !(i16 >= t.from && i16 < t.to)) {  // p = 0 there, and 0 times a stale Inf or NaN would not be
-                for (int c = 0; c < HD * 2; c += 16) *reinterpret_cast<uint4*>(sl.v + i16 * V_PITCH + c) = make_uint4(0u, 0u, 0u, 0u);
-            }
             fence_proxy_async_smem();
-            if (lane == 0) mbar_arrive_expect_tx(&sl.v_full, (uint32_t)(t.to - t.from) * HD * 2);
+            if (lane == 0) mbar_arrive_expect_tx(&sl.v_full, V_PIECES * PIECE);
             __syncwarp();
-            if (lane < 16 && i16 >= t.from && i16 < t.to)
-                bulk_copy(vb + i16 * V_PITCH, (const uint8_t*)t.v->data + ((t.row0 + i16) * n_kv + kvh) * HD * 2, HD * 2, vbar);
+            if (lane < V_PIECES) tma_load_3d(sl.v[lane], t.v, &sl.v_full, lane * 64, kvh, t.row0);
         };
 #pragma unroll
         for (int c = 0; c < HD / 16; c++) o[c][0] = o[c][1] = o[c][2] = o[c][3] = 0.0f;
@@ -146,8 +129,11 @@ struct RowsWarp {
             issue_k(0);
             issue_v(0);
         }
-        const uint32_t k_addr = kb + ((lane & 7) + 8 * ((lane >> 3) & 1)) * K_PITCH + (lane >> 4) * 16;
-        const uint32_t v_addr = vb + ((lane & 7) + 8 * (lane >> 4)) * V_PITCH + ((lane >> 3) & 1) * 16;
+        // ldmatrix: K plain, lane -> (row (lane & 7) + 8 * bit 3, 16-byte chunk + bit 4); V transposed, the two bits swapped.  Chunk c
+        // of a row lies in piece c / 8 at (c % 8) ^ (row & 7).
+        const uint32_t sw = lane & 7, k_addr = smem_u32(sl.k) + (sw + 8 * ((lane >> 3) & 1)) * 128, v_addr = smem_u32(sl.v) + (sw + 8 * (lane >> 4)) * 128;
+        const uint32_t k_bit = lane >> 4, v_bit = (lane >> 3) & 1;
+        auto at = [&](uint32_t base, uint32_t chunk) { return base + (chunk >> 3) * PIECE + (((chunk & 7) ^ sw) << 4); };
         const uint8_t* q_row = q_sm + g * Q_PITCH + t4 * (KQ8 ? 8 : 4);
         for (int i = 0; i < n; ++i) {
             KeyTile t;
@@ -158,36 +144,43 @@ struct RowsWarp {
                 uint4 sa[2], sc[2];  // 16 block scales of keys g and g + 8
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
-                    sa[h] = *reinterpret_cast<const uint4*>(sl.sc + g * SC_PITCH + 16 * h);
-                    sc[h] = *reinterpret_cast<const uint4*>(sl.sc + (g + 8) * SC_PITCH + 16 * h);
+                    sa[h] = *reinterpret_cast<const uint4*>(sl.sc + g * SC_ROW + 16 * h);
+                    sc[h] = *reinterpret_cast<const uint4*>(sl.sc + (g + 8) * SC_ROW + 16 * h);
                 }
                 const __half* ha = reinterpret_cast<const __half*>(sa);
                 const __half* hc = reinterpret_cast<const __half*>(sc);
 #pragma unroll
-                for (int b = 0; b < HD / 32; b++) {
-                    uint32_t x[4];
-                    ldsm_x4(k_addr + 32 * b, x);
-                    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                for (int b = 0; b < HD / 32; b += 2) {  // two blocks side by side: their MMAs do not wait for each other
+                    float acc[2][4] = {};
+                    uint32_t x[2][4];
+#pragma unroll
+                    for (int h = 0; h < 2; h++) ldsm_x4(at(k_addr, 2 * (b + h) + k_bit), x[h]);
 #pragma unroll
                     for (int cc = 0; cc < 2; cc++) {
-                        uint32_t a[4];
-                        bytes_to_f16(x[2 * cc], a[0], a[2]);
-                        bytes_to_f16(x[2 * cc + 1], a[1], a[3]);
-                        const uint2 q = *reinterpret_cast<const uint2*>(q_row + (2 * b + cc) * 32);
-                        mma16816(acc, a, q.x, q.y);
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            uint32_t a[4];
+                            bytes_to_f16(x[h][2 * cc], a[0], a[2]);
+                            bytes_to_f16(x[h][2 * cc + 1], a[1], a[3]);
+                            const uint2 q = *reinterpret_cast<const uint2*>(q_row + (2 * (b + h) + cc) * 32);
+                            mma16816(acc[h], a, q.x, q.y);
+                        }
                     }
-                    const float fa = __half2float(ha[b]), fc = __half2float(hc[b]);
-                    s[0] = fmaf(fa, acc[0], s[0]);
-                    s[1] = fmaf(fa, acc[1], s[1]);
-                    s[2] = fmaf(fc, acc[2], s[2]);
-                    s[3] = fmaf(fc, acc[3], s[3]);
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const float fa = __half2float(ha[b + h]), fc = __half2float(hc[b + h]);
+                        s[0] = fmaf(fa, acc[h][0], s[0]);
+                        s[1] = fmaf(fa, acc[h][1], s[1]);
+                        s[2] = fmaf(fc, acc[h][2], s[2]);
+                        s[3] = fmaf(fc, acc[h][3], s[3]);
+                    }
                 }
             } else {
                 float s1[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
                 for (int c = 0; c < HD / 16; c++) {
                     uint32_t a[4];
-                    ldsm_x4(k_addr + 32 * c, a);
+                    ldsm_x4(at(k_addr, 2 * c + k_bit), a);
                     const uint32_t b0 = *reinterpret_cast<const uint32_t*>(q_row + 32 * c), b1 = *reinterpret_cast<const uint32_t*>(q_row + 32 * c + 16);
                     mma16816((c & 1) ? s1 : s, a, b0, b1);
                 }
@@ -234,12 +227,22 @@ struct RowsWarp {
                 lo[h] = movmatrix_trans(pack_half2(p[2 * h] - f.x, p[2 * h + 1] - f.y));
             }
             mbar_wait(&sl.v_full, i & 1, status, 602, failed);
+            if (t.from > 0 || t.to < TILE) {  // p = 0 in the rows that are no keys, and 0 times a stale Inf or NaN would not be
+                for (int w = lane; w < V_PIECES * TILE * 8; w += 32) {
+                    const int r = (w >> 3) & (TILE - 1);
+                    if (r < t.from || r >= t.to) *reinterpret_cast<uint4*>(&sl.v[0][0] + 16 * w) = make_uint4(0u, 0u, 0u, 0u);
+                }
+                __syncwarp();
+            }
 #pragma unroll
-            for (int c = 0; c < HD / 16; c++) {
-                uint32_t a[4];
-                ldsm_x4_trans(v_addr + 32 * c, a);
-                mma16816(o[c], a, hi[0], hi[1]);
-                mma16816(o[c], a, lo[0], lo[1]);
+            for (int c = 0; c < HD / 16; c += 4) {  // four accumulators at a time: hi and lo of one would wait for each other
+                uint32_t a[4][4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) ldsm_x4_trans(at(v_addr, 2 * (c + k) + v_bit), a[k]);
+#pragma unroll
+                for (int k = 0; k < 4; k++) mma16816(o[c + k], a[k], hi[0], hi[1]);
+#pragma unroll
+                for (int k = 0; k < 4; k++) mma16816(o[c + k], a[k], lo[0], lo[1]);
             }
             __syncwarp();
             if (i + 1 < n) issue_v(i + 1);
@@ -281,20 +284,26 @@ __device__ __forceinline__ void stage_queries(uint8_t* q_sm, int live, RowPtr ro
 
 template <int HD, int G, bool KQ8, int WARPS>
 struct DecodeRowsSmem {
-    uint8_t q[8 * (HD * 2 + (KQ8 ? 32 : 16))];
     typename RowsWarp<HD, KQ8, G>::Slots w[WARPS];
+    uint8_t q[8 * (HD * 2 + (KQ8 ? 32 : 16))];
 };
 
 // Split-K partials.  Grid, split ranges and partials as decode_generic_kernel.
 template <int HD, int G, bool KQ8, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) decode_rows_kernel(const __half* __restrict__ q, const __grid_constant__ KvOperand kop,
+__global__ void __launch_bounds__(WARPS * 32) decode_rows_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_sc,
+                                                                 const __grid_constant__ CUtensorMap tm_v, const __half* __restrict__ q,
+                                                                 const __grid_constant__ KvOperand kop,
                                                                  const __grid_constant__ KvOperand vop, float* __restrict__ part,
                                                                  const uint32_t* __restrict__ step, int step_slot, uint32_t n_splits, float scale,
                                                                  uint32_t* status)
 {
     using W = RowsWarp<HD, KQ8, G>;
-    extern __shared__ __align__(128) uint8_t smem_raw[];
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
     DecodeRowsSmem<HD, G, KQ8, WARPS>& sm = *reinterpret_cast<DecodeRowsSmem<HD, G, KQ8, WARPS>*>(smem_raw);
+    if ((smem_u32(smem_raw) & 1023u) != 0u) {  // the swizzled tiles need it; never seen, but never assumed
+        if (threadIdx.x == 0) report_error(status, DEV_ERR_BOUNDS, 603, smem_u32(smem_raw), 0);
+        return;
+    }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kvh = blockIdx.x, n_kv = gridDim.x, split = blockIdx.y, n_q = n_kv * G;
     const uint32_t i = blockIdx.z, m_q = gridDim.z;
@@ -324,14 +333,15 @@ __global__ void __launch_bounds__(WARPS * 32) decode_rows_kernel(const __half* _
     const int64_t lo[2] = {0, 0}, hi[2] = {INT64_MAX, INT64_MAX};
     w.run(sm.w[warp], tiles > warp ? (tiles - warp + WARPS - 1) / WARPS : 0,
           [&](int n, KeyTile& t) {
-              t.row0 = t_begin + (size_t)(warp + n * WARPS) * TILE;
+              t.row0 = (int)(t_begin + (uint32_t)(warp + n * WARPS) * TILE);
               t.from = 0;
-              t.to = (int)min((size_t)TILE, t_end - t.row0);
+              t.to = min(TILE, (int)t_end - t.row0);
               t.pos0 = 0;
-              t.k = &kop;
-              t.v = &vop;
+              t.k = &tm_k;
+              t.sc = &tm_sc;
+              t.v = &tm_v;
           },
-          sm.q, kvh, n_kv, scale, lo, hi, status);
+          sm.q, kvh, scale, lo, hi, status);
     __syncthreads();
     bool odd = false;
     for (int idx = threadIdx.x; idx < G * HD; idx += WARPS * 32) {
@@ -381,8 +391,8 @@ __global__ void __launch_bounds__(WARPS * 32) decode_rows_kernel(const __half* _
 constexpr int V_HD = 128, V_G = 2, V_WARPS = 4, V_CTAS = 8, V_DPL = V_HD / 32;
 
 struct VerifySmem {
-    uint8_t q[8 * (V_HD * 2 + 16)];
     RowsWarp<V_HD, false, 8>::Slots w[V_WARPS];
+    uint8_t q[8 * (V_HD * 2 + 16)];
     float acc[8][V_HD], m[8], l[8];  // this CTA's merged rows, read by the cluster
 };
 
@@ -398,12 +408,17 @@ __device__ __forceinline__ void cluster_sync()
 }
 
 __global__ void __cluster_dims__(V_CTAS, 1, 1) __launch_bounds__(V_WARPS * 32)
-    verify_ring_kernel(const __half* __restrict__ q, const __grid_constant__ KvOperand k_ring, const __grid_constant__ KvOperand v_ring,
+    verify_ring_kernel(const __grid_constant__ CUtensorMap tm_kr, const __grid_constant__ CUtensorMap tm_vr, const __grid_constant__ CUtensorMap tm_kn,
+                       const __grid_constant__ CUtensorMap tm_vn, const __half* __restrict__ q, const __grid_constant__ KvOperand k_ring, const __grid_constant__ KvOperand v_ring,
                        const __grid_constant__ KvOperand k_new, const __grid_constant__ KvOperand v_new, float* __restrict__ out,
                        const uint32_t* __restrict__ step, uint32_t n_kv, uint32_t m_q, uint32_t window, uint32_t ring, float scale, uint32_t* status)
 {
-    extern __shared__ __align__(128) uint8_t smem_raw[];
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
     VerifySmem& sm = *reinterpret_cast<VerifySmem*>(smem_raw);
+    if ((smem_u32(smem_raw) & 1023u) != 0u) {  // the swizzled tiles need it; never seen, but never assumed
+        if (threadIdx.x == 0) report_error(status, DEV_ERR_BOUNDS, 604, smem_u32(smem_raw), 0);
+        return;
+    }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t4 = lane & 3;
     const int kvh = blockIdx.x / V_CTAS, rank = blockIdx.x % V_CTAS, n_q = (int)n_kv * V_G, rows = (int)m_q * V_G;
     if (lane == 0) {
@@ -434,21 +449,21 @@ __global__ void __cluster_dims__(V_CTAS, 1, 1) __launch_bounds__(V_WARPS * 32)
               const int it = me + n * V_CTAS * V_WARPS;
               if (it < n_hist) {
                   t.pos0 = first + (int64_t)it * TILE;
-                  t.row0 = (size_t)(t.pos0 % ring);
+                  t.row0 = (int)(t.pos0 % ring);
                   t.from = (int)max((int64_t)0, band_lo - t.pos0);
                   t.to = (int)min((int64_t)TILE, q0 - t.pos0);
-                  t.k = &k_ring;
-                  t.v = &v_ring;
+                  t.k = &tm_kr;
+                  t.v = &tm_vr;
               } else {
                   t.pos0 = q0;
                   t.row0 = 0;
                   t.from = 0;
                   t.to = (int)m_q;
-                  t.k = &k_new;
-                  t.v = &v_new;
+                  t.k = &tm_kn;
+                  t.v = &tm_vn;
               }
           },
-          sm.q, kvh, (int)n_kv, scale, lo, hi, status);
+          sm.q, kvh, scale, lo, hi, status);
     __syncthreads();
     for (int idx = threadIdx.x; idx < 8 * V_HD; idx += V_WARPS * 32) {
         const int r = idx / V_HD, d = idx % V_HD;
@@ -510,6 +525,15 @@ __global__ void __cluster_dims__(V_CTAS, 1, 1) __launch_bounds__(V_WARPS * 32)
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
+// [row][head][n] tensor of `elem`-byte values, boxes of n_box x 1 x 16 rows.
+int encode_tiles(const LaunchArgs& a, CUtensorMap* tm, const void* base, uint64_t rows, uint64_t heads, uint64_t n, uint32_t n_box, int elem, int swizzle)
+{
+    const uint64_t dims[3] = {n, heads, rows};
+    const uint64_t strides[2] = {n * elem, heads * n * elem};
+    const uint32_t box[3] = {n_box, 1, TILE};
+    return encode_tensor_map(a, tm, elem == 2, 3, const_cast<void*>(base), dims, strides, box, swizzle);
+}
+
 template <typename Kern>
 int allow_smem(const LaunchArgs& a, Kern kern, size_t smem)
 {
@@ -524,9 +548,11 @@ int allow_smem(const LaunchArgs& a, Kern kern, size_t smem)
 
 }  // namespace
 
-// The bulk copies need 16-byte aligned bases; anything else stays on the streaming kernel.
+// The copies need 16-byte aligned bases and row numbers within an int; anything else stays on the streaming kernel.
 bool decode_rows_takes(const KvOperand& k, const KvOperand& v, const void* q)
 {
+    for (const KvOperand* o : {&k, &v})
+        if (o->rows == 0 || o->rows >= (1u << 30)) return false;
     return aligned16(k.data) && aligned16(v.data) && aligned16(q) && (k.scales == nullptr || aligned16(k.scales));
 }
 
@@ -548,7 +574,13 @@ int launch_decode_rows(const LaunchArgs& a, const void* q, const KvOperand& k, c
             if (a.device < 64) attr_set[a.device] = true;
         }
     }
-    const cudaError_t e = launch_dependent(kern, dim3(n_kv, n_splits, m_q), dim3(WARPS * 32), smem, a.stream, (const __half*)q, k, v, (float*)part,
+    CUtensorMap tk, ts, tv;
+    if (int r = encode_tiles(a, &tk, k.data, k.rows, n_kv, HD, KQ8 ? 128 : 64, KQ8 ? 1 : 2, 3)) return r;
+    if (int r = encode_tiles(a, &tv, v.data, v.rows, n_kv, HD, 64, 2, 3)) return r;
+    ts = tk;
+    if (KQ8)
+        if (int r = encode_tiles(a, &ts, k.scales, k.rows, n_kv, HD / 32, HD / 32, 2, 0)) return r;
+    const cudaError_t e = launch_dependent(kern, dim3(n_kv, n_splits, m_q), dim3(WARPS * 32), smem, a.stream, tk, ts, tv, (const __half*)q, k, v, (float*)part,
                                            (const uint32_t*)step, step_slot, n_splits, scale, a.status);
     ++*a.launches;
     return check_cuda(a, e, "attn_decode");
@@ -564,7 +596,11 @@ int launch_verify_ring_d128(const LaunchArgs& a, const void* q, const KvOperand&
     constexpr size_t smem = sizeof(VerifySmem);
     static_assert(smem <= 100 * 1024, "two or more CTAs per SM");
     if (int r = allow_smem(a, verify_ring_kernel, smem)) return r;
-    const cudaError_t e = launch_dependent(verify_ring_kernel, dim3(n_kv * V_CTAS), dim3(V_WARPS * 32), smem, a.stream, (const __half*)q, k_ring, v_ring,
+    CUtensorMap tm[4];
+    const KvOperand* const ops[4] = {&k_ring, &v_ring, &k_new, &v_new};
+    for (int i = 0; i < 4; i++)
+        if (int r = encode_tiles(a, &tm[i], ops[i]->data, ops[i]->rows, n_kv, V_HD, 64, 2, 3)) return r;
+    const cudaError_t e = launch_dependent(verify_ring_kernel, dim3(n_kv * V_CTAS), dim3(V_WARPS * 32), smem, a.stream, tm[0], tm[1], tm[2], tm[3], (const __half*)q, k_ring, v_ring,
                                            k_new, v_new, (float*)out, (const uint32_t*)step, n_kv, m, window, ring, scale, a.status);
     ++*a.launches;
     return check_cuda(a, e, "attn_verify_sliding_ring");
