@@ -36,6 +36,7 @@ struct KernelEntry {
     uint32_t push_bytes;
     const char* signature;
     LaunchFn fn;
+    uint32_t writes;  // bit i: binding i is written; 0: ordered with every other dispatch of a recorded graph
 };
 
 // Host-side error helpers shared by the launchers (defined in sgb_runtime.cu).
