@@ -13,6 +13,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import operator
 import struct
 from dataclasses import dataclass
 from typing import Callable, Iterable, Optional, Sequence
@@ -304,10 +305,24 @@ def _push_bytes(push) -> bytes:
         return struct.pack("<I", int(push))
     if isinstance(push, (float, np.floating)):
         return struct.pack("<f", float(push))
-    out = b""
-    for v in push:  # a tuple of u32 / f32 fields, in declaration order
-        out += struct.pack("<f", float(v)) if isinstance(v, (float, np.floating)) else struct.pack("<I", int(v))
-    return out
+    fields = [(float(v), "f") if isinstance(v, (float, np.floating)) else (int(v), "I") for v in push]  # u32 / f32, in declaration order
+    return struct.pack("<" + "".join(f for _, f in fields), *[v for v, _ in fields])
+
+
+# sgb_dispatch as it is called here: bindings, push words and groups as packed bytes, which the library only reads.  A ctypes
+# structure per binding costs several times as much, more than the launch itself.
+_PACKED = [_vp, _vp, C.c_char_p, _u32, C.c_char_p, _sz, C.c_char_p]
+_U32 = 0xFFFFFFFF
+_packed_fns: dict = {}
+
+
+def _packed(name: str):
+    fn = _packed_fns.get(name)
+    if fn is None:
+        fn = lib()[name]  # a function object of its own: the prototypes of ABI stay as they are
+        fn.restype, fn.argtypes = _int, _PACKED
+        _packed_fns[name] = fn
+    return fn
 
 
 class GpuContext:
@@ -383,19 +398,22 @@ class GpuContext:
                                             info.signature.decode()))
 
     def _dispatch(self, fn, kernel: Kernel, bindings: Sequence[BufferBinding], push, groups: Sequence[int]) -> None:
-        arr = (_Binding * len(bindings))(*[_Binding(b.index, b.buf._h) for b in bindings])
+        flat: list = []
+        for b in bindings:
+            flat += (operator.index(b.index) & _U32, b.buf._h or 0)
+        n = len(bindings)
         pb = _push_bytes(push)
-        g = (C.c_uint32 * 3)(*(list(groups) + [1, 1, 1])[:3])
-        pbuf = C.create_string_buffer(pb, len(pb)) if pb else None
-        _check(fn(self._h, kernel._h, arr, len(bindings), C.cast(pbuf, C.c_void_p) if pbuf else None, len(pb), g))
+        g = (list(groups) + [1, 1, 1])[:3]
+        _check(fn(self._h, kernel._h, struct.pack("I4xP" * n, *flat), n, pb or None, len(pb),
+                  struct.pack("3I", operator.index(g[0]) & _U32, operator.index(g[1]) & _U32, operator.index(g[2]) & _U32)))
 
     def dispatch(self, kernel: Kernel, bindings: Sequence[BufferBinding], push, groups: Sequence[int]) -> None:
         """Enqueue (or, while recording, capture) one kernel (GraphRecorder::dispatch, graph.rs:203)."""
-        self._dispatch(lib().sgb_dispatch, kernel, bindings, push, groups)
+        self._dispatch(_packed("sgb_dispatch"), kernel, bindings, push, groups)
 
     def dispatch_blocking(self, kernel: Kernel, bindings: Sequence[BufferBinding], push, groups: Sequence[int]) -> None:
         """One-shot dispatch and wait (exec.rs:12-23)."""
-        self._dispatch(lib().sgb_dispatch_blocking, kernel, bindings, push, groups)
+        self._dispatch(_packed("sgb_dispatch_blocking"), kernel, bindings, push, groups)
 
     def sync(self, timeout_ms: int = 0) -> None:
         _check(lib().sgb_sync(self._h, timeout_ms))
