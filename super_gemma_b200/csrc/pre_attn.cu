@@ -217,20 +217,23 @@ __global__ void __launch_bounds__(PRE_THREADS) norm_rope_d128_kernel(const __hal
 
 // Q8_0 of the 32-value block that four consecutive lanes hold (8 values each): the arithmetic of
 // kv_quant_q8.wgsl:38-57 (see kv_codec.cu); the block maximum by two shuffles.  All lanes of the warp call it.
-__device__ __forceinline__ void quant_oct_f32(const float (&x)[8], __half& scale, uint2& packed)
+__device__ __forceinline__ void quant_oct_f32(const float2 (&x)[4], __half& scale, uint2& packed)
 {
     float amax = 0.0f;
 #pragma unroll
-    for (int i = 0; i < 8; i++) amax = fmaxf(amax, fabsf(x[i]));
+    for (int i = 0; i < 4; i++) amax = max3(amax, fabsf(x[i].x), fabsf(x[i].y));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
     const float d = __fmul_rn(amax, 1.0f / 127.0f);
-    const float id = d > 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
+    const float id = d > 0.0f ? __frcp_rn(d) : 0.0f;
     scale = __float2half_rn(d);
-    uint32_t p[2] = {0u, 0u};
+    uint32_t w[4];  // two quants each, in the low bytes
 #pragma unroll
-    for (int i = 0; i < 8; i++) p[i >> 2] |= (uint32_t)(__float2int_rn(__fmul_rn(x[i], id)) & 0xFF) << (8 * (i & 3));
-    packed = make_uint2(p[0], p[1]);
+    for (int i = 0; i < 4; i++) {
+        const float2 y = __fmul2_rn(x[i], make_float2(id, id));
+        w[i] = __byte_perm((uint32_t)__float2int_rn(y.x), (uint32_t)__float2int_rn(y.y), 0x0040);
+    }
+    packed = make_uint2(__byte_perm(w[0], w[1], 0x5410), __byte_perm(w[2], w[3], 0x5410));
 }
 
 // kv_norm_rope_append_paged_q8_d128: K rows (norm with k_w, rope) and V rows (weightless norm), both landing Q8_0-quantised at
@@ -261,17 +264,15 @@ __global__ void __launch_bounds__(PRE_THREADS)
     // rotation: dims [8 o, 8 o + 8) pair with +-64; half_rot is a multiple of 8 (checked on the host), so a whole octet turns or none
     const uint32_t pair0 = (uint32_t)(o & 7) * 8;
     const bool turns = pair0 < half_rot;
-    float c[8], sn[8];
+    float2 c[4], sn[4];
     if (turns) {
         const float4* cp = reinterpret_cast<const float4*>(cos_sin + (size_t)token * half_rot + pair0);
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const float4 cs = __ldg(cp + j);
-            c[2 * j] = cs.x;
-            c[2 * j + 1] = cs.z;
+            c[j] = make_float2(cs.x, cs.z);
             // low half: lo*c - hi*s with lo = own; high half: hi*c + lo*s with hi = own (x - y is x + (-y), bit for bit)
-            sn[2 * j] = o < 8 ? -cs.y : cs.y;
-            sn[2 * j + 1] = o < 8 ? -cs.w : cs.w;
+            sn[j] = o < 8 ? make_float2(-cs.y, -cs.w) : make_float2(cs.y, cs.w);
         }
     }
     size_t dst_row = 0;
@@ -298,51 +299,45 @@ __global__ void __launch_bounds__(PRE_THREADS)
         const uint32_t r = r0 + slot;
         const bool live = r < rows, is_q = r < n_q, is_v = r >= n_q + n_kv;
         const uint32_t head = is_q ? r : is_v ? r - n_q - n_kv : r - n_q;
-        float v[8];
-        float wv[8];
+        // pairs: packed f32x2 multiplies round each half like the scalar ones
+        float2 v[4], wv[4];
 #pragma unroll
-        for (int i = 0; i < 8; i++) wv[i] = 1.0f;
+        for (int j = 0; j < 4; j++) wv[j] = make_float2(1.0f, 1.0f);
         if (live && !is_v) {
             const float* w = (is_q ? q_w : k_w) + 8 * o;
             const float4 w0 = __ldg(reinterpret_cast<const float4*>(w)), w1 = __ldg(reinterpret_cast<const float4*>(w) + 1);
-            const float x[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+            const float2 x[4] = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w), make_float2(w1.x, w1.y), make_float2(w1.z, w1.w)};
 #pragma unroll
-            for (int i = 0; i < 8; i++) wv[i] = PLUS_ONE ? 1.0f + x[i] : x[i];
+            for (int j = 0; j < 4; j++) wv[j] = PLUS_ONE ? __fadd2_rn(make_float2(1.0f, 1.0f), x[j]) : x[j];
         }
+        float ss = 0.0f;
         {
             const __half2* h = reinterpret_cast<const __half2*>(&u);
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const float2 f = __half22float2(h[j]);
-                v[2 * j] = f.x;
-                v[2 * j + 1] = f.y;
+                v[j] = __half22float2(h[j]);
+                ss = fmaf(v[j].x, v[j].x, ss);
+                ss = fmaf(v[j].y, v[j].y, ss);
             }
         }
-        float ss = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 8; i++) ss = fmaf(v[i], v[i], ss);
 #pragma unroll
         for (int d = 1; d < 16; d <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);  // fixed tree: every lane gets the same bits
         const float inv = rsqrtf(ss / 128.0f + RMS_EPS);
         uint32_t own[4];  // the normed octet as f16 pairs: what the chain of kernels stores between norm and rotation
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            own[j] = pack_half2(v[2 * j] * inv * wv[2 * j], v[2 * j + 1] * inv * wv[2 * j + 1]);
-            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&own[j]));
-            v[2 * j] = f.x;
-            v[2 * j + 1] = f.y;
+            const float2 y = __fmul2_rn(__fmul2_rn(v[j], make_float2(inv, inv)), wv[j]);
+            own[j] = pack_half2(y.x, y.y);
+            v[j] = __half22float2(*reinterpret_cast<const __half2*>(&own[j]));
         }
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const uint32_t other = __shfl_xor_sync(0xffffffffu, own[j], 8);  // the partner octet, dims +-64
             if (turns && !is_v) {
                 const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&other));
-                const float a = __fadd_rn(__fmul_rn(v[2 * j], c[2 * j]), __fmul_rn(f.x, sn[2 * j]));
-                const float b = __fadd_rn(__fmul_rn(v[2 * j + 1], c[2 * j + 1]), __fmul_rn(f.y, sn[2 * j + 1]));
-                own[j] = pack_half2(a, b);
-                const float2 y = __half22float2(*reinterpret_cast<const __half2*>(&own[j]));
-                v[2 * j] = y.x;
-                v[2 * j + 1] = y.y;
+                // not packed: a packed multiply and add were contracted to one rounding
+                own[j] = pack_half2(__fadd_rn(__fmul_rn(v[j].x, c[j].x), __fmul_rn(f.x, sn[j].x)), __fadd_rn(__fmul_rn(v[j].y, c[j].y), __fmul_rn(f.y, sn[j].y)));
+                v[j] = __half22float2(*reinterpret_cast<const __half2*>(&own[j]));
             }
         }
         if (r0 + ROWS_PER_PASS <= n_q) {  // only q rows in this pass (uniform over the block)
