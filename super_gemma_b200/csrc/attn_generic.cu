@@ -1,6 +1,5 @@
-// Scalar (CUDA-core) attention kernels: every reference-shaped registry name, and the d128 cases
-// that are too small for a tensor-core tile (sliding decode, 4-token verify over the ring, the
-// 512-token sliding prefill).  They follow the reference's streaming-softmax statement per key
+// Scalar (CUDA-core) attention kernels: the statement of every reference-shaped registry name, for what the tensor-core kernels
+// do not take, and the launchers that choose between the two.  They follow the reference's streaming-softmax statement per key
 // (attn_decode_sliding.wgsl:84-107 and its siblings) with f32 math, one warp per key and the four
 // warps of a block merged in a fixed order, so reruns are bit-identical.
 #include "attn_merge.cuh"
@@ -361,9 +360,9 @@ int launch_prefill_generic(const LaunchArgs& a)
             return launch_verify_ring_d128(a, a.b[0].ptr, kh, vh, kc, vc, a.b[bi].ptr, a.b[bi + 1].ptr, n_kv, (uint32_t)m, WINDOW, RING, scale);
     }
     if constexpr (HD == 256 && !OUT_F32) {
-        if (prefill_wide_takes<HD, G, false, TWO_RANGE != 0>(a, kh, vh, kc, vc, a.b[0].ptr, scale))
-            return launch_prefill_wide<HD, G, false, TWO_RANGE != 0>(a, a.b[0].ptr, nullptr, kh, vh, kc, vc, a.b[bi].ptr, a.b[bi + 1].ptr, n_kv,
-                                                                     (uint32_t)m, WINDOW, RING, scale);
+        if (prefill_wide_takes<TWO_RANGE != 0>(kh, vh, kc, vc, a.b[0].ptr, a.b[bi].ptr, scale))
+            return launch_prefill_wide<TWO_RANGE != 0>(a, a.b[0].ptr, kh, vh, kc, vc, a.b[bi].ptr, a.b[bi + 1].ptr, n_kv, (uint32_t)m, WINDOW, RING,
+                                                       scale);
     }
     prefill_generic_kernel<HD, G, FMT_F16, FMT_F16, TWO_RANGE, OUT_F32><<<dim3(n_kv, (uint32_t)m), GEN_THREADS, 0, a.stream>>>(
         a.b[0].ptr, nullptr, kh, vh, kc, vc, a.b[bi].ptr, (const uint32_t*)a.b[bi + 1].ptr, WINDOW, RING, scale,
@@ -455,9 +454,8 @@ int launch_prefill_global_flash_ref(const LaunchArgs& a)
     if (int r = need_bytes(a, bi, m * n_q * HD * 2, "out")) return r;
     if (int r = need_bytes(a, bi + 1, 16, "step")) return r;
     if constexpr (VARIANT == 2) {
-        if (prefill_wide_takes<HD, G, true, false>(a, kop, vop, none, none, a.b[0].ptr, scale))
-            return launch_prefill_wide<HD, G, true, false>(a, a.b[0].ptr, q_scales, kop, vop, none, none, a.b[bi].ptr, a.b[bi + 1].ptr, N_KV,
-                                                           (uint32_t)m, 0, 0, scale);
+        if (prefill_int8_takes(kop, vop, a.b[0].ptr, scale))
+            return launch_prefill_int8(a, a.b[0].ptr, q_scales, kop, vop, a.b[bi].ptr, a.b[bi + 1].ptr, N_KV, (uint32_t)m, scale);
     }
     const dim3 grid(N_KV, (uint32_t)m);
     void* out = a.b[bi].ptr;

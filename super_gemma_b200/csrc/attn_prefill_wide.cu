@@ -1,25 +1,18 @@
-// Prefill attention for the reference model's own layers on tcgen05: head_dim 256 (sliding layers, f16 K/V, 2 query heads per
-// kv head, 1024-token window over a linear cache or ring history + chunk) and head_dim 512 (global layers, int8 Q and K with
-// f16 block scales, f16 V, 8 query heads per kv head).  Semantics: attn_prefill_sliding.wgsl:53-125,
-// attn_prefill_sliding_ring.wgsl:88-140, attn_prefill_global_flash_sp_iq.wgsl.
+// Prefill attention for the reference model's sliding layers on tcgen05: head_dim 256, f16 K/V, 2 query heads per kv head,
+// 1024-token window over a linear cache or ring history + chunk.  Semantics: attn_prefill_sliding.wgsl:53-125,
+// attn_prefill_sliding_ring.wgsl:88-140.
 //
-// A head of 512 dims fills tensor memory with a 128-row f32 output alone, so everything here is transposed: keys and output
-// dims are the M = 128 side of the MMAs, and a CTA's 64 query rows (64 / G tokens x the G query heads of one kv head, which
-// share every K/V tile) are the N side.  Per 128-key tile:
-//   S^T[128 keys x 64 rows]  = K Q^T    thread = key, so a Q8_0 key's scales are that thread's registers
-//   O^T[HD dims x 64 rows]  += V^T P^T  V is the MN-major A operand straight from its [key][dim] tile, P^T the MN-major B
-//                                       operand that each thread writes as one swizzled 128-byte row
-// Q8_0 scores: one kind::i8 MMA (K = 32) per scale block gives that block's whole-number dot product, exactly; the two f16
-// scales multiply it in f32 (f32(qs) * f32(ks) is exact), so the score is closer to f32(scale) * f32(q) arithmetic than an
-// f32 dot product.  Blocks go through four 64-column buffers, two per hand-over.
-// P keeps f32 precision: P = hi + lo with both halves f16 (22 bits), two MMAs per V tile.  The exponent carries +7, so that
+// A CTA owns 128 query rows (64 tokens x the 2 query heads of one kv head, which share every K/V tile).  Per 64-key tile
+// S[128 x 64] = Q K^T, softmax with two threads per row (32 keys each), O[128 x 256] += P V with P as the tensor-memory A
+// operand and V as the MN-major B operand straight from its [key][dim] tile.  (A transposed form, with V as the MN-major A
+// operand of 128 x 64 instructions, needed 160 cycles per instruction where K-major operands take 48: 38.6 us where this
+// one takes 22.7.)  Where two CTAs per unit fit the GPU at once a cluster of two shares a unit's key tiles; the halves
+// merge at the end through distributed shared memory, each CTA finishing 128 of the dims.
+// P keeps f32 precision: P = hi + lo with both halves f16 (22 bits), two MMAs per 16 keys.  The exponent carries +7, so that
 // lo stays clear of f16's subnormals (the factor cancels in O / l).
-// Roles: warps 0-7 softmax (two threads per key, 32 rows each), one MMA thread, one K and one V loader thread; mbarriers only.
-// The row maximum over keys runs across threads; it is only computed (32 values in 31 shuffles) when some score exceeds its
-// row's running maximum by 2^8, which one barrier with an OR finds out.
-//
-// Measured (us a call, streaming kernel before -> this one): 256 queries at 7936 + 256 keys, head_dim 512 int8: 13500 -> 500;
-// 256 queries, head_dim 256 over ring + chunk: about 790 -> 30.  The floors are 86 us (tensor) and 5.4 us (bytes).
+// Roles: warps 0-7 softmax, one MMA thread, one K and one V loader; mbarriers only.
+// Measured: 256 queries, 16 kv heads, ring + chunk: 795 us on the streaming kernel, 22.7 here; bound by the chain score -> softmax
+// -> P V of eight tiles plus set-up and merge (3000 cycles a tile, of which the MMAs need 1800).
 //
 // What a tile reads beyond a query's own keys must not matter: scores are masked by selection, V rows that hold no key are
 // zeroed.  A V row that is visible to some query of the tile and not finite is visible to all of them as 0 * Inf, so a CTA
@@ -35,123 +28,73 @@ namespace sgb {
 
 namespace {
 
-constexpr int ROWS = 64;       // query rows per CTA (N)
-constexpr int TILE_K = 128;    // keys per tile (M of S^T)
+constexpr int ROWS = 128;     // query rows per CTA (M)
+constexpr int TILE_K = 64;    // keys per tile
+constexpr int HD = 256, G = 2;
 constexpr int SOFT_THREADS = 256;
 constexpr int MMA_W = 8, K_W = 9, V_W = 10;
 constexpr int WIDE_THREADS = 352;
-constexpr int NV = 5;                          // V units in flight
-constexpr uint32_t Q_CHUNK = ROWS * 128;       // 128 bytes of every row
+constexpr int CHUNKS = 4, STAGES = 2;       // 128-byte chunks of a row of Q or K; K and V tiles in flight
+constexpr uint32_t Q_CHUNK = ROWS * 128;    // 128 bytes of every row
 constexpr uint32_t K_CHUNK = TILE_K * 128;
-constexpr uint32_t V_UNIT = 64 * 256;          // 64 keys x 128 dims f16, as two [64 keys][128 B] halves
-constexpr uint32_t P_TILE = TILE_K * ROWS * 2; // [128 keys][64 rows] f16
+constexpr uint32_t V_CHUNK = TILE_K * 128;  // 64 dims f16 of every key
+constexpr uint32_t V_TILE = 4 * V_CHUNK;
+constexpr uint32_t TMEM_O = 0, TMEM_S = 256, TMEM_COLS = 512;
 constexpr float EXP_BIAS = 7.0f, GROW_T = 8.0f;
 
 struct WideSmem {
-    uint8_t q[4][Q_CHUNK];
-    uint8_t k[4][K_CHUNK];
-    uint8_t p[2][P_TILE];  // hi, lo
-    uint8_t v[NV][V_UNIT];
-    float qs[16][ROWS];    // int8 Q: its scales, [block][row]
-    float red[4][ROWS];
-    float m_ref[ROWS], corr[ROWS];
-    uint64_t q_bar, k_full[4], k_free[4], v_full[NV], v_free[NV], v_ok[NV], s_ready[2], s_free[2], p_ready, pv_done;
+    uint8_t q[CHUNKS][Q_CHUNK];
+    uint8_t k[STAGES][CHUNKS][K_CHUNK];  // afterwards the other CTA's O of this CTA's 128 dims
+    uint8_t v[STAGES][V_TILE];
+    float red[2][ROWS];
+    float2 other_ml[ROWS];
+    uint64_t q_bar, k_full[STAGES], k_free[STAGES], v_full[STAGES], v_free[STAGES], v_ok[STAGES], s_ready[2], p_ready[2], pv_done[2];
     uint32_t tmem_base, abort, redo;
 };
-static_assert(sizeof(WideSmem) + 1024 <= 227 * 1024, "one CTA per SM");
+static_assert(sizeof(WideSmem) <= 227 * 1024, "one CTA per SM");
 
 struct WideParams {
     const uint32_t* step;
     __half* out;
     uint32_t* status;
-    const __half* q_scales;  // int8 Q
     uint32_t m_tokens, n_kv, window, ring;
     float scale;
+    uint32_t n_cta;          // CTAs of a cluster
     const void* q;           // for the streaming statement
     KvOperand k0, v0, k1, v1;
 };
 
-// tcgen05.mma kind::i8: int8 operands, int32 accumulator, K = 32 (32 bytes, like a K = 16 step of f16).
-__device__ __forceinline__ void umma_i8_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc)
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t smem_addr, uint32_t rank)
+{
+    uint32_t out;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(smem_addr), "r"(rank));
+    return out;
+}
+__device__ __forceinline__ void st_cluster_f4(uint32_t addr, float4 v)
+{
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t (&r)[16])
 {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, 0, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc)
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+          "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
         : "memory");
-}
-// Instruction descriptor of kind::i8: D format 2 = s32, A and B format 1 = signed 8 bit, both K-major.
-__host__ __device__ constexpr uint32_t umma_idesc_i8(uint32_t m, uint32_t n)
-{
-    return (2u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((m >> 4) << 24);
-}
-// Barrier over `threads` threads that also tells every one of them whether `pred` held for any.
-__device__ __forceinline__ bool named_barrier_or(uint32_t id, uint32_t threads, bool pred)
-{
-    uint32_t r;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %3, 0;\n\t"
-        "barrier.cta.red.or.pred q, %1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}\n"
-        : "=r"(r)
-        : "r"(id), "r"(threads), "r"((uint32_t)pred)
-        : "memory");
-    return r != 0;
-}
-
-// Reduce 32 values over the 32 lanes of a warp: lane c is left with the total of v[c].  Each step halves the values.
-template <bool MAX>
-__device__ __forceinline__ float transpose_reduce(float (&v)[32], int lane)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const bool upper = (lane & o) != 0;
-#pragma unroll
-        for (int i = 0; i < o; i++) {
-            const float send = upper ? v[i] : v[i + o], keep = upper ? v[i + o] : v[i];
-            const float r = __shfl_xor_sync(0xffffffffu, send, o);
-            v[i] = MAX ? fmaxf(keep, r) : keep + r;
-        }
-    }
-    return v[0];
 }
 
 // The rows of one CTA by the streaming statement, a warp per row.
-template <int HD, int G, bool QI8, bool TWO_SRC>
+template <bool TWO_SRC>
 __device__ __noinline__ void stream_rows(const WideParams& prm, uint32_t m0, int kvh)
 {
-    constexpr int DPL = HD / 32, KFMT = QI8 ? FMT_Q8 : FMT_F16;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d0 = lane * DPL, n_kv = (int)prm.n_kv, n_q = n_kv * G;
     const uint32_t q0 = prm.step[STEP_Q0];
-    for (int r = warp; r < ROWS; r += WIDE_THREADS / 32) {
-        const uint32_t i = m0 + r / G;
-        if (i >= prm.m_tokens) break;
-        const size_t qrow = (size_t)i * n_q + kvh * G + r % G;
-        float qr[DPL], kk[DPL], vv[DPL];
-        if constexpr (QI8)
-            load_q8<DPL>(reinterpret_cast<const int8_t*>(prm.q) + qrow * HD + d0, prm.q_scales + qrow * (HD / 32), d0, qr);
-        else
-            load_f16<DPL>(reinterpret_cast<const __half*>(prm.q) + qrow * HD + d0, qr);
-        Stream<1, DPL> st;
-        st.init();
-        const uint32_t qpos = q0 + i, begin = (prm.window != 0 && qpos + 1 > prm.window) ? qpos + 1 - prm.window : 0;
-        const uint32_t hist_end = TWO_SRC ? min(q0, qpos + 1) : qpos + 1;
-        for (uint32_t t = begin; t < hist_end; t++) {
-            const size_t row = prm.ring ? t % prm.ring : t;
-            if (row >= prm.k0.rows || row >= prm.v0.rows) break;  // reported where the tiles are laid out
-            load_row<HD, KFMT, DPL>(prm.k0, row, kvh, n_kv, d0, kk);
-            load_row<HD, FMT_F16, DPL>(prm.v0, row, kvh, n_kv, d0, vv);
-            st.step(0, qr, kk, vv, prm.scale);
-        }
-        if (TWO_SRC) {
-            for (uint32_t c = begin > q0 ? begin - q0 : 0; c <= i; c++) {
-                load_row<HD, FMT_F16, DPL>(prm.k1, c, kvh, n_kv, d0, kk);
-                load_row<HD, FMT_F16, DPL>(prm.v1, c, kvh, n_kv, d0, vv);
-                st.step(0, qr, kk, vv, prm.scale);
-            }
-        }
-#pragma unroll
-        for (int d = 0; d < DPL; d++) prm.out[qrow * HD + d0 + d] = __float2half_rn(st.acc[0][d] / st.l[0]);
-    }
+    for (int r = threadIdx.x >> 5; r < ROWS && m0 + r / G < prm.m_tokens; r += WIDE_THREADS / 32)
+        stream_prefill_row<HD, G, false, TWO_SRC>(prm.q, nullptr, prm.k0, prm.v0, prm.k1, prm.v1, prm.out, q0, m0 + r / G, kvh * G + r % G, (int)prm.n_kv,
+                                                  prm.window, prm.ring, prm.scale);
 }
 
 struct WideTile {
@@ -159,30 +102,28 @@ struct WideTile {
     int64_t pos0, lo, hi;   // position of key 0; positions this source really holds
 };
 
-template <int HD, int G, bool QI8, bool TWO_SRC>
+template <bool TWO_SRC>
 __global__ void __launch_bounds__(WIDE_THREADS, 1)
     wide_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k0,
                         const __grid_constant__ CUtensorMap tm_v0, const __grid_constant__ CUtensorMap tm_k1,
                         const __grid_constant__ CUtensorMap tm_v1, const __grid_constant__ WideParams prm)
 {
-    static_assert(HD * (QI8 ? 1 : 2) == 512, "a row of Q or K is four 128-byte chunks");
-    constexpr int TOK = ROWS / G, DB = HD / 128, UNITS = 2 * DB;  // V units per tile: (dim block, key half)
-    constexpr int GROUPS = QI8 ? 8 : 1;                           // S hand-overs per tile
-    constexpr uint32_t S_COLS = QI8 ? 128 : 64;                   // columns of one hand-over
-    constexpr uint32_t TMEM_O = 0, TMEM_S = DB * 64, TMEM_COLS = QI8 ? 512 : 256;
-    static_assert(TMEM_S + 2 * S_COLS <= TMEM_COLS, "O and two S buffers fit");
+    constexpr int TOK = ROWS / G, CE = 64;  // tokens; elements of a 128-byte chunk
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     WideSmem& sm = *reinterpret_cast<WideSmem*>(smem_raw);
-    if ((smem_u32(smem_raw) & 1023u) != 0u) {  // the swizzled tiles need it; never seen, but never assumed
-        if (threadIdx.x == 0) report_error(prm.status, DEV_ERR_BOUNDS, 500, smem_u32(smem_raw), 0);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t rank = blockIdx.x % prm.n_cta, unit = blockIdx.x / prm.n_cta;
+    const bool split = prm.n_cta == 2;  // the CTAs of a cluster share the keys
+    const bool aligned = (smem_u32(smem_raw) & 1023u) == 0u;  // the swizzled tiles need it; never seen, but never assumed
+    if (!aligned) {                                           // the same in every CTA: nobody waits for one that left
+        if (tid == 0) report_error(prm.status, DEV_ERR_BOUNDS, 500, smem_u32(smem_raw), 0);
         return;
     }
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     pdl_wait();  // the step words, q, K and V come from earlier kernels of the stream
     pdl_launch_dependents();
-    const int kvh = blockIdx.x % prm.n_kv;
+    const int kvh = unit % prm.n_kv;
     const uint32_t n_qt = (prm.m_tokens + TOK - 1) / TOK;
-    const uint32_t m0 = (n_qt - 1 - blockIdx.x / prm.n_kv) * TOK;  // latest query tile (most keys) first
+    const uint32_t m0 = (n_qt - 1 - unit / prm.n_kv) * TOK;  // latest query tile (most keys) first
     const uint32_t live_tok = min((uint32_t)TOK, prm.m_tokens - m0);
     const int64_t q0 = prm.step[STEP_Q0];
     const int64_t first_qpos = q0 + m0, last_qpos = first_qpos + live_tok - 1;
@@ -207,8 +148,15 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
         n_hist = end >= band_lo ? (int)(end / TILE_K - band_lo / TILE_K + 1) : 0;
         n_tiles = n_hist;
     }
+    int t_begin = 0;
+    if (split) {
+        const int per = (n_tiles + 1) / 2;
+        t_begin = min(n_tiles, (int)rank * per);
+        n_tiles = min(n_tiles, t_begin + per) - t_begin;
+    }
     auto tile_at = [&](int it) {
         WideTile t;
+        it += t_begin;
         if (it < n_hist) {
             t.src = 0;
             t.pos0 = hist_pos0 + (int64_t)it * TILE_K;
@@ -230,34 +178,21 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
 
     if (tid == 0) {
         mbar_init(&sm.q_bar, 1);
-        for (int i = 0; i < 4; i++) {
+        for (int i = 0; i < STAGES; i++) {
             mbar_init(&sm.k_full[i], 1);
             mbar_init(&sm.k_free[i], 1);
-        }
-        for (int i = 0; i < NV; i++) {
             mbar_init(&sm.v_full[i], 1);
             mbar_init(&sm.v_free[i], 1);
             mbar_init(&sm.v_ok[i], 1);
         }
         for (int i = 0; i < 2; i++) {
             mbar_init(&sm.s_ready[i], 1);
-            mbar_init(&sm.s_free[i], SOFT_THREADS);
+            mbar_init(&sm.p_ready[i], SOFT_THREADS / 32);  // an arrival per warp: they serialise on the barrier's word
+            mbar_init(&sm.pv_done[i], 1);
         }
-        mbar_init(&sm.p_ready, SOFT_THREADS);
-        mbar_init(&sm.pv_done, 1);
         sm.abort = 0;
         sm.redo = 0;
         mbar_fence_init();
-    }
-    if (tid < ROWS) sm.m_ref[tid] = NEG_SENTINEL;
-    if (QI8) {
-        for (int i = tid; i < 16 * ROWS; i += WIDE_THREADS) {
-            const int r = i >> 4, b = i & 15;
-            const uint32_t tok = m0 + r / G;
-            float s = 0.0f;
-            if (tok < prm.m_tokens) s = __half2float(__ldg(prm.q_scales + ((size_t)tok * (prm.n_kv * G) + kvh * G + r % G) * 16 + b));
-            sm.qs[b][r] = s;
-        }
     }
     if (warp == 0) {
         tmem_alloc(&sm.tmem_base, TMEM_COLS);
@@ -269,267 +204,161 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
     const uint32_t tmem = sm.tmem_base;
     bool failed = false;
 
+    const int kq = warp & 3, half = warp >> 2, row = kq * 32 + lane;  // softmax threads: row, keys 32 * half .. of a tile
+    const uint32_t lane_addr = tmem + ((uint32_t)(kq * 32) << 16);
+    float m_run = NEG_SENTINEL, l_run = 0.0f;
+
     if (warp == K_W) {
-        // ======================= Q and K loads: K(j) chunk by chunk as the MMAs of tile j - 1 let go of them ==========
+        // ======================= Q and K loads =======================
         if (lane == 0) {
-            constexpr int CE = QI8 ? 128 : 64;  // elements of a 128-byte chunk
-            mbar_arrive_expect_tx(&sm.q_bar, 4 * Q_CHUNK);
-            for (int c = 0; c < 4; c++) tma_load_3d(sm.q[c], &tm_q, &sm.q_bar, c * CE, kvh * G, (int)m0);
-            for (int j = 0; j < n_tiles && !failed; ++j) {
+            mbar_arrive_expect_tx(&sm.q_bar, CHUNKS * Q_CHUNK);
+            for (int c = 0; c < CHUNKS; c++) tma_load_3d(sm.q[c], &tm_q, &sm.q_bar, c * CE, kvh * G, (int)m0);
+            for (int j = 0; j < n_tiles; ++j) {
                 const WideTile t = tile_at(j);
                 const CUtensorMap* mk = (TWO_SRC && t.src) ? &tm_k1 : &tm_k0;
-                for (int c = 0; c < 4; c++) {
-                    if (j > 0) mbar_wait(&sm.k_free[c], (j - 1) & 1, prm.status, 511, failed, 50);
-                    if (failed) break;  // never write into a buffer that may still be read
-                    mbar_arrive_expect_tx(&sm.k_full[c], K_CHUNK);
-                    tma_load_3d(sm.k[c], mk, &sm.k_full[c], c * CE, kvh, t.row0);
-                }
+                const int st = j % STAGES;
+                if (j >= STAGES) mbar_wait(&sm.k_free[st], (j / STAGES - 1) & 1, prm.status, 511, failed, 50);
+                if (failed) break;  // never write into a buffer that may still be read
+                mbar_arrive_expect_tx(&sm.k_full[st], CHUNKS * K_CHUNK);
+                for (int c = 0; c < CHUNKS; c++) tma_load_3d(sm.k[st][c], mk, &sm.k_full[st], c * CE, kvh, t.row0);
             }
         }
     } else if (warp == V_W) {
-        // ======================= V loads in units of 64 keys x 128 dims =======================
-        int n = 0;
-        for (int j = 0; j < n_tiles && !failed; ++j) {
+        // ======================= V loads =======================
+        for (int j = 0; j < n_tiles; ++j) {
             const WideTile t = tile_at(j);
             const CUtensorMap* mv = (TWO_SRC && t.src) ? &tm_v1 : &tm_v0;
             const int64_t last = valid_end(t);
             const bool tail = t.pos0 + TILE_K - 1 > last;  // the MMA warp computes the same
-            for (int u = 0; u < UNITS; u++, n++) {
-                const int st = n % NV;
-                if (n >= NV) mbar_wait(&sm.v_free[st], (n / NV - 1) & 1, prm.status, 512, failed, 50);
+            const int st = j % STAGES;
+            if (j >= STAGES) mbar_wait(&sm.v_free[st], (j / STAGES - 1) & 1, prm.status, 512, failed, 50);
+            if (failed) break;
+            if (lane == 0) {
+                mbar_arrive_expect_tx(&sm.v_full[st], V_TILE);
+                for (int c = 0; c < 4; c++) tma_load_3d(sm.v[st] + c * V_CHUNK, mv, &sm.v_full[st], c * 64, kvh, t.row0);
+            }
+            if (tail) {
+                __syncwarp();
+                mbar_wait(&sm.v_full[st], (j / STAGES) & 1, prm.status, 513, failed);
                 if (failed) break;
-                const int kh = u & 1, db = u >> 1;
-                if (lane == 0) {
-                    mbar_arrive_expect_tx(&sm.v_full[st], V_UNIT);
-                    tma_load_3d(sm.v[st], mv, &sm.v_full[st], db * 128, kvh, t.row0 + kh * 64);
-                    tma_load_3d(sm.v[st] + V_UNIT / 2, mv, &sm.v_full[st], db * 128 + 64, kvh, t.row0 + kh * 64);
-                }
-                if (tail) {
-                    __syncwarp();
-                    mbar_wait(&sm.v_full[st], (n / NV) & 1, prm.status, 513, failed);
-                    if (failed) break;
-                    for (int r = lane; r < 64; r += 32) {
-                        if (t.pos0 + kh * 64 + r <= last) continue;
+                for (int r = lane; r < TILE_K; r += 32) {
+                    if (t.pos0 + r <= last) continue;
 #pragma unroll
-                        for (int h = 0; h < 2; h++) {
-                            uint4* row = reinterpret_cast<uint4*>(sm.v[st] + h * (V_UNIT / 2) + r * 128);
+                    for (int c = 0; c < 4; c++) {
+                        uint4* p = reinterpret_cast<uint4*>(sm.v[st] + c * V_CHUNK + r * 128);
 #pragma unroll
-                            for (int i = 0; i < 8; i++) row[i] = make_uint4(0u, 0u, 0u, 0u);
-                        }
+                        for (int i = 0; i < 8; i++) p[i] = make_uint4(0u, 0u, 0u, 0u);
                     }
-                    fence_proxy_async_smem();  // generic-proxy writes, read next by the tensor pipe
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&sm.v_ok[st]);
                 }
+                fence_proxy_async_smem();  // generic-proxy writes, read next by the tensor pipe
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sm.v_ok[st]);
             }
         }
     } else if (warp == MMA_W) {
         // ======================= MMA issue =======================
         if (lane == 0) {
-            constexpr uint32_t IDESC_QK = QI8 ? umma_idesc_i8(TILE_K, ROWS) : umma_idesc_f16(TILE_K, ROWS, 0, 0);
-            constexpr uint32_t IDESC_PV = umma_idesc_f16(128, ROWS, 1, 1);
-            const uint64_t dq = umma_desc_sw128(smem_u32(sm.q[0]), 16, 1024), dk = umma_desc_sw128(smem_u32(sm.k[0]), 16, 1024);
-            const uint64_t dv = umma_desc_sw128(smem_u32(sm.v[0]), V_UNIT / 2, 1024);
-            const uint64_t dp = umma_desc_sw128(smem_u32(sm.p[0]), 16, 1024);
-            uint32_t ok_phase = 0;  // of v_ok, a bit per slot: only tail tiles use it up
-            // S of (tile j, group g) into buffer n & 1, n = j * GROUPS + g
-            auto issue_qk = [&](int j, int g) {
-                const int n = j * GROUPS + g;
-                if (n >= 2) mbar_wait(&sm.s_free[n & 1], ((n - 2) >> 1) & 1, prm.status, 521, failed);
-                const uint32_t d = tmem + TMEM_S + (n & 1) * S_COLS;
-                if (QI8) {
-                    const int c = g >> 1;  // 128-byte chunk; the group is its lower or upper two blocks
-                    if ((g & 1) == 0) mbar_wait(&sm.k_full[c], j & 1, prm.status, 522, failed);
-                    if (failed) return;
-                    tc_fence_after_sync();
+            constexpr uint32_t IDESC_QK = umma_idesc_f16(ROWS, TILE_K, 0, 0);
+            constexpr uint32_t IDESC_PV = umma_idesc_f16(ROWS, HD, 0, 1);
+            const uint64_t dq = umma_desc_sw128(smem_u32(sm.q[0]), 16, 1024), dk = umma_desc_sw128(smem_u32(sm.k[0][0]), 16, 1024);
+            const uint64_t dv = umma_desc_sw128(smem_u32(sm.v[0]), V_CHUNK, 1024);
+            uint32_t ok_phase = 0;  // of v_ok, a bit per stage: only tail tiles use it up
+            // Q K^T of tile j, into S buffer j % 2 (free: P V of tile j - 2 was issued before)
+            auto issue_tile = [&](int j) {
+                const int st = j % STAGES;
+                mbar_wait(&sm.k_full[st], (j / STAGES) & 1, prm.status, 522, failed);
+                if (failed) return;
+                tc_fence_after_sync();
 #pragma unroll
-                    for (int e = 0; e < 2; e++) {
-                        const uint32_t off = 2 * (2 * (g & 1) + e);
-                        umma_i8_ss(d + e * 64, dk + c * (K_CHUNK >> 4) + off, dq + c * (Q_CHUNK >> 4) + off, IDESC_QK);
-                    }
-                    if (g & 1) umma_commit(&sm.k_free[c]);
-                } else {
+                for (int c = 0; c < CHUNKS; c++)
 #pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        mbar_wait(&sm.k_full[c], j & 1, prm.status, 522, failed);
-                        if (failed) return;
-                        tc_fence_after_sync();
-#pragma unroll
-                        for (int kk = 0; kk < 4; kk++)
-                            umma_f16_ss(d, dk + c * (K_CHUNK >> 4) + 2 * kk, dq + c * (Q_CHUNK >> 4) + 2 * kk, IDESC_QK, (c | kk) ? 1u : 0u);
-                        umma_commit(&sm.k_free[c]);
-                    }
-                }
-                umma_commit(&sm.s_ready[n & 1]);
+                    for (int kk = 0; kk < 4; kk++)
+                        umma_f16_ss(tmem + TMEM_S + (j & 1) * 64, dq + c * (Q_CHUNK >> 4) + 2 * kk, dk + (st * CHUNKS + c) * (K_CHUNK >> 4) + 2 * kk,
+                                    IDESC_QK, (c | kk) ? 1u : 0u);
+                umma_commit(&sm.s_ready[j & 1]);
+                umma_commit(&sm.k_free[st]);
             };
-            // O^T += V^T P^T for one unit of tile j
-            auto issue_pv = [&](int j, int u, bool tail) {
-                const int n = j * UNITS + u, st = n % NV, kh = u & 1, db = u >> 1;
-                mbar_wait(&sm.v_full[st], (n / NV) & 1, prm.status, 523, failed);
+            mbar_wait(&sm.q_bar, 0, prm.status, 520, failed);
+            for (int j = 0; j < 2 && j < n_tiles; j++) issue_tile(j);
+            for (int j = 0; j < n_tiles && !failed; ++j) {
+                const WideTile t = tile_at(j);
+                const bool tail = t.pos0 + TILE_K - 1 > valid_end(t);
+                const int st = j % STAGES;
+                mbar_wait(&sm.v_full[st], (j / STAGES) & 1, prm.status, 523, failed);
                 if (tail) {
                     mbar_wait(&sm.v_ok[st], (ok_phase >> st) & 1, prm.status, 524, failed);
                     ok_phase ^= 1u << st;
                 }
-                if (failed) return;
-                tc_fence_after_sync();
-                const uint64_t v = dv + (uint64_t)st * (V_UNIT >> 4), p = dp + kh * (64 * 128 >> 4);
-                const uint32_t d = tmem + TMEM_O + db * 64;
-#pragma unroll
-                for (int half = 0; half < 2; half++)
-#pragma unroll
-                    for (int kk = 0; kk < 4; kk++)
-                        umma_f16_ss(d, v + 128 * kk, p + half * (P_TILE >> 4) + 128 * kk, IDESC_PV, (j > 0 || kh || half || kk) ? 1u : 0u);
-                umma_commit(&sm.v_free[st]);
-            };
-            mbar_wait(&sm.q_bar, 0, prm.status, 520, failed);
-            if (n_tiles > 0)
-                for (int g = 0; g < GROUPS; g++) issue_qk(0, g);
-            for (int j = 0; j < n_tiles && !failed; ++j) {
-                const WideTile t = tile_at(j);
-                const bool tail = t.pos0 + TILE_K - 1 > valid_end(t), more = j + 1 < n_tiles;
-                // the next tile's scores go ahead of this tile's products, and between them (Q8_0)
-                int g = 0;
-                for (; more && g < (QI8 ? 2 : 1); g++) issue_qk(j + 1, g);
-                mbar_wait(&sm.p_ready, j & 1, prm.status, 525, failed);
+                mbar_wait(&sm.p_ready[j & 1], (j >> 1) & 1, prm.status, 525, failed);
                 if (failed) break;
                 tc_fence_after_sync();
-                for (int u = 0; u < UNITS; u++) {
-                    issue_pv(j, u, tail);
-                    if (u == UNITS - 1) umma_commit(&sm.pv_done);
-                    if (more && g < GROUPS) issue_qk(j + 1, g++);
+                // O += P V in eight instructions (hi and lo of four 16-key steps)
+                const uint32_t p = tmem + TMEM_S + (j & 1) * 64;
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const int kk = i >> 1;
+                    umma_f16_ts(tmem + TMEM_O, p + (i & 1) * 32 + kk * 8, dv + (uint64_t)st * (V_TILE >> 4) + 128 * kk, IDESC_PV, (j > 0 || i > 0) ? 1u : 0u);
                 }
+                umma_commit(&sm.pv_done[j & 1]);
+                umma_commit(&sm.v_free[st]);
+                if (j + 2 < n_tiles) issue_tile(j + 2);
             }
         }
     } else {
-        // ======================= softmax: thread = (key kq * 32 + lane, rows 32 * half ..) =======================
-        const int kq = warp & 3, half = warp >> 2, key = kq * 32 + lane;
-        const uint32_t lane_addr = tmem + ((uint32_t)(kq * 32) << 16);
+        // ======================= softmax =======================
         const float scale2 = prm.scale * 1.4426950408889634f;  // > 0 (checked on the host)
-        float2 l2[16];
-#pragma unroll
-        for (int i = 0; i < 16; i++) l2[i] = make_float2(0.0f, 0.0f);
-        uint4 ks_next[2] = {};
-        auto fetch_scales = [&](int it) {
-            const WideTile t = tile_at(it);
-            ks_next[0] = ks_next[1] = make_uint4(0u, 0u, 0u, 0u);
-            if (t.pos0 + key <= valid_end(t)) {
-                const uint4* p = reinterpret_cast<const uint4*>(prm.k0.scales + ((size_t)(t.row0 + key) * prm.n_kv + kvh) * 16);
-                ks_next[0] = __ldg(p);
-                ks_next[1] = __ldg(p + 1);
-            }
-        };
-        if (QI8 && n_tiles > 0) fetch_scales(0);
-
+        const uint32_t tok = m0 + row / G;
+        const int64_t qpos = q0 + tok, row_lo = (win && qpos + 1 > win) ? qpos + 1 - win : 0;
         for (int it = 0; it < n_tiles; ++it) {
             const WideTile t = tile_at(it);
+            const int b = it & 1;
             float s[32];
-            if constexpr (QI8) {
-                const uint4 ks4[2] = {ks_next[0], ks_next[1]};
-                if (it + 1 < n_tiles) fetch_scales(it + 1);
-                float2 a2[16];
-#pragma unroll
-                for (int i = 0; i < 16; i++) a2[i] = make_float2(0.0f, 0.0f);
-#pragma unroll
-                for (int g = 0; g < 8; g++) {
-                    mbar_wait(&sm.s_ready[g & 1], ((it * 8 + g) >> 1) & 1, prm.status, 531, failed);
-                    tc_fence_after_sync();
-                    uint32_t r0[32], r1[32];
-                    tmem_ld_32x32b_x32(lane_addr + TMEM_S + (g & 1) * S_COLS + 32 * half, r0);
-                    tmem_ld_32x32b_x32(lane_addr + TMEM_S + (g & 1) * S_COLS + 64 + 32 * half, r1);
-                    tc_wait_ld();
-                    tc_fence_before_sync();
-                    mbar_arrive(&sm.s_free[g & 1]);
-                    const uint32_t w = reinterpret_cast<const uint32_t*>(ks4)[g];
-                    const float2 ks = __half22float2(*reinterpret_cast<const __half2*>(&w));
-#pragma unroll
-                    for (int e = 0; e < 2; e++) {
-                        const float4* qs = reinterpret_cast<const float4*>(&sm.qs[2 * g + e][32 * half]);
-                        const float2 kk = e ? make_float2(ks.y, ks.y) : make_float2(ks.x, ks.x);
-#pragma unroll
-                        for (int i = 0; i < 8; i++) {
-                            const float4 f = qs[i];
-                            const uint32_t* r = (e ? r1 : r0) + 4 * i;
-                            a2[2 * i] = __ffma2_rn(make_float2((float)(int)r[0], (float)(int)r[1]), __fmul2_rn(kk, make_float2(f.x, f.y)), a2[2 * i]);
-                            a2[2 * i + 1] = __ffma2_rn(make_float2((float)(int)r[2], (float)(int)r[3]), __fmul2_rn(kk, make_float2(f.z, f.w)), a2[2 * i + 1]);
-                        }
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    s[2 * i] = a2[i].x;
-                    s[2 * i + 1] = a2[i].y;
-                }
-            } else {
-                mbar_wait(&sm.s_ready[it & 1], (it >> 1) & 1, prm.status, 531, failed);
+            {
+                mbar_wait(&sm.s_ready[b], (it >> 1) & 1, prm.status, 531, failed);
                 tc_fence_after_sync();
-                uint32_t r0[32];
-                tmem_ld_32x32b_x32(lane_addr + TMEM_S + (it & 1) * S_COLS + 32 * half, r0);
+                uint32_t r[32];
+                tmem_ld_32x32b_x32(lane_addr + TMEM_S + b * 64 + 32 * half, r);
                 tc_wait_ld();
                 tc_fence_before_sync();
-                mbar_arrive(&sm.s_free[it & 1]);
 #pragma unroll
-                for (int i = 0; i < 32; i++) s[i] = __uint_as_float(r0[i]);
+                for (int i = 0; i < 32; i++) s[i] = __uint_as_float(r[i]);
             }
-
             // masks only where the tile crosses a band edge or the end of its source
             if (t.pos0 + TILE_K - 1 > first_qpos || t.pos0 < last_lo || t.pos0 < t.lo || t.pos0 + TILE_K - 1 > t.hi) {
-                const int64_t pos = t.pos0 + key;
-                const bool real = pos >= t.lo && pos <= t.hi;
-                // row r (token r / G of the tile) sees the key from its own position on, and for `win` positions
-                const int from = real ? (int)(pos - first_qpos) : TOK, until = win ? from + (int)win : TOK;
+                const int64_t at = t.pos0 + 32 * half;
+                const int64_t lo64 = max(row_lo, t.lo) - at, hi64 = min(qpos, t.hi) - at;
+                const int lo = (int)max((int64_t)-1, min((int64_t)64, lo64)), hi = (int)max((int64_t)-1, min((int64_t)64, hi64));
 #pragma unroll
-                for (int i = 0; i < 32; i++) {
-                    const int tok = (32 * half + i) / G;
-                    if (tok < from || tok >= until) s[i] = -INFINITY;
-                }
+                for (int i = 0; i < 32; i++)
+                    if (i < lo || i > hi) s[i] = -INFINITY;
             }
-            // does any score exceed its row's reference by more than 2^8?
-            const float4* mr = reinterpret_cast<const float4*>(&sm.m_ref[32 * half]);
-            bool over = false;
-            {
-                const float2 sc2 = make_float2(scale2, scale2);
-                float top = -INFINITY;
+            float mx = max3(s[0], s[1], s[2]);
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const float4 f = mr[i];
-                    const float2 a = __ffma2_rn(make_float2(s[4 * i], s[4 * i + 1]), sc2, make_float2(-f.x, -f.y));
-                    const float2 b = __ffma2_rn(make_float2(s[4 * i + 2], s[4 * i + 3]), sc2, make_float2(-f.z, -f.w));
-                    top = max3(top, max3(a.x, a.y, b.x), b.y);
-                }
-                over = top > GROW_T;
-            }
-            if (named_barrier_or(1, SOFT_THREADS, over)) {
-                float c[32];
-#pragma unroll
-                for (int i = 0; i < 32; i++) c[i] = s[i];
-                sm.red[kq][32 * half + lane] = transpose_reduce<true>(c, lane);
-                named_barrier_sync(2, SOFT_THREADS);
-                if (tid < ROWS) {
-                    const float mx = fmaxf(fmaxf(sm.red[0][tid], sm.red[1][tid]), fmaxf(sm.red[2][tid], sm.red[3][tid])) * scale2;
-                    const float old = sm.m_ref[tid];
-                    const float now = mx > old + GROW_T ? mx : old;
-                    sm.corr[tid] = ex2(old - now);
-                    sm.m_ref[tid] = now;
-                }
-                named_barrier_sync(2, SOFT_THREADS);
-                const float4* cr = reinterpret_cast<const float4*>(&sm.corr[32 * half]);
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const float4 f = cr[i];
-                    l2[2 * i] = __fmul2_rn(l2[2 * i], make_float2(f.x, f.y));
-                    l2[2 * i + 1] = __fmul2_rn(l2[2 * i + 1], make_float2(f.z, f.w));
-                }
+            for (int i = 3; i < 31; i += 2) mx = max3(mx, s[i], s[i + 1]);
+            mx = fmaxf(mx, s[31]) * scale2;
+            // The two threads of a row agree on its maximum; it moves only when a score exceeds it by 2^8.  The barrier also
+            // stands between their reads of S and the writes of P over it.
+            const bool raise = named_barrier_or(1 + kq, 64, mx > m_run + GROW_T);
+            tc_fence_after_sync();
+            if (raise) {
+                sm.red[half][row] = mx;
+                named_barrier_sync(5 + kq, 64);
+                const float top = fmaxf(sm.red[0][row], sm.red[1][row]);
+                const float now = top > m_run + GROW_T ? top : m_run;
+                const float corr = ex2(m_run - now);
+                m_run = now;
+                l_run *= corr;
                 if (it > 0) {
-                    mbar_wait(&sm.pv_done, (it - 1) & 1, prm.status, 532, failed);
+                    mbar_wait(&sm.pv_done[b ^ 1], ((it - 1) >> 1) & 1, prm.status, 532, failed);
                     tc_fence_after_sync();
 #pragma unroll 1
-                    for (int db = 0; db < DB; db++) {
+                    for (int c = 0; c < 4; c++) {
                         uint32_t o[32];
-                        tmem_ld_32x32b_x32(lane_addr + TMEM_O + db * 64 + 32 * half, o);
+                        tmem_ld_32x32b_x32(lane_addr + TMEM_O + 128 * half + 32 * c, o);
                         tc_wait_ld();
 #pragma unroll
-                        for (int i = 0; i < 32; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * sm.corr[32 * half + i]);
-                        tmem_st_32x32b_x32(lane_addr + TMEM_O + db * 64 + 32 * half, o);
+                        for (int i = 0; i < 32; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * corr);
+                        tmem_st_32x32b_x32(lane_addr + TMEM_O + 128 * half + 32 * c, o);
                     }
                     tc_wait_st();
                 }
@@ -537,73 +366,120 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
             // P = 2^(s * scale2 - m + 7) as f16 hi + lo; l from the unrounded values
             uint32_t hi[16], lo[16];
             {
-                const float2 sc2 = make_float2(scale2, scale2);
+                const float2 sc2 = make_float2(scale2, scale2), neg = make_float2(EXP_BIAS - m_run, EXP_BIAS - m_run);
+                float2 l2[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
 #pragma unroll
                 for (int i = 0; i < 16; i++) {
-                    const float2 m = reinterpret_cast<const float2*>(mr)[i];
-                    const float2 x = __ffma2_rn(make_float2(s[2 * i], s[2 * i + 1]), sc2, make_float2(EXP_BIAS - m.x, EXP_BIAS - m.y));
+                    const float2 x = __ffma2_rn(make_float2(s[2 * i], s[2 * i + 1]), sc2, neg);
                     const float2 p = make_float2(ex2(x.x), ex2(x.y));
-                    l2[i] = __fadd2_rn(l2[i], p);
+                    l2[i & 1] = __fadd2_rn(l2[i & 1], p);
                     hi[i] = pack_half2(p.x, p.y);
                     const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hi[i]));
                     lo[i] = pack_half2(p.x - h.x, p.y - h.y);
                 }
+                l_run += (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y);
             }
-            if (it > 0) mbar_wait(&sm.pv_done, (it - 1) & 1, prm.status, 533, failed);  // P of the last tile has been read
-            {
-                uint8_t* row = sm.p[0] + key * 128;
-#pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    const uint32_t off = ((4 * half + c) ^ (key & 7)) << 4;
-                    *reinterpret_cast<uint4*>(row + off) = make_uint4(hi[4 * c], hi[4 * c + 1], hi[4 * c + 2], hi[4 * c + 3]);
-                    *reinterpret_cast<uint4*>(row + P_TILE + off) = make_uint4(lo[4 * c], lo[4 * c + 1], lo[4 * c + 2], lo[4 * c + 3]);
-                }
-            }
-            fence_proxy_async_smem();
+            const uint32_t p_at = lane_addr + TMEM_S + b * 64 + 16 * half;
+            tmem_st_32x32b_x16(p_at, hi);
+            tmem_st_32x32b_x16(p_at + 32, lo);
+            tc_wait_st();
             tc_fence_before_sync();
-            mbar_arrive(&sm.p_ready);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.p_ready[b]);
         }
+        if (n_tiles > 0) mbar_wait(&sm.pv_done[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1, prm.status, 534, failed);
+        sm.red[half][row] = l_run;
+    }
+    if (failed) sm.abort = 1;
+    tc_fence_before_sync();
+    __syncthreads();
+    if (prm.n_cta > 1) cluster_sync();  // neither CTA's shared memory is a target or a source any more
+    tc_fence_after_sync();
 
-        // ---- epilogue: thread = output dim db * 128 + key -----------------------------------------------
-        float l[32];
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            l[2 * i] = l2[i].x;
-            l[2 * i + 1] = l2[i].y;
-        }
-        named_barrier_sync(2, SOFT_THREADS);  // every thread is done with red and corr
-        sm.red[kq][32 * half + lane] = transpose_reduce<false>(l, lane);
-        named_barrier_sync(2, SOFT_THREADS);
-        if (tid < ROWS) sm.corr[tid] = 1.0f / ((sm.red[0][tid] + sm.red[1][tid]) + (sm.red[2][tid] + sm.red[3][tid]));
-        named_barrier_sync(2, SOFT_THREADS);
-        if (n_tiles > 0) mbar_wait(&sm.pv_done, (n_tiles - 1) & 1, prm.status, 534, failed);
-        tc_fence_after_sync();
-        bool odd = false;
+    // ---- out = O / l --------------------------------------------------------------------------------------
+    const bool soft = warp < SOFT_THREADS / 32;
+    float l = 0.0f, w_own = 1.0f, w_other = 0.0f;
+    if (soft) l = sm.red[0][row] + sm.red[1][row];
+    float4* xo = reinterpret_cast<float4*>(sm.k[0][0]);  // split: the other CTA's O of this CTA's 128 dims, [half][16][row]
+    static_assert(sizeof(WideSmem::k) >= 2 * 16 * ROWS * sizeof(float4), "the K stages hold it");
+    if (split) {
+        if (soft) {
+            const uint32_t dst = map_to_rank(smem_u32(xo + half * 16 * ROWS + row), rank ^ 1u);
 #pragma unroll 1
-        for (int db = 0; db < DB; db++) {
+            for (int c = 0; c < 2; c++) {
+                uint32_t o[32];
+                if (n_tiles > 0) {  // uniform over the CTA
+                    tmem_ld_32x32b_x32(lane_addr + TMEM_O + 128 * (rank ^ 1u) + 64 * half + 32 * c, o);
+                    tc_wait_ld();
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 32; i++) o[i] = 0u;
+                }
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                    st_cluster_f4(dst + (8 * c + i) * ROWS * 16, make_float4(__uint_as_float(o[4 * i]), __uint_as_float(o[4 * i + 1]),
+                                                                             __uint_as_float(o[4 * i + 2]), __uint_as_float(o[4 * i + 3])));
+            }
+            if (half == 0) {
+                const uint32_t ml = map_to_rank(smem_u32(&sm.other_ml[row]), rank ^ 1u);
+                asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(ml), "f"(m_run), "f"(l) : "memory");
+            }
+        }
+        __syncwarp();
+        cluster_sync();
+        if (soft) {
+            const float2 ml = sm.other_ml[row];
+            const float top = fmaxf(m_run, ml.x);
+            w_own = ex2(m_run - top);
+            w_other = ex2(ml.x - top);
+            l = rank == 0 ? fmaf(l, w_own, ml.y * w_other) : fmaf(ml.y, w_other, l * w_own);  // the same bits in both
+        }
+    }
+    if (soft) {
+        const float inv = 1.0f / l;
+        const bool live = (uint32_t)(row / G) < live_tok;
+        bool odd = false;
+        const int n_c = split ? 2 : 4, col0 = split ? 128 * (int)rank + 64 * half : 128 * half;
+        __half* orow = prm.out + ((size_t)(m0 + (live ? row / G : 0)) * (prm.n_kv * G) + kvh * G + row % G) * HD + col0;
+#pragma unroll 1
+        for (int c = 0; c < n_c; c++) {
             uint32_t o[32];
             if (n_tiles > 0) {  // uniform over the CTA
-                tmem_ld_32x32b_x32(lane_addr + TMEM_O + db * 64 + 32 * half, o);
+                tmem_ld_32x32b_x32(lane_addr + TMEM_O + col0 + 32 * c, o);
                 tc_wait_ld();
             } else {
 #pragma unroll
                 for (int i = 0; i < 32; i++) o[i] = 0u;
             }
+            float y[32];
 #pragma unroll
-            for (int i = 0; i < 32; i++) {
-                const int r = 32 * half + i;
-                const float y = __uint_as_float(o[i]) * sm.corr[r];
-                if ((uint32_t)(r / G) < live_tok) {
-                    odd |= !(fabsf(y) <= 3.4e38f);
-                    prm.out[((size_t)(m0 + r / G) * (prm.n_kv * G) + kvh * G + r % G) * HD + db * 128 + key] = __float2half_rn(y);
+            for (int i = 0; i < 32; i++) y[i] = __uint_as_float(o[i]);
+            if (split) {
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const float4 f = xo[(half * 16 + 8 * c + i) * ROWS + row];
+                    y[4 * i] = fmaf(f.x, w_other, y[4 * i] * w_own);
+                    y[4 * i + 1] = fmaf(f.y, w_other, y[4 * i + 1] * w_own);
+                    y[4 * i + 2] = fmaf(f.z, w_other, y[4 * i + 2] * w_own);
+                    y[4 * i + 3] = fmaf(f.w, w_other, y[4 * i + 3] * w_own);
                 }
+            }
+            if (live) {
+#pragma unroll
+                for (int i = 0; i < 32; i++) {
+                    y[i] *= inv;
+                    odd |= !(fabsf(y[i]) <= 3.4e38f);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    *reinterpret_cast<uint4*>(orow + 32 * c + 8 * i) = make_uint4(pack_half2(y[8 * i], y[8 * i + 1]), pack_half2(y[8 * i + 2], y[8 * i + 3]),
+                                                                                  pack_half2(y[8 * i + 4], y[8 * i + 5]), pack_half2(y[8 * i + 6], y[8 * i + 7]));
             }
         }
         if (odd) sm.redo = 1;
     }
     // A wait that ran out leaves copies and MMAs of this CTA in flight that nobody will wait for: give them a bounded
     // time to land before the shared and tensor memory they target is handed to the next CTA.
-    if (failed) sm.abort = 1;
     tc_fence_before_sync();
     __syncthreads();
     if (*(volatile uint32_t*)&sm.abort != 0u) {
@@ -611,49 +487,23 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
         __syncthreads();
     }
     if (warp == 0) tmem_dealloc(tmem, TMEM_COLS);
-    if (*(volatile uint32_t*)&sm.redo != 0u) stream_rows<HD, G, QI8, TWO_SRC>(prm, m0, kvh);
+    if (prm.n_cta > 1) {
+        // both CTAs have written their share: if either redoes the rows, its values are the last
+        __syncwarp();
+        cluster_sync();
+    }
+    if (*(volatile uint32_t*)&sm.redo != 0u) stream_rows<TWO_SRC>(prm, m0, kvh);
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// [row][head][HD] tensor of `elem`-byte values, boxes of 128 bytes x box_heads x box_rows.
-int encode_rows(const LaunchArgs& a, CUtensorMap* tm, const void* base, uint64_t rows, uint64_t heads, int hd, int elem, uint32_t box_heads, uint32_t box_rows)
+// [row][head][256] f16, boxes of 64 dims x box_heads x box_rows.
+int encode_rows(const LaunchArgs& a, CUtensorMap* tm, const void* base, uint64_t rows, uint64_t heads, uint32_t box_heads, uint32_t box_rows)
 {
-    const uint64_t dims[3] = {(uint64_t)hd, heads, rows};
-    const uint64_t strides[2] = {(uint64_t)hd * elem, heads * hd * elem};
-    const uint32_t box[3] = {128u / elem, box_heads, box_rows};
-    return encode_tensor_map(a, tm, elem == 2, 3, const_cast<void*>(base), dims, strides, box, 3);
-}
-
-template <int HD, int G, bool QI8, bool TWO_SRC>
-int run_wide(const LaunchArgs& a, const WideParams& prm)
-{
-    CUtensorMap tq, tk0, tv0, tk1, tv1;
-    const int e = QI8 ? 1 : 2;
-    if (int r = encode_rows(a, &tq, prm.q, prm.m_tokens, prm.n_kv * G, HD, e, G, ROWS / G)) return r;
-    if (int r = encode_rows(a, &tk0, prm.k0.data, prm.k0.rows, prm.n_kv, HD, e, 1, TILE_K)) return r;
-    if (int r = encode_rows(a, &tv0, prm.v0.data, prm.v0.rows, prm.n_kv, HD, 2, 1, 64)) return r;
-    tk1 = tk0;
-    tv1 = tv0;
-    if (TWO_SRC) {
-        if (int r = encode_rows(a, &tk1, prm.k1.data, prm.k1.rows, prm.n_kv, HD, e, 1, TILE_K)) return r;
-        if (int r = encode_rows(a, &tv1, prm.v1.data, prm.v1.rows, prm.n_kv, HD, 2, 1, 64)) return r;
-    }
-    const int smem = (int)sizeof(WideSmem);
-    auto kern = wide_prefill_kernel<HD, G, QI8, TWO_SRC>;
-    {
-        static std::mutex attr_mutex;
-        static bool attr_set[64] = {};
-        std::lock_guard<std::mutex> lock(attr_mutex);
-        if (a.device >= 64 || !attr_set[a.device]) {
-            if (int r = check_cuda(a, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "cudaFuncSetAttribute(wide_prefill)")) return r;
-            if (a.device < 64) attr_set[a.device] = true;
-        }
-    }
-    const uint32_t q_tiles = (prm.m_tokens + ROWS / G - 1) / (ROWS / G);
-    const cudaError_t err = launch_dependent(kern, dim3(q_tiles * prm.n_kv), dim3(WIDE_THREADS), smem, a.stream, tq, tk0, tv0, tk1, tv1, prm);
-    ++*a.launches;
-    return check_cuda(a, err, "attn_prefill (wide heads)");
+    const uint64_t dims[3] = {HD, heads, rows};
+    const uint64_t strides[2] = {HD * 2, heads * HD * 2};
+    const uint32_t box[3] = {64, box_heads, box_rows};
+    return encode_tensor_map(a, tm, 1, 3, const_cast<void*>(base), dims, strides, box, 3);
 }
 
 }  // namespace
@@ -661,34 +511,55 @@ int run_wide(const LaunchArgs& a, const WideParams& prm)
 // What the tensor-core kernel takes: a positive softmax scale (the row maximum is taken before it), operands whose rows the
 // copies can address (16-byte aligned bases, K and V with at least one row, row indexes within an int).  Everything else stays
 // on the streaming kernel.
-template <int HD, int G, bool QI8, bool TWO_SRC>
-bool prefill_wide_takes(const LaunchArgs& a, const KvOperand& k0, const KvOperand& v0, const KvOperand& k1, const KvOperand& v1, const void* q, float scale)
+template <bool TWO_SRC>
+bool prefill_wide_takes(const KvOperand& k0, const KvOperand& v0, const KvOperand& k1, const KvOperand& v1, const void* q, const void* out, float scale)
 {
-    (void)a;
-    if (!(scale > 0.0f) || !(scale < 1e30f) || !aligned16(q)) return false;
+    if (!(scale > 0.0f) || !(scale < 1e30f) || !aligned16(q) || !aligned16(out)) return false;
     const KvOperand* ops[4] = {&k0, &v0, &k1, &v1};
     for (int i = 0; i < (TWO_SRC ? 4 : 2); i++)
         if (ops[i]->rows == 0 || ops[i]->rows >= (1u << 30) || !aligned16(ops[i]->data)) return false;
-    return !QI8 || aligned16(k0.scales);
+    return true;
 }
 
-template <int HD, int G, bool QI8, bool TWO_SRC>
-int launch_prefill_wide(const LaunchArgs& a, const void* q, const __half* q_scales, const KvOperand& k0, const KvOperand& v0, const KvOperand& k1,
-                        const KvOperand& v1, void* out, const void* step, uint32_t n_kv, uint32_t m, uint32_t window, uint32_t ring, float scale)
+template <bool TWO_SRC>
+int launch_prefill_wide(const LaunchArgs& a, const void* q, const KvOperand& k0, const KvOperand& v0, const KvOperand& k1, const KvOperand& v1, void* out,
+                        const void* step, uint32_t n_kv, uint32_t m, uint32_t window, uint32_t ring, float scale)
 {
-    WideParams prm{(const uint32_t*)step, (__half*)out, a.status, q_scales, m, n_kv, window, ring, scale, q, k0, v0, k1, v1};
-    return run_wide<HD, G, QI8, TWO_SRC>(a, prm);
+    const uint32_t units = (m + ROWS / G - 1) / (ROWS / G) * n_kv;
+    const uint32_t n_cta = 2 * units <= (uint32_t)a.sm_count ? 2 : 1;  // one CTA per SM: two per unit while they fit at once
+    const WideParams prm{(const uint32_t*)step, (__half*)out, a.status, m, n_kv, window, ring, scale, n_cta, q, k0, v0, k1, v1};
+    CUtensorMap tq, tk0, tv0, tk1, tv1;
+    if (int r = encode_rows(a, &tq, q, m, n_kv * G, G, ROWS / G)) return r;
+    if (int r = encode_rows(a, &tk0, k0.data, k0.rows, n_kv, 1, TILE_K)) return r;
+    if (int r = encode_rows(a, &tv0, v0.data, v0.rows, n_kv, 1, TILE_K)) return r;
+    tk1 = tk0;
+    tv1 = tv0;
+    if (TWO_SRC) {
+        if (int r = encode_rows(a, &tk1, k1.data, k1.rows, n_kv, 1, TILE_K)) return r;
+        if (int r = encode_rows(a, &tv1, v1.data, v1.rows, n_kv, 1, TILE_K)) return r;
+    }
+    auto kern = wide_prefill_kernel<TWO_SRC>;
+    {
+        static std::mutex attr_mutex;
+        static bool attr_set[64] = {};
+        std::lock_guard<std::mutex> lock(attr_mutex);
+        if (a.device >= 64 || !attr_set[a.device]) {
+            if (int r = check_cuda(a, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WideSmem)),
+                                   "cudaFuncSetAttribute(wide_prefill)"))
+                return r;
+            if (a.device < 64) attr_set[a.device] = true;
+        }
+    }
+    const cudaError_t err = launch_dependent_clusters(kern, n_cta, dim3(units * n_cta), dim3(WIDE_THREADS), sizeof(WideSmem), a.stream, tq, tk0, tv0, tk1,
+                                                      tv1, prm);
+    ++*a.launches;
+    return check_cuda(a, err, "attn_prefill_sliding");
 }
-
-#define SGB_WIDE(HD, G, QI8, TWO)                                                                                                       \
-    template bool prefill_wide_takes<HD, G, QI8, TWO>(const LaunchArgs&, const KvOperand&, const KvOperand&, const KvOperand&,            \
-                                                      const KvOperand&, const void*, float);                                              \
-    template int launch_prefill_wide<HD, G, QI8, TWO>(const LaunchArgs&, const void*, const __half*, const KvOperand&, const KvOperand&,  \
-                                                      const KvOperand&, const KvOperand&, void*, const void*, uint32_t, uint32_t,         \
-                                                      uint32_t, uint32_t, float);
-SGB_WIDE(256, 2, false, false)
-SGB_WIDE(256, 2, false, true)
-SGB_WIDE(512, 8, true, false)
-#undef SGB_WIDE
+template bool prefill_wide_takes<false>(const KvOperand&, const KvOperand&, const KvOperand&, const KvOperand&, const void*, const void*, float);
+template bool prefill_wide_takes<true>(const KvOperand&, const KvOperand&, const KvOperand&, const KvOperand&, const void*, const void*, float);
+template int launch_prefill_wide<false>(const LaunchArgs&, const void*, const KvOperand&, const KvOperand&, const KvOperand&, const KvOperand&, void*,
+                                        const void*, uint32_t, uint32_t, uint32_t, uint32_t, float);
+template int launch_prefill_wide<true>(const LaunchArgs&, const void*, const KvOperand&, const KvOperand&, const KvOperand&, const KvOperand&, void*,
+                                       const void*, uint32_t, uint32_t, uint32_t, uint32_t, float);
 
 }  // namespace sgb

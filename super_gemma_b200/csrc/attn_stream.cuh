@@ -151,4 +151,41 @@ inline KvOperand linear_q8(const BufView& quants, const BufView& scales, int n_k
     return KvOperand{quants.ptr, (const __half*)scales.ptr, nullptr, 0, 1, quants.bytes / ((size_t)n_kv * hd)};
 }
 
+// One query row of prefill by the streaming statement, by a warp: history rows [begin, q0) or all rows [begin, qpos] of (k0, v0) at
+// t % ring, then (two sources) the chunk's rows of (k1, v1).  For rows whose tiled result is not finite.
+template <int HD, int G, bool QI8, bool TWO_SRC>
+__device__ __forceinline__ void stream_prefill_row(const void* q, const __half* q_scales, const KvOperand& k0, const KvOperand& v0, const KvOperand& k1,
+                                                   const KvOperand& v1, __half* out, uint32_t q0, uint32_t i, int head, int n_kv, uint32_t window,
+                                                   uint32_t ring, float scale)
+{
+    constexpr int DPL = HD / 32, KFMT = QI8 ? FMT_Q8 : FMT_F16;
+    const int d0 = (threadIdx.x & 31) * DPL, kvh = head / G;
+    const size_t qrow = (size_t)i * (n_kv * G) + head;
+    float qr[DPL], kk[DPL], vv[DPL];
+    if constexpr (QI8)
+        load_q8<DPL>(reinterpret_cast<const int8_t*>(q) + qrow * HD + d0, q_scales + qrow * (HD / 32), d0, qr);
+    else
+        load_f16<DPL>(reinterpret_cast<const __half*>(q) + qrow * HD + d0, qr);
+    Stream<1, DPL> st;
+    st.init();
+    const uint32_t qpos = q0 + i, begin = (window != 0 && qpos + 1 > window) ? qpos + 1 - window : 0;
+    const uint32_t hist_end = TWO_SRC ? min(q0, qpos + 1) : qpos + 1;
+    for (uint32_t t = begin; t < hist_end; t++) {
+        const size_t row = ring ? t % ring : t;
+        if (row >= k0.rows || row >= v0.rows) break;  // reported where the tiles are laid out
+        load_row<HD, KFMT, DPL>(k0, row, kvh, n_kv, d0, kk);
+        load_row<HD, FMT_F16, DPL>(v0, row, kvh, n_kv, d0, vv);
+        st.step(0, qr, kk, vv, scale);
+    }
+    if (TWO_SRC) {
+        for (uint32_t c = begin > q0 ? begin - q0 : 0; c <= i; c++) {
+            load_row<HD, FMT_F16, DPL>(k1, c, kvh, n_kv, d0, kk);
+            load_row<HD, FMT_F16, DPL>(v1, c, kvh, n_kv, d0, vv);
+            st.step(0, qr, kk, vv, scale);
+        }
+    }
+#pragma unroll
+    for (int d = 0; d < DPL; d++) out[qrow * HD + d0 + d] = __float2half_rn(st.acc[0][d] / st.l[0]);
+}
+
 }  // namespace sgb

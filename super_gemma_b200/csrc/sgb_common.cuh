@@ -220,6 +220,18 @@ __device__ __forceinline__ void named_barrier_sync(uint32_t id, uint32_t threads
 {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
+// Barrier over `threads` threads that also tells every one of them whether `pred` held for any.
+__device__ __forceinline__ bool named_barrier_or(uint32_t id, uint32_t threads, bool pred)
+{
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %3, 0;\n\t"
+        "barrier.cta.red.or.pred q, %1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}\n"
+        : "=r"(r)
+        : "r"(id), "r"(threads), "r"((uint32_t)pred)
+        : "memory");
+    return r != 0;
+}
 // Three-input maximum (one instruction on sm_100).
 __device__ __forceinline__ float max3(float a, float b, float c)
 {

@@ -115,12 +115,16 @@ int launch_decode_rows(const LaunchArgs&, const void* q, const KvOperand& k, con
 int launch_verify_ring_d128(const LaunchArgs&, const void* q, const KvOperand& k_ring, const KvOperand& v_ring, const KvOperand& k_new,
                             const KvOperand& v_new, void* out, const void* step, uint32_t n_kv, uint32_t m, uint32_t window, uint32_t ring, float scale);
 
-// attn_prefill_wide.cu: the tensor-core form of the reference-shaped prefill kernels (head_dim 256 f16, head_dim 512 int8 Q/K)
-template <int HD, int G, bool QI8, bool TWO_SRC>
-bool prefill_wide_takes(const LaunchArgs&, const KvOperand& k0, const KvOperand& v0, const KvOperand& k1, const KvOperand& v1, const void* q, float scale);
-template <int HD, int G, bool QI8, bool TWO_SRC>
-int launch_prefill_wide(const LaunchArgs&, const void* q, const __half* q_scales, const KvOperand& k0, const KvOperand& v0, const KvOperand& k1,
-                        const KvOperand& v1, void* out, const void* step, uint32_t n_kv, uint32_t m, uint32_t window, uint32_t ring, float scale);
+// attn_prefill_wide.cu, attn_prefill_int8.cu: the tensor-core form of the reference-shaped prefill kernels (head_dim 256 f16;
+// head_dim 512 with int8 Q and K)
+template <bool TWO_SRC>
+bool prefill_wide_takes(const KvOperand& k0, const KvOperand& v0, const KvOperand& k1, const KvOperand& v1, const void* q, const void* out, float scale);
+template <bool TWO_SRC>
+int launch_prefill_wide(const LaunchArgs&, const void* q, const KvOperand& k0, const KvOperand& v0, const KvOperand& k1, const KvOperand& v1, void* out,
+                        const void* step, uint32_t n_kv, uint32_t m, uint32_t window, uint32_t ring, float scale);
+bool prefill_int8_takes(const KvOperand& k, const KvOperand& v, const void* q, float scale);
+int launch_prefill_int8(const LaunchArgs&, const void* q, const __half* q_scales, const KvOperand& k, const KvOperand& v, void* out, const void* step,
+                        uint32_t n_kv, uint32_t m, float scale);
 
 // attn_exchange.cu
 int launch_reduce_exchange_d128(const LaunchArgs&);
