@@ -3,8 +3,8 @@
 //
 // All of them are a few query rows (<= 8: the query heads of a kv head, times the drafted tokens) against many keys, bound by
 // the bytes of K and V.  A warp takes 16 keys at a time: they arrive by TMA, 128 bytes of all 16 rows to a copy (128-byte
-// swizzle), in the warp's own slots (K and V apart, so that the next K is on its way while this V is used).  S = K Q^T and O^T += V^T P^T are mma.sync m16n8k16 with the keys or 16 dims as M and the rows as N: tcgen05 has
-// no tile this small.  Warps never wait for one another before the end, where their states merge in warp order.
+// swizzle), in the warp's own slots (K and V apart, so that the next K is on its way while this V is used).  S = K Q^T
+// and O^T += V^T P^T are mma.sync m16n8k16 with the keys or 16 dims as M and the rows as N: tcgen05 has no tile this small.  Warps never wait for one another before the end, where their states merge in warp order.
 // Precision is that of the f32 statement (attn_decode_sliding.wgsl:84-107): Q8_0 keys enter as whole numbers and every block's
 // sum is multiplied by its f32 scale; P = (hi + lo) * 2^-14 with both halves f16 (22 bits, the factor keeps lo out of f16's
 // subnormals); running maximum and sums in f32.
