@@ -454,7 +454,7 @@ int launch_prefill_global_flash_ref(const LaunchArgs& a)
     if (int r = need_bytes(a, bi, m * n_q * HD * 2, "out")) return r;
     if (int r = need_bytes(a, bi + 1, 16, "step")) return r;
     if constexpr (VARIANT == 2) {
-        if (prefill_int8_takes(kop, vop, a.b[0].ptr, scale))
+        if (prefill_int8_takes(kop, vop, a.b[0].ptr, a.b[bi].ptr, (uint32_t)m, scale))
             return launch_prefill_int8(a, a.b[0].ptr, q_scales, kop, vop, a.b[bi].ptr, a.b[bi + 1].ptr, N_KV, (uint32_t)m, scale);
     }
     const dim3 grid(N_KV, (uint32_t)m);

@@ -10,12 +10,21 @@
 // One kind::i8 MMA (K = 32) per scale block gives that block's whole-number dot product, exactly; the two f16 scales multiply
 // it in f32 (f32(qs) * f32(ks) is exact), so the score is closer to f32(scale) * f32(q) arithmetic than an f32 dot product.
 // Blocks go through four 64-column buffers, two per hand-over.
-// P keeps f32 precision: P = hi + lo with both halves f16 (22 bits), two MMAs per V tile.  The exponent carries +7, so that
-// lo stays clear of f16's subnormals (the factor cancels in O / l).
+// P = hi + lo, both halves f16, two MMAs per V tile: together they miss p by at most one unit of its last f32 place.  The exponent
+// carries +7, so that lo stays clear of f16's subnormals (the factor cancels in O / l); a p below 2^-32 of its row's reference
+// maximum is in l but too small for lo.
+// The tensor pipe truncates an accumulator each time it adds to it: in one accumulator, outputs shrank by 2e-9 of themselves per
+// key (1.7e-5 at 8192 keys, 6.7e-5 at 33280, where the error against 64 bits was 2.22e-4 instead of f16's own 2.08e-4).  From the
+// fifth tile on the softmax threads therefore settle one of the four dim blocks of O in every tile: the block, plus what was
+// settled of it before, added in f32 with rounding, splits into its upper 16 bits, which they keep in this CTA's share of the
+// output, and the exact rest, from which the tensor pipe goes on; what it adds to stays as small as the sum of four tiles.
+// Another block comes first in each tile's products, so that it can be settled while the tensor pipe is at the others.  Errors since:
+// 2.0762e-4 and 2.0773e-4 (streaming kernel: 2.0762e-4, 2.0774e-4), for 23 us of 533 at 8192 keys; all four blocks in every
+// fourth tile, with the tensor pipe waiting, took 44.
 // Roles: warps 0-7 softmax (two threads per key, 32 rows each), one MMA thread, one K and one V loader thread; mbarriers only.
 // The row maximum over keys runs across threads; it is only computed (32 values in 31 shuffles) when some score exceeds its
 // row's running maximum by 2^8, which one barrier with an OR finds out.
-// Measured: 256 queries at 7936 + 256 keys 13500 us on the streaming kernel, 500 here (floor 86).  Two things bound it: V as the
+// Measured: 256 queries at 7936 + 256 keys 13500 us on the streaming kernel, 533 here (floor 86).  Two things bound it: V as the
 // MN-major A operand costs 160 cycles per instruction (10000 of a tile's 14400), and every block's scores cross from tensor
 // memory to registers (16 x 32 KB a tile, 500 cycles each).  Rows as the M side with the 512 dims and the blocks split over
 // two CTAs that exchange partial scores took the first away and was slower, 787 us with 8 softmax warps and 741 with 16 (649
@@ -56,7 +65,7 @@ struct Int8Smem {
     float qs[16][ROWS];    // scales of Q, [block][row]
     float red[4][ROWS];
     float m_ref[ROWS], corr[ROWS];
-    uint64_t q_bar, k_full[4], k_free[4], v_full[NV], v_free[NV], v_ok[NV], s_ready[2], s_free[2], p_ready, pv_done;
+    uint64_t q_bar, k_full[4], k_free[4], v_full[NV], v_free[NV], v_ok[NV], s_ready[2], s_free[2], p_ready, first_done, pv_done;
     uint32_t tmem_base, abort, redo;
 };
 static_assert(sizeof(Int8Smem) + 1024 <= 227 * 1024, "one CTA per SM");
@@ -162,6 +171,7 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
             mbar_init(&sm.s_free[i], SOFT_THREADS / 32);
         }
         mbar_init(&sm.p_ready, SOFT_THREADS / 32);
+        mbar_init(&sm.first_done, 1);
         mbar_init(&sm.pv_done, 1);
         sm.abort = 0;
         sm.redo = 0;
@@ -186,6 +196,7 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
     tc_fence_after_sync();
     const uint32_t tmem = sm.tmem_base;
     bool failed = false;
+    auto block_at = [](int j, int u) { return ((u >> 1) + j) & (DB - 1); };  // dim block of V unit u of tile j: another one first in each tile
 
     if (warp == K_W) {
         // ======================= Q and K loads: K(j) chunk by chunk as the MMAs of tile j - 1 let go of them ==========
@@ -212,7 +223,7 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
                 const int st = n % NV;
                 if (n >= NV) mbar_wait(&sm.v_free[st], (n / NV - 1) & 1, prm.status, 512, failed, 50);
                 if (failed) break;
-                const int kh = u & 1, db = u >> 1;
+                const int kh = u & 1, db = block_at(j, u);
                 if (lane == 0) {
                     mbar_arrive_expect_tx(&sm.v_full[st], V_UNIT);
                     tma_load_3d(sm.v[st], &tm_v, &sm.v_full[st], db * 128, kvh, (int)pos0 + kh * 64);
@@ -265,7 +276,7 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
             };
             // O^T += V^T P^T for one unit of tile j
             auto issue_pv = [&](int j, int u, bool tail) {
-                const int n = j * UNITS + u, st = n % NV, kh = u & 1, db = u >> 1;
+                const int n = j * UNITS + u, st = n % NV, kh = u & 1, db = block_at(j, u);
                 mbar_wait(&sm.v_full[st], (n / NV) & 1, prm.status, 523, failed);
                 if (tail) {
                     mbar_wait(&sm.v_ok[st], (ok_phase >> st) & 1, prm.status, 524, failed);
@@ -295,6 +306,7 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
                 tc_fence_after_sync();
                 for (int u = 0; u < UNITS; u++) {
                     issue_pv(j, u, tail);
+                    if (u == 1) umma_commit(&sm.first_done);
                     if (u == UNITS - 1) umma_commit(&sm.pv_done);
                     if (more && g < GROUPS) issue_qk(j + 1, g++);
                 }
@@ -319,6 +331,40 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
             }
         };
         if (n_tiles > 0) fetch_scales(0);
+        // The settled part of this thread's O as 16-bit halves, in this CTA's own share of the output (64 rows x 512 dims x 2 bytes),
+        // which nobody reads before the end.  A step takes 16 of the 32 values of a block; 8 values c of step h at [2 * h + c][thread].
+        uint32_t settled = 0;  // a bit per block
+        auto settled_at = [&](int h, int c) {
+            const int e = 2 * h + c;
+            return reinterpret_cast<uint4*>(prm.out + ((size_t)(m0 + e / 2) * (prm.n_kv * G) + kvh * G) * HD) + (e & 1) * SOFT_THREADS + tid;
+        };
+        auto o_at = [&](int h) { return lane_addr + TMEM_O + (h >> 1) * 64 + 32 * half + 16 * (h & 1); };
+        auto fetch_settled = [&](int h, uint4 (&u)[2]) {
+            u[0] = *settled_at(h, 0);
+            u[1] = *settled_at(h, 1);
+        };
+        auto add_settled = [&](const uint4 (&u)[2], uint32_t (&o)[16]) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const uint32_t w = reinterpret_cast<const uint32_t*>(u)[i];
+                o[2 * i] = __float_as_uint(__fadd_rn(__uint_as_float(o[2 * i]), __uint_as_float(w << 16)));
+                o[2 * i + 1] = __float_as_uint(__fadd_rn(__uint_as_float(o[2 * i + 1]), __uint_as_float(w & 0xFFFF0000u)));
+            }
+        };
+        auto settle = [&](int h, uint32_t (&o)[16]) {  // o: whole values, left as the rest
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                uint32_t w[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    uint32_t &a = o[8 * c + 2 * k], &b = o[8 * c + 2 * k + 1];
+                    w[k] = __byte_perm(a, b, 0x7632);
+                    a = __float_as_uint(__uint_as_float(a) - __uint_as_float(a & 0xFFFF0000u));
+                    b = __float_as_uint(__uint_as_float(b) - __uint_as_float(b & 0xFFFF0000u));
+                }
+                *settled_at(h, c) = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+        };
 
         for (int it = 0; it < n_tiles; ++it) {
             float s[32];
@@ -353,6 +399,26 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
                             a2[2 * i + 1] = __ffma2_rn(make_float2((float)(int)r[2], (float)(int)r[3]), __fmul2_rn(kk, make_float2(f.z, f.w)), a2[2 * i + 1]);
                         }
                     }
+                    if (g == 3 && it >= 4) {
+                        // the last tile's products of its first block were issued ahead of these scores, and both S buffers are free: the
+                        // tensor pipe goes on meanwhile
+                        const int db = block_at(it - 1, 0);
+                        mbar_wait(&sm.first_done, (it - 1) & 1, prm.status, 535, failed);
+                        tc_fence_after_sync();
+#pragma unroll 1
+                        for (int h = 2 * db; h < 2 * db + 2; h++) {
+                            uint32_t o[16];
+                            uint4 u[2] = {};
+                            if ((settled >> db) & 1) fetch_settled(h, u);
+                            tmem_ld_32x32b_x16(o_at(h), o);
+                            tc_wait_ld();
+                            add_settled(u, o);
+                            settle(h, o);
+                            tmem_st_32x32b_x16(o_at(h), o);
+                        }
+                        tc_wait_st();
+                        settled |= 1u << db;
+                    }
                 }
 #pragma unroll
                 for (int i = 0; i < 16; i++) {
@@ -385,7 +451,8 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
                 }
                 over = top > GROW_T;
             }
-            if (named_barrier_or(1, SOFT_THREADS, over)) {
+            const bool raise = named_barrier_or(1, SOFT_THREADS, over);
+            if (raise) {
                 float c[32];
 #pragma unroll
                 for (int i = 0; i < 32; i++) c[i] = s[i];
@@ -406,20 +473,25 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
                     l2[2 * i] = __fmul2_rn(l2[2 * i], make_float2(f.x, f.y));
                     l2[2 * i + 1] = __fmul2_rn(l2[2 * i + 1], make_float2(f.z, f.w));
                 }
-                if (it > 0) {
-                    mbar_wait(&sm.pv_done, (it - 1) & 1, prm.status, 532, failed);
-                    tc_fence_after_sync();
+            }
+            if (raise && it > 0) {
+                mbar_wait(&sm.pv_done, (it - 1) & 1, prm.status, 532, failed);
+                tc_fence_after_sync();
 #pragma unroll 1
-                    for (int db = 0; db < DB; db++) {
-                        uint32_t o[32];
-                        tmem_ld_32x32b_x32(lane_addr + TMEM_O + db * 64 + 32 * half, o);
-                        tc_wait_ld();
+                for (int h = 0; h < 2 * DB; h++) {
+                    const bool in_parts = (settled >> (h >> 1)) & 1;
+                    uint32_t o[16];
+                    uint4 u[2];
+                    tmem_ld_32x32b_x16(o_at(h), o);
+                    if (in_parts) fetch_settled(h, u);
+                    tc_wait_ld();
+                    if (in_parts) add_settled(u, o);
 #pragma unroll
-                        for (int i = 0; i < 32; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * sm.corr[32 * half + i]);
-                        tmem_st_32x32b_x32(lane_addr + TMEM_O + db * 64 + 32 * half, o);
-                    }
-                    tc_wait_st();
+                    for (int i = 0; i < 16; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * sm.corr[32 * half + 16 * (h & 1) + i]);
+                    if (in_parts) settle(h, o);
+                    tmem_st_32x32b_x16(o_at(h), o);
                 }
+                tc_wait_st();
             }
             // P = 2^(s * scale2 - m + 7) as f16 hi + lo; l from the unrounded values
             uint32_t hi[16], lo[16];
@@ -466,6 +538,21 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
         named_barrier_sync(2, SOFT_THREADS);
         if (n_tiles > 0) mbar_wait(&sm.pv_done, (n_tiles - 1) & 1, prm.status, 534, failed);
         tc_fence_after_sync();
+        if (settled != 0) {  // whole again before the first result is written over a settled part
+#pragma unroll 1
+            for (int h = 0; h < 2 * DB; h++) {
+                if (((settled >> (h >> 1)) & 1) == 0) continue;
+                uint32_t o[16];
+                uint4 u[2];
+                tmem_ld_32x32b_x16(o_at(h), o);
+                fetch_settled(h, u);
+                tc_wait_ld();
+                add_settled(u, o);
+                tmem_st_32x32b_x16(o_at(h), o);
+            }
+            tc_wait_st();
+            named_barrier_sync(2, SOFT_THREADS);
+        }
         bool odd = false;
 #pragma unroll 1
         for (int db = 0; db < DB; db++) {
@@ -516,11 +603,11 @@ int encode_rows(const LaunchArgs& a, CUtensorMap* tm, const void* base, uint64_t
 }  // namespace
 
 // What the tensor-core kernel takes: a positive softmax scale (the row maximum is taken before it), operands whose rows the
-// copies can address (16-byte aligned bases, K and V with at least one row, row indexes within an int).  Everything else stays
-// on the streaming kernel.
-bool prefill_int8_takes(const KvOperand& k, const KvOperand& v, const void* q, float scale)
+// copies can address (16-byte aligned bases, K and V with at least one row, row indexes within an int), an output that can be
+// settled into (16-byte accesses, whole query tiles).  Everything else stays on the streaming kernel.
+bool prefill_int8_takes(const KvOperand& k, const KvOperand& v, const void* q, const void* out, uint32_t m, float scale)
 {
-    if (!(scale > 0.0f) || !(scale < 1e30f) || !aligned16(q) || !aligned16(k.scales)) return false;
+    if (!(scale > 0.0f) || !(scale < 1e30f) || !aligned16(q) || !aligned16(k.scales) || !aligned16(out) || m % (ROWS / G) != 0) return false;
     for (const KvOperand* o : {&k, &v})
         if (o->rows == 0 || o->rows >= (1u << 30) || !aligned16(o->data)) return false;
     return true;

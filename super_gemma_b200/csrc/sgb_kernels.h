@@ -122,7 +122,7 @@ bool prefill_wide_takes(const KvOperand& k0, const KvOperand& v0, const KvOperan
 template <bool TWO_SRC>
 int launch_prefill_wide(const LaunchArgs&, const void* q, const KvOperand& k0, const KvOperand& v0, const KvOperand& k1, const KvOperand& v1, void* out,
                         const void* step, uint32_t n_kv, uint32_t m, uint32_t window, uint32_t ring, float scale);
-bool prefill_int8_takes(const KvOperand& k, const KvOperand& v, const void* q, float scale);
+bool prefill_int8_takes(const KvOperand& k, const KvOperand& v, const void* q, const void* out, uint32_t m, float scale);
 int launch_prefill_int8(const LaunchArgs&, const void* q, const __half* q_scales, const KvOperand& k, const KvOperand& v, void* out, const void* step,
                         uint32_t n_kv, uint32_t m, float scale);
 

@@ -108,6 +108,33 @@ def test_global_int8_edges(ctx, m, q0):
     assert np.all(np.isfinite(got))
 
 
+def test_global_int8_long_history_is_not_biased(ctx):
+    """Over 32768 keys the outputs must not shrink: their projection on the f64 result is off by at most what the products of four
+    tiles, the longest sum left to the tensor pipe, lose to its truncation (64 additions of less than 2^-23 each: 7.6e-6), plus
+    the mean of 32768 f16 roundings (4 sigma of 2.1e-4 / sqrt(32768): 4.6e-6).  In one sum it was 6.7e-5."""
+    m, q0 = 16, 32752
+    q, k, v = _normal(31, m, 32, 512), _normal(32, q0 + m, 4, 512), _normal(33, q0 + m, 4, 512)
+    got, qd, kd = _iq(ctx, q, k, v, q0, m)
+    toks = np.array([0, m - 1], np.uint32)
+    want = O.attention_f64(qd, kd, v, m, q0, 32, 4, 512, 0.044194174, tokens=toks)
+    d = got[toks] - want
+    assert abs(np.vdot(d, want) / np.vdot(want, want)) <= 7.6e-6 + 4.6e-6
+    assert_close(got[toks], want, 1e-6, 1.05 * RTOL, "32768 keys")  # outputs of some 0.006: their own rounding, barely more
+
+
+@pytest.mark.parametrize("q0", [496, 500, 512, 624, 640, 1008, 1020, 1136, 2032])
+def test_global_int8_settled_parts(ctx, q0):
+    """Ends around the tiles in which a dim block is settled for the first or second time, with scores that keep raising the running maximum after parts were settled."""
+    m = 16
+    q, k, v = _normal(q0, m, 32, 512), _normal(q0 + 1, q0 + m, 4, 512), _normal(q0 + 2, q0 + m, 4, 512)
+    q = np.repeat(q[:, ::8], 8, axis=1)
+    for up, scale in ((0.0, 0.044194174), (1e-3, 200 / (q0 + m))):  # scores of up to some 100: rounded to 100 * 2^-24
+        kk = (k + (np.arange(q0 + m)[:, None, None] * up * q.mean(0)[::8][None])).astype(np.float16).astype(np.float32)
+        got, qd, kd = _iq(ctx, q, kk, v, q0, m, scale=scale)
+        want = O.attention_f64(qd, kd, v, m, q0, 32, 4, 512, scale)
+        assert_close(got, want, 2 * ATOL, RTOL, f"q0={q0} up={up}")
+
+
 def test_global_int8_peaked_scores(ctx):
     """Scores that grow along the keys by far more than 2^8: every tile raises the running maximum."""
     m, q0 = 16, 700
