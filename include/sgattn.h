@@ -65,7 +65,9 @@ int sgb_sync(sgb_ctx *ctx, uint32_t timeout_ms);
  * the host; here upload/download are explicit copies ordered on the context's stream.  The
  * *_async forms return at once (give them pinned host memory); the plain forms wait. */
 int sgb_buffer_create(sgb_ctx *ctx, size_t bytes, sgb_buffer **out);
-int sgb_buffer_adopt(sgb_ctx *ctx, void *device_ptr, size_t bytes, sgb_buffer **out); /* not owned */
+/* Adopted memory is not owned and may start anywhere; a dispatch whose kernel would access a binding misaligned (16 bytes for rows
+ * of f16 in general, 8 at head_dim 128 of the streaming kernels, otherwise the element's size) fails with SGB_ERR_VALIDATION. */
+int sgb_buffer_adopt(sgb_ctx *ctx, void *device_ptr, size_t bytes, sgb_buffer **out);
 int sgb_buffer_slice(sgb_buffer *parent, size_t offset, size_t bytes, sgb_buffer **out); /* Buffer::slice */
 void sgb_buffer_retain(sgb_buffer *buf);
 void sgb_buffer_release(sgb_buffer *buf);

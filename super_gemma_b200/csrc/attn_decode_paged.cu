@@ -639,8 +639,7 @@ int launch_decode_paged_q8kv_d128(const LaunchArgs& a)
     if (a.b[0].bytes < m_q * n_q * HD * 2) return fail_validation(a, "decode_paged: q buffer too small");
     if (int r = need_bytes(a, 6, m_q * n_q * p.n_splits * (HD + 2) * 4, "part")) return r;
     if (int r = need_bytes(a, 7, 16, "step")) return r;
-    for (int i = 1; i <= 4; i++)
-        if (reinterpret_cast<uintptr_t>(a.b[i].ptr) & 15) return fail_validation(a, "decode_paged: K/V pools must be 16-byte aligned");
+    if (int r = need_aligned(a, {8, 16, 16, 16, 16, 4, 8, 4})) return r;
 
     CUtensorMap tm[4];
     const void* const quants[2] = {a.b[1].ptr, a.b[3].ptr};
@@ -733,6 +732,10 @@ extern "C" int sgb_decode_paged_q8kv_d128_noalloc(int device, void* stream, cons
     if ((uint64_t)table_len * page < kv_len) return set_last_error(3, "decode_noalloc: page table shorter than kv_len");
     for (const void* p : {k_quants, k_scales, v_quants, v_scales})
         if (reinterpret_cast<uintptr_t>(p) & 15) return set_last_error(3, "decode_noalloc: K/V pools must be 16-byte aligned");
+    if ((reinterpret_cast<uintptr_t>(q) & 7) || (reinterpret_cast<uintptr_t>(out) & 7))
+        return set_last_error(3, "decode_noalloc: q and out must be 8-byte aligned");
+    if ((reinterpret_cast<uintptr_t>(page_table) & 3) || (reinterpret_cast<uintptr_t>(status) & 3))
+        return set_last_error(3, "decode_noalloc: page_table and status must be 4-byte aligned");
 
     int prev = 0;
     cudaError_t e = cudaGetDevice(&prev);

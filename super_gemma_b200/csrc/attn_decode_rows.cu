@@ -548,7 +548,8 @@ int allow_smem(const LaunchArgs& a, Kern kern, size_t smem)
 
 }  // namespace
 
-// The copies need 16-byte aligned bases and row numbers within an int; anything else stays on the streaming kernel.
+// The copies need 16-byte aligned bases and row numbers within an int.  What else the launcher accepts stays on the streaming kernel:
+// quants and scales of any alignment, head_dim 128 rows on 8 bytes (f16 rows of 256 and 512 need 16 there too).
 bool decode_rows_takes(const KvOperand& k, const KvOperand& v, const void* q)
 {
     for (const KvOperand* o : {&k, &v})

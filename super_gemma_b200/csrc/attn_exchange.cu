@@ -65,6 +65,7 @@ int run_reduce_exchange(const LaunchArgs& a, bool timed)
     if (int r = need_bytes(a, 3, rows * HD * 4, "out")) return r;
     if (timed)
         if (int r = need_bytes(a, 4, rows * 5 * 8, "stamps")) return r;
+    if (int r = timed ? need_aligned(a, {8, 16, 8, 8, 8}) : need_aligned(a, {8, 16, 8, 8})) return r;
     // The wait is counted in SM cycles; 2 cycles per nanosecond bounds the clock from above.
     const long long wait_cycles = (long long)p.wait_us * 2000;
     reduce_exchange_kernel<<<(uint32_t)rows, HD / 2, 0, a.stream>>>((const float*)a.b[0].ptr, (float*)a.b[1].ptr,

@@ -248,6 +248,9 @@ int launch_decode_generic(const LaunchArgs& a)
     if (q.bytes < m_q * n_q * HD * 2) return fail_validation(a, "decode: q buffer too small");
     if (int r = need_bytes(a, part_i, m_q * n_q * p.n_splits * (HD + 2) * 4, "part")) return r;
     if (int r = need_bytes(a, step_i, 16, "step")) return r;
+    static_assert(VFMT == FMT_F16, "the lists below name no V scales");
+    constexpr uint32_t ROW = row_alignment(HD);
+    if (int r = KFMT == FMT_Q8 ? need_aligned(a, {ROW, 4, 2, ROW, 4, 4}) : need_aligned(a, {ROW, ROW, ROW, 4, 4})) return r;
     if (decode_rows_takes(kop, vop, q.ptr))
         return launch_decode_rows<HD, G, KFMT == FMT_Q8>(a, q.ptr, kop, vop, a.b[part_i].ptr, a.b[step_i].ptr, STEP_SLOT, n_kv, p.n_splits, m_q, p.scale);
     decode_generic_kernel<HD, G, KFMT, VFMT><<<dim3(n_kv, p.n_splits, m_q), GEN_THREADS, 0, a.stream>>>(
@@ -287,6 +290,7 @@ int launch_decode_paged_q8kv_scalar_d128(const LaunchArgs& a)
     if (a.b[0].bytes < m_q * n_q * 128 * 2) return fail_validation(a, "decode_paged: q buffer too small");
     if (int r = need_bytes(a, 6, m_q * n_q * p.n_splits * 130 * 4, "part")) return r;
     if (int r = need_bytes(a, 7, 16, "step")) return r;
+    if (int r = need_aligned(a, {row_alignment(128), 4, 2, 4, 2, 4, 4, 4})) return r;
     decode_generic_kernel<128, 2, FMT_Q8, FMT_Q8><<<dim3(n_kv, p.n_splits, m_q), GEN_THREADS, 0, a.stream>>>(
         (const __half*)a.b[0].ptr, kop, vop, (float*)a.b[6].ptr, (const uint32_t*)a.b[7].ptr, STEP_KV_LEN_GLOBAL, p.n_splits,
         p.scale, a.status);
@@ -305,6 +309,7 @@ int launch_reduce(const LaunchArgs& a)
     if (int r = need_bytes(a, 0, rows * n_splits * (HD + 2) * 4, "part")) return r;
     const size_t out_bytes = OUT_MODE == 0 ? rows * HD * 2 : OUT_MODE == 1 ? rows * HD * 4 : rows * (HD + 2) * 4;
     if (int r = need_bytes(a, 1, out_bytes, "out")) return r;
+    if (int r = need_aligned(a, {8, OUT_MODE == 0 ? 4u : 8u})) return r;
     const cudaError_t e = launch_dependent(reduce_kernel<HD, OUT_MODE>, dim3((uint32_t)rows), dim3(HD / 2), 0, a.stream, (const float*)a.b[0].ptr,
                                            a.b[1].ptr, n_splits, 0);
     ++*a.launches;
@@ -326,6 +331,7 @@ int launch_combine_ranks_d128(const LaunchArgs& a)
         return fail_validation(a, "attn_combine_ranks: rows must be > 0 and n_ranks in 1..1024");
     if (int r = need_bytes(a, 0, rows * n_ranks * 130 * 4, "gathered partials")) return r;
     if (int r = need_bytes(a, 1, rows * 128 * 4, "out")) return r;
+    if (int r = need_aligned(a, {8, 8})) return r;
     reduce_kernel<128, 1><<<(uint32_t)rows, 64, 0, a.stream>>>((const float*)a.b[0].ptr, a.b[1].ptr, n_ranks, 1);
     ++*a.launches;
     return check_cuda(a, cudaGetLastError(), "attn_combine_ranks_d128");
@@ -354,6 +360,8 @@ int launch_prefill_generic(const LaunchArgs& a)
     if (a.b[0].bytes < m * n_q * HD * 2) return fail_validation(a, "attn_prefill: q buffer too small");
     if (int r = need_bytes(a, bi, m * n_q * HD * (OUT_F32 ? 4 : 2), "out")) return r;
     if (int r = need_bytes(a, bi + 1, 16, "step")) return r;
+    constexpr uint32_t ROW = row_alignment(HD), OUT = OUT_F32 ? 4 : 2;
+    if (int r = TWO_RANGE ? need_aligned(a, {ROW, ROW, ROW, ROW, ROW, OUT, 4}) : need_aligned(a, {ROW, ROW, ROW, OUT, 4})) return r;
     if constexpr (HD == 128 && TWO_RANGE) {
         // up to four queries are the eight rows of one MMA column; more queries are the streaming kernel's (or the flash kernel's)
         if (m <= 4 && decode_rows_takes(kh, vh, a.b[0].ptr) && decode_rows_takes(kc, vc, a.b[0].ptr))
@@ -400,6 +408,7 @@ int launch_prefill_paged_q8kv_scalar_d128(const LaunchArgs& a)
     if (a.b[0].bytes < m * n_q * 128 * 2) return fail_validation(a, "prefill_paged: q buffer too small");
     if (int r = need_bytes(a, 6, m * n_q * 128 * 4, "out")) return r;
     if (int r = need_bytes(a, 7, 16, "step")) return r;
+    if (int r = need_aligned(a, {row_alignment(128), 4, 2, 4, 2, 4, 4, 4})) return r;
     KvOperand none{};
     prefill_generic_kernel<128, 2, FMT_Q8, FMT_Q8, 0, 1><<<dim3(n_kv, (uint32_t)m), GEN_THREADS, 0, a.stream>>>(
         a.b[0].ptr, nullptr, kop, vop, none, none, a.b[6].ptr, (const uint32_t*)a.b[7].ptr, 0, 0, p.scale, a.status);
@@ -453,6 +462,10 @@ int launch_prefill_global_flash_ref(const LaunchArgs& a)
     }
     if (int r = need_bytes(a, bi, m * n_q * HD * 2, "out")) return r;
     if (int r = need_bytes(a, bi + 1, 16, "step")) return r;
+    if (int r = VARIANT == 0   ? need_aligned(a, {16, 16, 16, 2, 4})
+                : VARIANT == 1 ? need_aligned(a, {16, 4, 2, 4, 2, 2, 4})
+                               : need_aligned(a, {4, 2, 4, 2, 16, 2, 4}))
+        return r;
     if constexpr (VARIANT == 2) {
         if (prefill_int8_takes(kop, vop, a.b[0].ptr, a.b[bi].ptr, (uint32_t)m, scale))
             return launch_prefill_int8(a, a.b[0].ptr, q_scales, kop, vop, a.b[bi].ptr, a.b[bi + 1].ptr, N_KV, (uint32_t)m, scale);

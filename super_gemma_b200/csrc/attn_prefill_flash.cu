@@ -534,7 +534,6 @@ int encode_qkv_map(const LaunchArgs& a, CUtensorMap* tm, const BufView& buf, uin
 {
     const uint64_t rows = buf.bytes / (heads * HD * 2);
     if (rows == 0) return fail_validation(a, std::string(what) + ": buffer holds no complete row");
-    if (reinterpret_cast<uintptr_t>(buf.ptr) & 15) return fail_validation(a, std::string(what) + ": buffer must be 16-byte aligned");
     const uint64_t dims[3] = {HD, heads, rows};
     const uint64_t strides[2] = {HD * 2, heads * HD * 2};
     const uint32_t box[3] = {64, box_heads, box_rows};
@@ -552,7 +551,6 @@ int run_flash(const LaunchArgs& a, const BufView& q, const BufView& k0, const Bu
     if (q.bytes < (size_t)m_tokens * n_q * HD * 2) return fail_validation(a, "flash prefill: q buffer too small");
     if (out.bytes < (size_t)m_tokens * n_q * HD * 4) return fail_validation(a, "flash prefill: out buffer too small");
     if (step.bytes < 16) return fail_validation(a, "flash prefill: the step buffer holds 4 x u32");
-    if (reinterpret_cast<uintptr_t>(out.ptr) & 15) return fail_validation(a, "flash prefill: out must be 16-byte aligned");
     CUtensorMap tq, tk0, tv0, tk1, tv1;
     if (int r = encode_qkv_map(a, &tq, BufView{q.ptr, (size_t)m_tokens * n_q * HD * 2}, n_q, G, BLOCK_TOK, "q")) return r;
     if (int r = encode_qkv_map(a, &tk0, k0, n_kv, 1, BLOCK_N, "k")) return r;
@@ -647,6 +645,7 @@ int run_flash(const LaunchArgs& a, const BufView& q, const BufView& k0, const Bu
 int launch_prefill_flash_f16_d128(const LaunchArgs& a)
 {
     const PushScaleWindow p = *(const PushScaleWindow*)a.push;
+    if (int r = need_aligned(a, {16, 16, 16, 16, 4})) return r;
     return run_flash<false>(a, a.b[0], a.b[1], a.b[2], nullptr, nullptr, a.b[3], a.b[4], a.groups[0], a.groups[1], p.scale,
                             p.window, 0);
 }
@@ -655,6 +654,7 @@ int launch_prefill_flash_f16_d128(const LaunchArgs& a)
 int launch_prefill_sliding_ring_flash_d128(const LaunchArgs& a)
 {
     const float scale = *(const float*)a.push;
+    if (int r = need_aligned(a, {16, 16, 16, 16, 16, 16, 4})) return r;
     return run_flash<true>(a, a.b[0], a.b[1], a.b[2], &a.b[3], &a.b[4], a.b[5], a.b[6], a.groups[0], a.groups[1], scale, 1024,
                            1024);
 }
@@ -666,6 +666,7 @@ int launch_prefill_paged_q8kv_flash_d128(const LaunchArgs& a)
     const PushScalePage p = *(const PushScalePage*)a.push;
     const uint32_t n_kv = a.groups[0];
     if (n_kv == 0 || p.page == 0) return fail_validation(a, "paged flash prefill: kv heads and page must be > 0");
+    if (int r = need_aligned(a, {16, 16, 2, 16, 2, 4, 16, 16, 16, 4})) return r;
     const uint32_t row_len = n_kv * HD;
     if (int r = run_kv_dequant_paged(a, a.b[2], a.b[1], a.b[5], a.b[6], a.b[9], row_len, p.page)) return r;
     if (int r = run_kv_dequant_paged(a, a.b[4], a.b[3], a.b[5], a.b[7], a.b[9], row_len, p.page)) return r;

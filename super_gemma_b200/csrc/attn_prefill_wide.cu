@@ -500,8 +500,9 @@ int encode_rows(const LaunchArgs& a, CUtensorMap* tm, const void* base, uint64_t
 }  // namespace
 
 // What the tensor-core kernel takes: a positive softmax scale (the row maximum is taken before it), operands whose rows the
-// copies can address (16-byte aligned bases, K and V with at least one row, row indexes within an int).  Everything else stays
-// on the streaming kernel.
+// copies can address (K and V with at least one row, row indexes within an int; the launcher refuses bases that are not 16-byte
+// aligned, which the streaming kernel's loads need too) and a 16-byte aligned output.  What else the launcher accepts stays on the
+// streaming kernel.
 template <bool TWO_SRC>
 bool prefill_wide_takes(const KvOperand& k0, const KvOperand& v0, const KvOperand& k1, const KvOperand& v1, const void* q, const void* out, float scale)
 {

@@ -142,6 +142,9 @@ __device__ __forceinline__ bool resolve_row(const KvOperand& op, size_t t, size_
     return true;
 }
 
+// What load_f16 asks of the base of rows of `hd` f16 values: a lane reads hd / 32 of them with accesses of up to 16 bytes.
+constexpr uint32_t row_alignment(int hd) { return hd / 32 % 8 == 0 ? 16 : 8; }
+
 inline KvOperand linear_f16(const BufView& b, int n_kv, int hd)
 {
     return KvOperand{b.ptr, nullptr, nullptr, 0, 1, b.bytes / ((size_t)n_kv * hd * 2)};

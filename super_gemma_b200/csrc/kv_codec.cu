@@ -239,6 +239,7 @@ int launch_kv_quant_q8(const LaunchArgs& a)
     if (int r = need_bytes(a, 1, n_blocks * 2, "scales")) return r;
     if (int r = need_bytes(a, 2, n_blocks * 32, "quants")) return r;
     if (n_blocks == 0) return 0;
+    if (int r = need_aligned(a, {16, 2, 16})) return r;
     const cudaError_t e = launch_dependent(kv_quant_q8_kernel, dim3(blocks_for(n_blocks, CODEC_THREADS)), dim3(CODEC_THREADS), 0, a.stream,
         (const __half*)a.b[0].ptr, (__half*)a.b[1].ptr, (int8_t*)a.b[2].ptr, n_blocks);
     ++*a.launches;
@@ -253,6 +254,7 @@ int launch_kv_dequant_q8(const LaunchArgs& a)
     if (int r = need_bytes(a, 0, n_blocks * 2, "scales")) return r;
     if (int r = need_bytes(a, 1, n_blocks * 32, "quants")) return r;
     if (n_blocks == 0) return 0;
+    if (int r = need_aligned(a, {2, 16, 16})) return r;
     const cudaError_t e = launch_dependent(kv_dequant_q8_kernel, dim3(blocks_for(n_blocks * 2, CODEC_THREADS)), dim3(CODEC_THREADS), 0, a.stream,
         (const __half*)a.b[0].ptr, (const int8_t*)a.b[1].ptr, (__half*)a.b[2].ptr, n_blocks * 2);
     ++*a.launches;
@@ -270,6 +272,7 @@ int launch_kv_append(const LaunchArgs& a)
     const size_t dst_rows = a.b[1].bytes / (ROW_LEN * 2);
     if (RING > 0 && dst_rows < (size_t)RING) return fail_validation(a, "kv_append: ring buffer smaller than the ring");
     if (n_vec == 0) return 0;
+    if (int r = need_aligned(a, {16, 16, 4})) return r;
     const cudaError_t e = launch_dependent(kv_append_kernel<ROW_LEN, RING>, dim3(blocks_for(n_vec, CODEC_THREADS)), dim3(CODEC_THREADS), 0, a.stream,
         (const uint4*)a.b[0].ptr, (uint4*)a.b[1].ptr, (const uint32_t*)a.b[2].ptr, n_vec, dst_rows, a.status);
     ++*a.launches;
@@ -290,6 +293,7 @@ int launch_kv_append_global_q8(const LaunchArgs& a)
     if (a.b[1].bytes / 2 < dst_rows * (ROW_LEN / 32))
         return fail_validation(a, "kv_append_global_q8: scales buffer shorter than the quants buffer implies");
     if (n_blocks == 0) return 0;
+    if (int r = need_aligned(a, {16, 2, 16, 4})) return r;
     const cudaError_t e = launch_dependent(kv_append_q8_kernel, dim3(blocks_for(n_blocks, CODEC_THREADS)), dim3(CODEC_THREADS), 0, a.stream,
         (const __half*)a.b[0].ptr, (__half*)a.b[1].ptr, (int8_t*)a.b[2].ptr, nullptr, 0, 1, (const uint32_t*)a.b[3].ptr, ROW_LEN / 32,
         n_blocks, dst_rows, a.status);
@@ -316,6 +320,7 @@ int launch_kv_append_paged_q8_d128(const LaunchArgs& a)
     if (a.b[1].bytes / 2 < dst_rows * (p.row_len / 32))
         return fail_validation(a, "kv_append_paged_q8_d128: scales buffer too short for the quants buffer");
     if (n_blocks == 0) return 0;
+    if (int r = need_aligned(a, {16, 2, 16, 4, 4})) return r;
     const cudaError_t e = launch_dependent(kv_append_q8_kernel, dim3(blocks_for(n_blocks, CODEC_THREADS)), dim3(CODEC_THREADS), 0, a.stream,
         (const __half*)a.b[0].ptr, (__half*)a.b[1].ptr, (int8_t*)a.b[2].ptr, (const uint32_t*)a.b[3].ptr, (uint32_t)(a.b[3].bytes / 4),
         p.page, (const uint32_t*)a.b[4].ptr, p.row_len / 32, n_blocks, dst_rows, a.status);
@@ -349,6 +354,7 @@ int launch_kv_dequant_paged_q8_d128(const LaunchArgs& a)
     if (p.row_len == 0 || p.row_len % 128 || p.page == 0)
         return fail_validation(a, "kv_dequant_paged_q8_d128: row_len must be n_kv_heads*128 and page > 0");
     if (int r = need_bytes(a, 4, 16, "step")) return r;
+    if (int r = need_aligned(a, {2, 16, 4, 16, 4})) return r;
     return run_kv_dequant_paged(a, a.b[0], a.b[1], a.b[2], a.b[3], a.b[4], p.row_len, p.page);
 }
 

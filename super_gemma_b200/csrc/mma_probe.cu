@@ -124,6 +124,7 @@ int launch_diag_mma_cycles(const LaunchArgs& a)
         return fail_validation(a, "diag_mma_cycles: shape 0..3, n_mma a multiple of 16 up to 2^20, groups[0] = CTAs per SM (1 or 2)");
     const uint32_t ctas = (uint32_t)a.sm_count * per_sm;
     if (int r = need_bytes(a, 0, (size_t)ctas * 16, "cycles")) return r;
+    if (int r = need_aligned(a, {8})) return r;
     if (a.groups[1] > 2) return fail_validation(a, "diag_mma_cycles: groups[1] = operand data, 0 or 1 (ones) or 2 (seeded values)");
     typedef void (*ProbeKernel)(uint32_t, unsigned long long*, uint32_t*, uint32_t);
     const ProbeKernel kern = p.shape == 0 ? mma_probe_kernel<0> : p.shape == 1 ? mma_probe_kernel<1> : p.shape == 2 ? mma_probe_kernel<2> : mma_probe_kernel<3>;

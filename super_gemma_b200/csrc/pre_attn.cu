@@ -399,6 +399,7 @@ int launch_rmsnorm(const LaunchArgs& a)
     if (int r = need_bytes(a, 2, a.b[0].bytes, "y")) return r;
     const size_t n_blocks = a.b[0].bytes / 64;
     if (n_blocks == 0) return 0;
+    if (int r = need_aligned(a, {16, 4, 16})) return r;
     const cudaError_t e = launch_dependent(rmsnorm_kernel<ROW_LEN / 32, PLUS_ONE != 0>, dim3(grid_for(n_blocks)), dim3(PRE_THREADS), 0, a.stream, (const __half*)a.b[0].ptr, (const float*)a.b[1].ptr, (__half*)a.b[2].ptr, n_blocks);
     ++*a.launches;
     return check_cuda(a, e, "rmsnorm");
@@ -416,6 +417,7 @@ int launch_rope(const LaunchArgs& a)
     const size_t pairs = rows * (ROT_DIMS / 2);
     if (int r = need_bytes(a, 1, rows / N_HEADS * (ROT_DIMS / 2) * 8, "cos_sin")) return r;
     if (pairs == 0) return 0;
+    if (int r = need_aligned(a, {2, 8})) return r;
     const cudaError_t e = launch_dependent(rope_kernel, dim3(grid_for(pairs)), dim3(PRE_THREADS), 0, a.stream, (__half*)a.b[0].ptr, (const float2*)a.b[1].ptr, HEAD_DIM, ROT_DIMS / 2, N_HEADS, pairs);
     ++*a.launches;
     return check_cuda(a, e, "rope");
@@ -437,7 +439,7 @@ int launch_norm_rope_d128(const LaunchArgs& a)
     if (int r = need_bytes(a, 3, a.b[0].bytes, "y")) return r;
     if (rows == 0) return 0;
     if (rows >= (1u << 27)) return fail_validation(a, "attn_norm_rope_d128: at most 2^27 rows per launch");
-    if (reinterpret_cast<uintptr_t>(a.b[2].ptr) & 15) return fail_validation(a, "attn_norm_rope_d128: cos_sin must be 16-byte aligned");
+    if (int r = need_aligned(a, {16, 16, 16, 16})) return r;
     auto kern = p.plus_one ? norm_rope_d128_kernel<true> : norm_rope_d128_kernel<false>;
     const cudaError_t e = launch_dependent(kern, dim3(grid_for(rows * 16)), dim3(PRE_THREADS), 0, a.stream, (const __half*)a.b[0].ptr, (const float*)a.b[1].ptr, (const float2*)a.b[2].ptr, (__half*)a.b[3].ptr, p.n_heads, p.rot_dims / 2, (uint32_t)rows);
     ++*a.launches;
@@ -464,7 +466,7 @@ int launch_kv_norm_rope_append_paged_q8_d128(const LaunchArgs& a)
     const size_t kv_rows = a.b[0].bytes / 256;
     if (kv_rows == 0) return 0;
     if (kv_rows >= (1u << 26)) return fail_validation(a, "kv_norm_rope_append_paged_q8_d128: at most 2^26 (token, head) rows per launch");
-    if (reinterpret_cast<uintptr_t>(a.b[3].ptr) & 15) return fail_validation(a, "kv_norm_rope_append_paged_q8_d128: cos_sin must be 16-byte aligned");
+    if (int r = need_aligned(a, {16, 16, 16, 16, 2, 8, 2, 8, 4, 4})) return r;
     auto kern = p.plus_one ? kv_norm_rope_append_kernel<true> : kv_norm_rope_append_kernel<false>;
     const cudaError_t e = launch_dependent(kern, append_grid(a, tokens, 2 * (p.row_len / 128)), dim3(PRE_THREADS), 0, a.stream,
         nullptr, nullptr, nullptr, 0u,
@@ -500,7 +502,7 @@ int launch_qkv_norm_rope_append_paged_q8_d128(const LaunchArgs& a)
     if (kv_rows == 0) return 0;
     if (kv_rows >= (1u << 26) || q_rows >= (1u << 26))
         return fail_validation(a, "qkv_norm_rope_append_paged_q8_d128: at most 2^26 (token, head) rows of q and of k per launch");
-    if (reinterpret_cast<uintptr_t>(kv[3].ptr) & 15) return fail_validation(a, "qkv_norm_rope_append_paged_q8_d128: cos_sin must be 16-byte aligned");
+    if (int r = need_aligned(a, {16, 16, 16, 16, 16, 16, 16, 2, 8, 2, 8, 4, 4})) return r;
     auto kern = p.plus_one ? kv_norm_rope_append_kernel<true> : kv_norm_rope_append_kernel<false>;
     const cudaError_t e = launch_dependent(kern, append_grid(a, tokens, p.n_q_heads + 2 * (p.row_len / 128)), dim3(PRE_THREADS), 0, a.stream,
         (const __half*)a.b[0].ptr, (const float*)a.b[1].ptr, (__half*)a.b[2].ptr, p.n_q_heads, (const __half*)kv[0].ptr,

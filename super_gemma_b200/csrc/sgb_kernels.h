@@ -6,6 +6,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <initializer_list>
+
 #include <string>
 
 namespace sgb {
@@ -44,6 +46,8 @@ int set_last_error(int code, const std::string& msg);  // records the text sgb_l
 int fail_validation(const LaunchArgs& a, const std::string& msg);
 int check_cuda(const LaunchArgs& a, cudaError_t e, const char* what);
 int need_bytes(const LaunchArgs& a, int binding, size_t bytes, const char* what);
+// The alignment in bytes that the kernels' accesses ask of bindings 0, 1, ... (adopted pointers carry no promise of their own).
+int need_aligned(const LaunchArgs& a, std::initializer_list<uint32_t> bytes);
 
 // Tensor-map encoder resolved at run time through the CUDA runtime (no link-time libcuda).
 // dims/strides innermost first; strides[i] is the byte stride of dimension i+1.

@@ -61,6 +61,20 @@ int need_bytes(const LaunchArgs& a, int binding, size_t bytes, const char* what)
     return fail_validation(a, buf);
 }
 
+int need_aligned(const LaunchArgs& a, std::initializer_list<uint32_t> bytes)
+{
+    int binding = 0;
+    for (const uint32_t n : bytes) {
+        if (reinterpret_cast<uintptr_t>(a.b[binding].ptr) & (n - 1)) {
+            char buf[160];
+            snprintf(buf, sizeof buf, "binding %d must be %u-byte aligned", binding, n);
+            return fail_validation(a, buf);
+        }
+        binding++;
+    }
+    return SGB_OK;
+}
+
 // cuTensorMapEncodeTiled, looked up through the runtime so the library has no link-time
 // dependency on libcuda (it must load, and export its symbols, on a machine without a driver).
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -447,6 +461,7 @@ void sgb_host_free(void* p)
 int sgb_step_write(sgb_buffer* step, uint32_t pos, uint32_t kv_len_sliding, uint32_t kv_len_global, uint32_t q0)
 {
     if (!step || step->bytes < 16) return set_error(SGB_ERR_VALIDATION, "sgb_step_write: the step buffer holds 4 x u32");
+    if (reinterpret_cast<uintptr_t>(step->ptr) & 3) return set_error(SGB_ERR_VALIDATION, "sgb_step_write: the step buffer must be 4-byte aligned");
     if (step->ctx->recording) return set_error(SGB_ERR_STATE, "sgb_step_write while recording: the step buffer is per-replay state");
     // The four words travel as kernel arguments: stream-ordered after every launch queued before
     // it, and no host memory has to outlive the call.
