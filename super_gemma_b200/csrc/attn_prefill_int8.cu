@@ -221,8 +221,7 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
             const bool tail = pos0 + TILE_K - 1 > valid_end;  // the MMA warp computes the same
             for (int u = 0; u < UNITS; u++, n++) {
                 const int st = n % NV;
-                if (n >= NV) mbar_wait(&sm.v_free[st], (n / NV - 1) & 1, prm.status, 512, failed, 50);
-                if (failed) break;
+                if (n >= NV && !mbar_wait_warp(&sm.v_free[st], (n / NV - 1) & 1, prm.status, 512, failed, 50)) break;
                 const int kh = u & 1, db = block_at(j, u);
                 if (lane == 0) {
                     mbar_arrive_expect_tx(&sm.v_full[st], V_UNIT);
@@ -231,8 +230,7 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
                 }
                 if (tail) {
                     __syncwarp();
-                    mbar_wait(&sm.v_full[st], (n / NV) & 1, prm.status, 513, failed);
-                    if (failed) break;
+                    if (!mbar_wait_warp(&sm.v_full[st], (n / NV) & 1, prm.status, 513, failed)) break;
                     for (int r = lane; r < 64; r += 32) {
                         if (pos0 + kh * 64 + r <= valid_end) continue;
 #pragma unroll
@@ -582,7 +580,7 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
     tc_fence_before_sync();
     __syncthreads();
     if (*(volatile uint32_t*)&sm.abort != 0u) {
-        for (int i = 0; i < 50; i++) __nanosleep(1000);
+        let_copies_land();
         __syncthreads();
     }
     if (warp == 0) tmem_dealloc(tmem, TMEM_COLS);

@@ -222,16 +222,14 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
             const int64_t last = valid_end(t);
             const bool tail = t.pos0 + TILE_K - 1 > last;  // the MMA warp computes the same
             const int st = j % STAGES;
-            if (j >= STAGES) mbar_wait(&sm.v_free[st], (j / STAGES - 1) & 1, prm.status, 512, failed, 50);
-            if (failed) break;
+            if (j >= STAGES && !mbar_wait_warp(&sm.v_free[st], (j / STAGES - 1) & 1, prm.status, 512, failed, 50)) break;
             if (lane == 0) {
                 mbar_arrive_expect_tx(&sm.v_full[st], V_TILE);
                 for (int c = 0; c < 4; c++) tma_load_3d(sm.v[st] + c * V_CHUNK, mv, &sm.v_full[st], c * 64, kvh, t.row0);
             }
             if (tail) {
                 __syncwarp();
-                mbar_wait(&sm.v_full[st], (j / STAGES) & 1, prm.status, 513, failed);
-                if (failed) break;
+                if (!mbar_wait_warp(&sm.v_full[st], (j / STAGES) & 1, prm.status, 513, failed)) break;
                 for (int r = lane; r < TILE_K; r += 32) {
                     if (t.pos0 + r <= last) continue;
 #pragma unroll
@@ -474,7 +472,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
     tc_fence_before_sync();
     __syncthreads();
     if (*(volatile uint32_t*)&sm.abort != 0u) {
-        for (int i = 0; i < 50; i++) __nanosleep(1000);
+        let_copies_land();
         __syncthreads();
     }
     if (warp == 0) tmem_dealloc(tmem, TMEM_COLS);

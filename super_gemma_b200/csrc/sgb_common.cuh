@@ -85,6 +85,22 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
     }
 }
 
+// The same by all lanes of a warp that leaves its loop when the wait has run out: they agree on it.  A limit that runs out in some
+// lanes as the barrier completes for the others would send the first out of the loop and leave the rest at its next
+// __syncwarp() for good.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, uint32_t* status, uint32_t site, bool& failed,
+                                               uint32_t backoff_ns = 0)
+{
+    mbar_wait(bar, parity, status, site, failed, backoff_ns);
+    failed = __any_sync(0xffffffffu, failed);
+    return !failed;
+}
+// What a wait that ran out leaves in flight gets a bounded time to land before its target is handed to the next CTA.
+__device__ __forceinline__ void let_copies_land()
+{
+    for (int i = 0; i < 50; i++) __nanosleep(1000);
+}
+
 // ---- TMA: every copy targets the issuing CTA only ---------------------------------------------
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m)
 {

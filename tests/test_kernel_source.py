@@ -1,0 +1,21 @@
+"""Rules of the kernels' sources that no run on a healthy GPU shows."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "super_gemma_b200", "csrc")
+
+
+def _source(name):
+    with open(os.path.join(CSRC, name)) as f:
+        return re.sub(r"//[^\n]*", "", f.read())
+
+
+@pytest.mark.parametrize("name", ["attn_prefill_wide.cu", "attn_prefill_int8.cu"])
+def test_v_loader_warps_agree_on_a_wait_that_ran_out(name):
+    """The V loader is a whole warp that breaks out of its loop, with __syncwarp() inside: every wait of its is voted on."""
+    s = _source(name)
+    role = s[s.index("warp == V_W"):s.index("warp == MMA_W")]
+    assert "__syncwarp" in role and "break" in role
+    assert len(re.findall(r"\bmbar_wait_warp\(", role)) == 2 and not re.search(r"\bmbar_wait\(", role)
