@@ -408,11 +408,13 @@ __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
 
         // Refill this slot for iteration it + NSTAGES; every lane is done reading it.
         __syncwarp();
-        if (lane < 4 && it + NSTAGES < n_iter) {
+        if (lane < 4 && it + NSTAGES < n_iter && !failed) {  // after a wait that ran out: no more copies, and no more waiting
             issue(it + NSTAGES, next_pp);
             if (it + NSTAGES + 1 < n_iter) next_pp = lookup(s_begin + (it + NSTAGES + 1) * n_sub);
         }
     }
+
+    if (__any_sync(0xffffffffu, failed)) let_copies_land();  // into this warp's ring, which is written next
 
     // ---- remove the +1152 offsets, total the denominators --------------------------------------------
 #pragma unroll

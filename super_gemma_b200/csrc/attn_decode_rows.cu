@@ -138,7 +138,7 @@ struct RowsWarp {
         for (int i = 0; i < n; ++i) {
             KeyTile t;
             tile(i, t);
-            mbar_wait(&sl.k_full, i & 1, status, 601, failed);
+            if (!mbar_wait_warp(&sl.k_full, i & 1, status, 601, failed)) break;
             float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // keys g (0, 1) and g + 8 (2, 3) x rows 2*t4, 2*t4 + 1
             if constexpr (KQ8) {
                 uint4 sa[2], sc[2];  // 16 block scales of keys g and g + 8
@@ -226,7 +226,7 @@ struct RowsWarp {
                 hi[h] = movmatrix_trans(w);
                 lo[h] = movmatrix_trans(pack_half2(p[2 * h] - f.x, p[2 * h + 1] - f.y));
             }
-            mbar_wait(&sl.v_full, i & 1, status, 602, failed);
+            if (!mbar_wait_warp(&sl.v_full, i & 1, status, 602, failed)) break;
             if (t.from > 0 || t.to < TILE) {  // p = 0 in the rows that are no keys, and 0 times a stale Inf or NaN would not be
                 for (int w = lane; w < V_PIECES * TILE * 8; w += 32) {
                     const int r = (w >> 3) & (TILE - 1);
@@ -247,6 +247,7 @@ struct RowsWarp {
             __syncwarp();
             if (i + 1 < n) issue_v(i + 1);
         }
+        if (failed) let_copies_land();  // into this warp's slots, one of which is written next
         // the state for the merge: [row][HD], m, l
         l[0] = key_sum(l[0]);
         l[1] = key_sum(l[1]);

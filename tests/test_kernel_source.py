@@ -19,3 +19,15 @@ def test_v_loader_warps_agree_on_a_wait_that_ran_out(name):
     role = s[s.index("warp == V_W"):s.index("warp == MMA_W")]
     assert "__syncwarp" in role and "break" in role
     assert len(re.findall(r"\bmbar_wait_warp\(", role)) == 2 and not re.search(r"\bmbar_wait\(", role)
+
+
+def test_decode_warps_stop_at_a_wait_that_ran_out():
+    """A warp whose copy did not arrive asks for no more (a slot would have two copies under way and its barrier more arrivals
+    than it counts), and lets those in flight land before their target is used for the merge or left to another CTA."""
+    s = _source("attn_decode_rows.cu")
+    waits = re.findall(r"[^\n]*\bmbar_wait(?:_warp)?\([^\n]*", s)
+    assert len(waits) == 2 and all(re.search(r"if \(!mbar_wait_warp\(.*\) break;", w) for w in waits)
+    assert 0 < s.index("if (failed) let_copies_land();", s.rindex("mbar_wait_warp("))
+    s = _source("attn_decode_paged.cu")
+    refill = s.index("n_iter && !failed)", s.index("mbar_wait("))
+    assert s.index("issue(it + NSTAGES", refill) < s.index("let_copies_land();", refill)
