@@ -12,8 +12,8 @@
 // (206 MB, 5.1 TB/s on the 128 SMs that 4 x 32 CTAs occupy); head_dim 256, 1024 slots, 16 splits 12.3 -> 5.7; verify of 4 tokens over
 // the ring, 16 kv heads 148 -> 8.4.
 // A bulk copy per row instead (48 a tile at head_dim 512) took 41.8 us.
-// V rows that hold no visible key are zeroed once they have arrived, and a CTA whose result is not finite computes it again by the
-// streaming statement: a tile multiplies by p = 0 what that statement skips.
+// V rows that hold no visible key are zeroed once they have arrived, and rows that are not finite are computed again by the streaming
+// statement: a tile multiplies by p = 0 what that statement skips (all of them at 32768 tokens: 427 us on the streaming kernel).
 #include <mutex>
 #include <string>
 
@@ -287,16 +287,15 @@ template <int HD, int G, bool KQ8, int WARPS>
 struct DecodeRowsSmem {
     typename RowsWarp<HD, KQ8, G>::Slots w[WARPS];
     uint8_t q[8 * (HD * 2 + (KQ8 ? 32 : 16))];
+    uint32_t redo;  // rows that are not finite, a bit each
 };
 
 // Split-K partials.  Grid, split ranges and partials as decode_generic_kernel.
 template <int HD, int G, bool KQ8, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) decode_rows_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_sc,
-                                                                 const __grid_constant__ CUtensorMap tm_v, const __half* __restrict__ q,
-                                                                 const __grid_constant__ KvOperand kop,
-                                                                 const __grid_constant__ KvOperand vop, float* __restrict__ part,
-                                                                 const uint32_t* __restrict__ step, int step_slot, uint32_t n_splits, float scale,
-                                                                 uint32_t* status)
+__global__ void __launch_bounds__(WARPS * 32, HD == 512 ? 1 : HD == 256 ? 3 : 6)  // CTAs that the slots let an SM hold
+    decode_rows_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_sc, const __grid_constant__ CUtensorMap tm_v,
+                       const __half* __restrict__ q, const __grid_constant__ KvOperand kop, const __grid_constant__ KvOperand vop,
+                       float* __restrict__ part, const uint32_t* __restrict__ step, int step_slot, uint32_t n_splits, float scale, uint32_t* status)
 {
     using W = RowsWarp<HD, KQ8, G>;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -313,6 +312,7 @@ __global__ void __launch_bounds__(WARPS * 32) decode_rows_kernel(const __grid_co
         mbar_init(&sm.w[warp].v_full, 1);
         mbar_fence_init();
     }
+    if (threadIdx.x == 0) sm.redo = 0;
     pdl_wait();
     pdl_launch_dependents();
     const uint32_t kv_len = __ldg(step + step_slot);
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(WARPS * 32) decode_rows_kernel(const __grid_co
           },
           sm.q, kvh, scale, lo, hi, status);
     __syncthreads();
-    bool odd = false;
+    uint32_t odd = 0;
     for (int idx = threadIdx.x; idx < G * HD; idx += WARPS * 32) {
         const int r = idx / HD, d = idx % HD;
         float big = sm.w[0].m[r];
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(WARPS * 32) decode_rows_kernel(const __grid_co
             acc = fmaf(f, reinterpret_cast<const float*>(sm.w[k].v)[idx], acc);
             l = fmaf(f, sm.w[k].l[r], l);
         }
-        odd |= !(fabsf(acc) <= 3.4e38f) || !(fabsf(l) <= 3.4e38f);
+        if (!(fabsf(acc) <= 3.4e38f) || !(fabsf(l) <= 3.4e38f)) odd |= 1u << r;
         float* row = part + (((size_t)i * n_q + kvh * G + r) * n_splits + split) * (HD + 2);
         row[d] = acc;
         if (d == 0) {
@@ -365,18 +365,17 @@ __global__ void __launch_bounds__(WARPS * 32) decode_rows_kernel(const __grid_co
             row[HD + 1] = l;
         }
     }
+    if (odd != 0) atomicOr(&sm.redo, odd);
     if (__syncthreads_or(odd)) {  // again by the streaming statement, a warp per row
         constexpr int DPL = HD / 32;
+        const uint32_t redo = sm.redo;
         for (int r = warp; r < G; r += WARPS) {
-            float qr[DPL], kk[DPL], vv[DPL];
-            load_f16<DPL>(q_row(r) + lane * DPL, qr);
+            if (((redo >> r) & 1) == 0) continue;
+            float qr[1][DPL];
+            load_f16<DPL>(q_row(r) + lane * DPL, qr[0]);
             Stream<1, DPL> st;
             st.init();
-            for (size_t t = t_begin; t < t_end; t++) {
-                load_row<HD, KQ8 ? FMT_Q8 : FMT_F16, DPL>(kop, t, kvh, n_kv, lane * DPL, kk);
-                load_row<HD, FMT_F16, DPL>(vop, t, kvh, n_kv, lane * DPL, vv);
-                st.step(0, qr, kk, vv, scale);
-            }
+            stream_keys<HD, KQ8 ? FMT_Q8 : FMT_F16, 1, HD == 128 ? 4 : 8>(st, qr, kop, vop, t_begin, t_end, 0, kvh, n_kv, scale);
             float* row = part + (((size_t)i * n_q + kvh * G + r) * n_splits + split) * (HD + 2);
 #pragma unroll
             for (int d = 0; d < DPL; d++) row[lane * DPL + d] = st.acc[0][d];
@@ -508,17 +507,13 @@ __global__ void __cluster_dims__(V_CTAS, 1, 1) __launch_bounds__(V_WARPS * 32)
     cluster_sync();  // nobody leaves while its shared memory is read
     if (__syncthreads_or(odd) && warp == 0) {  // this CTA's row again, by the streaming statement
         const uint32_t i = rank / V_G, qpos = (uint32_t)q0 + i, begin = qpos + 1 > window ? qpos + 1 - window : 0;
-        float qr[V_DPL], kk[V_DPL], vv[V_DPL];
-        load_f16<V_DPL>(q_row(rank) + lane * V_DPL, qr);
+        float qr[1][V_DPL];
+        load_f16<V_DPL>(q_row(rank) + lane * V_DPL, qr[0]);
         Stream<1, V_DPL> st;
         st.init();
-        for (uint32_t t = begin; t <= qpos; t++) {
-            const bool old = t < (uint32_t)q0;
-            const size_t row = old ? t % ring : t - (uint32_t)q0;
-            load_row<V_HD, FMT_F16, V_DPL>(old ? k_ring : k_new, row, kvh, (int)n_kv, lane * V_DPL, kk);
-            load_row<V_HD, FMT_F16, V_DPL>(old ? v_ring : v_new, row, kvh, (int)n_kv, lane * V_DPL, vv);
-            st.step(0, qr, kk, vv, scale);
-        }
+        stream_keys<V_HD, FMT_F16, 1, 8>(st, qr, k_ring, v_ring, begin, (uint32_t)q0, ring, kvh, (int)n_kv, scale);
+        const uint32_t c0 = begin > (uint32_t)q0 ? begin - (uint32_t)q0 : 0;
+        stream_keys<V_HD, FMT_F16, 1, 4>(st, qr, k_new, v_new, c0, i + 1, 0, kvh, (int)n_kv, scale);
 #pragma unroll
         for (int d = 0; d < V_DPL; d++) out[((size_t)i * n_q + kvh * V_G + rank % V_G) * V_HD + lane * V_DPL + d] = st.acc[0][d] / st.l[0];
     }

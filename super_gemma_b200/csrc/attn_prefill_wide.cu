@@ -15,8 +15,9 @@
 // -> P V of eight tiles plus set-up and merge (3000 cycles a tile, of which the MMAs need 1800).
 //
 // What a tile reads beyond a query's own keys must not matter: scores are masked by selection, V rows that hold no key are
-// zeroed.  A V row that is visible to some query of the tile and not finite is visible to all of them as 0 * Inf, so a CTA
-// with a non-finite output computes its rows again by the streaming statement, which reads what each query sees.
+// zeroed.  A V row that is visible to some query of the tile and not finite is visible to all of them as 0 * Inf, so rows that are
+// not finite are computed again by the streaming statement, which reads what each query sees (all of 256 queries over the
+// ring: 807 us on the streaming kernel, 793 here; eight of them 238).
 #include <mutex>
 #include <string>
 
@@ -49,7 +50,8 @@ struct WideSmem {
     float red[2][ROWS];
     float2 other_ml[ROWS];
     uint64_t q_bar, k_full[STAGES], k_free[STAGES], v_full[STAGES], v_free[STAGES], v_ok[STAGES], s_ready[2], p_ready[2], pv_done[2];
-    uint32_t tmem_base, abort, redo;
+    uint32_t tmem_base, abort;
+    __align__(16) uint32_t redo[2][2][ROWS / 32];  // rows that are not finite, a bit each: [found by this CTA or the other][dim half][row / 32]
 };
 static_assert(sizeof(WideSmem) <= 227 * 1024, "one CTA per SM");
 
@@ -74,18 +76,25 @@ __device__ __forceinline__ void st_cluster_f4(uint32_t addr, float4 v)
 {
     asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
+__device__ __forceinline__ void st_cluster_u32(uint32_t addr, uint32_t v)
+{
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
 __device__ __forceinline__ void cluster_sync()
 {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// The rows of one CTA by the streaming statement, a warp per row.
+// The rows that are not finite by the streaming statement, a warp per token (G = 2 rows); the CTAs of a cluster take turns.
 template <bool TWO_SRC>
-__device__ __noinline__ void stream_rows(const WideParams& prm, uint32_t m0, int kvh)
+__device__ __noinline__ void stream_rows(const WideParams& prm, const WideSmem& sm, uint32_t m0, int kvh, uint32_t rank)
 {
     const uint32_t q0 = prm.step[STEP_Q0];
-    for (int r = threadIdx.x >> 5; r < ROWS && m0 + r / G < prm.m_tokens; r += WIDE_THREADS / 32)
-        stream_prefill_row<HD, G, false, TWO_SRC>(prm.q, nullptr, prm.k0, prm.v0, prm.k1, prm.v1, prm.out, q0, m0 + r / G, kvh * G + r % G, (int)prm.n_kv,
-                                                  prm.window, prm.ring, prm.scale);
+    for (uint32_t tok = threadIdx.x >> 5; tok < ROWS / G; tok += WIDE_THREADS / 32) {
+        const uint32_t i = tok / 16, redo = sm.redo[0][0][i] | sm.redo[0][1][i] | sm.redo[1][0][i] | sm.redo[1][1][i], which = (redo >> (2 * tok % 32)) & 3u;
+        if (which == 0 || (prm.n_cta == 2 && tok % 2 != rank)) continue;
+        stream_prefill_rows<HD, G, false, TWO_SRC>(prm.q, nullptr, prm.k0, prm.v0, prm.k1, prm.v1, prm.out, q0, m0 + tok, kvh * G, which, (int)prm.n_kv,
+                                                   prm.window, prm.ring, prm.scale);
+    }
 }
 
 struct WideTile {
@@ -182,9 +191,9 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
             mbar_init(&sm.pv_done[i], 1);
         }
         sm.abort = 0;
-        sm.redo = 0;
         mbar_fence_init();
     }
+    if (tid < 4 * ROWS / 32) (&sm.redo[0][0][0])[tid] = 0;
     if (warp == 0) {
         tmem_alloc(&sm.tmem_base, TMEM_COLS);
         tmem_relinquish();
@@ -465,7 +474,11 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
                                                                                   pack_half2(y[8 * i + 4], y[8 * i + 5]), pack_half2(y[8 * i + 6], y[8 * i + 7]));
             }
         }
-        if (odd) sm.redo = 1;
+        const uint32_t rows_odd = __ballot_sync(0xffffffffu, odd);
+        if (rows_odd != 0 && lane == 0) {
+            sm.redo[0][half][kq] = rows_odd;
+            if (split) st_cluster_u32(map_to_rank(smem_u32(&sm.redo[1][half][kq]), rank ^ 1u), rows_odd);
+        }
     }
     // A wait that ran out leaves copies and MMAs of this CTA in flight that nobody will wait for: give them a bounded
     // time to land before the shared and tensor memory they target is handed to the next CTA.
@@ -477,11 +490,16 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
     }
     if (warp == 0) tmem_dealloc(tmem, TMEM_COLS);
     if (prm.n_cta > 1) {
-        // both CTAs have written their share: if either redoes the rows, its values are the last
+        // both CTAs have written their share and know of each other's rows: what is written again is the last
         __syncwarp();
         cluster_sync();
     }
-    if (*(volatile uint32_t*)&sm.redo != 0u) stream_rows<TWO_SRC>(prm, m0, kvh);
+    const uint4* redo = reinterpret_cast<const uint4*>(sm.redo);
+    static_assert(sizeof(WideSmem::redo) == 4 * sizeof(uint4), "four words of rows / 32 bits each");
+    uint32_t any = 0;
+#pragma unroll
+    for (int i = 0; i < 4; i++) any |= redo[i].x | redo[i].y | redo[i].z | redo[i].w;
+    if (any != 0) stream_rows<TWO_SRC>(prm, sm, m0, kvh, rank);
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }

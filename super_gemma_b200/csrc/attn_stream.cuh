@@ -1,6 +1,6 @@
 // The reference's streaming-softmax statement, one key at a time in f32 (attn_decode_sliding.wgsl:84-107): row loads in every
-// cache format and the per-warp state.  The scalar kernels are built from it, and the tensor-core kernels fall back to it
-// for rows whose tiled result is not finite.
+// cache format and the per-warp state.  The scalar kernels are built from it, and the tensor-core kernels fall back to its form of
+// several keys at a time for rows whose tiled result is not finite.
 #pragma once
 
 #include "sgb_common.cuh"
@@ -154,41 +154,167 @@ inline KvOperand linear_q8(const BufView& quants, const BufView& scales, int n_k
     return KvOperand{quants.ptr, (const __half*)scales.ptr, nullptr, 0, 1, quants.bytes / ((size_t)n_kv * hd)};
 }
 
-// One query row of prefill by the streaming statement, by a warp: history rows [begin, q0) or all rows [begin, qpos] of (k0, v0) at
-// t % ring, then (two sources) the chunk's rows of (k1, v1).  For rows whose tiled result is not finite.
-template <int HD, int G, bool QI8, bool TWO_SRC>
-__device__ __forceinline__ void stream_prefill_row(const void* q, const __half* q_scales, const KvOperand& k0, const KvOperand& v0, const KvOperand& k1,
-                                                   const KvOperand& v1, __half* out, uint32_t q0, uint32_t i, int head, int n_kv, uint32_t window,
-                                                   uint32_t ring, float scale)
+// warp_sum of N values (a power of two): the lanes share out the values while they add, about 2 N shuffles instead of 5 N.
+template <int N>
+__device__ __forceinline__ void warp_sums(float* v)
 {
-    constexpr int DPL = HD / 32, KFMT = QI8 ? FMT_Q8 : FMT_F16;
-    const int d0 = (threadIdx.x & 31) * DPL, kvh = head / G;
-    const size_t qrow = (size_t)i * (n_kv * G) + head;
-    float qr[DPL], kk[DPL], vv[DPL];
-    if constexpr (QI8)
-        load_q8<DPL>(reinterpret_cast<const int8_t*>(q) + qrow * HD + d0, q_scales + qrow * (HD / 32), d0, qr);
-    else
-        load_f16<DPL>(reinterpret_cast<const __half*>(q) + qrow * HD + d0, qr);
-    Stream<1, DPL> st;
-    st.init();
-    const uint32_t qpos = q0 + i, begin = (window != 0 && qpos + 1 > window) ? qpos + 1 - window : 0;
-    const uint32_t hist_end = TWO_SRC ? min(q0, qpos + 1) : qpos + 1;
-    for (uint32_t t = begin; t < hist_end; t++) {
-        const size_t row = ring ? t % ring : t;
-        if (row >= k0.rows || row >= v0.rows) break;  // reported where the tiles are laid out
-        load_row<HD, KFMT, DPL>(k0, row, kvh, n_kv, d0, kk);
-        load_row<HD, FMT_F16, DPL>(v0, row, kvh, n_kv, d0, vv);
-        st.step(0, qr, kk, vv, scale);
-    }
-    if (TWO_SRC) {
-        for (uint32_t c = begin > q0 ? begin - q0 : 0; c <= i; c++) {
-            load_row<HD, FMT_F16, DPL>(k1, c, kvh, n_kv, d0, kk);
-            load_row<HD, FMT_F16, DPL>(v1, c, kvh, n_kv, d0, vv);
-            st.step(0, qr, kk, vv, scale);
+    const int lane = threadIdx.x & 31;
+    int o = 16;
+#pragma unroll
+    for (int n = N / 2; n > 0; n >>= 1, o >>= 1) {
+        const bool upper = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < n; i++) {
+            const float send = upper ? v[i] : v[i + n], keep = upper ? v[i + n] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
         }
     }
+    float total = v[0];  // of value lane / (32 / N)
 #pragma unroll
-    for (int d = 0; d < DPL; d++) out[qrow * HD + d0 + d] = __float2half_rn(st.acc[0][d] / st.l[0]);
+    for (o = 16 / N; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+#pragma unroll
+    for (int i = 0; i < N; i++) v[i] = __shfl_sync(0xffffffffu, total, i * (32 / N));
+}
+
+// ---- the same by one warp, several keys at a time: for the rows whose tiled result is not finite ----------------------------
+// A slice of a row as it lies in memory.
+template <int FMT, int DPL>
+struct RawSlice {
+    uint32_t w[FMT == FMT_F16 ? DPL / 2 : DPL / 4];
+    float s;
+    __device__ __forceinline__ void load(const char* p)
+    {
+        constexpr int N = sizeof(w) / 4;
+        if constexpr (FMT == FMT_F16 && N % 4 == 0) {
+#pragma unroll
+            for (int i = 0; i < N / 4; i++) {
+                const uint4 u = __ldg(reinterpret_cast<const uint4*>(p) + i);
+                w[4 * i] = u.x, w[4 * i + 1] = u.y, w[4 * i + 2] = u.z, w[4 * i + 3] = u.w;
+            }
+        } else if constexpr (FMT == FMT_F16) {
+#pragma unroll
+            for (int i = 0; i < N / 2; i++) {
+                const uint2 u = __ldg(reinterpret_cast<const uint2*>(p) + i);
+                w[2 * i] = u.x, w[2 * i + 1] = u.y;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < N; i++) w[i] = __ldg(reinterpret_cast<const uint32_t*>(p) + i);
+        }
+    }
+    __device__ __forceinline__ float at(int d) const
+    {
+        if constexpr (FMT == FMT_F16) {
+            const float2 f = __half22float2(reinterpret_cast<const __half2*>(w)[d / 2]);
+            return (d & 1) ? f.y : f.x;
+        } else {
+            return __fmul_rn(s, (float)(int8_t)((w[d / 4] >> (8 * (d & 3))) & 0xFF));
+        }
+    }
+};
+
+// H query heads of a kv head against the keys [begin, end), key t in row t, or t % ring.  One key at a time a warp waits for memory
+// at every step (490 ns a key); KEYS of them cost one wait, and share the rescale.
+template <int HD, int KFMT, int H, int KEYS>
+__device__ __forceinline__ void stream_keys(Stream<H, HD / 32>& st, const float (&qr)[H][HD / 32], const KvOperand& k, const KvOperand& v,
+                                            uint32_t begin, uint32_t end, uint32_t ring, int kvh, int n_kv, float scale)
+{
+    constexpr int DPL = HD / 32;
+    const int d0 = (threadIdx.x & 31) * DPL;
+    const uint32_t k_pitch = (uint32_t)n_kv * HD * (KFMT == FMT_F16 ? 2 : 1), v_pitch = (uint32_t)n_kv * HD * 2, s_pitch = (uint32_t)n_kv * (HD / 32);
+    const char* k_base = reinterpret_cast<const char*>(k.data) + (kvh * HD + d0) * (KFMT == FMT_F16 ? 2 : 1);
+    const char* v_base = reinterpret_cast<const char*>(v.data) + (kvh * HD + d0) * 2;
+    for (uint32_t t0 = begin; t0 < end; t0 += KEYS) {
+        // Past the end the last key once more, with a score of -inf and zeros for its value: no branches between the keys
+        RawSlice<KFMT, DPL> kk[KEYS];
+        RawSlice<FMT_F16, DPL> vv[KEYS];
+        const uint32_t row0 = ring ? t0 % ring : t0;
+#pragma unroll
+        for (int j = 0; j < KEYS; j++) {
+            uint32_t row = row0 + min((uint32_t)j, end - 1 - t0);
+            if (ring && row >= ring) row -= ring;
+            kk[j].load(k_base + (uint64_t)row * k_pitch);
+            if constexpr (KFMT != FMT_F16) kk[j].s = __half2float(__ldg(k.scales + (uint64_t)row * s_pitch + kvh * (HD / 32) + d0 / 32));
+            vv[j].load(v_base + (uint64_t)row * v_pitch);
+        }
+        float s[KEYS][H];
+#pragma unroll
+        for (int j = 0; j < KEYS; j++) {
+#pragma unroll
+            for (int h = 0; h < H; h++) s[j][h] = 0.0f;
+#pragma unroll
+            for (int d = 0; d < DPL; d++) {
+                const float x = kk[j].at(d);
+#pragma unroll
+                for (int h = 0; h < H; h++) s[j][h] = fmaf(qr[h][d], x, s[j][h]);
+            }
+        }
+        warp_sums<KEYS * H>(&s[0][0]);
+#pragma unroll
+        for (int h = 0; h < H; h++) {
+            float top = st.m[h];
+#pragma unroll
+            for (int j = 0; j < KEYS; j++) {
+                s[j][h] = t0 + j < end ? s[j][h] * scale : -INFINITY;
+                top = fmaxf(top, s[j][h]);
+            }
+            const float corr = __expf(st.m[h] - top);
+            st.m[h] = top;
+            st.l[h] *= corr;
+#pragma unroll
+            for (int d = 0; d < DPL; d++) st.acc[h][d] *= corr;
+#pragma unroll
+            for (int j = 0; j < KEYS; j++) {
+                s[j][h] = __expf(s[j][h] - top);
+                st.l[h] += s[j][h];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < KEYS; j++) {
+#pragma unroll
+            for (int d = 0; d < DPL; d++) {
+                const float x = t0 + j < end ? vv[j].at(d) : 0.0f;
+#pragma unroll
+                for (int h = 0; h < H; h++) st.acc[h][d] = fmaf(s[j][h], x, st.acc[h][d]);
+            }
+        }
+    }
+}
+
+// Two heads (head0 and the next, of one kv head) of prefill token i by a warp: history rows [begin, q0) or all rows [begin, qpos] of
+// (k0, v0) at t % ring, then (two sources) the chunk's rows of (k1, v1).  Writes the heads in `which`.
+template <int HD, int G, bool QI8, bool TWO_SRC>
+__device__ __forceinline__ void stream_prefill_rows(const void* q, const __half* q_scales, const KvOperand& k0, const KvOperand& v0, const KvOperand& k1,
+                                                    const KvOperand& v1, __half* out, uint32_t q0, uint32_t i, int head0, uint32_t which, int n_kv,
+                                                    uint32_t window, uint32_t ring, float scale)
+{
+    constexpr int DPL = HD / 32, KFMT = QI8 ? FMT_Q8 : FMT_F16, KEYS = 4;
+    static_assert(G % 2 == 0, "a pair of heads shares its kv head");
+    const int d0 = (threadIdx.x & 31) * DPL, kvh = head0 / G;
+    const size_t qrow = (size_t)i * (n_kv * G) + head0;
+    float qr[2][DPL];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        if constexpr (QI8)
+            load_q8<DPL>(reinterpret_cast<const int8_t*>(q) + (qrow + h) * HD + d0, q_scales + (qrow + h) * (HD / 32), d0, qr[h]);
+        else
+            load_f16<DPL>(reinterpret_cast<const __half*>(q) + (qrow + h) * HD + d0, qr[h]);
+    }
+    Stream<2, DPL> st;
+    st.init();
+    const uint32_t qpos = q0 + i, begin = (window != 0 && qpos + 1 > window) ? qpos + 1 - window : 0;
+    uint32_t hist_end = TWO_SRC ? min(q0, qpos + 1) : qpos + 1;
+    if (ring == 0) hist_end = (uint32_t)min((size_t)hist_end, min(k0.rows, v0.rows));  // reported where the tiles are laid out
+    stream_keys<HD, KFMT, 2, KEYS>(st, qr, k0, v0, begin, hist_end, ring, kvh, n_kv, scale);
+    if constexpr (TWO_SRC)
+        stream_keys<HD, FMT_F16, 2, KEYS>(st, qr, k1, v1, begin > q0 ? begin - q0 : 0, i + 1, 0, kvh, n_kv, scale);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        if ((which >> h) & 1) {
+#pragma unroll
+            for (int d = 0; d < DPL; d++) out[(qrow + h) * HD + d0 + d] = __float2half_rn(st.acc[h][d] / st.l[h]);
+        }
+    }
 }
 
 }  // namespace sgb

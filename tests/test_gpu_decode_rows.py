@@ -134,3 +134,17 @@ def test_verify_ring_value_only_the_later_token_sees(ctx):
     assert np.all(got[3, 2:, 9] == np.inf)
     got[3, 2:, 9] = clean[3, 2:, 9]
     assert_close(got, clean, ATOL, 1e-5, "everything else")
+
+
+@pytest.mark.parametrize("kind", KINDS, ids=lambda k: k[0])
+def test_only_rows_that_are_not_finite_are_computed_again(ctx, kind):
+    """A NaN in one query row leaves the other rows' bits alone."""
+    _, _, n_kv, g, hd, _, _ = kind
+    n, splits = 300, 3
+    q, k, v = _case(kind, 91, n)
+    clean, _, _ = _decode(ctx, kind, q, k, v, n, splits)
+    row = n_kv * g - 1
+    q[row, 3] = np.nan
+    got, _, _ = _decode(ctx, kind, q, k, v, n, splits)
+    assert np.all(np.isnan(got[row]))
+    assert np.array_equal(got[:row].view(np.uint32), clean[:row].view(np.uint32))

@@ -85,8 +85,11 @@ def test_sliding_ring_wrapped(ctx, q0, m):
     assert_close(got[toks], want, ATOL, RTOL, f"wrapped q0={q0} m={m}")
 
 
-def _iq(ctx, q, k, v, q0, m, scale=0.044194174, pad=80, v_bits=None):
+def _iq(ctx, q, k, v, q0, m, scale=0.044194174, pad=80, v_bits=None, poison=None):
     qs, qq, qd = O.q8_quant_div(q.ravel())
+    if poison is not None:  # a scale of q
+        qs = qs.copy()
+        qs.view(np.uint16)[poison] = NAN16
     ks, kq, kd = O.q8_quant_div(k.ravel())
     up = lambda b: ctx.buffer_from_iter(np.ascontiguousarray(b))
     tail = np.full(pad * 2048, NAN16, np.uint16)
@@ -187,3 +190,54 @@ def test_reruns_give_the_same_bits(ctx):
     q, k, v, _ = _sliding_case(15, 1500, 96, 16)
     a, b = (_sliding(ctx, q, k, v, 1500, 96, 16, True) for _ in range(2))
     assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
+@pytest.mark.parametrize("n_kv", [2, 80])  # two CTAs per unit, one
+def test_only_rows_that_are_not_finite_are_computed_again(ctx, n_kv):
+    """A NaN in one query row leaves every other row's bits alone, also those of its own tile and of the other CTA of its cluster."""
+    m, q0 = 64, 300
+    q, k, v, _ = _sliding_case(21, q0, m, n_kv)
+    clean = _sliding(ctx, q, k, v, q0, m, n_kv, True)
+    for tok, head in ((37, 1), (0, 2), (63, 3)):
+        q2 = q.copy()
+        q2[tok, head, 100] = np.nan
+        got = _sliding(ctx, q2, k, v, q0, m, n_kv, True)
+        assert np.all(np.isnan(got[tok, head]))
+        got[tok, head] = clean[tok, head]
+        assert np.array_equal(got.view(np.uint32), clean.view(np.uint32))
+
+
+def test_global_int8_only_rows_that_are_not_finite_are_computed_again(ctx):
+    """... and of a row whose scales hold a NaN in the int8 form."""
+    m, q0 = 16, 600
+    q, k, v = _normal(41, m, 32, 512), _normal(42, q0 + m, 4, 512), _normal(43, q0 + m, 4, 512)
+    clean, _, _ = _iq(ctx, q, k, v, q0, m)
+    for tok, head in ((0, 0), (5, 13), (15, 31)):
+        got, _, _ = _iq(ctx, q, k, v, q0, m, poison=(tok * 32 + head) * 16 + 7)
+        assert np.all(np.isnan(got[tok, head]))
+        got[tok, head] = clean[tok, head]
+        assert np.array_equal(got.view(np.uint32), clean.view(np.uint32))
+
+
+@pytest.mark.parametrize("n_kv", [2, 80])
+def test_a_value_that_everybody_sees(ctx, n_kv):
+    """Inf in the first visible value of one dim: all rows of that kv head are computed again, by both CTAs of a cluster."""
+    m, q0 = 65, 200
+    q, k, v, _ = _sliding_case(23, q0, m, n_kv)
+    clean = _sliding(ctx, q, k, v, q0, m, n_kv, True)
+    v[0, 1, 200] = np.inf
+    got = _sliding(ctx, q, k, v, q0, m, n_kv, True)
+    assert np.all(got[:, 2:4, 200] == np.inf)
+    got[:, 2:4, 200] = clean[:, 2:4, 200]
+    assert_close(got, clean, ATOL, 2 * RTOL, "everything else")  # two statements, each rounded to f16
+
+
+def test_global_int8_value_that_everybody_sees(ctx):
+    m, q0 = 16, 333
+    q, k, v = _normal(51, m, 32, 512), _normal(52, q0 + m, 4, 512), _normal(53, q0 + m, 4, 512)
+    clean, _, _ = _iq(ctx, q, k, v, q0, m)
+    v[2, 3, 500] = -np.inf
+    got, _, _ = _iq(ctx, q, k, v, q0, m)
+    assert np.all(got[:, 24:, 500] == -np.inf)
+    got[:, 24:, 500] = clean[:, 24:, 500]
+    assert_close(got, clean, ATOL, 2 * RTOL, "everything else")
