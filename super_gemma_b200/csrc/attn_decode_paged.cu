@@ -143,8 +143,8 @@ template <int NSTAGES, int MIN_CTAS, int SUB, bool CLUSTERED>
 __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
     decode_paged_kernel(const __grid_constant__ CUtensorMap tm_kq, const __grid_constant__ CUtensorMap tm_ks,
                         const __grid_constant__ CUtensorMap tm_vq, const __grid_constant__ CUtensorMap tm_vs,
-                        const __half* __restrict__ q, const uint32_t* __restrict__ page_table, uint32_t table_len, uint32_t page,
-                        uint32_t pool_pages, float* __restrict__ part, const uint32_t* __restrict__ step, uint32_t n_kv,
+                        const __half* q, const uint32_t* page_table, uint32_t table_len, uint32_t page,
+                        uint32_t pool_pages, float* __restrict__ part, const uint32_t* step, uint32_t n_kv,
                         uint32_t n_splits, float scale, uint32_t m_q, uint32_t* status)
 {
     extern __shared__ uint8_t smem_raw[];
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
     }
     pdl_wait();  // everything below reads what earlier kernels of the stream wrote (step words, q, the appended rows)
     pdl_launch_dependents();
-    const uint32_t kv_len = __ldg(step + STEP_KV_LEN_GLOBAL);
+    const uint32_t kv_len = ld_global(step + STEP_KV_LEN_GLOBAL);
     const uint32_t chunk = (kv_len + n_splits - 1) / n_splits;
     const uint32_t t_begin = min((uint32_t)split * chunk, kv_len);
     const uint32_t t_end = min(t_begin + chunk, kv_len);
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
         const uint32_t lp = (stage * STAGE_TOK) >> page_shift;  // page is a power of two (checked on the host)
         uint32_t pp = 0;
         if (lp < table_len) {
-            pp = __ldg(page_table + lp);
+            pp = ld_global(page_table + lp);
         } else {
             report_error(status, DEV_ERR_BOUNDS, 302, lp, table_len);
         }
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
             for (int cc = 0; cc < 2; cc++) {
                 const int c = 2 * b + cc;
                 uint2 w = make_uint2(0u, 0u);
-                if (q_live) w = __ldg(reinterpret_cast<const uint2*>(qrow + 16 * c + 4 * t4));
+                if (q_live) w = ld_global(reinterpret_cast<const uint2*>(qrow + 16 * c + 4 * t4));
                 qb[c][0] = w.x;
                 qb[c][1] = w.y;
                 const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&w.x));
@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
         }
     }
 
-    if (__any_sync(0xffffffffu, failed)) let_copies_land();  // into this warp's ring, which is written next
+    if (failed) let_copies_land();  // into this warp's ring, which is written next
 
     // ---- remove the +1152 offsets, total the denominators --------------------------------------------
 #pragma unroll

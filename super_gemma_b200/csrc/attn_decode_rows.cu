@@ -278,7 +278,7 @@ __device__ __forceinline__ void stage_queries(uint8_t* q_sm, int live, RowPtr ro
     for (int i = threadIdx.x; i < 8 * HD / 8; i += blockDim.x) {
         const int r = i / (HD / 8), c = i % (HD / 8);
         uint4 u = make_uint4(0u, 0u, 0u, 0u);
-        if (r < live) u = __ldg(reinterpret_cast<const uint4*>(row_ptr(r)) + c);
+        if (r < live) u = ld_global(reinterpret_cast<const uint4*>(row_ptr(r)) + c);
         *reinterpret_cast<uint4*>(q_sm + r * Q_PITCH + 16 * c) = u;
     }
 }
@@ -294,8 +294,8 @@ struct DecodeRowsSmem {
 template <int HD, int G, bool KQ8, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, HD == 512 ? 1 : HD == 256 ? 3 : 6)  // CTAs that the slots let an SM hold
     decode_rows_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_sc, const __grid_constant__ CUtensorMap tm_v,
-                       const __half* __restrict__ q, const __grid_constant__ KvOperand kop, const __grid_constant__ KvOperand vop,
-                       float* __restrict__ part, const uint32_t* __restrict__ step, int step_slot, uint32_t n_splits, float scale, uint32_t* status)
+                       const __half* q, const __grid_constant__ KvOperand kop, const __grid_constant__ KvOperand vop,
+                       float* __restrict__ part, const uint32_t* step, int step_slot, uint32_t n_splits, float scale, uint32_t* status)
 {
     using W = RowsWarp<HD, KQ8, G>;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(WARPS * 32, HD == 512 ? 1 : HD == 256 ? 3 : 6)
     if (threadIdx.x == 0) sm.redo = 0;
     pdl_wait();
     pdl_launch_dependents();
-    const uint32_t kv_len = __ldg(step + step_slot);
+    const uint32_t kv_len = ld_global(step + step_slot);
     const uint32_t chunk = (kv_len + n_splits - 1) / n_splits;
     const uint32_t t_begin = min((uint32_t)split * chunk, kv_len);
     uint32_t t_end = min(t_begin + chunk, kv_len);
@@ -409,9 +409,9 @@ __device__ __forceinline__ void cluster_sync()
 
 __global__ void __cluster_dims__(V_CTAS, 1, 1) __launch_bounds__(V_WARPS * 32)
     verify_ring_kernel(const __grid_constant__ CUtensorMap tm_kr, const __grid_constant__ CUtensorMap tm_vr, const __grid_constant__ CUtensorMap tm_kn,
-                       const __grid_constant__ CUtensorMap tm_vn, const __half* __restrict__ q, const __grid_constant__ KvOperand k_ring, const __grid_constant__ KvOperand v_ring,
+                       const __grid_constant__ CUtensorMap tm_vn, const __half* q, const __grid_constant__ KvOperand k_ring, const __grid_constant__ KvOperand v_ring,
                        const __grid_constant__ KvOperand k_new, const __grid_constant__ KvOperand v_new, float* __restrict__ out,
-                       const uint32_t* __restrict__ step, uint32_t n_kv, uint32_t m_q, uint32_t window, uint32_t ring, float scale, uint32_t* status)
+                       const uint32_t* step, uint32_t n_kv, uint32_t m_q, uint32_t window, uint32_t ring, float scale, uint32_t* status)
 {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     VerifySmem& sm = *reinterpret_cast<VerifySmem*>(smem_raw);
@@ -428,7 +428,7 @@ __global__ void __cluster_dims__(V_CTAS, 1, 1) __launch_bounds__(V_WARPS * 32)
     }
     pdl_wait();
     pdl_launch_dependents();
-    const int64_t q0 = __ldg(step + STEP_Q0);
+    const int64_t q0 = ld_global(step + STEP_Q0);
     const int64_t band_lo = q0 + 1 > window ? q0 + 1 - window : 0;  // the first query's
     const int64_t first = band_lo / TILE * TILE;
     const int n_hist = q0 > band_lo ? (int)((q0 - 1) / TILE - first / TILE + 1) : 0, tiles = n_hist + 1;  // the draft is one tile

@@ -51,9 +51,9 @@ __device__ __forceinline__ void merge_warps(Stream<G, DPL>& st, float* sm_acc, f
 // Split-K decode partials.  Grid (kv head, split, query token); the reference's grid is the first
 // two (attn_decode_sliding.wgsl:53-62).  part row = i * H + qh.
 template <int HD, int G, int KFMT, int VFMT>
-__global__ void __launch_bounds__(GEN_THREADS) decode_generic_kernel(const __half* __restrict__ q, KvOperand kop, KvOperand vop,
+__global__ void __launch_bounds__(GEN_THREADS) decode_generic_kernel(const __half* q, KvOperand kop, KvOperand vop,
                                                                      float* __restrict__ part,
-                                                                     const uint32_t* __restrict__ step, int step_slot,
+                                                                     const uint32_t* step, int step_slot,
                                                                      uint32_t n_splits, float scale, uint32_t* status)
 {
     constexpr int DPL = HD / 32;
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(GEN_THREADS) decode_generic_kernel(const __hal
 constexpr int REDUCE_MAX_SPLITS = 1024;
 
 template <int HD, int OUT_MODE>
-__global__ void __launch_bounds__(HD / 2) reduce_kernel(const float* __restrict__ part, void* __restrict__ out, uint32_t n_splits,
+__global__ void __launch_bounds__(HD / 2) reduce_kernel(const float* part, void* __restrict__ out, uint32_t n_splits,
                                                        int split_major)
 {
     const size_t row = blockIdx.x, rows = gridDim.x;
@@ -139,10 +139,10 @@ __global__ void __launch_bounds__(HD / 2) reduce_kernel(const float* __restrict_
 // QFMT = FMT_Q8: q holds int8 quants [M x H x HD] with f16 scales q_scales [M x H x HD/32]
 // (attn_prefill_global_flash_sp_iq.wgsl:24-25).
 template <int HD, int G, int KFMT, int VFMT, int TWO_RANGE, int OUT_F32, int QFMT = FMT_F16>
-__global__ void __launch_bounds__(GEN_THREADS) prefill_generic_kernel(const void* __restrict__ q, const __half* __restrict__ q_scales,
+__global__ void __launch_bounds__(GEN_THREADS) prefill_generic_kernel(const void* q, const __half* q_scales,
                                                                       KvOperand k_hist, KvOperand v_hist, KvOperand k_chunk,
                                                                       KvOperand v_chunk, void* __restrict__ out,
-                                                                      const uint32_t* __restrict__ step, uint32_t window,
+                                                                      const uint32_t* step, uint32_t window,
                                                                       uint32_t ring, float scale, uint32_t* status)
 {
     constexpr int DPL = HD / 32;

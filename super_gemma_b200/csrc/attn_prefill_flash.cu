@@ -449,7 +449,7 @@ __global__ void __launch_bounds__(FLASH_THREADS, 2) flash_prefill_kernel(const _
 // Merge the pieces of every row: out = sum_p 2^(m_p - M) O_p / sum_p 2^(m_p - M) l_p, pieces in index
 // order (fixed order => bit-identical reruns).  One warp per row, lane = 4 dims.
 constexpr int MAX_PIECES = 16;
-__global__ void __launch_bounds__(256) combine_pieces_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
+__global__ void __launch_bounds__(256) combine_pieces_kernel(const float* part_acc, const float* part_ml,
                                                              float* __restrict__ out, uint32_t rows, uint32_t pieces)
 {
     pdl_wait();  // the partials come from the kernel before this one

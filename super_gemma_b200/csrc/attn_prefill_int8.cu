@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
             const int r = i >> 4, b = i & 15;
             const uint32_t tok = m0 + r / G;
             float s = 0.0f;
-            if (tok < prm.m_tokens) s = __half2float(__ldg(prm.q_scales + ((size_t)tok * (prm.n_kv * G) + kvh * G + r % G) * 16 + b));
+            if (tok < prm.m_tokens) s = __half2float(ld_global(prm.q_scales + ((size_t)tok * (prm.n_kv * G) + kvh * G + r % G) * 16 + b));
             sm.qs[b][r] = s;
         }
     }
@@ -329,8 +329,8 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
             ks_next[0] = ks_next[1] = make_uint4(0u, 0u, 0u, 0u);
             if ((int64_t)pos <= valid_end) {
                 const uint4* p = reinterpret_cast<const uint4*>(prm.k0.scales + (pos * prm.n_kv + kvh) * 16);
-                ks_next[0] = __ldg(p);
-                ks_next[1] = __ldg(p + 1);
+                ks_next[0] = ld_global(p);
+                ks_next[1] = ld_global(p + 1);
             }
         };
         if (n_tiles > 0) fetch_scales(0);

@@ -28,7 +28,7 @@ __device__ __forceinline__ void load_f16(const __half* p, float (&out)[DPL])
     if constexpr (DPL % 8 == 0) {
 #pragma unroll
         for (int i = 0; i < DPL / 8; i++) {
-            const uint4 u = __ldg(reinterpret_cast<const uint4*>(p) + i);
+            const uint4 u = ld_global(reinterpret_cast<const uint4*>(p) + i);
             const __half2* h = reinterpret_cast<const __half2*>(&u);
 #pragma unroll
             for (int j = 0; j < 4; j++) {
@@ -41,7 +41,7 @@ __device__ __forceinline__ void load_f16(const __half* p, float (&out)[DPL])
         static_assert(DPL % 4 == 0, "lanes own 4 or more dims");
 #pragma unroll
         for (int i = 0; i < DPL / 4; i++) {
-            const uint2 u = __ldg(reinterpret_cast<const uint2*>(p) + i);
+            const uint2 u = ld_global(reinterpret_cast<const uint2*>(p) + i);
             const __half2* h = reinterpret_cast<const __half2*>(&u);
 #pragma unroll
             for (int j = 0; j < 2; j++) {
@@ -58,10 +58,10 @@ __device__ __forceinline__ void load_f16(const __half* p, float (&out)[DPL])
 template <int DPL>
 __device__ __forceinline__ void load_q8(const int8_t* q, const __half* scales, int d0, float (&out)[DPL])
 {
-    const float s = __half2float(__ldg(scales + d0 / 32));
+    const float s = __half2float(ld_global(scales + d0 / 32));
 #pragma unroll
     for (int i = 0; i < DPL / 4; i++) {
-        const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(q) + i);
+        const uint32_t w = ld_global(reinterpret_cast<const uint32_t*>(q) + i);
         out[4 * i] = __fmul_rn(s, (float)(int8_t)(w & 0xFF));
         out[4 * i + 1] = __fmul_rn(s, (float)(int8_t)((w >> 8) & 0xFF));
         out[4 * i + 2] = __fmul_rn(s, (float)(int8_t)((w >> 16) & 0xFF));
@@ -188,18 +188,18 @@ struct RawSlice {
         if constexpr (FMT == FMT_F16 && N % 4 == 0) {
 #pragma unroll
             for (int i = 0; i < N / 4; i++) {
-                const uint4 u = __ldg(reinterpret_cast<const uint4*>(p) + i);
+                const uint4 u = ld_global(reinterpret_cast<const uint4*>(p) + i);
                 w[4 * i] = u.x, w[4 * i + 1] = u.y, w[4 * i + 2] = u.z, w[4 * i + 3] = u.w;
             }
         } else if constexpr (FMT == FMT_F16) {
 #pragma unroll
             for (int i = 0; i < N / 2; i++) {
-                const uint2 u = __ldg(reinterpret_cast<const uint2*>(p) + i);
+                const uint2 u = ld_global(reinterpret_cast<const uint2*>(p) + i);
                 w[2 * i] = u.x, w[2 * i + 1] = u.y;
             }
         } else {
 #pragma unroll
-            for (int i = 0; i < N; i++) w[i] = __ldg(reinterpret_cast<const uint32_t*>(p) + i);
+            for (int i = 0; i < N; i++) w[i] = ld_global(reinterpret_cast<const uint32_t*>(p) + i);
         }
     }
     __device__ __forceinline__ float at(int d) const
@@ -234,7 +234,7 @@ __device__ __forceinline__ void stream_keys(Stream<H, HD / 32>& st, const float 
             uint32_t row = row0 + min((uint32_t)j, end - 1 - t0);
             if (ring && row >= ring) row -= ring;
             kk[j].load(k_base + (uint64_t)row * k_pitch);
-            if constexpr (KFMT != FMT_F16) kk[j].s = __half2float(__ldg(k.scales + (uint64_t)row * s_pitch + kvh * (HD / 32) + d0 / 32));
+            if constexpr (KFMT != FMT_F16) kk[j].s = __half2float(ld_global(k.scales + (uint64_t)row * s_pitch + kvh * (HD / 32) + d0 / 32));
             vv[j].load(v_base + (uint64_t)row * v_pitch);
         }
         float s[KEYS][H];

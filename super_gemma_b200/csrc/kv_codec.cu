@@ -53,7 +53,7 @@ __device__ __forceinline__ void load_block(const __half* src, size_t blk, uint4 
 {
     const uint4* p = reinterpret_cast<const uint4*>(src + blk * 32);
 #pragma unroll
-    for (int i = 0; i < 4; i++) in[i] = __ldg(p + i);
+    for (int i = 0; i < 4; i++) in[i] = ld_global(p + i);
 }
 
 __device__ __forceinline__ void store_quants(int8_t* quants, size_t blk, const uint32_t (&packed)[8])
@@ -64,7 +64,7 @@ __device__ __forceinline__ void store_quants(int8_t* quants, size_t blk, const u
 }
 
 // kv_quant_q8 (crates/sg-gpu/shaders/kv_quant_q8.wgsl:24-57).
-__global__ void __launch_bounds__(CODEC_THREADS) kv_quant_q8_kernel(const __half* __restrict__ src,
+__global__ void __launch_bounds__(CODEC_THREADS) kv_quant_q8_kernel(const __half* src,
                                                                     __half* __restrict__ scales,
                                                                     int8_t* __restrict__ quants, size_t n_blocks)
 {
@@ -82,8 +82,8 @@ __global__ void __launch_bounds__(CODEC_THREADS) kv_quant_q8_kernel(const __half
 }
 
 // kv_dequant_q8 (crates/sg-gpu/shaders/kv_dequant_q8.wgsl:9-29): one thread per 16 values.
-__global__ void __launch_bounds__(CODEC_THREADS) kv_dequant_q8_kernel(const __half* __restrict__ scales,
-                                                                      const int8_t* __restrict__ quants,
+__global__ void __launch_bounds__(CODEC_THREADS) kv_dequant_q8_kernel(const __half* scales,
+                                                                      const int8_t* quants,
                                                                       __half* __restrict__ dst, size_t n_halfblocks)
 {
     pdl_wait();
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(CODEC_THREADS) kv_dequant_q8_kernel(const __ha
     const size_t hb = (size_t)blockIdx.x * CODEC_THREADS + threadIdx.x;
     if (hb >= n_halfblocks) return;
     const float d = __half2float(scales[hb >> 1]);
-    const uint4 qw = __ldg(reinterpret_cast<const uint4*>(quants) + hb);
+    const uint4 qw = ld_global(reinterpret_cast<const uint4*>(quants) + hb);
     const uint32_t w[4] = {qw.x, qw.y, qw.z, qw.w};
     uint32_t o[8];
 #pragma unroll
@@ -110,8 +110,8 @@ __global__ void __launch_bounds__(CODEC_THREADS) kv_dequant_q8_kernel(const __ha
 
 // kv_append (crates/sg-gpu/shaders/kv_append.wgsl:15-37): rows of ROW_LEN f16, slot from step[0].
 template <int ROW_LEN, int RING>
-__global__ void __launch_bounds__(CODEC_THREADS) kv_append_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst,
-                                                                  const uint32_t* __restrict__ step, size_t n_vec,
+__global__ void __launch_bounds__(CODEC_THREADS) kv_append_kernel(const uint4* src, uint4* __restrict__ dst,
+                                                                  const uint32_t* step, size_t n_vec,
                                                                   size_t dst_rows, uint32_t* status)
 {
     constexpr int VEC_PER_ROW = ROW_LEN / 8;
@@ -126,17 +126,17 @@ __global__ void __launch_bounds__(CODEC_THREADS) kv_append_kernel(const uint4* _
         report_error(status, DEV_ERR_BOUNDS, 101, (uint32_t)slot, (uint32_t)dst_rows);
         return;
     }
-    dst[slot * VEC_PER_ROW + j] = __ldg(src + i);
+    dst[slot * VEC_PER_ROW + j] = ld_global(src + i);
 }
 
 // kv_append_global_q8 (crates/sg-gpu/shaders/kv_append_global_q8.wgsl:19-60), plus the page-table
 // row mapping when page_table != nullptr: row = page_table[t / page] * page + t % page.
-__global__ void __launch_bounds__(CODEC_THREADS) kv_append_q8_kernel(const __half* __restrict__ src,
+__global__ void __launch_bounds__(CODEC_THREADS) kv_append_q8_kernel(const __half* src,
                                                                      __half* __restrict__ scales,
                                                                      int8_t* __restrict__ quants,
-                                                                     const uint32_t* __restrict__ page_table,
+                                                                     const uint32_t* page_table,
                                                                      uint32_t table_len, uint32_t page,
-                                                                     const uint32_t* __restrict__ step,
+                                                                     const uint32_t* step,
                                                                      uint32_t blocks_per_row, size_t n_blocks,
                                                                      size_t dst_rows, uint32_t* status)
 {
@@ -173,12 +173,12 @@ __global__ void __launch_bounds__(CODEC_THREADS) kv_append_q8_kernel(const __hal
 // the rows up to the next multiple of 64):
 // dst[t][j] = f16(scale * q) read at row page_table[t / page] * page + t % page.  The dequantised
 // value is the one attn_prefill_global_flash_sp_q8.wgsl:100-104 builds in its LDS slab.
-__global__ void __launch_bounds__(CODEC_THREADS) kv_dequant_paged_kernel(const __half* __restrict__ scales,
-                                                                         const int8_t* __restrict__ quants,
-                                                                         const uint32_t* __restrict__ page_table,
+__global__ void __launch_bounds__(CODEC_THREADS) kv_dequant_paged_kernel(const __half* scales,
+                                                                         const int8_t* quants,
+                                                                         const uint32_t* page_table,
                                                                          uint32_t table_len, uint32_t page,
                                                                          __half* __restrict__ dst,
-                                                                         const uint32_t* __restrict__ step,
+                                                                         const uint32_t* step,
                                                                          uint32_t row_len, size_t dst_rows,
                                                                          size_t src_rows, uint32_t* status)
 {
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(CODEC_THREADS) kv_dequant_paged_kernel(const _
             return;
         }
         const float d = __half2float(scales[row * (row_len / 32) + (hb >> 1)]);
-        const uint4 qw = __ldg(reinterpret_cast<const uint4*>(quants + row * row_len) + hb);
+        const uint4 qw = ld_global(reinterpret_cast<const uint4*>(quants + row * row_len) + hb);
         const uint32_t w[4] = {qw.x, qw.y, qw.z, qw.w};
         uint32_t o[8];
 #pragma unroll

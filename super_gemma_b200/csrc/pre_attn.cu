@@ -29,7 +29,7 @@ __device__ __forceinline__ void load_f16x32(const __half* p, float (&x)[32])
     const uint4* v = reinterpret_cast<const uint4*>(p);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const uint4 u = __ldg(v + i);
+        const uint4 u = ld_global(v + i);
         const __half2* h = reinterpret_cast<const __half2*>(&u);
 #pragma unroll
         for (int j = 0; j < 4; j++) {
@@ -71,19 +71,19 @@ __device__ __forceinline__ float row_inv_rms(const float (&x)[32])
 
 // y = f16(x * inv * weight) for this thread's block; PLUS_ONE: weight = 1 + w (rmsnorm.wgsl:52-58); w == nullptr: 1.
 template <bool PLUS_ONE>
-__device__ __forceinline__ void apply_norm(float (&x)[32], float inv, const float* __restrict__ w)
+__device__ __forceinline__ void apply_norm(float (&x)[32], float inv, const float* w)
 {
 #pragma unroll
     for (int i = 0; i < 32; i++) {
         float weight = 1.0f;
-        if (w != nullptr) weight = PLUS_ONE ? 1.0f + __ldg(w + i) : __ldg(w + i);
+        if (w != nullptr) weight = PLUS_ONE ? 1.0f + ld_global(w + i) : ld_global(w + i);
         x[i] = round_f16(x[i] * inv * weight);
     }
 }
 
 // rmsnorm_<ROW_LEN>[_plus1]: x f16[rows x ROW_LEN], w f32[ROW_LEN], y f16.  grid [rows].
 template <int BPR, bool PLUS_ONE>
-__global__ void __launch_bounds__(PRE_THREADS) rmsnorm_kernel(const __half* __restrict__ x, const float* __restrict__ w,
+__global__ void __launch_bounds__(PRE_THREADS) rmsnorm_kernel(const __half* x, const float* w,
                                                               __half* __restrict__ y, size_t n_blocks)
 {
     pdl_wait();
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(PRE_THREADS) rmsnorm_kernel(const __half* __re
 }
 
 // rope_*: in place over rows [token x head x head_dim], one thread per (row, live pair) (rope.wgsl:36-52).
-__global__ void __launch_bounds__(PRE_THREADS) rope_kernel(__half* __restrict__ xs, const float2* __restrict__ cos_sin,
+__global__ void __launch_bounds__(PRE_THREADS) rope_kernel(__half* __restrict__ xs, const float2* cos_sin,
                                                            uint32_t head_dim, uint32_t half_rot, uint32_t n_heads, size_t pairs_total)
 {
     pdl_wait();
@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(PRE_THREADS) rope_kernel(__half* __restrict__ 
     const size_t row = g / half_rot;
     const uint32_t pair = (uint32_t)(g % half_rot);
     const size_t token = row / n_heads;
-    const float2 cs = __ldg(cos_sin + token * half_rot + pair);
+    const float2 cs = ld_global(cos_sin + token * half_rot + pair);
     __half* lo = xs + row * head_dim + pair;
     __half* hi = lo + head_dim / 2;
     const float a = __half2float(*lo), b = __half2float(*hi);
@@ -131,12 +131,12 @@ __global__ void __launch_bounds__(PRE_THREADS) rope_kernel(__half* __restrict__ 
 // rotation partner's normalised values (dims +-64, lane o ^ 8) by shuffle.  Every lane of the warp must call
 // it (dead lanes with live = false), and half_rot must be the same for the whole warp.
 template <bool PLUS_ONE>
-__device__ __forceinline__ void norm_rope_oct_d128(const __half* __restrict__ row_ptr, const float* __restrict__ w,
-                                                    const float2* __restrict__ cs_row, uint32_t half_rot, int o, bool live,
+__device__ __forceinline__ void norm_rope_oct_d128(const __half* row_ptr, const float* w,
+                                                    const float2* cs_row, uint32_t half_rot, int o, bool live,
                                                     float (&v)[8])
 {
     if (live) {
-        const uint4 u = __ldg(reinterpret_cast<const uint4*>(row_ptr + 8 * o));
+        const uint4 u = ld_global(reinterpret_cast<const uint4*>(row_ptr + 8 * o));
         const __half2* h = reinterpret_cast<const __half2*>(&u);
 #pragma unroll
         for (int j = 0; j < 4; j++) {
@@ -158,7 +158,7 @@ __device__ __forceinline__ void norm_rope_oct_d128(const __half* __restrict__ ro
 #pragma unroll
     for (int i = 0; i < 8; i++) wv[i] = 1.0f;
     if (w != nullptr && live) {
-        const float4 w0 = __ldg(reinterpret_cast<const float4*>(w + 8 * o)), w1 = __ldg(reinterpret_cast<const float4*>(w + 8 * o) + 1);
+        const float4 w0 = ld_global(reinterpret_cast<const float4*>(w + 8 * o)), w1 = ld_global(reinterpret_cast<const float4*>(w + 8 * o) + 1);
         const float t[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
         for (int i = 0; i < 8; i++) wv[i] = PLUS_ONE ? 1.0f + t[i] : t[i];
@@ -174,7 +174,7 @@ __device__ __forceinline__ void norm_rope_oct_d128(const __half* __restrict__ ro
     const float4* cp = reinterpret_cast<const float4*>(cs_row + pair0);  // (cos, sin) pairs; 16-byte aligned: half_rot % 8 == 0
 #pragma unroll
     for (int j = 0; j < 4; j++) {  // half_rot is a multiple of 8 (checked on the host): all 8 pairs of a live piece rotate
-        const float4 cs = __ldg(cp + j);
+        const float4 cs = ld_global(cp + j);
         const float c[2] = {cs.x, cs.z}, sn[2] = {cs.y, cs.w};
 #pragma unroll
         for (int e = 0; e < 2; e++) {
@@ -199,8 +199,8 @@ __device__ __forceinline__ uint4 pack_f16x8(const float (&v)[8])
 
 // attn_norm_rope_d128: x f16[rows x 128] (rows = tokens x n_heads), w f32[128], cos_sin f32[tokens x rot/2 x 2], y f16.
 template <bool PLUS_ONE>
-__global__ void __launch_bounds__(PRE_THREADS) norm_rope_d128_kernel(const __half* __restrict__ x, const float* __restrict__ w,
-                                                                     const float2* __restrict__ cos_sin, __half* __restrict__ y,
+__global__ void __launch_bounds__(PRE_THREADS) norm_rope_d128_kernel(const __half* x, const float* w,
+                                                                     const float2* cos_sin, __half* __restrict__ y,
                                                                      uint32_t n_heads, uint32_t half_rot, uint32_t rows)
 {
     pdl_wait();
@@ -250,11 +250,11 @@ constexpr int ROWS_AHEAD = 4;  // loads of a thread under way at a time
 
 template <bool PLUS_ONE>
 __global__ void __launch_bounds__(PRE_THREADS)
-    kv_norm_rope_append_kernel(const __half* __restrict__ q_raw, const float* __restrict__ q_w, __half* __restrict__ q_out,
-                               uint32_t n_q, const __half* __restrict__ k_raw, const __half* __restrict__ v_raw, const float* __restrict__ k_w,
-                               const float2* __restrict__ cos_sin, __half* __restrict__ k_scales, int8_t* __restrict__ k_quants,
-                               __half* __restrict__ v_scales, int8_t* __restrict__ v_quants, const uint32_t* __restrict__ page_table,
-                               uint32_t table_len, uint32_t page, const uint32_t* __restrict__ step, uint32_t n_kv, uint32_t half_rot,
+    kv_norm_rope_append_kernel(const __half* q_raw, const float* q_w, __half* __restrict__ q_out,
+                               uint32_t n_q, const __half* k_raw, const __half* v_raw, const float* k_w,
+                               const float2* cos_sin, __half* __restrict__ k_scales, int8_t* __restrict__ k_quants,
+                               __half* __restrict__ v_scales, int8_t* __restrict__ v_quants, const uint32_t* page_table,
+                               uint32_t table_len, uint32_t page, const uint32_t* step, uint32_t n_kv, uint32_t half_rot,
                                size_t dst_rows, uint32_t* status)
 {
     pdl_wait();  // the raw q, k, v rows come from earlier kernels of the stream
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(PRE_THREADS)
         const float4* cp = reinterpret_cast<const float4*>(cos_sin + (size_t)token * half_rot + pair0);
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const float4 cs = __ldg(cp + j);
+            const float4 cs = ld_global(cp + j);
             c[j] = make_float2(cs.x, cs.z);
             // low half: lo*c - hi*s with lo = own; high half: hi*c + lo*s with hi = own (x - y is x + (-y), bit for bit)
             sn[j] = o < 8 ? make_float2(-cs.y, -cs.w) : make_float2(cs.y, cs.w);
@@ -278,8 +278,8 @@ __global__ void __launch_bounds__(PRE_THREADS)
     size_t dst_row = 0;
     bool placed = true;
     {
-        const uint32_t t = __ldg(step + STEP_POS) + token, p = t / page;
-        if (p < table_len) dst_row = (size_t)__ldg(page_table + p) * page + (t - p * page);
+        const uint32_t t = ld_global(step + STEP_POS) + token, p = t / page;
+        if (p < table_len) dst_row = (size_t)ld_global(page_table + p) * page + (t - p * page);
         placed = p < table_len && dst_row < dst_rows;
         if (!placed && threadIdx.x == 0 && blockIdx.y == 0) {
             if (p >= table_len)
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(PRE_THREADS)
         const __half* src = r < n_q           ? q_raw + ((size_t)token * n_q + r) * 128
                             : r < n_q + n_kv ? k_raw + ((size_t)token * n_kv + (r - n_q)) * 128
                                              : v_raw + ((size_t)token * n_kv + (r - n_q - n_kv)) * 128;
-        return __ldg(reinterpret_cast<const uint4*>(src + 8 * o));
+        return ld_global(reinterpret_cast<const uint4*>(src + 8 * o));
     };
     auto work = [&](uint32_t r0, const uint4& u) {
         const uint32_t r = r0 + slot;
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(PRE_THREADS)
         for (int j = 0; j < 4; j++) wv[j] = make_float2(1.0f, 1.0f);
         if (live && !is_v) {
             const float* w = (is_q ? q_w : k_w) + 8 * o;
-            const float4 w0 = __ldg(reinterpret_cast<const float4*>(w)), w1 = __ldg(reinterpret_cast<const float4*>(w) + 1);
+            const float4 w0 = ld_global(reinterpret_cast<const float4*>(w)), w1 = ld_global(reinterpret_cast<const float4*>(w) + 1);
             const float2 x[4] = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w), make_float2(w1.x, w1.y), make_float2(w1.z, w1.w)};
 #pragma unroll
             for (int j = 0; j < 4; j++) wv[j] = PLUS_ONE ? __fadd2_rn(make_float2(1.0f, 1.0f), x[j]) : x[j];

@@ -6,6 +6,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 namespace sgb {
 
@@ -248,6 +249,34 @@ __device__ __forceinline__ float ex2(float x)
 // soon as every CTA of this grid has called it.  Both are no-ops for a plain launch.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Loads of what an earlier kernel of the stream may have written: not ld.global.nc, whose data has to be constant for as long as the
+// kernel lives, and a kernel that starts before its predecessor has ended lives while that one still writes.  For the same
+// reason no const pointer of such a kernel is __restrict__ (the compiler turns reads through one into ld.global.nc and may
+// move them ahead of pdl_wait(); a volatile asm stays behind it).
+template <typename T>
+__device__ __forceinline__ T ld_global(const T* p)
+{
+    static_assert(sizeof(T) == 2 || sizeof(T) == 4 || sizeof(T) == 8 || sizeof(T) == 16, "one load");
+    T v;
+    if constexpr (sizeof(T) == 2) {
+        uint16_t x;
+        asm volatile("ld.global.b16 %0, [%1];" : "=h"(x) : "l"(p));
+        memcpy(&v, &x, 2);
+    } else if constexpr (sizeof(T) == 4) {
+        uint32_t x;
+        asm volatile("ld.global.b32 %0, [%1];" : "=r"(x) : "l"(p));
+        memcpy(&v, &x, 4);
+    } else if constexpr (sizeof(T) == 8) {
+        uint2 x;
+        asm volatile("ld.global.v2.b32 {%0, %1}, [%2];" : "=r"(x.x), "=r"(x.y) : "l"(p));
+        memcpy(&v, &x, 8);
+    } else {
+        uint4 x;
+        asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w) : "l"(p));
+        memcpy(&v, &x, 16);
+    }
+    return v;
+}
 // Barrier `id` (1..15; 0 is __syncthreads) over `threads` threads of the CTA, a multiple of 32.
 __device__ __forceinline__ void named_barrier_sync(uint32_t id, uint32_t threads)
 {

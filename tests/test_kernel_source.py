@@ -31,3 +31,15 @@ def test_decode_warps_stop_at_a_wait_that_ran_out():
     s = _source("attn_decode_paged.cu")
     refill = s.index("n_iter && !failed)", s.index("mbar_wait("))
     assert s.index("issue(it + NSTAGES", refill) < s.index("let_copies_land();", refill)
+
+
+def test_dependent_kernels_read_nothing_as_constant():
+    """A kernel that waits for its predecessor (pdl_wait) lives while that one still writes: no ld.global.nc, neither asked for nor
+    invited by a const __restrict__ pointer."""
+    names = sorted(n for n in os.listdir(CSRC) if n.endswith((".cu", ".cuh")))
+    dependent = [n for n in names if "pdl_wait()" in _source(n)]
+    assert len(dependent) >= 6
+    for n in names:
+        assert not re.search(r"\b__ldg\b|ld\.global\.nc", _source(n)), n
+    for n in dependent:
+        assert not re.search(r"\bconst\s+[\w ]+\*\s*__restrict__", _source(n)), n
