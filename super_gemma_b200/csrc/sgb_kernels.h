@@ -74,7 +74,9 @@ cudaError_t launch_dependent_clusters(void (*kern)(KArgs...), uint32_t cluster, 
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = cluster > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+    if (e != cudaSuccess) (void)cudaGetLastError();  // reported here, not by whichever launch asks next
+    return e;
 }
 template <typename... KArgs, typename... Args>
 cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args)

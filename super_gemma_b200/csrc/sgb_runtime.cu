@@ -48,6 +48,7 @@ int fail_validation(const LaunchArgs& a, const std::string& msg)
 int check_cuda(const LaunchArgs& a, cudaError_t e, const char* what)
 {
     if (e == cudaSuccess) return SGB_OK;
+    (void)cudaGetLastError();  // reported once
     if (a.err) *a.err = std::string(what) + ": " + cudaGetErrorString(e);
     return SGB_ERR_CUDA;
 }
@@ -244,7 +245,10 @@ struct sgb_timer {
 #define CUDA_TRY(expr, what)                                                                      \
     do {                                                                                          \
         cudaError_t e__ = (expr);                                                                 \
-        if (e__ != cudaSuccess) return set_error(SGB_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e__)); \
+        if (e__ != cudaSuccess) {                                                                 \
+            (void)cudaGetLastError(); /* reported here, not by whichever launch asks next */      \
+            return set_error(SGB_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e__));   \
+        }                                                                                         \
     } while (0)
 
 extern "C" {

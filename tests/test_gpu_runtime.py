@@ -114,3 +114,30 @@ def test_decode_splits_hint_fills_the_sms():
     assert n == sms * 16 // 32 and (16 * n * 2) % 4 == 0  # two warps per (kv head, split), 16 warps per SM
     assert ctx.decode_splits_hint(16, 2048) == 4           # at least 512 tokens per split
     assert ctx.decode_splits_hint(16, 10) == 1
+
+
+@pytest.mark.parametrize("recorded", [False, True])
+def test_a_launch_that_fails_is_reported_once(recorded):
+    """More splits than a grid has rows: the launch is refused with an error of its own, and the next dispatch, whose launcher asks
+    for the last error, does not inherit it."""
+    import super_gemma_b200 as sg
+
+    ctx = sg.GpuContext(0)
+    splits = 70000
+    k = ctx.new_buffer(16 * 256, np.uint16)
+    args = bind(ctx.new_buffer(2 * 256, np.uint16), k, k, ctx.new_buffer(2 * splits * 258, np.float32), ctx.new_step_buffer())
+    part = np.zeros((1, 4, 130), np.float32)
+    part[..., 5], part[..., 129] = 2.0, 1.0
+    gathered, out = ctx.buffer_from_iter(part), ctx.new_buffer(4 * 128, np.float32)
+
+    def run(c):
+        with pytest.raises(sg.CudaError, match="attn_decode"):
+            c.dispatch(c.load_kernel("attn_decode_sliding"), args, (splits, 0.1), [1, splits, 1])
+        c.dispatch(c.load_kernel("attn_combine_ranks_d128"), bind(gathered, out), 1, [4, 1, 1])
+
+    if recorded:
+        ctx.submit_blocking(ctx.record_graph(run))
+    else:
+        run(ctx)
+    got = out.read().reshape(4, 128)
+    assert np.all(got[:, 5] == 2.0) and np.all(np.delete(got, 5, 1) == 0)
