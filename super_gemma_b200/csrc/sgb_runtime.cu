@@ -634,10 +634,10 @@ int sgb_dispatch(sgb_ctx* c, const sgb_kernel* k, const sgb_binding* bindings, u
     LaunchArgs a{c->stream, views, push, {groups[0], groups[1], groups[2]}, c->status_dev, c->sm_count, c->device, &err,
                  &launched};
     const int r = e->fn(a);
-    if (c->recording) {
-        if (int r2 = record_after(c, &op, after)) return r2;
-    }
+    const int recorded = c->recording ? record_after(c, &op, after) : SGB_OK;
+    // the launcher's own message first: what broke the launch may have ended the capture as well
     if (r != SGB_OK) return set_error(r, err.empty() ? std::string(e->name) + " failed" : err);
+    if (recorded != SGB_OK) return recorded;
     if (c->recording) {
         c->recording_launches += launched;
         for (uint32_t i = 0; i < n_bindings; i++) {

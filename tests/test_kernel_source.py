@@ -43,3 +43,10 @@ def test_dependent_kernels_read_nothing_as_constant():
         assert not re.search(r"\b__ldg\b|ld\.global\.nc", _source(n)), n
     for n in dependent:
         assert not re.search(r"\bconst\s+[\w ]+\*\s*__restrict__", _source(n)), n
+
+
+def test_a_failed_launch_is_reported_by_its_own_message():
+    """What breaks a launch while recording can end the capture too; the launcher's message must not be lost to that."""
+    s = _source("sgb_runtime.cu")
+    body = s[s.index("e->fn(a)"):]
+    assert body.index("record_after(") < body.index("set_error(r,") < body.index("return recorded")
