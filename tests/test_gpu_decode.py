@@ -205,3 +205,23 @@ def test_bad_page_id_is_reported_not_followed(ctx):
     c.bufs[5] = ctx.buffer_from_iter(c.table)
     _, got = c.run(4)  # the context is still usable
     assert_close(got, c.want(), what="after a reported bounds error")
+
+
+@pytest.mark.parametrize("kv_len,n_splits,m_q", [(131072, 32, 4), (131072, 74, 1), (131072, 148, 1), (65536, 296, 1), (65536, 592, 1), (65536, 1000, 1),
+                                                 (65536, 1, 1)])  # on 148 SMs: 32, 16, 8, 4, 2 and 1 warps per split, and one split of 32
+def test_every_stage_counts_once(ctx, kv_len, n_splits, m_q):
+    """All scores equal, and the value of the 16-token stage i is 1 in dim i % 128: a dim's result is 64 stages' worth (32 at 65536), so
+    one stage too few or twice, let alone a page, moves it by 1/64.  Normal values cannot show that: their mean over so many
+    keys is as small as what a page adds to it.  Allowed: half of it."""
+    c = PagedCase(ctx, 9, kv_len, m_q=m_q, n_kv=2)
+    k = np.broadcast_to(normal_f16(10, 1, 2, D), (kv_len, 2, D))
+    v = np.zeros((kv_len, 2, D), np.float16)
+    v[np.arange(kv_len), :, (np.arange(kv_len) // 16) % D] = 1
+    kp, vp = q8_pool(k, c.table, PAGE, len(c.table) + 1, 11), q8_pool(v, c.table, PAGE, len(c.table) + 1, 12)
+    up = ctx.buffer_from_iter
+    c.bufs = [up(c.q16), up(kp.quants), up(kp.scales), up(vp.quants), up(vp.scales), up(c.table)]
+    _, got = c.run(n_splits)
+    seen = kv_len - m_q + 1 + np.arange(m_q)  # of query i; the last stage is cut short for the first queries
+    counts = np.stack([np.bincount((np.arange(s) // 16) % D, minlength=D) / s for s in seen])
+    one = vp.deq[0, 0, 0]  # 1 as Q8_0 holds it
+    assert_close(got / one, np.broadcast_to(counts[:, None, :], got.shape), 0, 1 / 128, f"kv_len={kv_len} splits={n_splits}")

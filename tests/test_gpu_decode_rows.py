@@ -148,3 +148,39 @@ def test_only_rows_that_are_not_finite_are_computed_again(ctx, kind):
     got, _, _ = _decode(ctx, kind, q, k, v, n, splits)
     assert np.all(np.isnan(got[row]))
     assert np.array_equal(got[:row].view(np.uint32), clean[:row].view(np.uint32))
+
+
+@pytest.mark.parametrize("kind", KINDS, ids=lambda k: k[0])
+@pytest.mark.parametrize("n,splits,m_q", [(50, 7, 4), (50, 7, 2), (17, 16, 3), (4, 2, 4), (200, 3, 2)])
+def test_decode_of_a_draft_is_causal(ctx, kind, n, splits, m_q):
+    """groups[2] query tokens: query i sees t <= n - m_q + i.  In (50, 7), (17, 16) and (4, 2) the last split begins between the
+    queries' last visible keys, so that it is empty for the first of them."""
+    name, red, n_kv, g, hd, q8, slot = kind
+    q, k, v = normal_f16(n, m_q, n_kv * g, hd), normal_f16(n + 1, n, n_kv, hd), normal_f16(n + 2, n, n_kv, hd)
+    up = lambda b: ctx.buffer_from_iter(np.ascontiguousarray(b))
+    if q8:
+        ks, kq, kd = O.q8_quant_div(k.astype(np.float32).ravel())
+        bufs = [up(kq), up(ks)]
+    else:
+        kd, bufs = k.astype(np.float32), [up(k)]
+    rows = m_q * n_kv * g
+    part, out = ctx.new_buffer(rows * splits * (hd + 2), np.float32), ctx.new_buffer(rows * hd, np.float32 if "f32" in red else np.uint16)
+    ctx.dispatch(ctx.load_kernel(name), bind(up(q), *bufs, up(v), part, _step(ctx, **{slot: n})), (splits, hd**-0.5), [n_kv, splits, m_q])
+    ctx.dispatch_blocking(ctx.load_kernel(red), bind(part, out), splits, [rows, 1, 1])
+    got = out.read() if "f32" in red else O.f16_bits_to_f32(out.read())
+    want = O.attention_f64(q.astype(np.float32), kd.reshape(k.shape), v.astype(np.float32), m_q, n - m_q, n_kv * g, n_kv, hd, hd**-0.5)
+    assert_close(got.reshape(want.shape), want, ATOL, 1e-5 if "f32" in red else 2.0**-11, name)
+
+
+@pytest.mark.parametrize("kind", KINDS[1:3], ids=lambda k: k[0])
+@pytest.mark.parametrize("splits", [1, 32])
+def test_every_tile_counts_once(ctx, kind, splits):
+    """All scores equal, and the value of tile i is 1 in dim i % 512: over 32768 keys a dim's result is 4 tiles' worth, and one tile
+    too few or twice is a quarter of it (allowed: the weights' f32 sums and the output's f16)."""
+    _, _, n_kv, g, hd, _, _ = kind
+    n = 32768
+    q, _, _ = _case(kind, 3, 1)
+    k, v = np.broadcast_to(normal_f16(4, 1, n_kv, hd), (n, n_kv, hd)), np.zeros((n, n_kv, hd), np.float16)
+    v[np.arange(n), :, (np.arange(n) // 16) % hd] = 1
+    got, _, _ = _decode(ctx, kind, q, k, v, n, splits)
+    assert_close(got, np.full_like(got, 1 / hd), 0, 2.0**-11 + 1e-5, "equal weights")

@@ -193,3 +193,38 @@ def test_one_launch_qkv_equals_the_two_kernels(ctx, tokens, n_kv):
     for x, y in zip(a, b):
         assert np.array_equal(x.read(), y.read())
     assert np.any(a[1].read() != 0)
+
+
+@pytest.mark.parametrize("tokens,n_kv", [(295, 4), (296, 4), (700, 16), (301, 1)])
+def test_one_launch_qkv_of_a_long_chunk(ctx, tokens, n_kv):
+    """From two tokens per SM on a block takes one token and walks its rows in several passes (296 on 148 SMs): the bits of
+    attn_norm_rope_d128 on q and on k and v, then kv_append_paged_q8_d128."""
+    import super_gemma_b200 as sg
+
+    n_q, page, rot, pos = 2 * n_kv, 64, 128, 70
+    pages = -(-(pos + tokens) // page)
+    row, rows = n_kv * 128, (pages + 1) * page
+    rng = np.random.default_rng(tokens)
+    q_raw, k_raw, v_raw = (rng.standard_normal(tokens * h * 128, dtype=np.float32).astype(np.float16) for h in (n_q, n_kv, n_kv))
+    q_w, k_w = rng.standard_normal(128, dtype=np.float32), rng.standard_normal(128, dtype=np.float32)
+    cs = O.cos_sin_table(O.inv_freqs(rot, 1e6), pos, tokens)
+    up = ctx.buffer_from_iter
+    qr, kr, vr, qw, kw, csb = up(q_raw), up(k_raw), up(v_raw), up(q_w), up(k_w), up(cs)
+    table = up(np.random.default_rng(7).permutation(pages + 1)[:pages].astype(np.uint32))
+    step = ctx.new_step_buffer()
+    sg.StepState(pos=pos).write_to(step)
+    mk = lambda dt, n: ctx.new_buffer(n, dt)
+    a, b = ([mk(np.uint16, rows * row // 32), mk(np.int8, rows * row), mk(np.uint16, rows * row // 32), mk(np.int8, rows * row)] for _ in range(2))
+    q1, q2 = mk(np.uint16, tokens * n_q * 128), mk(np.uint16, tokens * n_q * 128)
+    ctx.dispatch_blocking(ctx.load_kernel("qkv_norm_rope_append_paged_q8_d128"), bind(qr, qw, q1, kr, vr, kw, csb, *a, table, step),
+                          (n_q, row, page, rot, 0), [1, 1, 1])
+    nr, app = ctx.load_kernel("attn_norm_rope_d128"), ctx.load_kernel("kv_append_paged_q8_d128")
+    k16, v16, ones = mk(np.uint16, tokens * row), mk(np.uint16, tokens * row), up(np.ones(128, np.float32))
+    ctx.dispatch(nr, bind(qr, qw, csb, q2), (n_q, rot, 0), [1, 1, 1])
+    ctx.dispatch(nr, bind(kr, kw, csb, k16), (n_kv, rot, 0), [1, 1, 1])
+    ctx.dispatch(nr, bind(vr, ones, csb, v16), (n_kv, 0, 0), [1, 1, 1])
+    ctx.dispatch(app, bind(k16, b[0], b[1], table, step), (row, page), app.groups_for(tokens * row // 32))
+    ctx.dispatch_blocking(app, bind(v16, b[2], b[3], table, step), (row, page), app.groups_for(tokens * row // 32))
+    assert np.array_equal(q1.read(), q2.read()) and np.any(q1.read() != 0)
+    for x, y in zip(a, b):
+        assert np.array_equal(x.read(), y.read()) and np.any(x.read() != 0)
