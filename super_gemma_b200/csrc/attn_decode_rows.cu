@@ -94,6 +94,7 @@ struct RowsWarp {
 
     float o[HD / 16][4];  // dims 16c + g, 16c + g + 8 x rows 2*t4, 2*t4 + 1
     float m[2], l[2];
+    uint32_t odd;  // rows with an infinite Q8_0 scale among their keys, as far as this lane saw
 
     // All tiles of this warp.  n tiles; tile(i, KeyTile&) describes the i-th.  row_lo/row_hi: positions rows 2*t4 + e may see.
     // q_sm: [8][q_pitch] f16 query rows.
@@ -124,6 +125,7 @@ struct RowsWarp {
         for (int c = 0; c < HD / 16; c++) o[c][0] = o[c][1] = o[c][2] = o[c][3] = 0.0f;
         m[0] = m[1] = NEG_SENTINEL;
         l[0] = l[1] = 0.0f;
+        odd = 0;
         bool failed = false;
         if (n > 0) {
             issue_k(0);
@@ -194,7 +196,11 @@ struct RowsWarp {
                 s[e] *= scale;
                 const int key = g + 8 * (e >> 1);
                 const int64_t pos = t.pos0 + key;
-                if (key < t.from || key >= t.to || pos < row_lo[e & 1] || pos > row_hi[e & 1]) s[e] = -INFINITY;
+                const bool seen = key >= t.from && key < t.to && pos >= row_lo[e & 1] && pos <= row_hi[e & 1];
+                // Finite scales cannot give it.  An infinite one times a whole sum that is negative would pass as a weight of 0; the
+                // statement multiplies the scale with every quant, and infinities of both signs make a NaN.
+                if (KQ8 && seen && s[e] == -INFINITY) odd |= 1u << (2 * t4 + (e & 1));
+                if (!seen) s[e] = -INFINITY;
             }
             float p[4];
             const float n0 = fmaxf(m[0], key_max(fmaxf(s[0], s[2]))), n1 = fmaxf(m[1], key_max(fmaxf(s[1], s[3])));
@@ -344,7 +350,7 @@ __global__ void __launch_bounds__(WARPS * 32, HD == 512 ? 1 : HD == 256 ? 3 : 6)
           },
           sm.q, kvh, scale, lo, hi, status);
     __syncthreads();
-    uint32_t odd = 0;
+    uint32_t odd = KQ8 ? w.odd : 0;
     for (int idx = threadIdx.x; idx < G * HD; idx += WARPS * 32) {
         const int r = idx / HD, d = idx % HD;
         float big = sm.w[0].m[r];

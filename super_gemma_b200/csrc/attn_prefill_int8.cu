@@ -21,7 +21,7 @@
 // Another block comes first in each tile's products, so that it can be settled while the tensor pipe is at the others.  Errors since:
 // 2.0762e-4 and 2.0773e-4 (streaming kernel: 2.0762e-4, 2.0774e-4), for 23 us of 533 at 8192 keys; all four blocks in every
 // fourth tile, with the tensor pipe waiting, took 44.
-// Roles: warps 0-7 softmax (two threads per key, 32 rows each), one MMA thread, one K and one V loader thread; mbarriers only.
+// Roles: warps 0-7 softmax (two threads per key, 32 rows each), one MMA thread, one K and one V loader; mbarriers only.
 // The row maximum over keys runs across threads; it is only computed (32 values in 31 shuffles) when some score exceeds its
 // row's running maximum by 2^8, which one barrier with an OR finds out.
 // Measured: 256 queries at 7936 + 256 keys 13500 us on the streaming kernel, 533 here (floor 86).  Two things bound it: V as the
@@ -220,9 +220,22 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
         }
     } else if (warp == V_W) {
         // ======================= V loads in units of 64 keys x 128 dims =======================
+        // It also looks at the scales of K.  An infinite one times a whole sum that is negative would pass as a weight of 0; the
+        // statement multiplies it with every quant, and infinities of both signs make a NaN.  A key with such a scale sends all
+        // rows to that statement.  (The softmax threads, which hold the scales anyway, took 5 us of 530 for it.)
+        uint32_t sc_top = 0;  // largest magnitudes as f16 bits, two at a time: from 0x7C00 on, not finite
         int n = 0;
         for (int j = 0; j < n_tiles && !failed; ++j) {
             const int64_t pos0 = (int64_t)j * TILE_K;
+            uint4 sc[8];  // used at the end of the tile
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int64_t pos = pos0 + 32 * i + lane;
+                const uint4* p = reinterpret_cast<const uint4*>(prm.k0.scales + ((size_t)pos * prm.n_kv + kvh) * 16);
+                const bool key = pos <= min(end, valid_end);
+                sc[2 * i] = key ? ld_global(p) : make_uint4(0u, 0u, 0u, 0u);
+                sc[2 * i + 1] = key ? ld_global(p + 1) : make_uint4(0u, 0u, 0u, 0u);
+            }
             const bool tail = pos0 + TILE_K - 1 > valid_end;  // the MMA warp computes the same
             for (int u = 0; u < UNITS; u++, n++) {
                 const int st = n % NV;
@@ -250,7 +263,10 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
                     if (lane == 0) mbar_arrive(&sm.v_ok[st]);
                 }
             }
+#pragma unroll
+            for (int i = 0; i < 32; i++) sc_top = __vmaxu2(sc_top, reinterpret_cast<const uint32_t*>(sc)[i] & 0x7FFF7FFFu);
         }
+        if ((sc_top & 0xFFFFu) >= 0x7C00u || (sc_top >> 16) >= 0x7C00u) sm.redo[0] = sm.redo[1] = 0xFFFFFFFFu;
     } else if (warp == MMA_W) {
         // ======================= MMA issue =======================
         if (lane == 0) {
@@ -556,7 +572,9 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
             tc_wait_st();
             named_barrier_sync(2, SOFT_THREADS);
         }
-        uint32_t odd = 0;
+        uint32_t odd = 0;  // also a row with a scale of Q that is not finite (see the V loader)
+        for (int b = 4 * kq; b < 4 * kq + 4; b++)
+            if (!(fabsf(sm.qs[b][32 * half + lane]) <= 65504.0f)) odd |= 1u << lane;
 #pragma unroll 1
         for (int db = 0; db < DB; db++) {
             uint32_t o[32];

@@ -35,7 +35,7 @@ def _step(ctx, **kw):
     return s
 
 
-def _decode(ctx, kind, q, k, v, n, splits, rows=None):
+def _decode(ctx, kind, q, k, v, n, splits, rows=None, k_scale=None):
     name, red, n_kv, g, hd, q8, slot = kind
     up = lambda b: ctx.buffer_from_iter(np.ascontiguousarray(b))
     junk = np.full((37, n_kv, hd), NAN16, np.uint16)
@@ -43,6 +43,9 @@ def _decode(ctx, kind, q, k, v, n, splits, rows=None):
     if q8:
         ks, kq, kd = O.q8_quant_div(k.astype(np.float32).ravel())
         kd = kd.reshape(k.shape)
+        if k_scale is not None:
+            ks = ks.copy()
+            ks.view(np.uint16)[k_scale] = 0x7C00
         pad = lambda x, w, fill: up(np.concatenate([x.reshape(n, w), np.full((37, w), fill, x.dtype)])[:rows])
         bufs = [pad(kq, n_kv * hd, 99), pad(ks.view(np.uint16), n_kv * hd // 32, NAN16)]
     else:
@@ -184,3 +187,14 @@ def test_every_tile_counts_once(ctx, kind, splits):
     v[np.arange(n), :, (np.arange(n) // 16) % hd] = 1
     got, _, _ = _decode(ctx, kind, q, k, v, n, splits)
     assert_close(got, np.full_like(got, 1 / hd), 0, 2.0**-11 + 1e-5, "equal weights")
+
+
+def test_decode_infinite_scale_of_a_key(ctx):
+    """The statement multiplies the scale with every quant: infinities of both signs, NaN for every head of that kv head."""
+    n = 300
+    q, k, v = _case(KINDS[2], 95, n)
+    clean, _, _ = _decode(ctx, KINDS[2], q, k, v, n, 3)
+    got, _, _ = _decode(ctx, KINDS[2], q, k, v, n, 3, k_scale=(170 * 4 + 1) * 16 + 9)
+    assert np.all(np.isnan(got[8:16]))
+    got[8:16] = clean[8:16]
+    assert np.array_equal(got.view(np.uint32), clean.view(np.uint32))

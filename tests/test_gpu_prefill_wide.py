@@ -85,12 +85,15 @@ def test_sliding_ring_wrapped(ctx, q0, m):
     assert_close(got[toks], want, ATOL, RTOL, f"wrapped q0={q0} m={m}")
 
 
-def _iq(ctx, q, k, v, q0, m, scale=0.044194174, pad=80, v_bits=None, poison=None):
+def _iq(ctx, q, k, v, q0, m, scale=0.044194174, pad=80, v_bits=None, poison=None, k_scale=None):
     qs, qq, qd = O.q8_quant_div(q.ravel())
     if poison is not None:  # a scale of q
         qs = qs.copy()
         qs.view(np.uint16)[poison] = NAN16
     ks, kq, kd = O.q8_quant_div(k.ravel())
+    if k_scale is not None:  # an infinite scale of K
+        ks = ks.copy()
+        ks.view(np.uint16)[k_scale] = 0x7C00
     up = lambda b: ctx.buffer_from_iter(np.ascontiguousarray(b))
     tail = np.full(pad * 2048, NAN16, np.uint16)
     bufs = [up(qq), up(qs), up(np.concatenate([kq, np.full(pad * 2048, 77, np.int8)])),
@@ -241,3 +244,16 @@ def test_global_int8_value_that_everybody_sees(ctx):
     assert np.all(got[:, 24:, 500] == -np.inf)
     got[:, 24:, 500] = clean[:, 24:, 500]
     assert_close(got, clean, ATOL, 2 * RTOL, "everything else")
+
+
+def test_global_int8_infinite_scale_of_a_key(ctx):
+    """The statement multiplies the scale with every quant: infinities of both signs, NaN for every row that sees the key, also where
+    the block's whole sum is negative."""
+    m, q0 = 32, 200
+    q, k, v = _normal(61, m, 32, 512), _normal(62, q0 + m, 4, 512), _normal(63, q0 + m, 4, 512)
+    clean, _, _ = _iq(ctx, q, k, v, q0, m)
+    got, _, _ = _iq(ctx, q, k, v, q0, m, k_scale=((q0 + 13) * 4 + 2) * 16 + 5)  # seen by queries 13 and later, kv head 2
+    assert np.all(np.isnan(got[13:, 16:24]))
+    assert_close(got[:13], clean[:13], ATOL, 2 * RTOL, "queries before it")
+    assert np.array_equal(got[:, :16].view(np.uint32), clean[:, :16].view(np.uint32))
+    assert np.array_equal(got[:, 24:].view(np.uint32), clean[:, 24:].view(np.uint32))
