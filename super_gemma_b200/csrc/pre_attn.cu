@@ -240,27 +240,32 @@ __device__ __forceinline__ void quant_oct_f32(const float2 (&x)[4], __half& scal
 // row page_table[t / page] * page + t % page with t = step[0] + token; and, for qkv_norm_rope_append_paged_q8_d128, Q rows
 // (norm with q_w, rope, f16 out): the whole pre-attention step of a layer in one launch.
 //
-// A block works on one token (blockIdx.x) and, of that token's rows (q heads, k heads, v heads in this order), on every
-// gridDim.y-th group of ROWS_PER_PASS: a thread keeps its octet of dims for all of them, so the token's cos/sin values and the
-// page lookup are read once and stay in registers instead of once per row (they were four times the bytes of a row's own
-// octet, and made the kernel issue-bound).  The launcher gives a long chunk one block per token and a short one as
-// many blocks per token as there are groups, where latency counts.
-constexpr int ROWS_PER_PASS = PRE_THREADS / 16;
+// 2^slot_bits groups of 16 lanes (and gridDim.y times as many) share the rows of a token (q heads, k heads, v heads in this order),
+// one row of 16 bytes a lane at a time: a thread keeps its octet of dims for all of its rows, so the token's cos/sin values and
+// the page lookup are read once and stay in registers instead of once per row (they were four times the bytes of a row's own
+// octet, and made the kernel issue-bound).  What the launcher chooses is at append_shape.
+constexpr int APPEND_THREADS = 128;
+constexpr int MOST_SLOTS = 16;  // groups per token and grid row
 constexpr int ROWS_AHEAD = 4;  // loads of a thread under way at a time
 
 template <bool PLUS_ONE>
-__global__ void __launch_bounds__(PRE_THREADS)
+__global__ void __launch_bounds__(APPEND_THREADS, 8)
     kv_norm_rope_append_kernel(const __half* q_raw, const float* q_w, __half* __restrict__ q_out,
                                uint32_t n_q, const __half* k_raw, const __half* v_raw, const float* k_w,
                                const float2* cos_sin, __half* __restrict__ k_scales, int8_t* __restrict__ k_quants,
                                __half* __restrict__ v_scales, int8_t* __restrict__ v_quants, const uint32_t* page_table,
                                uint32_t table_len, uint32_t page, const uint32_t* step, uint32_t n_kv, uint32_t half_rot,
-                               size_t dst_rows, uint32_t* status)
+                               size_t dst_rows, uint32_t tokens, uint32_t slot_bits, uint32_t* status)
 {
     pdl_wait();  // the raw q, k, v rows come from earlier kernels of the stream
     pdl_launch_dependents();
-    const uint32_t token = blockIdx.x, rows = n_q + 2 * n_kv;
-    const int o = threadIdx.x & 15, slot = threadIdx.x >> 4;
+    const int o = threadIdx.x & 15;
+    const uint32_t rows = n_q + 2 * n_kv, group = blockIdx.x * (APPEND_THREADS / 16) + (threadIdx.x >> 4);
+    uint32_t token = group >> slot_bits, slot = group & ((1u << slot_bits) - 1);
+    if (token >= tokens) {  // behind the last token: no row of the first
+        token = 0;
+        slot = rows;
+    }
     // rotation: dims [8 o, 8 o + 8) pair with +-64; half_rot is a multiple of 8 (checked on the host), so a whole octet turns or none
     const uint32_t pair0 = (uint32_t)(o & 7) * 8;
     const bool turns = pair0 < half_rot;
@@ -281,7 +286,7 @@ __global__ void __launch_bounds__(PRE_THREADS)
         const uint32_t t = ld_global(step + STEP_POS) + token, p = t / page;
         if (p < table_len) dst_row = (size_t)ld_global(page_table + p) * page + (t - p * page);
         placed = p < table_len && dst_row < dst_rows;
-        if (!placed && threadIdx.x == 0 && blockIdx.y == 0) {
+        if (!placed && slot == 0 && o == 0 && blockIdx.y == 0) {
             if (p >= table_len)
                 report_error(status, DEV_ERR_BOUNDS, 104, p, table_len);
             else
@@ -340,8 +345,8 @@ __global__ void __launch_bounds__(PRE_THREADS)
                 v[j] = __half22float2(*reinterpret_cast<const __half2*>(&own[j]));
             }
         }
-        if (r0 + ROWS_PER_PASS <= n_q) {  // only q rows in this pass (uniform over the block)
-            *reinterpret_cast<uint4*>(q_out + ((size_t)token * n_q + head) * 128 + 8 * o) = make_uint4(own[0], own[1], own[2], own[3]);
+        if (r0 + (1u << slot_bits) <= n_q) {  // only q rows in this pass (uniform over the block)
+            if (live) *reinterpret_cast<uint4*>(q_out + ((size_t)token * n_q + head) * 128 + 8 * o) = make_uint4(own[0], own[1], own[2], own[3]);
             return;
         }
         __half s;
@@ -356,8 +361,8 @@ __global__ void __launch_bounds__(PRE_THREADS)
             *reinterpret_cast<uint2*>((is_v ? v_quants : k_quants) + drow * 128 + 8 * o) = packed;
         }
     };
-    const uint32_t stride = gridDim.y * ROWS_PER_PASS;
-    for (uint32_t base = blockIdx.y * ROWS_PER_PASS; base < rows; base += ROWS_AHEAD * stride) {
+    const uint32_t stride = gridDim.y << slot_bits;
+    for (uint32_t base = blockIdx.y << slot_bits; base < rows; base += ROWS_AHEAD * stride) {
         uint4 u[ROWS_AHEAD];
 #pragma unroll
         for (int k = 0; k < ROWS_AHEAD; k++) u[k] = octet(base + k * stride + slot);
@@ -369,11 +374,23 @@ __global__ void __launch_bounds__(PRE_THREADS)
     }
 }
 
-// Blocks per token: one for chunks that fill the GPU by themselves (two 256-thread blocks per SM and more), else one per group of rows.
-inline dim3 append_grid(const LaunchArgs& a, size_t tokens, uint32_t rows)
+struct AppendShape {
+    dim3 grid;
+    uint32_t slot_bits;
+};
+// Slots and blocks.  While all rows of the launch can be under way at once (64 a SM: eight blocks of eight groups), one row
+// per group, which takes least time for one; beyond, ROWS_AHEAD of them, which takes least instructions per row, so few rows
+// (few kv heads) put several tokens into a block.  us in a recorded chain, 1 row | 4 rows: 16 kv heads with q, 64 tokens
+// 2.7 | 3.7, 290 tokens 6.0 | 4.7, 4096 tokens 63 | 39; 4 kv heads without q, 1000 tokens 3.7 | 4.5, 2000 tokens 5.9 | 5.1,
+// 8192 tokens 17.3 | 11.7 (a block per token whatever its rows: 33).  Blocks of 256 threads: 41 where these take 39.
+inline AppendShape append_shape(const LaunchArgs& a, size_t tokens, uint32_t rows)
 {
-    const uint32_t groups = min(1024u, (rows + ROWS_PER_PASS - 1) / ROWS_PER_PASS);
-    return dim3((uint32_t)tokens, tokens >= 2 * (size_t)a.sm_count ? 1 : groups);
+    const uint32_t per_thread = tokens * rows <= (size_t)64 * a.sm_count ? 1 : ROWS_AHEAD;
+    uint32_t bits = 0;
+    while ((1u << bits) < MOST_SLOTS && (per_thread << bits) < rows) bits++;
+    const size_t groups = tokens << bits;  // < 2^29: at most 2^26 rows of q and of k
+    const uint32_t per_token = (rows + (1u << bits) - 1) >> bits;
+    return {dim3((uint32_t)((groups * 16 + APPEND_THREADS - 1) / APPEND_THREADS), per_thread == 1 ? min(1024u, per_token) : 1), bits};
 }
 
 inline uint32_t grid_for(size_t n) { return (uint32_t)((n + PRE_THREADS - 1) / PRE_THREADS); }
@@ -468,11 +485,12 @@ int launch_kv_norm_rope_append_paged_q8_d128(const LaunchArgs& a)
     if (kv_rows >= (1u << 26)) return fail_validation(a, "kv_norm_rope_append_paged_q8_d128: at most 2^26 (token, head) rows per launch");
     if (int r = need_aligned(a, {16, 16, 16, 16, 2, 8, 2, 8, 4, 4})) return r;
     auto kern = p.plus_one ? kv_norm_rope_append_kernel<true> : kv_norm_rope_append_kernel<false>;
-    const cudaError_t e = launch_dependent(kern, append_grid(a, tokens, 2 * (p.row_len / 128)), dim3(PRE_THREADS), 0, a.stream,
+    const AppendShape shape = append_shape(a, tokens, 2 * (p.row_len / 128));
+    const cudaError_t e = launch_dependent(kern, shape.grid, dim3(APPEND_THREADS), 0, a.stream,
         nullptr, nullptr, nullptr, 0u,
         (const __half*)a.b[0].ptr, (const __half*)a.b[1].ptr, (const float*)a.b[2].ptr, (const float2*)a.b[3].ptr, (__half*)a.b[4].ptr,
         (int8_t*)a.b[5].ptr, (__half*)a.b[6].ptr, (int8_t*)a.b[7].ptr, (const uint32_t*)a.b[8].ptr, (uint32_t)(a.b[8].bytes / 4), p.page,
-        (const uint32_t*)a.b[9].ptr, p.row_len / 128, p.rot_dims / 2, dst_rows, a.status);
+        (const uint32_t*)a.b[9].ptr, p.row_len / 128, p.rot_dims / 2, dst_rows, (uint32_t)tokens, shape.slot_bits, a.status);
     ++*a.launches;
     return check_cuda(a, e, "kv_norm_rope_append_paged_q8_d128");
 }
@@ -504,11 +522,12 @@ int launch_qkv_norm_rope_append_paged_q8_d128(const LaunchArgs& a)
         return fail_validation(a, "qkv_norm_rope_append_paged_q8_d128: at most 2^26 (token, head) rows of q and of k per launch");
     if (int r = need_aligned(a, {16, 16, 16, 16, 16, 16, 16, 2, 8, 2, 8, 4, 4})) return r;
     auto kern = p.plus_one ? kv_norm_rope_append_kernel<true> : kv_norm_rope_append_kernel<false>;
-    const cudaError_t e = launch_dependent(kern, append_grid(a, tokens, p.n_q_heads + 2 * (p.row_len / 128)), dim3(PRE_THREADS), 0, a.stream,
+    const AppendShape shape = append_shape(a, tokens, p.n_q_heads + 2 * (p.row_len / 128));
+    const cudaError_t e = launch_dependent(kern, shape.grid, dim3(APPEND_THREADS), 0, a.stream,
         (const __half*)a.b[0].ptr, (const float*)a.b[1].ptr, (__half*)a.b[2].ptr, p.n_q_heads, (const __half*)kv[0].ptr,
         (const __half*)kv[1].ptr, (const float*)kv[2].ptr, (const float2*)kv[3].ptr, (__half*)kv[4].ptr, (int8_t*)kv[5].ptr,
         (__half*)kv[6].ptr, (int8_t*)kv[7].ptr, (const uint32_t*)kv[8].ptr, (uint32_t)(kv[8].bytes / 4), p.page,
-        (const uint32_t*)kv[9].ptr, p.row_len / 128, p.rot_dims / 2, dst_rows, a.status);
+        (const uint32_t*)kv[9].ptr, p.row_len / 128, p.rot_dims / 2, dst_rows, (uint32_t)tokens, shape.slot_bits, a.status);
     ++*a.launches;
     return check_cuda(a, e, "qkv_norm_rope_append_paged_q8_d128");
 }

@@ -195,10 +195,11 @@ def test_one_launch_qkv_equals_the_two_kernels(ctx, tokens, n_kv):
     assert np.any(a[1].read() != 0)
 
 
-@pytest.mark.parametrize("tokens,n_kv", [(295, 4), (296, 4), (700, 16), (301, 1)])
+@pytest.mark.parametrize("tokens,n_kv", [(295, 4), (296, 4), (592, 4), (593, 4), (700, 16), (301, 1), (2371, 1), (803, 3), (485, 5)])
 def test_one_launch_qkv_of_a_long_chunk(ctx, tokens, n_kv):
-    """From two tokens per SM on a block takes one token and walks its rows in several passes (296 on 148 SMs): the bits of
-    attn_norm_rope_d128 on q and on k and v, then kv_append_paged_q8_d128."""
+    """Beyond 64 rows per SM (592 tokens of 16 rows on 148 SMs) a thread walks several rows of its token, and few kv heads put
+    several tokens into a block, the last one short of them: the bits of attn_norm_rope_d128 on q and on k and v, then
+    kv_append_paged_q8_d128."""
     import super_gemma_b200 as sg
 
     n_q, page, rot, pos = 2 * n_kv, 64, 128, 70
