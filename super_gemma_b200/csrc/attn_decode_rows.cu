@@ -332,7 +332,14 @@ __global__ void __launch_bounds__(WARPS * 32, HD == 512 ? 1 : HD == 256 ? 3 : 6)
         if (threadIdx.x == 0) report_error(status, DEV_ERR_BOUNDS, kop.rows <= vop.rows ? 202 : 204, (uint32_t)have, (uint32_t)have);
         t_end = max((uint32_t)have, t_begin);
     }
-    const int tiles = t_end > t_begin ? (int)((t_end - t_begin + TILE - 1) / TILE) : 0;
+    if (t_end <= t_begin) {  // an empty split (a short sequence, many splits): nothing to wait for
+        for (int idx = threadIdx.x; idx < G * (HD + 2); idx += WARPS * 32) {
+            const int r = idx / (HD + 2), d = idx % (HD + 2);
+            part[(((size_t)i * n_q + kvh * G + r) * n_splits + split) * (HD + 2) + d] = d == HD ? NEG_SENTINEL : 0.0f;
+        }
+        return;
+    }
+    const int tiles = (int)((t_end - t_begin + TILE - 1) / TILE);
     auto q_row = [&](int r) { return q + ((size_t)i * n_q + kvh * G + r) * HD; };
     stage_queries<HD, KQ8>(sm.q, G, q_row);
     __syncthreads();

@@ -251,7 +251,11 @@ int launch_decode_generic(const LaunchArgs& a)
     static_assert(VFMT == FMT_F16, "the lists below name no V scales");
     constexpr uint32_t ROW = row_alignment(HD);
     if (int r = KFMT == FMT_Q8 ? need_aligned(a, {ROW, 4, 2, ROW, 4, 4}) : need_aligned(a, {ROW, ROW, ROW, 4, 4})) return r;
-    if (decode_rows_takes(kop, vop, q.ptr))
+    // The tiled kernel pays its set-up for each of the many CTAs that many splits make (us, streaming | tiled, 1024 cached tokens: head_dim
+    // 256, 16 splits 9.9 | 5.4, 32 splits 7.1 | 7.5, 256 splits 11 | 34; head_dim 128, 32 splits 6.4 | 4.1, 64 splits 5.0 | 6.3;
+    // head_dim 512, 64 splits 19 | 16, 128 splits 28 | 32; 4096 tokens, 256 splits 66 | 55).  The length is on the device, the rows are known.
+    constexpr size_t ROWS_PER_SPLIT = HD == 256 ? 64 : HD == 128 ? 32 : 16;
+    if (min(kop.rows, vop.rows) >= ROWS_PER_SPLIT * p.n_splits && decode_rows_takes(kop, vop, q.ptr))
         return launch_decode_rows<HD, G, KFMT == FMT_Q8>(a, q.ptr, kop, vop, a.b[part_i].ptr, a.b[step_i].ptr, STEP_SLOT, n_kv, p.n_splits, m_q, p.scale);
     decode_generic_kernel<HD, G, KFMT, VFMT><<<dim3(n_kv, p.n_splits, m_q), GEN_THREADS, 0, a.stream>>>(
         (const __half*)q.ptr, kop, vop, (float*)a.b[part_i].ptr, (const uint32_t*)a.b[step_i].ptr, STEP_SLOT, p.n_splits,

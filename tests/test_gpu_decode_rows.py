@@ -35,10 +35,16 @@ def _step(ctx, **kw):
     return s
 
 
+def _spare(n, splits):
+    """Rows behind the n keys: 64 per split in all, as many as the tiled kernels want."""
+    return max(37, 64 * splits - n)
+
+
 def _decode(ctx, kind, q, k, v, n, splits, rows=None, k_scale=None):
     name, red, n_kv, g, hd, q8, slot = kind
     up = lambda b: ctx.buffer_from_iter(np.ascontiguousarray(b))
-    junk = np.full((37, n_kv, hd), NAN16, np.uint16)
+    spare = _spare(n, splits)
+    junk = np.full((spare, n_kv, hd), NAN16, np.uint16)
     v_up = up(np.concatenate([v.view(np.uint16), junk])[:rows])
     if q8:
         ks, kq, kd = O.q8_quant_div(k.astype(np.float32).ravel())
@@ -46,7 +52,7 @@ def _decode(ctx, kind, q, k, v, n, splits, rows=None, k_scale=None):
         if k_scale is not None:
             ks = ks.copy()
             ks.view(np.uint16)[k_scale] = 0x7C00
-        pad = lambda x, w, fill: up(np.concatenate([x.reshape(n, w), np.full((37, w), fill, x.dtype)])[:rows])
+        pad = lambda x, w, fill: up(np.concatenate([x.reshape(n, w), np.full((spare, w), fill, x.dtype)])[:rows])
         bufs = [pad(kq, n_kv * hd, 99), pad(ks.view(np.uint16), n_kv * hd // 32, NAN16)]
     else:
         kd, bufs = k.astype(np.float32), [up(np.concatenate([k.view(np.uint16), junk])[:rows])]
@@ -73,6 +79,20 @@ def test_decode_lengths(ctx, kind, n, splits):
     assert_close(got, want, ATOL, 1e-5 if got.dtype == np.float32 and "f32" in kind[1] else 2.0**-11, f"{kind[0]} n={n} splits={splits}")
     chunk = -(-n // splits)
     empty = [s for s in range(splits) if s * chunk >= n]
+    assert np.all(part[:, empty, hd] == np.float32(-3.0e38)) and np.all(part[:, empty, hd + 1] == 0) and np.all(part[:, empty, :hd] == 0)
+
+
+@pytest.mark.parametrize("kind", KINDS, ids=lambda k: k[0])
+@pytest.mark.parametrize("n,splits,rows", [(300, 10, 639), (300, 10, 640), (300, 10, 319), (300, 10, 320), (150, 10, 159), (150, 10, 160), (300, 300, 300), (5, 64, 4096)])
+def test_decode_few_rows_per_split(ctx, kind, n, splits, rows):
+    """Both sides of the line between the streaming and the tiled kernel: 64 rows of the cache per split at head_dim 256, 32 at
+    128, 16 at 512."""
+    _, _, n_kv, g, hd, _, _ = kind
+    q, k, v = _case(kind, rows, n)
+    got, kd, part = _decode(ctx, kind, q, k, v, n, splits, rows=rows)
+    want = O.attention_f64(q.astype(np.float32)[None], kd, v.astype(np.float32), 1, n - 1, n_kv * g, n_kv, hd, hd**-0.5)[0]
+    assert_close(got, want, ATOL, 1e-5 if "f32" in kind[1] else 2.0**-11, f"{kind[0]} rows={rows}")
+    empty = np.arange(splits) * -(-n // splits) >= n
     assert np.all(part[:, empty, hd] == np.float32(-3.0e38)) and np.all(part[:, empty, hd + 1] == 0) and np.all(part[:, empty, :hd] == 0)
 
 
@@ -163,12 +183,13 @@ def test_decode_of_a_draft_is_causal(ctx, kind, n, splits, m_q):
     up = lambda b: ctx.buffer_from_iter(np.ascontiguousarray(b))
     if q8:
         ks, kq, kd = O.q8_quant_div(k.astype(np.float32).ravel())
-        bufs = [up(kq), up(ks)]
+        bufs = [up(np.resize(x, (n + _spare(n, splits)) * (x.size // n))) for x in (kq, ks)]
     else:
-        kd, bufs = k.astype(np.float32), [up(k)]
+        kd, bufs = k.astype(np.float32), [up(np.resize(k, (n + _spare(n, splits), n_kv, hd)))]
     rows = m_q * n_kv * g
     part, out = ctx.new_buffer(rows * splits * (hd + 2), np.float32), ctx.new_buffer(rows * hd, np.float32 if "f32" in red else np.uint16)
-    ctx.dispatch(ctx.load_kernel(name), bind(up(q), *bufs, up(v), part, _step(ctx, **{slot: n})), (splits, hd**-0.5), [n_kv, splits, m_q])
+    ctx.dispatch(ctx.load_kernel(name), bind(up(q), *bufs, up(np.resize(v, (n + _spare(n, splits), n_kv, hd))), part,
+                                            _step(ctx, **{slot: n})), (splits, hd**-0.5), [n_kv, splits, m_q])
     ctx.dispatch_blocking(ctx.load_kernel(red), bind(part, out), splits, [rows, 1, 1])
     got = out.read() if "f32" in red else O.f16_bits_to_f32(out.read())
     want = O.attention_f64(q.astype(np.float32), kd.reshape(k.shape), v.astype(np.float32), m_q, n - m_q, n_kv * g, n_kv, hd, hd**-0.5)
