@@ -125,7 +125,7 @@ struct RowsWarp {
         for (int c = 0; c < HD / 16; c++) o[c][0] = o[c][1] = o[c][2] = o[c][3] = 0.0f;
         m[0] = m[1] = NEG_SENTINEL;
         l[0] = l[1] = 0.0f;
-        odd = 0;
+        float most[2] = {0.0f, 0.0f};  // largest magnitude of the rows' scores, whole tiles (Q8_0 keys)
         bool failed = false;
         if (n > 0) {
             issue_k(0);
@@ -191,16 +191,14 @@ struct RowsWarp {
             }
             __syncwarp();
             if (i + 1 < n) issue_k(i + 1);
+            if (KQ8)
+                for (int e = 0; e < 2; e++) most[e] = max3(most[e], fabsf(s[e]), fabsf(s[2 + e]));
 #pragma unroll
             for (int e = 0; e < 4; e++) {
                 s[e] *= scale;
                 const int key = g + 8 * (e >> 1);
                 const int64_t pos = t.pos0 + key;
-                const bool seen = key >= t.from && key < t.to && pos >= row_lo[e & 1] && pos <= row_hi[e & 1];
-                // Finite scales cannot give it.  An infinite one times a whole sum that is negative would pass as a weight of 0; the
-                // statement multiplies the scale with every quant, and infinities of both signs make a NaN.
-                if (KQ8 && seen && s[e] == -INFINITY) odd |= 1u << (2 * t4 + (e & 1));
-                if (!seen) s[e] = -INFINITY;
+                if (key < t.from || key >= t.to || pos < row_lo[e & 1] || pos > row_hi[e & 1]) s[e] = -INFINITY;
             }
             float p[4];
             const float n0 = fmaxf(m[0], key_max(fmaxf(s[0], s[2]))), n1 = fmaxf(m[1], key_max(fmaxf(s[1], s[3])));
@@ -254,6 +252,12 @@ struct RowsWarp {
             if (i + 1 < n) issue_v(i + 1);
         }
         if (failed) let_copies_land();  // into this warp's slots, one of which is written next
+        // Finite scales cannot give an infinite score.  An infinite one times a block's whole sum could pass as a weight of 0; the statement
+        // multiplies the scale with every quant, and infinities of both signs make a NaN.  (Rows that are no keys count here
+        // too: the statement then only confirms the row.)
+        odd = 0;
+        for (int e = 0; e < 2; e++)
+            if (most[e] == INFINITY) odd |= 1u << (2 * t4 + e);
         // the state for the merge: [row][HD], m, l
         l[0] = key_sum(l[0]);
         l[1] = key_sum(l[1]);
@@ -298,7 +302,7 @@ struct DecodeRowsSmem {
 
 // Split-K partials.  Grid, split ranges and partials as decode_generic_kernel.
 template <int HD, int G, bool KQ8, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, HD == 512 ? 1 : HD == 256 ? 3 : 6)  // CTAs that the slots let an SM hold
+__global__ void __launch_bounds__(WARPS * 32, HD == 512 ? 1 : HD == 256 ? 3 : 5)  // CTAs that the slots let an SM hold, one less at 128 (6: 80 registers, slower)
     decode_rows_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_sc, const __grid_constant__ CUtensorMap tm_v,
                        const __half* q, const __grid_constant__ KvOperand kop, const __grid_constant__ KvOperand vop,
                        float* __restrict__ part, const uint32_t* step, int step_slot, uint32_t n_splits, float scale, uint32_t* status)
