@@ -138,7 +138,11 @@ __device__ __forceinline__ void cluster_sync()
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// CLUSTERED: the sub-splits of a (kv head, split) spread over a cluster of CTAs as well, SUB = 4 in each.
+// CLUSTERED: the sub-splits of a (kv head, split) spread over a cluster of CTAs as well, SUB = 4 in each.  What the launcher cannot
+// know is how long the sequence is: a split of up to ALONE_STAGES is the first CTA's alone, which has no other's part to wait for
+// (us, 16 kv heads, without that | with it | no cluster: 64 tokens in one split 5.1 | 4.4 | 3.7, in 8 splits 5.7 | 4.4 | 3.5; 600 tokens in 8
+// splits 7.4 | 6.7 | 4.4; 16 stages: 2000 tokens in 8 splits 7.8 | 10.3).
+constexpr uint32_t ALONE_STAGES = 8;
 template <int NSTAGES, int MIN_CTAS, int SUB, bool CLUSTERED>
 __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
     decode_paged_kernel(const __grid_constant__ CUtensorMap tm_kq, const __grid_constant__ CUtensorMap tm_ks,
@@ -156,7 +160,6 @@ __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
     constexpr int HEADS_PER_CTA = WPC / SUB;
     const int n_cta = CLUSTERED ? (int)cluster_ctas() : 1, rank = CLUSTERED ? (int)blockIdx.x % n_cta : 0;
     const int kvh = ((int)blockIdx.x / n_cta) * HEADS_PER_CTA + warp / SUB, sub = warp % SUB, split = blockIdx.y;
-    const uint32_t n_sub = SUB * n_cta, first_sub = rank * SUB + sub;  // sub-splits of a split; this warp's
     const int n_q = (int)n_kv * G;
     const bool active = kvh < (int)n_kv;  // idle warps of the last CTA when n_kv * SUB is not a multiple of 4
     const int g = lane >> 2, t4 = lane & 3;
@@ -174,8 +177,11 @@ __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
     const uint32_t chunk = (kv_len + n_splits - 1) / n_splits;
     const uint32_t t_begin = min((uint32_t)split * chunk, kv_len);
     const uint32_t t_end = min(t_begin + chunk, kv_len);
-    const uint32_t s_begin = t_begin / STAGE_TOK + first_sub;  // this warp's first stage; it then strides by n_sub
     const uint32_t n_stages = t_begin < t_end ? (t_end + STAGE_TOK - 1) / STAGE_TOK - t_begin / STAGE_TOK : 0;
+    const bool alone = CLUSTERED && n_stages <= ALONE_STAGES;  // the same in all CTAs of a cluster
+    if (alone && rank != 0) return;
+    const uint32_t n_sub = alone ? SUB : SUB * n_cta, first_sub = rank * SUB + sub;  // sub-splits of a split; this warp's
+    const uint32_t s_begin = t_begin / STAGE_TOK + first_sub;  // this warp's first stage; it then strides by n_sub
     const uint32_t n_iter = active && n_stages > first_sub ? (n_stages - first_sub + n_sub - 1) / n_sub : 0;
     __syncwarp();
 
@@ -466,7 +472,7 @@ __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
 
     // ---- merge the CTAs of a cluster in rank order ------------------------------------------------------
     // Each leaves its state where warp 0's K ring was; rank r then owns every n_cta-th stretch of 16 dims of all rows.
-    if constexpr (CLUSTERED) {
+    if (CLUSTERED && !alone) {
         float* mine = reinterpret_cast<float*>(sm.kq[0][0]);
         __syncthreads();  // the merge above has read what the other warps left
         if (warp == 0) {
@@ -589,7 +595,9 @@ cudaError_t launch_decode_variant(cudaStream_t stream, int device, const CUtenso
 // four CTAs = 16 warps live on an SM.  The number of sub-splits per (kv head, split) is the largest
 // of 32, 16, 8 (clusters of 8, 4, 2 CTAs), 4, 2, 1 for which all warps still fit on the GPU at once (one wave): extra waves
 // cost more than the parallelism buys, while few splits (a short sequence) leave most of the chip idle and every warp a long
-// chain of stages: 1000 tokens, one split, 16 kv heads took 18.2 us a launch with 4 sub-splits per split, 7.1 with 32.
+// chain of stages: 1000 tokens, one split, 16 kv heads took 17.7 us a launch with 4 sub-splits per split, 6.3 with 32.  A
+// cluster costs 1 to 2 us, so it wants splits of more than ALONE_STAGES: 16 kv heads, 1000 tokens, 8 splits 5.3 us with 4
+// sub-splits, 7.4 with 16.
 // SGB_DECODE_SUB=1|2|4|8|16|32 overrides the choice (tuning aid; results agree
 // within rounding, each choice is bit-reproducible).
 cudaError_t launch_decode(cudaStream_t stream, int device, int sm_count, const CUtensorMap (&tm)[4], const __half* q,
@@ -604,6 +612,7 @@ cudaError_t launch_decode(cudaStream_t stream, int device, int sm_count, const C
     const uint64_t tasks = (uint64_t)n_kv * n_splits;
     int sub = 32;
     while (sub > 1 && tasks * sub > slots) sub /= 2;
+    if (sub > 4 && (uint64_t)table_len * page <= (uint64_t)n_splits * ALONE_STAGES * STAGE_TOK) sub = 4;  // no split can be longer
     if (forced >= 1 && forced <= 4 * MAX_CLUSTER && (forced & (forced - 1)) == 0) sub = forced;
 #define SGB_DECODE_ARGS stream, device, tm, q, page_table, table_len, page, pool_pages, part, step, n_kv, n_splits, scale, m_q, status
     if (sub > 4) return launch_decode_variant<3, 4, 4, true>(SGB_DECODE_ARGS, sub / 4);

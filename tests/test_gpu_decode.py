@@ -225,3 +225,17 @@ def test_every_stage_counts_once(ctx, kv_len, n_splits, m_q):
     counts = np.stack([np.bincount((np.arange(s) // 16) % D, minlength=D) / s for s in seen])
     one = vp.deq[0, 0, 0]  # 1 as Q8_0 holds it
     assert_close(got / one, np.broadcast_to(counts[:, None, :], got.shape), 0, 1 / 128, f"kv_len={kv_len} splits={n_splits}")
+
+
+@pytest.mark.parametrize("kv_len", [1, 16, 17, 128, 129, 250, 300])
+@pytest.mark.parametrize("n_splits", [1, 2, 8])
+@pytest.mark.parametrize("spare_pages", [0, 200])
+def test_short_sequence_in_a_short_or_long_table(ctx, kv_len, n_splits, spare_pages):
+    """The launcher gives few splits clusters of CTAs unless the table ends first (8 stages of 16 tokens a split), and splits of at
+    most 8 stages stay with a cluster's first CTA.  Entries behind the sequence name no page of the pool."""
+    c = PagedCase(ctx, 0x51 + kv_len, kv_len, page=64)
+    c.bufs[5] = ctx.buffer_from_iter(np.concatenate([c.table, np.full(spare_pages, 0xFFFFFFF, np.uint32)]))
+    part, got = c.run(n_splits)
+    assert_close(got, c.want(), what=f"kv_len={kv_len} splits={n_splits} spare={spare_pages}")
+    empty = np.arange(n_splits) * -(-kv_len // n_splits) >= kv_len
+    assert np.all(part[:, empty, D] == np.float32(-3.0e38)) and np.all(part[:, empty, D + 1] == 0)
