@@ -4,13 +4,17 @@
 // All of them are a few query rows (<= 8: the query heads of a kv head, times the drafted tokens) against many keys, bound by
 // the bytes of K and V.  A warp takes 16 keys at a time: they arrive by TMA, 128 bytes of all 16 rows to a copy (128-byte
 // swizzle), in the warp's own slots (K and V apart, so that the next K is on its way while this V is used).  S = K Q^T
-// and O^T += V^T P^T are mma.sync m16n8k16 with the keys or 16 dims as M and the rows as N: tcgen05 has no tile this small.  Warps never wait for one another before the end, where their states merge in warp order.
+// and O^T += V^T P^T are mma.sync m16n8k16 with the keys or 16 dims as M and the rows as N: tcgen05 has no tile this small.
+// Warps never wait for one another before the end, where their states merge in warp order.
 // Precision is that of the f32 statement (attn_decode_sliding.wgsl:84-107): Q8_0 keys enter as whole numbers and every block's
-// sum is multiplied by its f32 scale; P = (hi + lo) * 2^-14 with both halves f16 (22 bits, the factor keeps lo out of f16's
-// subnormals); running maximum and sums in f32.
+// sum is multiplied by its f32 scale; products of f16 keys are added up 16 at a time in f32, for the tensor pipe truncates what it
+// adds to; P = (hi + lo) * 2^-14, both halves f16, which together miss p by at most one unit of its last f32 place (the factor keeps
+// lo out of f16's subnormals; a p below 2^-39 of its row's maximum is in l but too small for lo); running maximum and sums in f32.
+// Error of the verify step against 64 bits, streaming kernel | this one: 60 cached tokens 1.56e-7 | 1.49e-7 (2.2e-7 while scores were
+// summed in the tensor pipe and hi went first), 700 tokens 3.0e-7 | 1.9e-7, 9000 tokens 3.5e-7 | 2.1e-7.
 // Measured (us a call, streaming kernel before -> this one): head_dim 512, Q8_0 keys, 32768 tokens, 32 splits 427 -> 40.6
 // (206 MB, 5.1 TB/s on the 128 SMs that 4 x 32 CTAs occupy); head_dim 256, 1024 slots, 16 splits 12.3 -> 5.7; verify of 4 tokens over
-// the ring, 16 kv heads 148 -> 8.4.
+// the ring, 16 kv heads 145 -> 8.2.
 // A bulk copy per row instead (48 a tile at head_dim 512) took 41.8 us.
 // V rows that hold no visible key are zeroed once they have arrived, and rows that are not finite are computed again by the streaming
 // statement: a tile multiplies by p = 0 what that statement skips (all of them at 32768 tokens: 427 us on the streaming kernel).
@@ -178,16 +182,20 @@ struct RowsWarp {
                     }
                 }
             } else {
-                float s1[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                // every product starts from 0 and is added in f32: the tensor pipe truncates what it adds to
 #pragma unroll
-                for (int c = 0; c < HD / 16; c++) {
-                    uint32_t a[4];
-                    ldsm_x4(at(k_addr, 2 * c + k_bit), a);
-                    const uint32_t b0 = *reinterpret_cast<const uint32_t*>(q_row + 32 * c), b1 = *reinterpret_cast<const uint32_t*>(q_row + 32 * c + 16);
-                    mma16816((c & 1) ? s1 : s, a, b0, b1);
+                for (int c = 0; c < HD / 16; c += 2) {
+                    float acc[2][4] = {};
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        uint32_t a[4];
+                        ldsm_x4(at(k_addr, 2 * (c + h) + k_bit), a);
+                        const uint32_t b0 = *reinterpret_cast<const uint32_t*>(q_row + 32 * (c + h)), b1 = *reinterpret_cast<const uint32_t*>(q_row + 32 * (c + h) + 16);
+                        mma16816(acc[h], a, b0, b1);
+                    }
+#pragma unroll
+                    for (int e = 0; e < 4; e++) s[e] += acc[0][e] + acc[1][e];
                 }
-#pragma unroll
-                for (int e = 0; e < 4; e++) s[e] += s1[e];
             }
             __syncwarp();
             if (i + 1 < n) issue_k(i + 1);
@@ -244,9 +252,9 @@ struct RowsWarp {
 #pragma unroll
                 for (int k = 0; k < 4; k++) ldsm_x4_trans(at(v_addr, 2 * (c + k) + v_bit), a[k]);
 #pragma unroll
-                for (int k = 0; k < 4; k++) mma16816(o[c + k], a[k], hi[0], hi[1]);
+                for (int k = 0; k < 4; k++) mma16816(o[c + k], a[k], lo[0], lo[1]);  // before hi: the first tile's is then exact in o
 #pragma unroll
-                for (int k = 0; k < 4; k++) mma16816(o[c + k], a[k], lo[0], lo[1]);
+                for (int k = 0; k < 4; k++) mma16816(o[c + k], a[k], hi[0], hi[1]);
             }
             __syncwarp();
             if (i + 1 < n) issue_v(i + 1);

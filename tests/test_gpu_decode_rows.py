@@ -2,7 +2,7 @@
 the warps' strides, empty and one-key splits, rows past the end that hold NaN, the ring's wrap, values that are not finite,
 lengths past the buffer.
 
-Tolerance against the f64 oracle: P keeps 22 bits, sums and exponentials are f32 (1e-5 of the largest |v|, below 5 for these
+Tolerance against the f64 oracle: P keeps f32's last place, sums and exponentials are f32 (1e-5 of the largest |v|, below 5 for these
 normals), and the output's own f16 rounding (2^-11) where it is f16."""
 import numpy as np
 import pytest
@@ -138,6 +138,24 @@ def test_verify_ring(ctx, m, q0):
                                up(np.concatenate([v[hist:].view(np.uint16), junk])), out, _step(ctx, q0=q0)), hd**-0.5, [n_kv, m, 1])
     want = O.attention_f64(q.astype(np.float32), k.astype(np.float32), v.astype(np.float32), m, hist, 2 * n_kv, n_kv, hd, hd**-0.5, window=1024)
     assert_close(out.read().reshape(m, 2 * n_kv, hd), want, ATOL, 1e-5, f"m={m} q0={q0}")
+
+
+def test_verify_ring_keeps_the_precision_of_the_f32_statement(ctx):
+    """The streaming kernel's 2-norm error on such inputs is 1.6e-7 of the result; scores summed in the tensor pipe gave 2.2e-7."""
+    n_kv, hd, m, q0 = 16, 128, 4, 60
+    q, k, v = normal_f16(1, m, 2 * n_kv, hd), normal_f16(2, q0 + m, n_kv, hd), normal_f16(3, q0 + m, n_kv, hd)
+    up = lambda b: ctx.buffer_from_iter(np.ascontiguousarray(b))
+    ring = lambda x: up(np.concatenate([x[:q0], np.zeros((R - q0, n_kv, hd), np.float16)]))
+    out = ctx.new_buffer(m * 2 * n_kv * hd, np.float32)
+    ctx.dispatch_blocking(ctx.load_kernel("attn_verify_sliding_ring_d128"), bind(up(q), ring(k), ring(v), up(k[q0:]), up(v[q0:]), out, _step(ctx, q0=q0)),
+                          hd**-0.5, [n_kv, m, 1])
+    q, k, v = (x.astype(np.float64) for x in (q, k, v))
+    s = np.einsum("mhd,khd->mhk", q, np.repeat(k, 2, 1)) * hd**-0.5
+    seen = np.arange(q0 + m)[None, None, :] <= q0 + np.arange(m)[:, None, None]
+    p = np.where(seen, np.exp(s - s.max(-1, keepdims=True)), 0)
+    want = np.einsum("mhk,khd->mhd", p / p.sum(-1, keepdims=True), np.repeat(v, 2, 1))
+    got = out.read().reshape(want.shape).astype(np.float64)
+    assert np.linalg.norm(got - want) < 1.8e-7 * np.linalg.norm(want)
 
 
 def test_verify_ring_value_only_the_later_token_sees(ctx):
