@@ -11,7 +11,7 @@
 //     sub-splits of a head take its 16-token stages round-robin and are merged in fixed order at
 //     the end, so the grid fills the SMs in one wave whatever n_splits the caller chose (the
 //     partials keep the reference's [row][split][130] layout).  Every warp runs its own
-//     pipeline: lane 0 issues the TMA loads of its head's 16-token stages (K quants, V quants, and
+//     pipeline: lanes 0-3 issue the TMA loads of its head's 16-token stages (K quants, V quants, and
 //     the 16-byte scale pairs of its head and its neighbour) NSTAGES ahead, through the page
 //     table, into the warp's private ring of shared-memory stages; the only synchronisation is the
 //     warp's own "full" mbarrier per stage -- no producer warp, no cross-warp barrier;
@@ -23,11 +23,16 @@
 //   * the per-block scales never touch the int8 data: QK^T is accumulated per 32-wide block and
 //     multiplied by f32(scale) afterwards (sum_b s_b * sum_d q_d k_d == sum_d q_d (s_b k_d), i.e.
 //     the reference's exact product f32(scale)*f32(q), no f16 re-rounding); for PV the scale is
-//     folded into P.  The +1152 offsets are removed exactly: the QK accumulator starts at
-//     -1152 * sum(q) and PV subtracts 1152 * sum(P') gathered by one extra MMA against ones;
+//     folded into P.  K keeps its +1152 (the accumulator of a block starts at -1152 * sum(q)); V loses
+//     it pair by pair: left in and taken off the sums at the end (1152 * sum(P'), an MMA against ones per
+//     block), it swamped them, for outputs shrink with the length as the offset's share grows.
+//     131072 tokens of a nearly flat softmax: error against 64 bits 2.2e-2 then, 3.0e-4 now, and the 32
+//     subtractions cost less than the four MMAs (a call 117.6 -> 113.7 us; 32768 tokens 45.5 -> 43.5);
 //   * online softmax in registers (base 2, row max by warp shuffles over the 4 lanes of a row,
-//     rescale only when the max grows by more than 2^8).  A head's tokens are walked by one warp
-//     in order, so the partials need no cross-warp merge and reruns are bit-identical.
+//     rescale only when the max grows by more than 2^8).  P and P * scale are f16, relative to the
+//     warp's own running maximum, so how many warps share a split moves results within that rounding
+//     (error against 64 bits, 1000 tokens in one split: 2.9e-4 with 4 warps, 2.3e-4 with 32).  States
+//     merge in a fixed order, so reruns are bit-identical.
 #include <cstdio>
 #include <cstdlib>
 #include <initializer_list>
@@ -68,6 +73,12 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], 
     asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// q + 1152 -> q, as f16 pairs, exactly.
+__device__ __forceinline__ uint32_t less_offset(uint32_t x)
+{
+    const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&x), __float2half2_rn(OFFSET));
+    return *reinterpret_cast<const uint32_t*>(&r);
 }
 // Transpose an 8x8 matrix of 16-bit elements held one row-pair per lane (the mma C/B layouts).
 __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a)
@@ -290,12 +301,8 @@ __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
     const float scale2 = scale * 1.4426950408889634f;
     float m_run[2] = {NEG_SENTINEL, NEG_SENTINEL}, l_part[2] = {0.0f, 0.0f};
     float o[8][4];     // o[c]: dims 16c + 2g (c0, c1) and 16c + 2g + 1 (c2, c3) x query rows 2*t4 (c0, c2), 2*t4 + 1 (c1, c3)
-    float osum[4][4];  // per block: sum over tokens of P'_b, same column layout
 #pragma unroll
     for (int c = 0; c < 8; c++) o[c][0] = o[c][1] = o[c][2] = o[c][3] = 0.0f;
-#pragma unroll
-    for (int b = 0; b < 4; b++) osum[b][0] = osum[b][1] = osum[b][2] = osum[b][3] = 0.0f;
-    const uint32_t ones[4] = {0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u};
 
     bool failed = false;
     for (uint32_t it = 0; it < n_iter; ++it) {
@@ -365,13 +372,6 @@ __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
                 o[c][2] *= c0;
                 o[c][3] *= c1;
             }
-#pragma unroll
-            for (int b = 0; b < 4; b++) {
-                osum[b][0] *= c0;
-                osum[b][1] *= c1;
-                osum[b][2] *= c0;
-                osum[b][3] *= c1;
-            }
         }
         const float p00 = ex2(s[0][0] - m_run[0]), p01 = ex2(s[0][1] - m_run[1]);
         const float p10 = ex2(s[1][0] - m_run[0]), p11 = ex2(s[1][1] - m_run[1]);
@@ -405,11 +405,10 @@ __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
 #pragma unroll
             for (int cc = 0; cc < 2; cc++) {
                 const uint32_t y0 = y[2 * cc] ^ 0x80808080u, y1 = y[2 * cc + 1] ^ 0x80808080u;
-                const uint32_t a[4] = {__byte_perm(y0, MAGIC, 0x4240), __byte_perm(y0, MAGIC, 0x4341),
-                                       __byte_perm(y1, MAGIC, 0x4240), __byte_perm(y1, MAGIC, 0x4341)};
+                const uint32_t a[4] = {less_offset(__byte_perm(y0, MAGIC, 0x4240)), less_offset(__byte_perm(y0, MAGIC, 0x4341)),
+                                       less_offset(__byte_perm(y1, MAGIC, 0x4240)), less_offset(__byte_perm(y1, MAGIC, 0x4341))};
                 mma16816(o[2 * b + cc], a, pb0, pb1);
             }
-            mma16816(osum[b], ones, pb0, pb1);
         }
 
         // Refill this slot for iteration it + NSTAGES; every lane is done reading it.
@@ -422,12 +421,6 @@ __global__ void __launch_bounds__(WPC * 32, MIN_CTAS)
 
     if (failed) let_copies_land();  // into this warp's ring, which is written next
 
-    // ---- remove the +1152 offsets, total the denominators --------------------------------------------
-#pragma unroll
-    for (int c = 0; c < 8; c++) {
-#pragma unroll
-        for (int i = 0; i < 4; i++) o[c][i] -= OFFSET * osum[c >> 1][i];
-    }
     float l_row[2] = {tok_sum(l_part[0]), tok_sum(l_part[1])};
 
     // ---- merge the SUB sub-splits of a head in fixed order (sub 0 <- 1 <- 2 <- 3) ----------------------
