@@ -813,7 +813,7 @@ def main():
                 del c2
                 torch.cuda.empty_cache()
                 best = None
-                # the library's hint (74 on 148 SMs: 16 kv heads x 74 splits x 2 warps fill every SM evenly) beside 32 / 64
+                # the library's hint (one split per 512 tokens here: 64; 74 from 37 888 tokens on) beside 32 / 64
                 hint = dev.ctx.decode_splits_hint(KV, 32768)
                 for ns in sorted({32, 64, hint}):
                     d3 = run_decode(dev, rank, world, 40, 5, dist, 32768, 1, ns, 0x5603)

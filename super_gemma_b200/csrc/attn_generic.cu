@@ -426,9 +426,10 @@ int launch_prefill_paged_q8kv_scalar_d128(const LaunchArgs& a)
 //   VARIANT 0  attn_prefill_global_flash, attn_prefill_global_flash_sp: q f16, k f16, v f16, out, step
 //   VARIANT 1  attn_prefill_global_flash_sp_q8: q f16, k_quants, k_scales, v_quants, v_scales, out, step
 //   VARIANT 2  attn_prefill_global_flash_sp_iq: q_i8, q_scales, k_quants, k_scales, v f16, out, step
-// Served by the streaming kernel on the dequantised values (the reference's own test compares the int8
-// kernel with attention over the dequantised Q and K, tests/parity_attn.rs:689-768).  Rows past the last
-// visible key are never read, so K/V need not be padded to a 64-key tile as the reference's callers do.
+// The first two are the streaming kernel's, on the dequantised values (the reference's own test compares the int8 kernel with
+// attention over the dequantised Q and K, tests/parity_attn.rs:689-768); the third, the one the reference's graph
+// dispatches, is int8_prefill_kernel's where that takes the call.  K/V need not be padded to a 64-key tile as the
+// reference's callers do: rows past the last visible key do not count.
 template <int VARIANT>
 int launch_prefill_global_flash_ref(const LaunchArgs& a)
 {

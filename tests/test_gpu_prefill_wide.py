@@ -3,7 +3,7 @@ Q and K) where its tiles can go wrong: query counts around the 64- and 16-token 
 and the ring's wrap, rows past the end that hold NaN, values that are not finite, and the calls it leaves to the streaming
 kernel.
 
-Tolerance against the f64 oracle: the output is f16 (relative 2^-11), P keeps 22 bits, sums and exponentials are f32:
+Tolerance against the f64 oracle: the output is f16 (relative 2^-11), P keeps f32's last place, sums and exponentials are f32:
 1e-5 of the largest |v| (below 5 for these normals)."""
 import numpy as np
 import pytest
