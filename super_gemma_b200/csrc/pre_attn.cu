@@ -9,8 +9,8 @@
 //   kv_norm_rope_append_paged_q8_d128         norm(k) + rope(k) + norm(v) + Q8_0 quantise + paged append
 // The fused kernels round to f16 exactly where the chain stores f16 (after the norm, after the rotation), so
 // they give the bits of their own unfused pieces.  All of it is HBM-bound: the head_dim-128 kernels give a row to 16
-// consecutive lanes (16-byte accesses, partner dims and block maxima by shuffle), the reference-named ones a 32-value
-// block to a thread; the row's sum of squares always goes through a fixed shuffle tree (deterministic).
+// consecutive lanes (16-byte accesses, partner dims and block maxima by shuffle), the append 8 (both partners in a lane), the
+// reference-named ones a 32-value block to a thread; the row's sum of squares always goes through a fixed shuffle tree (deterministic).
 //
 // Arithmetic (f32): inv = 1/sqrt(sum(x^2)/n + 1e-6); y = f16(x * inv * w)  [w or 1 + w];
 // rope pair i couples dims (i, i + n/2), live for i < rot_dims/2: lo' = f16(lo*c - hi*s), hi' = f16(hi*c + lo*s).
@@ -215,41 +215,95 @@ __global__ void __launch_bounds__(PRE_THREADS) norm_rope_d128_kernel(const __hal
     if (live) *reinterpret_cast<uint4*>(y + (size_t)row * 128 + 8 * o) = pack_f16x8(v);
 }
 
-// Q8_0 of the 32-value block that four consecutive lanes hold (8 values each): the arithmetic of
-// kv_quant_q8.wgsl:38-57 (see kv_codec.cu); the block maximum by two shuffles.  All lanes of the warp call it.
-__device__ __forceinline__ void quant_oct_f32(const float2 (&x)[4], __half& scale, uint2& packed)
+// Multiplies and additions of pairs, each half rounded by itself: ptxas contracts a packed multiply and add that do not say .rn.
+__device__ __forceinline__ float2 mul2_rn(float2 a, float2 b)
 {
-    float amax = 0.0f;
+    float2 r;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ float2 add2_rn(float2 a, float2 b)
+{
+    float2 r;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ float2 unpack_half2(uint32_t u) { return __half22float2(*reinterpret_cast<const __half2*>(&u)); }
+
+// Q8_0 of the 32-value blocks that four consecutive lanes hold (8 values each, two blocks side by side): the arithmetic of
+// kv_quant_q8.wgsl:38-57 (see kv_codec.cu).  The values are f16, so the block maxima are taken of f16 pairs, both blocks' in one
+// word and two shuffles; the conversion adds 1.5 * 2^23, which leaves the nearest whole number in the low bytes and costs an
+// eighth of a convert instruction.  Blocks that hold an infinity or a NaN convert value by value.  All lanes of the warp call it.
+__device__ __forceinline__ void quant_2x8(const uint32_t (&x)[8], __half (&scale)[2], uint2 (&packed)[2])
+{
+    auto habs = [](uint32_t u) { return __habs2(*reinterpret_cast<const __half2*>(&u)); };
+    __half2 top[2];
 #pragma unroll
-    for (int i = 0; i < 4; i++) amax = max3(amax, fabsf(x[i].x), fabsf(x[i].y));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-    const float d = __fmul_rn(amax, 1.0f / 127.0f);
-    const float id = d > 0.0f ? __frcp_rn(d) : 0.0f;
-    scale = __float2half_rn(d);
-    uint32_t w[4];  // two quants each, in the low bytes
+    for (int e = 0; e < 2; e++) top[e] = __hmax2_nan(__hmax2_nan(habs(x[4 * e]), habs(x[4 * e + 1])), __hmax2_nan(habs(x[4 * e + 2]), habs(x[4 * e + 3])));
+    __half2 both = __hmax2_nan(__lows2half2(top[0], top[1]), __highs2half2(top[0], top[1]));
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const float2 y = __fmul2_rn(x[i], make_float2(id, id));
-        w[i] = __byte_perm((uint32_t)__float2int_rn(y.x), (uint32_t)__float2int_rn(y.y), 0x0040);
+    for (int d = 1; d < 4; d <<= 1) {
+        const uint32_t o = __shfl_xor_sync(0xffffffffu, *reinterpret_cast<const uint32_t*>(&both), d);
+        both = __hmax2_nan(both, *reinterpret_cast<const __half2*>(&o));
     }
-    packed = make_uint2(__byte_perm(w[0], w[1], 0x5410), __byte_perm(w[2], w[3], 0x5410));
+    float2 amax = __half22float2(both);
+    const bool odd = __any_sync(0xffffffffu, !(fmaxf(amax.x, amax.y) <= 65504.0f) || amax.x != amax.x || amax.y != amax.y);
+    if (odd) {  // the maximum of what is a number
+        float m[2] = {0.0f, 0.0f};
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const float2 f = unpack_half2(x[i]);
+            m[i >> 2] = max3(m[i >> 2], fabsf(f.x), fabsf(f.y));
+        }
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            m[e] = fmaxf(m[e], __shfl_xor_sync(0xffffffffu, m[e], 1));
+            m[e] = fmaxf(m[e], __shfl_xor_sync(0xffffffffu, m[e], 2));
+        }
+        amax = make_float2(m[0], m[1]);
+    }
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+        const float d = __fmul_rn(e ? amax.y : amax.x, 1.0f / 127.0f);
+        const float id = d > 0.0f ? __frcp_rn(d) : 0.0f;
+        scale[e] = __float2half_rn(d);
+        uint32_t w[4];  // two quants each, in the low bytes
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float2 y = mul2_rn(unpack_half2(x[4 * e + i]), make_float2(id, id));
+            if (odd) {
+                w[i] = __byte_perm((uint32_t)__float2int_rn(y.x), (uint32_t)__float2int_rn(y.y), 0x0040);
+            } else {
+                const float2 n = add2_rn(y, make_float2(12582912.0f, 12582912.0f));
+                w[i] = __byte_perm(__float_as_uint(n.x), __float_as_uint(n.y), 0x0040);
+            }
+        }
+        packed[e] = make_uint2(__byte_perm(w[0], w[1], 0x5410), __byte_perm(w[2], w[3], 0x5410));
+    }
 }
 
 // kv_norm_rope_append_paged_q8_d128: K rows (norm with k_w, rope) and V rows (weightless norm), both landing Q8_0-quantised at
 // row page_table[t / page] * page + t % page with t = step[0] + token; and, for qkv_norm_rope_append_paged_q8_d128, Q rows
 // (norm with q_w, rope, f16 out): the whole pre-attention step of a layer in one launch.
 //
-// 2^slot_bits groups of 16 lanes (and gridDim.y times as many) share the rows of a token (q heads, k heads, v heads in this order),
-// one row of 16 bytes a lane at a time: a thread keeps its octet of dims for all of its rows, so the token's cos/sin values and
-// the page lookup are read once and stay in registers instead of once per row (they were four times the bytes of a row's own
-// octet, and made the kernel issue-bound).  What the launcher chooses is at append_shape.
-constexpr int APPEND_THREADS = 128;
+// 2^slot_bits groups of 8 lanes (and gridDim.y times as many) share the rows of a token (q heads, k heads, v heads in this order).
+// A lane has the octet of dims 8 o .. and the one 64 dims further on that it turns with, so the rotation stays in the lane; it
+// keeps its octets for all of its rows, so the token's cos/sin values and the page lookup are read once and stay in
+// registers.  Bound by issued instructions: 16 lanes a row, which exchanged partners by shuffle and converted what they got,
+// took 40.5 us for 4096 tokens of q, k and v with 16 kv heads, this form 33.0 (120 MB: 18.4 at the copy bandwidth).  What the launcher
+// chooses is at append_shape.
+constexpr int APPEND_THREADS = 128, APPEND_BLOCKS = 6;
+constexpr int ROW_LANES = 8;
 constexpr int MOST_SLOTS = 16;  // groups per token and grid row
-constexpr int ROWS_AHEAD = 4;  // loads of a thread under way at a time
+constexpr int ROWS_EACH = 4;   // rows of a group where a launch has more than it takes to fill the GPU
+constexpr int ROWS_AHEAD = 2;  // whose loads are under way at a time
 
 template <bool PLUS_ONE>
-__global__ void __launch_bounds__(APPEND_THREADS, 8)
+__global__ void __launch_bounds__(APPEND_THREADS, APPEND_BLOCKS)
     kv_norm_rope_append_kernel(const __half* q_raw, const float* q_w, __half* __restrict__ q_out,
                                uint32_t n_q, const __half* k_raw, const __half* v_raw, const float* k_w,
                                const float2* cos_sin, __half* __restrict__ k_scales, int8_t* __restrict__ k_quants,
@@ -259,25 +313,25 @@ __global__ void __launch_bounds__(APPEND_THREADS, 8)
 {
     pdl_wait();  // the raw q, k, v rows come from earlier kernels of the stream
     pdl_launch_dependents();
-    const int o = threadIdx.x & 15;
-    const uint32_t rows = n_q + 2 * n_kv, group = blockIdx.x * (APPEND_THREADS / 16) + (threadIdx.x >> 4);
+    const int o = threadIdx.x & (ROW_LANES - 1);
+    const uint32_t rows = n_q + 2 * n_kv, group = blockIdx.x * (APPEND_THREADS / ROW_LANES) + threadIdx.x / ROW_LANES;
     uint32_t token = group >> slot_bits, slot = group & ((1u << slot_bits) - 1);
     if (token >= tokens) {  // behind the last token: no row of the first
         token = 0;
         slot = rows;
     }
-    // rotation: dims [8 o, 8 o + 8) pair with +-64; half_rot is a multiple of 8 (checked on the host), so a whole octet turns or none
-    const uint32_t pair0 = (uint32_t)(o & 7) * 8;
-    const bool turns = pair0 < half_rot;
-    float2 c[4], sn[4];
+    // rotation: dims 8 o + i and 64 + 8 o + i; half_rot is a multiple of 8 (checked on the host), so a whole octet turns or none
+    const bool turns = 8 * (uint32_t)o < half_rot;
+    float c[8], sn[8];
     if (turns) {
-        const float4* cp = reinterpret_cast<const float4*>(cos_sin + (size_t)token * half_rot + pair0);
+        const float4* cp = reinterpret_cast<const float4*>(cos_sin + (size_t)token * half_rot + 8 * o);
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const float4 cs = ld_global(cp + j);
-            c[j] = make_float2(cs.x, cs.z);
-            // low half: lo*c - hi*s with lo = own; high half: hi*c + lo*s with hi = own (x - y is x + (-y), bit for bit)
-            sn[j] = o < 8 ? make_float2(-cs.y, -cs.w) : make_float2(cs.y, cs.w);
+            c[2 * j] = cs.x;
+            sn[2 * j] = cs.y;
+            c[2 * j + 1] = cs.z;
+            sn[2 * j + 1] = cs.w;
         }
     }
     size_t dst_row = 0;
@@ -293,79 +347,87 @@ __global__ void __launch_bounds__(APPEND_THREADS, 8)
                 report_error(status, DEV_ERR_BOUNDS, 105, (uint32_t)dst_row, (uint32_t)dst_rows);
         }
     }
-    auto octet = [&](uint32_t r) {
-        if (r >= rows) return make_uint4(0u, 0u, 0u, 0u);
+    struct Octets {
+        uint4 lo, hi;
+    };
+    auto octets = [&](uint32_t r) {
+        if (r >= rows) return Octets{make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
         const __half* src = r < n_q           ? q_raw + ((size_t)token * n_q + r) * 128
                             : r < n_q + n_kv ? k_raw + ((size_t)token * n_kv + (r - n_q)) * 128
                                              : v_raw + ((size_t)token * n_kv + (r - n_q - n_kv)) * 128;
-        return ld_global(reinterpret_cast<const uint4*>(src + 8 * o));
+        const uint4* p = reinterpret_cast<const uint4*>(src + 8 * o);
+        return Octets{ld_global(p), ld_global(p + 8)};
     };
-    auto work = [&](uint32_t r0, const uint4& u) {
+    auto work = [&](uint32_t r0, const Octets& u) {
         const uint32_t r = r0 + slot;
         const bool live = r < rows, is_q = r < n_q, is_v = r >= n_q + n_kv;
         const uint32_t head = is_q ? r : is_v ? r - n_q - n_kv : r - n_q;
-        // pairs: packed f32x2 multiplies round each half like the scalar ones
-        float2 v[4], wv[4];
+        uint32_t own[8] = {u.lo.x, u.lo.y, u.lo.z, u.lo.w, u.hi.x, u.hi.y, u.hi.z, u.hi.w};
+        float ss[2] = {0.0f, 0.0f};
+        float2 v[8];
 #pragma unroll
-        for (int j = 0; j < 4; j++) wv[j] = make_float2(1.0f, 1.0f);
-        if (live && !is_v) {
-            const float* w = (is_q ? q_w : k_w) + 8 * o;
-            const float4 w0 = ld_global(reinterpret_cast<const float4*>(w)), w1 = ld_global(reinterpret_cast<const float4*>(w) + 1);
-            const float2 x[4] = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w), make_float2(w1.x, w1.y), make_float2(w1.z, w1.w)};
-#pragma unroll
-            for (int j = 0; j < 4; j++) wv[j] = PLUS_ONE ? __fadd2_rn(make_float2(1.0f, 1.0f), x[j]) : x[j];
+        for (int j = 0; j < 8; j++) {
+            v[j] = unpack_half2(own[j]);
+            ss[j >> 2] = fmaf(v[j].x, v[j].x, ss[j >> 2]);
+            ss[j >> 2] = fmaf(v[j].y, v[j].y, ss[j >> 2]);
         }
-        float ss = 0.0f;
-        {
-            const __half2* h = reinterpret_cast<const __half2*>(&u);
+        // a fixed tree, every lane gets the same bits: the sixteen octets by 1, 2, 4 and 8
+#pragma unroll
+        for (int d = 1; d < ROW_LANES; d <<= 1) {
+            ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], d);
+            ss[1] += __shfl_xor_sync(0xffffffffu, ss[1], d);
+        }
+        const float inv = rsqrtf((ss[0] + ss[1]) / 128.0f + RMS_EPS);
+#pragma unroll
+        for (int j = 0; j < 8; j++) v[j] = mul2_rn(v[j], make_float2(inv, inv));
+        if (live && !is_v) {
+            const float4* w = reinterpret_cast<const float4*>((is_q ? q_w : k_w) + 8 * o);
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                v[j] = __half22float2(h[j]);
-                ss = fmaf(v[j].x, v[j].x, ss);
-                ss = fmaf(v[j].y, v[j].y, ss);
+                const float4 f = ld_global(w + (j >> 1) * 16 + (j & 1));
+                const float2 one = make_float2(1.0f, 1.0f), w0 = make_float2(f.x, f.y), w1 = make_float2(f.z, f.w);
+                v[2 * j] = mul2_rn(v[2 * j], PLUS_ONE ? add2_rn(one, w0) : w0);
+                v[2 * j + 1] = mul2_rn(v[2 * j + 1], PLUS_ONE ? add2_rn(one, w1) : w1);
             }
         }
+        // the normed octets as f16 pairs: what the chain of kernels stores between norm and rotation
 #pragma unroll
-        for (int d = 1; d < 16; d <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);  // fixed tree: every lane gets the same bits
-        const float inv = rsqrtf(ss / 128.0f + RMS_EPS);
-        uint32_t own[4];  // the normed octet as f16 pairs: what the chain of kernels stores between norm and rotation
+        for (int j = 0; j < 8; j++) own[j] = pack_half2(v[j].x, v[j].y);
+        if (turns && !is_v) {
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const float2 y = __fmul2_rn(__fmul2_rn(v[j], make_float2(inv, inv)), wv[j]);
-            own[j] = pack_half2(y.x, y.y);
-            v[j] = __half22float2(*reinterpret_cast<const __half2*>(&own[j]));
-        }
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const uint32_t other = __shfl_xor_sync(0xffffffffu, own[j], 8);  // the partner octet, dims +-64
-            if (turns && !is_v) {
-                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&other));
-                // not packed: a packed multiply and add were contracted to one rounding
-                own[j] = pack_half2(__fadd_rn(__fmul_rn(v[j].x, c[j].x), __fmul_rn(f.x, sn[j].x)), __fadd_rn(__fmul_rn(v[j].y, c[j].y), __fmul_rn(f.y, sn[j].y)));
-                v[j] = __half22float2(*reinterpret_cast<const __half2*>(&own[j]));
+            for (int j = 0; j < 4; j++) {
+                const float2 a = unpack_half2(own[j]), b = unpack_half2(own[4 + j]);
+                const float c0 = c[2 * j], c1 = c[2 * j + 1], s0 = sn[2 * j], s1 = sn[2 * j + 1];
+                own[j] = pack_half2(__fsub_rn(__fmul_rn(a.x, c0), __fmul_rn(b.x, s0)), __fsub_rn(__fmul_rn(a.y, c1), __fmul_rn(b.y, s1)));
+                own[4 + j] = pack_half2(__fadd_rn(__fmul_rn(b.x, c0), __fmul_rn(a.x, s0)), __fadd_rn(__fmul_rn(b.y, c1), __fmul_rn(a.y, s1)));
             }
         }
-        if (r0 + (1u << slot_bits) <= n_q) {  // only q rows in this pass (uniform over the block)
-            if (live) *reinterpret_cast<uint4*>(q_out + ((size_t)token * n_q + head) * 128 + 8 * o) = make_uint4(own[0], own[1], own[2], own[3]);
-            return;
+        if (is_q && live) {
+            uint4* to = reinterpret_cast<uint4*>(q_out + ((size_t)token * n_q + head) * 128 + 8 * o);
+            to[0] = make_uint4(own[0], own[1], own[2], own[3]);
+            to[8] = make_uint4(own[4], own[5], own[6], own[7]);
         }
-        __half s;
-        uint2 packed;
-        quant_oct_f32(v, s, packed);
-        if (!live) return;
-        if (is_q) {
-            *reinterpret_cast<uint4*>(q_out + ((size_t)token * n_q + head) * 128 + 8 * o) = make_uint4(own[0], own[1], own[2], own[3]);
-        } else if (placed) {
+        if (r0 + (1u << slot_bits) <= n_q) return;  // only q rows in this pass (uniform over the block)
+        __half s[2];
+        uint2 packed[2];
+        quant_2x8(own, s, packed);
+        if (live && !is_q && placed) {
             const size_t drow = dst_row * n_kv + head;  // row of [128] quants / [4] scales
-            if ((o & 3) == 0) (is_v ? v_scales : k_scales)[drow * 4 + (o >> 2)] = s;
-            *reinterpret_cast<uint2*>((is_v ? v_quants : k_quants) + drow * 128 + 8 * o) = packed;
+            if ((o & 3) == 0) {
+                __half* to = (is_v ? v_scales : k_scales) + drow * 4 + (o >> 2);
+                to[0] = s[0];
+                to[2] = s[1];
+            }
+            uint2* to = reinterpret_cast<uint2*>((is_v ? v_quants : k_quants) + drow * 128 + 8 * o);
+            to[0] = packed[0];
+            to[8] = packed[1];
         }
     };
     const uint32_t stride = gridDim.y << slot_bits;
     for (uint32_t base = blockIdx.y << slot_bits; base < rows; base += ROWS_AHEAD * stride) {
-        uint4 u[ROWS_AHEAD];
+        Octets u[ROWS_AHEAD];
 #pragma unroll
-        for (int k = 0; k < ROWS_AHEAD; k++) u[k] = octet(base + k * stride + slot);
+        for (int k = 0; k < ROWS_AHEAD; k++) u[k] = octets(base + k * stride + slot);
 #pragma unroll
         for (int k = 0; k < ROWS_AHEAD; k++) {
             if (base + k * stride >= rows) break;  // uniform over the block
@@ -378,19 +440,18 @@ struct AppendShape {
     dim3 grid;
     uint32_t slot_bits;
 };
-// Slots and blocks.  While all rows of the launch can be under way at once (64 a SM: eight blocks of eight groups), one row
-// per group, which takes least time for one; beyond, ROWS_AHEAD of them, which takes least instructions per row, so few rows
-// (few kv heads) put several tokens into a block.  us in a recorded chain, 1 row | 4 rows: 16 kv heads with q, 64 tokens
-// 2.7 | 3.7, 290 tokens 6.0 | 4.7, 4096 tokens 63 | 39; 4 kv heads without q, 1000 tokens 3.7 | 4.5, 2000 tokens 5.9 | 5.1,
-// 8192 tokens 17.3 | 11.7 (a block per token whatever its rows: 33).  Blocks of 256 threads: 41 where these take 39.
+// Slots and blocks.  Few rows: one per group, which takes least time for one; beyond, ROWS_EACH of them, which takes least
+// instructions per row, and few rows a token (few kv heads) put several tokens into a block.  us in a recorded chain, 1 row | 4 rows: 16 kv
+// heads with q, 64 tokens 2.7 | 4.3, 150 tokens 3.5 | 4.6, 290 tokens 4.8 | 4.8, 600 tokens 7.6 | 7.0, 4096 tokens 44 | 31.6; 4 kv
+// heads, 1000 tokens 5.2 | 4.7, 8192 tokens 22.3 | 15.2.
 inline AppendShape append_shape(const LaunchArgs& a, size_t tokens, uint32_t rows)
 {
-    const uint32_t per_thread = tokens * rows <= (size_t)64 * a.sm_count ? 1 : ROWS_AHEAD;
+    const uint32_t per_thread = tokens * rows <= (size_t)96 * a.sm_count ? 1 : ROWS_EACH;
     uint32_t bits = 0;
     while ((1u << bits) < MOST_SLOTS && (per_thread << bits) < rows) bits++;
     const size_t groups = tokens << bits;  // < 2^29: at most 2^26 rows of q and of k
     const uint32_t per_token = (rows + (1u << bits) - 1) >> bits;
-    return {dim3((uint32_t)((groups * 16 + APPEND_THREADS - 1) / APPEND_THREADS), per_thread == 1 ? min(1024u, per_token) : 1), bits};
+    return {dim3((uint32_t)((groups * ROW_LANES + APPEND_THREADS - 1) / APPEND_THREADS), per_thread == 1 ? min(1024u, per_token) : 1), bits};
 }
 
 inline uint32_t grid_for(size_t n) { return (uint32_t)((n + PRE_THREADS - 1) / PRE_THREADS); }

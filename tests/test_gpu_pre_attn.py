@@ -229,3 +229,35 @@ def test_one_launch_qkv_of_a_long_chunk(ctx, tokens, n_kv):
     assert np.array_equal(q1.read(), q2.read()) and np.any(q1.read() != 0)
     for x, y in zip(a, b):
         assert np.array_equal(x.read(), y.read()) and np.any(x.read() != 0)
+
+
+@pytest.mark.parametrize("tokens", [2, 4001])  # a row per group; four, sixteen tokens to a block and the last one short of them
+@pytest.mark.parametrize("rot", [0, 32, 128])
+def test_fused_kv_append_of_values_that_are_not_finite(ctx, rot, tokens):
+    """Weights that make infinities and NaN of some dims: blocks that hold one quantise value by value, with a maximum over what is a number,
+    as the unfused pieces do, bit for bit."""
+    import super_gemma_b200 as sg
+
+    n_kv, page, pos = 2, 64, 5
+    pages = -(-(pos + tokens) // page)
+    row, rows = n_kv * 128, pages * page
+    rng = np.random.default_rng(rot + tokens)
+    k_raw, v_raw = (rng.standard_normal(tokens * row, dtype=np.float32).astype(np.float16) for _ in range(2))
+    v_raw[130] = np.inf
+    k_w = rng.standard_normal(128, dtype=np.float32)
+    k_w[[5, 40, 100]] = np.inf, np.nan, 1e38
+    cs = O.cos_sin_table(O.inv_freqs(rot, 1e6), pos, tokens) if rot else np.zeros(2, np.float32)
+    up, mk = ctx.buffer_from_iter, lambda dt, n: ctx.new_buffer(n, dt)
+    kr, vr, kw, csb, table = up(k_raw), up(v_raw), up(k_w), up(cs), up(np.arange(pages, dtype=np.uint32))
+    step = ctx.new_step_buffer()
+    sg.StepState(pos=pos).write_to(step)
+    a, b = ([mk(np.uint16, rows * row // 32), mk(np.int8, rows * row), mk(np.uint16, rows * row // 32), mk(np.int8, rows * row)] for _ in range(2))
+    ctx.dispatch_blocking(ctx.load_kernel("kv_norm_rope_append_paged_q8_d128"), bind(kr, vr, kw, csb, *a, table, step), (row, page, rot, 0), [1, 1, 1])
+    nr, app = ctx.load_kernel("attn_norm_rope_d128"), ctx.load_kernel("kv_append_paged_q8_d128")
+    k16, v16, ones = mk(np.uint16, tokens * row), mk(np.uint16, tokens * row), up(np.ones(128, np.float32))
+    ctx.dispatch(nr, bind(kr, kw, csb, k16), (n_kv, rot, 0), [1, 1, 1])
+    ctx.dispatch(nr, bind(vr, ones, csb, v16), (n_kv, 0, 0), [1, 1, 1])
+    ctx.dispatch(app, bind(k16, b[0], b[1], table, step), (row, page), app.groups_for(tokens * row // 32))
+    ctx.dispatch_blocking(app, bind(v16, b[2], b[3], table, step), (row, page), app.groups_for(tokens * row // 32))
+    for x, y in zip(a, b):
+        assert np.array_equal(x.read(), y.read())
