@@ -262,10 +262,10 @@ __global__ void __launch_bounds__(FLASH_THREADS, 2) flash_prefill_kernel(const _
                 const uint64_t k0 = b ? dk[1][0] : dk[0][0], k1 = b ? dk[1][1] : dk[0][1];
                 const uint32_t d = tmem + TMEM_S + b * BLOCK_N;
 #pragma unroll
-                for (int kk = 0; kk < 4; kk++) umma_f16_ss(d, dq[0] + 2 * kk, k0 + 2 * kk, IDESC_QK, kk ? 1u : 0u);
+                for (int kk = 0; kk < 4; kk++) umma_f16_ss(d, dq[0] + 2 * kk, k0 + 2 * kk, IDESC_QK, kk ? 1u : 0u, 1u);
 #pragma unroll
-                for (int kk = 0; kk < 4; kk++) umma_f16_ss(d, dq[1] + 2 * kk, k1 + 2 * kk, IDESC_QK, 1u);
-                umma_commit(&sm.s_ready[b]);
+                for (int kk = 0; kk < 4; kk++) umma_f16_ss(d, dq[1] + 2 * kk, k1 + 2 * kk, IDESC_QK, 1u, 1u);
+                umma_commit(&sm.s_ready[b], 1u);
             };
             mbar_wait(&sm.q_bar, 0, prm.status, 401, failed);
             if (n_tiles > 0) issue_qk(0);
@@ -280,11 +280,11 @@ __global__ void __launch_bounds__(FLASH_THREADS, 2) flash_prefill_kernel(const _
                     // P(j) lives in the first 32 columns of S[b] (packed f16 pairs), written by the softmax warps
                     const uint64_t v0 = b ? dv[1] : dv[0];
                     const uint32_t pa = tmem + TMEM_S + b * BLOCK_N;
-                    umma_f16_ts(tmem + TMEM_O, pa, v0, IDESC_PV, j ? 1u : 0u);
+                    umma_f16_ts(tmem + TMEM_O, pa, v0, IDESC_PV, j ? 1u : 0u, 1u);
 #pragma unroll
-                    for (int kk = 1; kk < 4; kk++) umma_f16_ts(tmem + TMEM_O, pa + kk * 8, v0 + 128 * kk, IDESC_PV, 1u);
+                    for (int kk = 1; kk < 4; kk++) umma_f16_ts(tmem + TMEM_O, pa + kk * 8, v0 + 128 * kk, IDESC_PV, 1u, 1u);
                 }
-                umma_commit(&sm.pv_done[b]);
+                umma_commit(&sm.pv_done[b], 1u);
                 if (j + 2 < n_tiles) {
                     // S[b] may be overwritten: the softmax warps read it before they produced P(j), waited for above
                     issue_qk(j + 2);

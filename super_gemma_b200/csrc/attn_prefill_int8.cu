@@ -1,34 +1,30 @@
 // Prefill attention for the reference model's global layers on tcgen05: head_dim 512, int8 Q and K with f16 block scales, f16 V,
 // 8 query heads per kv head (attn_prefill_global_flash_sp_iq.wgsl).
 //
-// A head of 512 dims fills tensor memory with a 128-row f32 output alone, so everything here is transposed: keys and output
-// dims are the M = 128 side of the MMAs, and a CTA's 64 query rows (8 tokens x the 8 query heads of one kv head, which
-// share every K/V tile) are the N side.  Per 128-key tile:
-//   S^T[128 keys x 64 rows]  = K Q^T    thread = key, so a key's scales are that thread's registers
-//   O^T[512 dims x 64 rows] += V^T P^T  V is the MN-major A operand straight from its [key][dim] tile, P^T the MN-major B
-//                                       operand that each thread writes as one swizzled 128-byte row
-// One kind::i8 MMA (K = 32) per scale block gives that block's whole-number dot product, exactly; the two f16 scales multiply
-// it in f32 (f32(qs) * f32(ks) is exact), so the score is closer to f32(scale) * f32(q) arithmetic than an f32 dot product.
-// Blocks go through four 64-column buffers, two per hand-over.
+// Two CTAs share one MMA (pair.cuh): 64 query rows each (8 tokens x the 8 query heads of one kv head), M = 128.  64 rows of 512 dims
+// are 256 columns of tensor memory that way, so O fits beside the scores with the rows as the M side.  Per 128-key tile:
+//   S[64 rows x 128 keys]  = Q K^T   per 32-value scale block, two blocks at a time into one of two buffers of 128 columns
+//   O[64 rows x 512 dims] += P V     V as the MN-major B operand straight from its [key][dim] tile, 256 dims an instruction
+// of which each CTA loads half the keys of K and half the dims of V.
+// Scores: Q's quants are exact as f16.  A key's quants times their f16 scale are whole multiples of the scale's last place, 19 bits, which
+// f16 hi + lo hold exactly; four warps make them from the cache's bytes.  A block's sum so lacks only the scale of Q, which is the
+// row's, and the softmax threads have nothing left to do for it but one multiply-add.  (Whole-number sums of int8 MMAs, scaled by
+// both scales in the softmax threads: they then read 16 x 128 scales a tile through shared memory, which the MMAs read their
+// operands from; 364 us.  The transposed form before it, keys and dims as M, took V as the MN-major A operand, 160 cycles
+// an instruction where 48 would do, and converted every sum with an instruction of a sixteenth of the rate: 529 us.)
 // P = hi + lo, both halves f16, two MMAs per V tile: together they miss p by at most one unit of its last f32 place.  The exponent
 // carries +7, so that lo stays clear of f16's subnormals (the factor cancels in O / l); a p below 2^-32 of its row's reference
 // maximum is in l but too small for lo.
 // The tensor pipe truncates an accumulator each time it adds to it: in one accumulator, outputs shrank by 2e-9 of themselves per
 // key (1.7e-5 at 8192 keys, 6.7e-5 at 33280, where the error against 64 bits was 2.22e-4 instead of f16's own 2.08e-4).  From the
-// fifth tile on the softmax threads therefore settle one of the four dim blocks of O in every tile: the block, plus what was
+// fifth tile on the softmax threads therefore settle one of the two dim blocks of O in every other tile: the block, plus what was
 // settled of it before, added in f32 with rounding, splits into its upper 16 bits, which they keep in this CTA's share of the
-// output, and the exact rest, from which the tensor pipe goes on; what it adds to stays as small as the sum of four tiles.
-// Another block comes first in each tile's products, so that it can be settled while the tensor pipe is at the others.  Errors since:
-// 2.0762e-4 and 2.0773e-4 (streaming kernel: 2.0762e-4, 2.0774e-4), for 23 us of 533 at 8192 keys; all four blocks in every
-// fourth tile, with the tensor pipe waiting, took 44.
-// Roles: warps 0-7 softmax (two threads per key, 32 rows each), one MMA thread, one K and one V loader; mbarriers only.
-// The row maximum over keys runs across threads; it is only computed (32 values in 31 shuffles) when some score exceeds its
-// row's running maximum by 2^8, which one barrier with an OR finds out.
-// Measured: 256 queries at 7936 + 256 keys 13500 us on the streaming kernel, 533 here (floor 86).  Two things bound it: V as the
-// MN-major A operand costs 160 cycles per instruction (10000 of a tile's 14400), and every block's scores cross from tensor
-// memory to registers (16 x 32 KB a tile, 500 cycles each).  Rows as the M side with the 512 dims and the blocks split over
-// two CTAs that exchange partial scores took the first away and was slower, 787 us with 8 softmax warps and 741 with 16 (649
-// without the remote stores): the second then stands in one chain with the softmax.
+// output, and the exact rest, from which the tensor pipe goes on; what it adds to stays as small as the sum of a few tiles.
+// The block comes first in the products before it is settled, so the tensor pipe is at the other meanwhile.
+// Roles: warps 0-7 softmax (a row in four threads), 8-11 K, one MMA warp (the even CTA's issues for both), one V loader; mbarriers only.
+// Measured, 256 queries at 7936 + 256 keys: 13500 us on the streaming kernel, 529 in the transposed form, 346 here (floor 82).  A tile takes
+// 9000 cycles, of which the MMAs need 4900; the softmax threads wait for scores 1700, read and scale them 3100, settle 1500
+// and turn them into P 1700.
 //
 // What a tile reads beyond a query's own keys must not matter: scores are masked by selection, V rows that hold no key are
 // zeroed.  A V row that is visible to some query of the tile and not finite is visible to all of them as 0 * Inf, so rows that are
@@ -38,6 +34,7 @@
 #include <string>
 
 #include "attn_stream.cuh"
+#include "pair.cuh"
 #include "sgb_common.cuh"
 #include "sgb_kernels.h"
 
@@ -46,31 +43,38 @@ namespace sgb {
 namespace {
 
 constexpr int HD = 512, G = 8;
-constexpr int ROWS = 64;       // query rows per CTA (N)
-constexpr int TILE_K = 128;    // keys per tile (M of S^T)
-constexpr int SOFT_THREADS = 256;
-constexpr int MMA_W = 8, K_W = 9, V_W = 10;
-constexpr int INT8_THREADS = 352;
-constexpr int NV = 5;                          // V units in flight
-constexpr uint32_t Q_CHUNK = ROWS * 128;       // 128 bytes of every row
-constexpr uint32_t K_CHUNK = TILE_K * 128;
+constexpr int ROWS = 64;       // query rows per CTA: 8 tokens x G heads
+constexpr int PAIR_TOK = 2 * ROWS / G;  // tokens of a pair of CTAs
+constexpr int TILE_K = 128;    // keys per tile
+constexpr int SOFT_THREADS = 256, SOFT_WARPS = SOFT_THREADS / 32;
+constexpr int K_WARPS = 4, MMA_W = SOFT_WARPS + K_WARPS, V_W = MMA_W + 1;
+constexpr int INT8_THREADS = 32 * (V_W + 1);
+constexpr int NK = 3;                          // K chunks in flight
+constexpr int NV = 4;                          // V units in flight
+constexpr uint32_t Q_CHUNK = ROWS * 128;       // 64 dims f16 of every row
+constexpr uint32_t K_CHUNK = 64 * 128;         // 64 dims f16 of this CTA's half of a tile's keys
 constexpr uint32_t V_UNIT = 64 * 256;          // 64 keys x 128 dims f16, as two [64 keys][128 B] halves
-constexpr uint32_t P_TILE = TILE_K * ROWS * 2; // [128 keys][64 rows] f16
+constexpr uint32_t P_HALF = ROWS * 128;        // [64 rows][64 keys] f16
+constexpr uint32_t P_TILE = 2 * P_HALF;
+constexpr int GROUPS = 8;                      // S hand-overs per tile, two scale blocks each
+constexpr uint32_t S_COLS = 128;               // columns of one hand-over
+constexpr uint32_t TMEM_O = 0, TMEM_S = 256, TMEM_COLS = 512;
+static_assert(TMEM_S + 2 * S_COLS <= TMEM_COLS, "O and two S buffers fit");
+constexpr int SETTLE_AT = 5;                   // the hand-over whose scores the tensor pipe computes behind the first block's products
 constexpr float EXP_BIAS = 7.0f, GROW_T = 8.0f;
 
 struct Int8Smem {
-    uint8_t q[4][Q_CHUNK];
-    uint8_t k[4][K_CHUNK];
-    uint8_t p[2][P_TILE];  // hi, lo
+    uint8_t q[HD / 64][Q_CHUNK];  // quants
+    uint8_t k[NK][2][K_CHUNK];    // quants times scales: hi, lo
+    uint8_t p[2][P_TILE];  // hi, lo; each [key half][row][64 keys]
     uint8_t v[NV][V_UNIT];
-    float qs[16][ROWS];    // scales of Q, [block][row]
+    float qs[HD / 32][ROWS];      // scales of Q, [block][row]
     float red[4][ROWS];
-    float m_ref[ROWS], corr[ROWS];
-    uint64_t q_bar, k_full[4], k_free[4], v_full[NV], v_free[NV], v_ok[NV], s_ready[2], s_free[2], p_ready, first_done, pv_done;
+    uint64_t k_full[NK], k_free[NK], v_full[NV], v_free[NV], v_here[NV], v_ok[NV], s_ready[2], s_free[2], p_ready, first_done, pv_done;
     uint32_t tmem_base, abort;
     uint32_t redo[ROWS / 32];  // rows that are not finite, a bit each
 };
-static_assert(sizeof(Int8Smem) + 1024 <= 227 * 1024, "one CTA per SM");
+static_assert(sizeof(Int8Smem) <= 227 * 1024, "one CTA per SM");
 
 struct Int8Params {
     const uint32_t* step;
@@ -83,35 +87,20 @@ struct Int8Params {
     KvOperand k0, v0;
 };
 
-// tcgen05.mma kind::i8: int8 operands, int32 accumulator, K = 32 (32 bytes, like a K = 16 step of f16).
-__device__ __forceinline__ void umma_i8_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc)
+// Eight signed bytes as f16 pairs, exactly: 0x6400 | (q + 128) is the f16 of q + 1152.
+__device__ __forceinline__ void whole_f16x8(uint2 q, __half2 (&out)[4])
 {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, 0, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc)
-        : "memory");
-}
-// Instruction descriptor of kind::i8: D format 2 = s32, A and B format 1 = signed 8 bit, both K-major.
-__host__ __device__ constexpr uint32_t umma_idesc_i8(uint32_t m, uint32_t n)
-{
-    return (2u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((m >> 4) << 24);
-}
-// Reduce 32 values over the 32 lanes of a warp: lane c is left with the total of v[c].  Each step halves the values.
-template <bool MAX>
-__device__ __forceinline__ float transpose_reduce(float (&v)[32], int lane)
-{
+    const uint32_t x[2] = {q.x ^ 0x80808080u, q.y ^ 0x80808080u};
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const bool upper = (lane & o) != 0;
-#pragma unroll
-        for (int i = 0; i < o; i++) {
-            const float send = upper ? v[i] : v[i + o], keep = upper ? v[i + o] : v[i];
-            const float r = __shfl_xor_sync(0xffffffffu, send, o);
-            v[i] = MAX ? fmaxf(keep, r) : keep + r;
-        }
+    for (int i = 0; i < 4; i++) {
+        const uint32_t u = __byte_perm(x[i >> 1], 0x64646464u, (i & 1) ? 0x4342 : 0x4140);
+        out[i] = __hsub2(*reinterpret_cast<const __half2*>(&u), __float2half2_rn(1152.0f));
     }
-    return v[0];
+}
+__device__ __forceinline__ uint4 as_uint4(const __half2 (&h)[4])
+{
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(h);
+    return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
 // The rows that are not finite by the streaming statement, a warp per pair of heads.
@@ -127,29 +116,25 @@ __device__ __noinline__ void stream_rows(const Int8Params& prm, const Int8Smem& 
 }
 
 __global__ void __launch_bounds__(INT8_THREADS, 1)
-    int8_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
-                        const __grid_constant__ Int8Params prm)
+    int8_prefill_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ Int8Params prm)
 {
-    constexpr int TOK = ROWS / G, DB = HD / 128, UNITS = 2 * DB;  // V units per tile: (dim block, key half)
-    constexpr int GROUPS = 8;  // S hand-overs per tile
-    constexpr uint32_t S_COLS = 128;  // columns of one hand-over
-    constexpr uint32_t TMEM_O = 0, TMEM_S = DB * 64, TMEM_COLS = 512;
-    static_assert(TMEM_S + 2 * S_COLS <= TMEM_COLS, "O and two S buffers fit");
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     Int8Smem& sm = *reinterpret_cast<Int8Smem*>(smem_raw);
-    if ((smem_u32(smem_raw) & 1023u) != 0u) {  // the swizzled tiles need it; never seen, but never assumed
+    if ((smem_u32(smem_raw) & 1023u) != 0u) {  // the swizzled tiles need it; never seen, but never assumed (the same in both CTAs)
         if (threadIdx.x == 0) report_error(prm.status, DEV_ERR_BOUNDS, 500, smem_u32(smem_raw), 0);
         return;
     }
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
+    const uint32_t rank = pair_rank();  // 0 issues the pair's MMAs
     pdl_wait();  // the step words, q, K and V come from earlier kernels of the stream
     pdl_launch_dependents();
-    const int kvh = blockIdx.x % prm.n_kv;
-    const uint32_t n_qt = (prm.m_tokens + TOK - 1) / TOK;
-    const uint32_t m0 = (n_qt - 1 - blockIdx.x / prm.n_kv) * TOK;  // latest query tile (most keys) first
-    const uint32_t live_tok = min((uint32_t)TOK, prm.m_tokens - m0);
+    const uint32_t pair = blockIdx.x / 2;
+    const int kvh = pair % prm.n_kv;
+    const uint32_t n_qt = prm.m_tokens / PAIR_TOK;
+    const uint32_t pair_m0 = (n_qt - 1 - pair / prm.n_kv) * PAIR_TOK;  // latest query tile (most keys) first
+    const uint32_t m0 = pair_m0 + rank * (ROWS / G);
     const int64_t q0 = prm.step[STEP_Q0];
-    const int64_t first_qpos = q0 + m0, last_qpos = first_qpos + live_tok - 1;
+    const int64_t first_qpos = q0 + m0, last_qpos = q0 + pair_m0 + PAIR_TOK - 1;
     const int64_t rows0 = (int64_t)min(prm.k0.rows, prm.v0.rows);
     int64_t end = last_qpos;  // positions that hold a visible key end here
     if (end >= rows0) {
@@ -161,203 +146,238 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
     const int64_t valid_end = min(rows0 - 1, q0 + (int64_t)prm.m_tokens - 1);
 
     if (tid == 0) {
-        mbar_init(&sm.q_bar, 1);
-        for (int i = 0; i < 4; i++) {
-            mbar_init(&sm.k_full[i], 1);
+        for (int i = 0; i < NK; i++) {
+            mbar_init(&sm.k_full[i], 2 * K_WARPS);
             mbar_init(&sm.k_free[i], 1);
         }
         for (int i = 0; i < NV; i++) {
             mbar_init(&sm.v_full[i], 1);
             mbar_init(&sm.v_free[i], 1);
-            mbar_init(&sm.v_ok[i], 1);
+            mbar_init(&sm.v_here[i], 1);
+            mbar_init(&sm.v_ok[i], 2);
         }
         for (int i = 0; i < 2; i++) {
             mbar_init(&sm.s_ready[i], 1);
-            mbar_init(&sm.s_free[i], SOFT_THREADS / 32);
+            mbar_init(&sm.s_free[i], 2 * SOFT_WARPS);
         }
-        mbar_init(&sm.p_ready, SOFT_THREADS / 32);
+        mbar_init(&sm.p_ready, 2 * SOFT_WARPS);
         mbar_init(&sm.first_done, 1);
         mbar_init(&sm.pv_done, 1);
         sm.abort = 0;
         sm.redo[0] = sm.redo[1] = 0;
         mbar_fence_init();
     }
-    if (tid < ROWS) sm.m_ref[tid] = NEG_SENTINEL;
-    {
-        for (int i = tid; i < 16 * ROWS; i += INT8_THREADS) {
-            const int r = i >> 4, b = i & 15;
-            const uint32_t tok = m0 + r / G;
-            float s = 0.0f;
-            if (tok < prm.m_tokens) s = __half2float(ld_global(prm.q_scales + ((size_t)tok * (prm.n_kv * G) + kvh * G + r % G) * 16 + b));
-            sm.qs[b][r] = s;
-        }
-    }
     if (warp == 0) {
-        tmem_alloc(&sm.tmem_base, TMEM_COLS);
-        tmem_relinquish();
+        tmem_alloc_pair(&sm.tmem_base, TMEM_COLS);
     }
+    // this CTA's query rows: quants as f16, which holds them exactly, K-major in 128-byte rows; scales in f32
+    for (int i = tid; i < ROWS * (HD / 16); i += INT8_THREADS) {
+        const int r = i / (HD / 16), c = i % (HD / 16);
+        const size_t at = (size_t)(m0 + r / G) * (prm.n_kv * G) + kvh * G + r % G;
+        const uint4 u = ld_global(reinterpret_cast<const uint4*>((const int8_t*)prm.q + at * HD) + c);
+        __half2 h[2][4];
+        whole_f16x8(make_uint2(u.x, u.y), h[0]);
+        whole_f16x8(make_uint2(u.z, u.w), h[1]);
+#pragma unroll
+        for (int e = 0; e < 2; e++) *reinterpret_cast<uint4*>(sm.q[c / 4] + r * 128 + (((2 * (c & 3) + e) ^ (r & 7)) << 4)) = as_uint4(h[e]);
+    }
+    for (int i = tid; i < ROWS * (HD / 32); i += INT8_THREADS) {
+        const int r = i / (HD / 32), b = i % (HD / 32);
+        const size_t at = (size_t)(m0 + r / G) * (prm.n_kv * G) + kvh * G + r % G;
+        sm.qs[b][r] = __half2float(ld_global(prm.q_scales + at * (HD / 32) + b));
+    }
+    fence_proxy_async_smem();  // read by the tensor pipe
     tc_fence_before_sync();
     __syncthreads();
+    pair_sync();  // the other CTA's barriers are there
     tc_fence_after_sync();
     const uint32_t tmem = sm.tmem_base;
     bool failed = false;
-    auto block_at = [](int j, int u) { return ((u >> 1) + j) & (DB - 1); };  // dim block of V unit u of tile j: another one first in each tile
+    // V unit u of tile j: 64 keys (half u & 1) of this CTA's 128 of the 256 dims of block dim_block(j, u); the blocks take turns in
+    // coming first, so that the first can be settled while the tensor pipe is at the other
+    auto dim_block = [](int j, int u) { return ((u >> 1) + (j >> 1)) & 1; };
 
-    if (warp == K_W) {
-        // ======================= Q and K loads: K(j) chunk by chunk as the MMAs of tile j - 1 let go of them ==========
-        if (lane == 0) {
-            constexpr int CE = 128;  // elements of a 128-byte chunk
-            mbar_arrive_expect_tx(&sm.q_bar, 4 * Q_CHUNK);
-            for (int c = 0; c < 4; c++) tma_load_3d(sm.q[c], &tm_q, &sm.q_bar, c * CE, kvh * G, (int)m0);
-            for (int j = 0; j < n_tiles && !failed; ++j) {
-                for (int c = 0; c < 4; c++) {
-                    if (j > 0) mbar_wait(&sm.k_free[c], (j - 1) & 1, prm.status, 511, failed, 50);
-                    if (failed) break;  // never write into a buffer that may still be read
-                    mbar_arrive_expect_tx(&sm.k_full[c], K_CHUNK);
-                    tma_load_3d(sm.k[c], &tm_k, &sm.k_full[c], c * CE, kvh, j * TILE_K);
+    if (warp >= SOFT_WARPS && warp < MMA_W) {
+        // ======================= K: quants times scales as f16 hi + lo, 64 dims of this CTA's 64 keys at a time =======================
+        // A thread has a key's 32-value block: hi = f16(s * q), lo = s * q - hi, which f16 holds exactly (s * q is a multiple of s's last
+        // place, and hi misses it by 64 of those at most).  What overflows f16, or has a scale that is not finite, makes
+        // infinities of both signs, so NaN scores, and its rows are computed again.
+        const int t = tid - 32 * SOFT_WARPS, key = t >> 1, half = t & 1;
+        const int64_t key_rows = rows0 - (int)rank * 64 - key;  // tiles that start before this hold the key
+        const size_t row_q = (size_t)prm.n_kv * HD, row_s = (size_t)prm.n_kv * (HD / 32);
+        const int8_t* quants = (const int8_t*)prm.k0.data + ((size_t)rank * 64 + key) * row_q + (size_t)kvh * HD + 32 * half;
+        const __half* scales = prm.k0.scales + ((size_t)rank * 64 + key) * row_s + (size_t)kvh * (HD / 32) + half;
+        const int n_chunks = n_tiles * (HD / 64);
+        struct Block {
+            uint4 q[2];
+            __half s;
+        };
+        auto fetch = [&](int n, Block& b) {
+            const int64_t pos0 = (int64_t)(n >> 3) * TILE_K;
+            b.q[0] = b.q[1] = make_uint4(0u, 0u, 0u, 0u);
+            b.s = __float2half_rn(0.0f);
+            if (n >= n_chunks || pos0 >= key_rows) return;
+            const uint4* p = reinterpret_cast<const uint4*>(quants + pos0 * row_q + 64 * (n & 7));
+            b.q[0] = ld_global(p);
+            b.q[1] = ld_global(p + 1);
+            b.s = ld_global(scales + pos0 * row_s + 2 * (n & 7));
+        };
+        auto convert = [&](int n, const Block& b) {
+            const int st = n % NK;
+            if (n >= NK && !mbar_wait_warp(&sm.k_free[st], (n / NK - 1) & 1, prm.status, 511, failed)) return;
+            const __half2 s2 = __half2half2(b.s);
+            const uint2* q = reinterpret_cast<const uint2*>(b.q);
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                __half2 whole[4], hi[4], lo[4];
+                whole_f16x8(q[c], whole);
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    hi[i] = __hmul2(s2, whole[i]);
+                    lo[i] = __hfma2(s2, whole[i], __hneg2(hi[i]));
                 }
+                const uint32_t off = key * 128 + (((4 * half + c) ^ (key & 7)) << 4);
+                *reinterpret_cast<uint4*>(sm.k[st][0] + off) = as_uint4(hi);
+                *reinterpret_cast<uint4*>(sm.k[st][1] + off) = as_uint4(lo);
             }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_pair(at_leader(&sm.k_full[st]));
+        };
+        Block even, odd;  // two chunks' loads under way
+        fetch(0, even);
+        fetch(1, odd);
+        for (int n = 0; n < n_chunks && !failed; n += 2) {
+            convert(n, even);
+            fetch(n + 2, even);
+            if (failed) break;
+            convert(n + 1, odd);
+            fetch(n + 3, odd);
         }
     } else if (warp == V_W) {
         // ======================= V loads in units of 64 keys x 128 dims =======================
-        // It also looks at the scales of K.  An infinite one times a whole sum that is negative would pass as a weight of 0; the
-        // statement multiplies it with every quant, and infinities of both signs make a NaN.  A key with such a scale sends all
-        // rows to that statement.  (The softmax threads, which hold the scales anyway, took 5 us of 530 for it.)
-        uint32_t sc_top = 0;  // largest magnitudes as f16 bits, two at a time: from 0x7C00 on, not finite
         int n = 0;
         for (int j = 0; j < n_tiles && !failed; ++j) {
             const int64_t pos0 = (int64_t)j * TILE_K;
-            uint4 sc[8];  // used at the end of the tile
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int64_t pos = pos0 + 32 * i + lane;
-                const uint4* p = reinterpret_cast<const uint4*>(prm.k0.scales + ((size_t)pos * prm.n_kv + kvh) * 16);
-                const bool key = pos <= min(end, valid_end);
-                sc[2 * i] = key ? ld_global(p) : make_uint4(0u, 0u, 0u, 0u);
-                sc[2 * i + 1] = key ? ld_global(p + 1) : make_uint4(0u, 0u, 0u, 0u);
-            }
-            const bool tail = pos0 + TILE_K - 1 > valid_end;  // the MMA warp computes the same
-            for (int u = 0; u < UNITS; u++, n++) {
+            const bool tail = pos0 + TILE_K - 1 > valid_end;  // the last tile at most: v_here and v_ok of a slot have one phase.  The MMA warp computes the same
+            for (int u = 0; u < 4; u++, n++) {
                 const int st = n % NV;
                 if (n >= NV && !mbar_wait_warp(&sm.v_free[st], (n / NV - 1) & 1, prm.status, 512, failed, 50)) break;
-                const int kh = u & 1, db = block_at(j, u);
-                if (lane == 0) {
-                    mbar_arrive_expect_tx(&sm.v_full[st], V_UNIT);
-                    tma_load_3d(sm.v[st], &tm_v, &sm.v_full[st], db * 128, kvh, (int)pos0 + kh * 64);
-                    tma_load_3d(sm.v[st] + V_UNIT / 2, &tm_v, &sm.v_full[st], db * 128 + 64, kvh, (int)pos0 + kh * 64);
-                }
-                if (tail) {
-                    __syncwarp();
-                    if (!mbar_wait_warp(&sm.v_full[st], (n / NV) & 1, prm.status, 513, failed)) break;
-                    for (int r = lane; r < 64; r += 32) {
-                        if (pos0 + kh * 64 + r <= valid_end) continue;
-#pragma unroll
-                        for (int h = 0; h < 2; h++) {
-                            uint4* row = reinterpret_cast<uint4*>(sm.v[st] + h * (V_UNIT / 2) + r * 128);
-#pragma unroll
-                            for (int i = 0; i < 8; i++) row[i] = make_uint4(0u, 0u, 0u, 0u);
-                        }
+                const int kh = u & 1, dim = dim_block(j, u) * 256 + (int)rank * 128;
+                if (!tail) {
+                    if (lane == 0) {
+                        if (rank == 0) mbar_arrive_expect_tx(&sm.v_full[st], 2 * V_UNIT);
+                        tma_load_3d_pair(sm.v[st], &tm_v, at_leader(&sm.v_full[st]), dim, kvh, (int)pos0 + kh * 64);
+                        tma_load_3d_pair(sm.v[st] + V_UNIT / 2, &tm_v, at_leader(&sm.v_full[st]), dim + 64, kvh, (int)pos0 + kh * 64);
                     }
-                    fence_proxy_async_smem();  // generic-proxy writes, read next by the tensor pipe
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&sm.v_ok[st]);
+                    continue;
                 }
-            }
+                if (lane == 0) {
+                    mbar_arrive_expect_tx(&sm.v_here[st], V_UNIT);
+                    tma_load_3d(sm.v[st], &tm_v, &sm.v_here[st], dim, kvh, (int)pos0 + kh * 64);
+                    tma_load_3d(sm.v[st] + V_UNIT / 2, &tm_v, &sm.v_here[st], dim + 64, kvh, (int)pos0 + kh * 64);
+                }
+                __syncwarp();
+                if (!mbar_wait_warp(&sm.v_here[st], 0, prm.status, 513, failed)) break;
+                for (int r = lane; r < 64; r += 32) {
+                    if (pos0 + kh * 64 + r <= valid_end) continue;
 #pragma unroll
-            for (int i = 0; i < 32; i++) sc_top = __vmaxu2(sc_top, reinterpret_cast<const uint32_t*>(sc)[i] & 0x7FFF7FFFu);
+                    for (int h = 0; h < 2; h++) {
+                        uint4* row = reinterpret_cast<uint4*>(sm.v[st] + h * (V_UNIT / 2) + r * 128);
+#pragma unroll
+                        for (int i = 0; i < 8; i++) row[i] = make_uint4(0u, 0u, 0u, 0u);
+                    }
+                }
+                fence_proxy_async_smem();  // generic-proxy writes, read next by the tensor pipe
+                __syncwarp();
+                if (lane == 0) mbar_arrive_pair(at_leader(&sm.v_ok[st]));
+            }
         }
-        if ((sc_top & 0xFFFFu) >= 0x7C00u || (sc_top >> 16) >= 0x7C00u) sm.redo[0] = sm.redo[1] = 0xFFFFFFFFu;
     } else if (warp == MMA_W) {
-        // ======================= MMA issue =======================
-        if (lane == 0) {
-            constexpr uint32_t IDESC_QK = umma_idesc_i8(TILE_K, ROWS);
-            constexpr uint32_t IDESC_PV = umma_idesc_f16(128, ROWS, 1, 1);
-            const uint64_t dq = umma_desc_sw128(smem_u32(sm.q[0]), 16, 1024), dk = umma_desc_sw128(smem_u32(sm.k[0]), 16, 1024);
+        // ======================= MMA issue, for both CTAs =======================
+        if (rank == 0) {
+            const uint32_t one = elect_one(), tm = warp_uniform(tmem);
+            const int tiles = warp_uniform(n_tiles);
+            constexpr uint32_t IDESC_QK = umma_idesc_f16(2 * ROWS, TILE_K, 0, 0);
+            constexpr uint32_t IDESC_PV = umma_idesc_f16(2 * ROWS, 256, 0, 1);
+            const uint64_t dq = umma_desc_sw128(smem_u32(sm.q[0]), 16, 1024), dk = umma_desc_sw128(smem_u32(sm.k[0][0]), 16, 1024);
             const uint64_t dv = umma_desc_sw128(smem_u32(sm.v[0]), V_UNIT / 2, 1024);
             const uint64_t dp = umma_desc_sw128(smem_u32(sm.p[0]), 16, 1024);
-            uint32_t ok_phase = 0;  // of v_ok, a bit per slot: only tail tiles use it up
             // S of (tile j, group g) into buffer n & 1, n = j * GROUPS + g
             auto issue_qk = [&](int j, int g) {
                 const int n = j * GROUPS + g;
-                if (n >= 2) mbar_wait(&sm.s_free[n & 1], ((n - 2) >> 1) & 1, prm.status, 521, failed);
-                const uint32_t d = tmem + TMEM_S + (n & 1) * S_COLS;
-                const int c = g >> 1;  // 128-byte chunk; the group is its lower or upper two blocks
-                if ((g & 1) == 0) mbar_wait(&sm.k_full[c], j & 1, prm.status, 522, failed);
+                if (n >= 2) mbar_wait_warp(&sm.s_free[n & 1], ((n - 2) >> 1) & 1, prm.status, 521, failed);
+                const uint32_t d = tm + TMEM_S + (n & 1) * S_COLS;
+                const int st = n % NK;
+                mbar_wait_warp(&sm.k_full[st], (n / NK) & 1, prm.status, 522, failed);
                 if (failed) return;
                 tc_fence_after_sync();
 #pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    const uint32_t off = 2 * (2 * (g & 1) + e);
-                    umma_i8_ss(d + e * 64, dk + c * (K_CHUNK >> 4) + off, dq + c * (Q_CHUNK >> 4) + off, IDESC_QK);
-                }
-                if (g & 1) umma_commit(&sm.k_free[c]);
-                umma_commit(&sm.s_ready[n & 1]);
+                for (int e = 0; e < 2; e++)  // the scale blocks of the chunk
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {  // lo, then hi
+                        const uint32_t off = 2 * (2 * e + (i & 1)), hl = 1 - (i >> 1);
+                        umma2_f16_ss(d + e * 64, dq + g * (Q_CHUNK >> 4) + off, dk + (2 * st + hl) * (K_CHUNK >> 4) + off, IDESC_QK, i ? 1u : 0u, one);
+                    }
+                umma2_commit(&sm.k_free[st], one);
+                umma2_commit(&sm.s_ready[n & 1], one);
             };
-            // O^T += V^T P^T for one unit of tile j
-            auto issue_pv = [&](int j, int u, bool tail) {
-                const int n = j * UNITS + u, st = n % NV, kh = u & 1, db = block_at(j, u);
-                mbar_wait(&sm.v_full[st], (n / NV) & 1, prm.status, 523, failed);
-                if (tail) {
-                    mbar_wait(&sm.v_ok[st], (ok_phase >> st) & 1, prm.status, 524, failed);
-                    ok_phase ^= 1u << st;
+            // O += P V for one unit of tile j, the upper or lower halves of P
+            auto issue_pv = [&](int j, int u, int half, bool tail) {
+                const int n = 4 * j + u, st = n % NV, kh = u & 1;
+                if (half == 0) {
+                    if (tail)
+                        mbar_wait_warp(&sm.v_ok[st], 0, prm.status, 524, failed);
+                    else
+                        mbar_wait_warp(&sm.v_full[st], (n / NV) & 1, prm.status, 523, failed);
                 }
                 if (failed) return;
                 tc_fence_after_sync();
-                const uint64_t v = dv + (uint64_t)st * (V_UNIT >> 4), p = dp + kh * (64 * 128 >> 4);
-                const uint32_t d = tmem + TMEM_O + db * 64;
+                const uint64_t v = dv + (uint64_t)st * (V_UNIT >> 4), p = dp + half * (P_TILE >> 4) + kh * (P_HALF >> 4);
+                const uint32_t d = tm + TMEM_O + dim_block(j, u) * 128;
 #pragma unroll
-                for (int half = 0; half < 2; half++)
-#pragma unroll
-                    for (int kk = 0; kk < 4; kk++)
-                        umma_f16_ss(d, v + 128 * kk, p + half * (P_TILE >> 4) + 128 * kk, IDESC_PV, (j > 0 || kh || half || kk) ? 1u : 0u);
-                umma_commit(&sm.v_free[st]);
+                for (int kk = 0; kk < 4; kk++) umma2_f16_ss(d, p + 2 * kk, v + 128 * kk, IDESC_PV, (j > 0 || kh || half || kk) ? 1u : 0u, one);
+                if (half) umma2_commit(&sm.v_free[st], one);
             };
-            mbar_wait(&sm.q_bar, 0, prm.status, 520, failed);
-            if (n_tiles > 0)
-                for (int g = 0; g < GROUPS; g++) issue_qk(0, g);
-            for (int j = 0; j < n_tiles && !failed; ++j) {
-                const bool tail = (int64_t)j * TILE_K + TILE_K - 1 > valid_end, more = j + 1 < n_tiles;
+            for (int g = 0; g < GROUPS; g++) issue_qk(0, g);
+            for (int j = 0; j < tiles && !failed; ++j) {
+                const bool tail = warp_uniform((int)((int64_t)j * TILE_K + TILE_K - 1 > valid_end)) != 0, more = j + 1 < tiles;
                 // the next tile's scores go ahead of this tile's products, and between them
                 int g = 0;
                 for (; more && g < 2; g++) issue_qk(j + 1, g);
-                mbar_wait(&sm.p_ready, j & 1, prm.status, 525, failed);
+                mbar_wait_warp(&sm.p_ready, j & 1, prm.status, 525, failed);
                 if (failed) break;
-                tc_fence_after_sync();
-                for (int u = 0; u < UNITS; u++) {
-                    issue_pv(j, u, tail);
-                    if (u == 1) umma_commit(&sm.first_done);
-                    if (u == UNITS - 1) umma_commit(&sm.pv_done);
+                for (int i = 0; i < 8; i++) {
+                    issue_pv(j, i >> 1, i & 1, tail);
+                    if (i == 3) umma2_commit(&sm.first_done, one);
+                    if (i == 7) umma2_commit(&sm.pv_done, one);
                     if (more && g < GROUPS) issue_qk(j + 1, g++);
                 }
             }
         }
     } else {
-        // ======================= softmax: thread = (key kq * 32 + lane, rows 32 * half ..) =======================
-        const int kq = warp & 3, half = warp >> 2, key = kq * 32 + lane;
-        const uint32_t lane_addr = tmem + ((uint32_t)(kq * 32) << 16);
+        // ======================= softmax: thread = (row, 32 keys of a tile; 64 dims of each block of O) =======================
+        // A row is in lane `row` (keys 0..63, dims 0..127 of a block) and lane 64 + row (the others) of tensor memory, each shared by two warps.
+        const int quarter = warp & 3, half = warp >> 2, tl = quarter * 32 + lane, row = tl & 63, kh = tl >> 6;
+        const int key0 = 64 * kh + 32 * half;  // of the tile
+        const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
+        const uint32_t s_free[2] = {at_leader(&sm.s_free[0]), at_leader(&sm.s_free[1])}, p_ready = at_leader(&sm.p_ready);
+        const int64_t last_key = min(first_qpos + row / G, rows0 - 1) - key0;  // minus the tile's first: the last of this thread's keys that the row sees
         const float scale2 = prm.scale * 1.4426950408889634f;  // > 0 (checked on the host)
-        float2 l2[16];
+        const size_t out_row = ((size_t)(m0 + row / G) * (prm.n_kv * G) + kvh * G + row % G) * HD;
+        bool odd = false;  // a scale or a result that is not finite
 #pragma unroll
-        for (int i = 0; i < 16; i++) l2[i] = make_float2(0.0f, 0.0f);
-        uint4 ks_next[2] = {};
-        auto fetch_scales = [&](int it) {
-            const size_t pos = (size_t)it * TILE_K + key;
-            ks_next[0] = ks_next[1] = make_uint4(0u, 0u, 0u, 0u);
-            if ((int64_t)pos <= valid_end) {
-                const uint4* p = reinterpret_cast<const uint4*>(prm.k0.scales + (pos * prm.n_kv + kvh) * 16);
-                ks_next[0] = ld_global(p);
-                ks_next[1] = ld_global(p + 1);
-            }
-        };
-        if (n_tiles > 0) fetch_scales(0);
+        for (int b = 0; b < 16; b++) odd |= !(fabsf(sm.qs[b][row]) <= 65504.0f);
+        float m_ref = NEG_SENTINEL;
+        float2 l2[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
         // The settled part of this thread's O as 16-bit halves, in this CTA's own share of the output (64 rows x 512 dims x 2 bytes),
-        // which nobody reads before the end.  A step takes 16 of the 32 values of a block; 8 values c of step h at [2 * h + c][thread].
+        // which nobody reads before the end.  A step takes 16 of the 64 values of a block; 8 values c of step h at [2 * h + c][thread].
         uint32_t settled = 0;  // a bit per block
         auto settled_at = [&](int h, int c) {
             const int e = 2 * h + c;
             return reinterpret_cast<uint4*>(prm.out + ((size_t)(m0 + e / 2) * (prm.n_kv * G) + kvh * G) * HD) + (e & 1) * SOFT_THREADS + tid;
         };
-        auto o_at = [&](int h) { return lane_addr + TMEM_O + (h >> 1) * 64 + 32 * half + 16 * (h & 1); };
+        auto o_at = [&](int h) { return lane_addr + TMEM_O + (h >> 2) * 128 + 64 * half + 16 * (h & 3); };
         auto fetch_settled = [&](int h, uint4 (&u)[2]) {
             u[0] = *settled_at(h, 0);
             u[1] = *settled_at(h, 1);
@@ -386,142 +406,108 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
         };
 
         for (int it = 0; it < n_tiles; ++it) {
-            float s[32];
-            {
-                const uint4 ks4[2] = {ks_next[0], ks_next[1]};
-                if (it + 1 < n_tiles) fetch_scales(it + 1);
-                float2 a2[16];
+            float2 s[16];
 #pragma unroll
-                for (int i = 0; i < 16; i++) a2[i] = make_float2(0.0f, 0.0f);
+            for (int i = 0; i < 16; i++) s[i] = make_float2(0.0f, 0.0f);
 #pragma unroll
-                for (int g = 0; g < 8; g++) {
-                    mbar_wait(&sm.s_ready[g & 1], ((it * 8 + g) >> 1) & 1, prm.status, 531, failed);
+            for (int g = 0; g < GROUPS; g++) {
+                mbar_wait(&sm.s_ready[g & 1], ((it * GROUPS + g) >> 1) & 1, prm.status, 531, failed);
+                tc_fence_after_sync();
+                // a block's sums times the row's scale; the second block's are on their way meanwhile
+                auto add = [&](const uint32_t (&r)[32], int block) {
+                    const float q = sm.qs[block][row];
+#pragma unroll
+                    for (int i = 0; i < 16; i++)
+                        s[i] = __ffma2_rn(make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), make_float2(q, q), s[i]);
+                };
+                uint32_t r0[32], r1[32];
+                tmem_ld_32x32b_x32(lane_addr + TMEM_S + (g & 1) * S_COLS + 32 * half, r0);
+                tmem_ld_32x32b_x32(lane_addr + TMEM_S + (g & 1) * S_COLS + 64 + 32 * half, r1);
+                tc_wait_ld();
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_pair(s_free[g & 1]);  // one arrival per warp: they serialise on the barrier's word
+                add(r0, 2 * g);
+                add(r1, 2 * g + 1);
+                if (g == SETTLE_AT && it >= 4 && (it & 1) == 0) {
+                    // the last tile's products of its first block are done, or soon; the tensor pipe goes on with the other's meanwhile
+                    const int db = dim_block(it - 1, 0);
+                    mbar_wait(&sm.first_done, (it - 1) & 1, prm.status, 535, failed);
                     tc_fence_after_sync();
-                    uint32_t r0[32], r1[32];
-                    tmem_ld_32x32b_x32(lane_addr + TMEM_S + (g & 1) * S_COLS + 32 * half, r0);
-                    tmem_ld_32x32b_x32(lane_addr + TMEM_S + (g & 1) * S_COLS + 64 + 32 * half, r1);
-                    tc_wait_ld();
-                    tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&sm.s_free[g & 1]);  // one arrival per warp: they serialise on the barrier's word
-                    const uint32_t w = reinterpret_cast<const uint32_t*>(ks4)[g];
-                    const float2 ks = __half22float2(*reinterpret_cast<const __half2*>(&w));
+                    // every load is under way before the first is used
+                    uint4 u[4][2] = {};
+                    if ((settled >> db) & 1)
 #pragma unroll
-                    for (int e = 0; e < 2; e++) {
-                        const float4* qs = reinterpret_cast<const float4*>(&sm.qs[2 * g + e][32 * half]);
-                        const float2 kk = e ? make_float2(ks.y, ks.y) : make_float2(ks.x, ks.x);
+                        for (int h = 0; h < 4; h++) fetch_settled(4 * db + h, u[h]);
 #pragma unroll
-                        for (int i = 0; i < 8; i++) {
-                            const float4 f = qs[i];
-                            const uint32_t* r = (e ? r1 : r0) + 4 * i;
-                            a2[2 * i] = __ffma2_rn(make_float2((float)(int)r[0], (float)(int)r[1]), __fmul2_rn(kk, make_float2(f.x, f.y)), a2[2 * i]);
-                            a2[2 * i + 1] = __ffma2_rn(make_float2((float)(int)r[2], (float)(int)r[3]), __fmul2_rn(kk, make_float2(f.z, f.w)), a2[2 * i + 1]);
-                        }
+                    for (int h = 0; h < 4; h++) {
+                        uint32_t o[16];
+                        tmem_ld_32x32b_x16(o_at(4 * db + h), o);
+                        tc_wait_ld();
+                        add_settled(u[h], o);
+                        settle(4 * db + h, o);
+                        tmem_st_32x32b_x16(o_at(4 * db + h), o);
                     }
-                    if (g == 3 && it >= 4) {
-                        // the last tile's products of its first block were issued ahead of these scores, and both S buffers are free: the
-                        // tensor pipe goes on meanwhile
-                        const int db = block_at(it - 1, 0);
-                        mbar_wait(&sm.first_done, (it - 1) & 1, prm.status, 535, failed);
-                        tc_fence_after_sync();
-#pragma unroll 1
-                        for (int h = 2 * db; h < 2 * db + 2; h++) {
-                            uint32_t o[16];
-                            uint4 u[2] = {};
-                            if ((settled >> db) & 1) fetch_settled(h, u);
-                            tmem_ld_32x32b_x16(o_at(h), o);
-                            tc_wait_ld();
-                            add_settled(u, o);
-                            settle(h, o);
-                            tmem_st_32x32b_x16(o_at(h), o);
-                        }
-                        tc_wait_st();
-                        settled |= 1u << db;
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    s[2 * i] = a2[i].x;
-                    s[2 * i + 1] = a2[i].y;
+                    tc_wait_st();
+                    settled |= 1u << db;
                 }
             }
 
-            // masks only where the tile crosses the diagonal or the end of the cache: row r (token r / G of the tile) sees the key
-            // from its own position on
+            // masks only where the tile crosses the diagonal or the end of the cache
             const int64_t pos0 = (int64_t)it * TILE_K;
             if (pos0 + TILE_K - 1 > min(first_qpos, rows0 - 1)) {
-                const int from = pos0 + key <= rows0 - 1 ? (int)(pos0 + key - first_qpos) : TOK;
+                const int last = (int)max((int64_t)-1, min((int64_t)TILE_K, last_key - pos0));
 #pragma unroll
-                for (int i = 0; i < 32; i++)
-                    if ((32 * half + i) / G < from) s[i] = -INFINITY;
+                for (int i = 0; i < 16; i++) {
+                    if (2 * i > last) s[i].x = -INFINITY;
+                    if (2 * i + 1 > last) s[i].y = -INFINITY;
+                }
             }
             // does any score exceed its row's reference by more than 2^8?
-            const float4* mr = reinterpret_cast<const float4*>(&sm.m_ref[32 * half]);
-            bool over = false;
-            {
-                const float2 sc2 = make_float2(scale2, scale2);
-                float top = -INFINITY;
+            const float2 sc2 = make_float2(scale2, scale2);
+            float top[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const float4 f = mr[i];
-                    const float2 a = __ffma2_rn(make_float2(s[4 * i], s[4 * i + 1]), sc2, make_float2(-f.x, -f.y));
-                    const float2 b = __ffma2_rn(make_float2(s[4 * i + 2], s[4 * i + 3]), sc2, make_float2(-f.z, -f.w));
-                    top = max3(top, max3(a.x, a.y, b.x), b.y);
-                }
-                over = top > GROW_T;
-            }
-            const bool raise = named_barrier_or(1, SOFT_THREADS, over);
+            for (int i = 0; i < 16; i++) top[i & 3] = max3(top[i & 3], s[i].x, s[i].y);
+            const float most = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])) * scale2;
+            const bool raise = named_barrier_or(1, SOFT_THREADS, most > m_ref + GROW_T);
             if (raise) {
-                float c[32];
-#pragma unroll
-                for (int i = 0; i < 32; i++) c[i] = s[i];
-                sm.red[kq][32 * half + lane] = transpose_reduce<true>(c, lane);
+                sm.red[2 * kh + half][row] = most;
                 named_barrier_sync(2, SOFT_THREADS);
-                if (tid < ROWS) {
-                    const float mx = fmaxf(fmaxf(sm.red[0][tid], sm.red[1][tid]), fmaxf(sm.red[2][tid], sm.red[3][tid])) * scale2;
-                    const float old = sm.m_ref[tid];
-                    const float now = mx > old + GROW_T ? mx : old;
-                    sm.corr[tid] = ex2(old - now);
-                    sm.m_ref[tid] = now;
-                }
-                named_barrier_sync(2, SOFT_THREADS);
-                const float4* cr = reinterpret_cast<const float4*>(&sm.corr[32 * half]);
+                const float mx = fmaxf(fmaxf(sm.red[0][row], sm.red[1][row]), fmaxf(sm.red[2][row], sm.red[3][row]));
+                const float now = mx > m_ref + GROW_T ? mx : m_ref;
+                const float corr = ex2(m_ref - now);
+                m_ref = now;
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const float4 f = cr[i];
-                    l2[2 * i] = __fmul2_rn(l2[2 * i], make_float2(f.x, f.y));
-                    l2[2 * i + 1] = __fmul2_rn(l2[2 * i + 1], make_float2(f.z, f.w));
-                }
-            }
-            if (raise && it > 0) {
-                mbar_wait(&sm.pv_done, (it - 1) & 1, prm.status, 532, failed);
-                tc_fence_after_sync();
+                for (int i = 0; i < 2; i++) l2[i] = __fmul2_rn(l2[i], make_float2(corr, corr));
+                if (it > 0) {
+                    mbar_wait(&sm.pv_done, (it - 1) & 1, prm.status, 532, failed);
+                    tc_fence_after_sync();
 #pragma unroll 1
-                for (int h = 0; h < 2 * DB; h++) {
-                    const bool in_parts = (settled >> (h >> 1)) & 1;
-                    uint32_t o[16];
-                    uint4 u[2];
-                    tmem_ld_32x32b_x16(o_at(h), o);
-                    if (in_parts) fetch_settled(h, u);
-                    tc_wait_ld();
-                    if (in_parts) add_settled(u, o);
+                    for (int h = 0; h < 8; h++) {
+                        const bool in_parts = (settled >> (h >> 2)) & 1;
+                        uint32_t o[16];
+                        uint4 u[2];
+                        tmem_ld_32x32b_x16(o_at(h), o);
+                        if (in_parts) fetch_settled(h, u);
+                        tc_wait_ld();
+                        if (in_parts) add_settled(u, o);
 #pragma unroll
-                    for (int i = 0; i < 16; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * sm.corr[32 * half + 16 * (h & 1) + i]);
-                    if (in_parts) settle(h, o);
-                    tmem_st_32x32b_x16(o_at(h), o);
+                        for (int i = 0; i < 16; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * corr);
+                        if (in_parts) settle(h, o);
+                        tmem_st_32x32b_x16(o_at(h), o);
+                    }
+                    tc_wait_st();
                 }
-                tc_wait_st();
             }
             // P = 2^(s * scale2 - m + 7) as f16 hi + lo; l from the unrounded values
             uint32_t hi[16], lo[16];
             {
-                const float2 sc2 = make_float2(scale2, scale2);
+                const float2 less = make_float2(EXP_BIAS - m_ref, EXP_BIAS - m_ref);
 #pragma unroll
                 for (int i = 0; i < 16; i++) {
-                    const float2 m = reinterpret_cast<const float2*>(mr)[i];
-                    const float2 x = __ffma2_rn(make_float2(s[2 * i], s[2 * i + 1]), sc2, make_float2(EXP_BIAS - m.x, EXP_BIAS - m.y));
+                    const float2 x = __ffma2_rn(s[i], sc2, less);
                     const float2 p = make_float2(ex2(x.x), ex2(x.y));
-                    l2[i] = __fadd2_rn(l2[i], p);
+                    l2[i & 1] = __fadd2_rn(l2[i & 1], p);
                     hi[i] = pack_half2(p.x, p.y);
                     const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hi[i]));
                     lo[i] = pack_half2(p.x - h.x, p.y - h.y);
@@ -529,38 +515,31 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
             }
             if (it > 0) mbar_wait(&sm.pv_done, (it - 1) & 1, prm.status, 533, failed);  // P of the last tile has been read
             {
-                uint8_t* row = sm.p[0] + key * 128;
+                uint8_t* to = sm.p[0] + kh * P_HALF + row * 128;
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
-                    const uint32_t off = ((4 * half + c) ^ (key & 7)) << 4;
-                    *reinterpret_cast<uint4*>(row + off) = make_uint4(hi[4 * c], hi[4 * c + 1], hi[4 * c + 2], hi[4 * c + 3]);
-                    *reinterpret_cast<uint4*>(row + P_TILE + off) = make_uint4(lo[4 * c], lo[4 * c + 1], lo[4 * c + 2], lo[4 * c + 3]);
+                    const uint32_t off = ((4 * half + c) ^ (row & 7)) << 4;
+                    *reinterpret_cast<uint4*>(to + off) = make_uint4(hi[4 * c], hi[4 * c + 1], hi[4 * c + 2], hi[4 * c + 3]);
+                    *reinterpret_cast<uint4*>(to + P_TILE + off) = make_uint4(lo[4 * c], lo[4 * c + 1], lo[4 * c + 2], lo[4 * c + 3]);
                 }
             }
             fence_proxy_async_smem();
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.p_ready);
+            if (lane == 0) mbar_arrive_pair(p_ready);
         }
 
-        // ---- epilogue: thread = output dim db * 128 + key -----------------------------------------------
-        float l[32];
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            l[2 * i] = l2[i].x;
-            l[2 * i + 1] = l2[i].y;
-        }
-        named_barrier_sync(2, SOFT_THREADS);  // every thread is done with red and corr
-        sm.red[kq][32 * half + lane] = transpose_reduce<false>(l, lane);
+        // ---- epilogue -----------------------------------------------
+        named_barrier_sync(2, SOFT_THREADS);  // every thread is done with red
+        sm.red[2 * kh + half][row] = (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y);
         named_barrier_sync(2, SOFT_THREADS);
-        if (tid < ROWS) sm.corr[tid] = 1.0f / ((sm.red[0][tid] + sm.red[1][tid]) + (sm.red[2][tid] + sm.red[3][tid]));
-        named_barrier_sync(2, SOFT_THREADS);
-        if (n_tiles > 0) mbar_wait(&sm.pv_done, (n_tiles - 1) & 1, prm.status, 534, failed);
+        const float inv = 1.0f / ((sm.red[0][row] + sm.red[1][row]) + (sm.red[2][row] + sm.red[3][row]));
+        mbar_wait(&sm.pv_done, (n_tiles - 1) & 1, prm.status, 534, failed);
         tc_fence_after_sync();
         if (settled != 0) {  // whole again before the first result is written over a settled part
 #pragma unroll 1
-            for (int h = 0; h < 2 * DB; h++) {
-                if (((settled >> (h >> 1)) & 1) == 0) continue;
+            for (int h = 0; h < 8; h++) {
+                if (((settled >> (h >> 2)) & 1) == 0) continue;
                 uint32_t o[16];
                 uint4 u[2];
                 tmem_ld_32x32b_x16(o_at(h), o);
@@ -572,31 +551,22 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
             tc_wait_st();
             named_barrier_sync(2, SOFT_THREADS);
         }
-        uint32_t odd = 0;  // also a row with a scale of Q that is not finite (see the V loader)
-        for (int b = 4 * kq; b < 4 * kq + 4; b++)
-            if (!(fabsf(sm.qs[b][32 * half + lane]) <= 65504.0f)) odd |= 1u << lane;
 #pragma unroll 1
-        for (int db = 0; db < DB; db++) {
-            uint32_t o[32];
-            if (n_tiles > 0) {  // uniform over the CTA
-                tmem_ld_32x32b_x32(lane_addr + TMEM_O + db * 64 + 32 * half, o);
-                tc_wait_ld();
-            } else {
+        for (int h = 0; h < 8; h++) {
+            uint32_t o[16], w[8];
+            tmem_ld_32x32b_x16(o_at(h), o);
+            tc_wait_ld();
 #pragma unroll
-                for (int i = 0; i < 32; i++) o[i] = 0u;
+            for (int i = 0; i < 8; i++) {
+                const float a = __uint_as_float(o[2 * i]) * inv, b = __uint_as_float(o[2 * i + 1]) * inv;
+                odd |= !(fabsf(a) <= 3.4e38f) || !(fabsf(b) <= 3.4e38f);
+                w[i] = pack_half2(a, b);
             }
-#pragma unroll
-            for (int i = 0; i < 32; i++) {
-                const int r = 32 * half + i;
-                const float y = __uint_as_float(o[i]) * sm.corr[r];
-                if ((uint32_t)(r / G) < live_tok) {
-                    if (!(fabsf(y) <= 3.4e38f)) odd |= 1u << i;
-                    prm.out[((size_t)(m0 + r / G) * (prm.n_kv * G) + kvh * G + r % G) * HD + db * 128 + key] = __float2half_rn(y);
-                }
-            }
+            uint4* to = reinterpret_cast<uint4*>(prm.out + out_row + (h >> 2) * 256 + kh * 128 + 64 * half + 16 * (h & 3));
+            to[0] = make_uint4(w[0], w[1], w[2], w[3]);
+            to[1] = make_uint4(w[4], w[5], w[6], w[7]);
         }
-        odd = __reduce_or_sync(0xffffffffu, odd);
-        if (odd != 0 && lane == 0) atomicOr(&sm.redo[half], odd);
+        if (odd) atomicOr(&sm.redo[row / 32], 1u << (row % 32));
     }
     // A wait that ran out leaves copies and MMAs of this CTA in flight that nobody will wait for: give them a bounded
     // time to land before the shared and tensor memory they target is handed to the next CTA.
@@ -607,7 +577,8 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
         let_copies_land();
         __syncthreads();
     }
-    if (warp == 0) tmem_dealloc(tmem, TMEM_COLS);
+    pair_sync();  // the pair's MMAs and arrivals reach into both CTAs
+    if (warp == 0) tmem_dealloc_pair(tmem, TMEM_COLS);
     if ((*(volatile uint32_t*)&sm.redo[0] | *(volatile uint32_t*)&sm.redo[1]) != 0) stream_rows(prm, sm, m0, kvh);
 }
 
@@ -630,7 +601,7 @@ int encode_rows(const LaunchArgs& a, CUtensorMap* tm, const void* base, uint64_t
 // bytes, scales and output on 2.
 bool prefill_int8_takes(const KvOperand& k, const KvOperand& v, const void* q, const void* out, uint32_t m, float scale)
 {
-    if (!(scale > 0.0f) || !(scale < 1e30f) || !aligned16(q) || !aligned16(k.scales) || !aligned16(out) || m % (ROWS / G) != 0) return false;
+    if (!(scale > 0.0f) || !(scale < 1e30f) || !aligned16(q) || !aligned16(k.scales) || !aligned16(out) || m % PAIR_TOK != 0) return false;
     for (const KvOperand* o : {&k, &v})
         if (o->rows == 0 || o->rows >= (1u << 30) || !aligned16(o->data)) return false;
     return true;
@@ -640,9 +611,7 @@ int launch_prefill_int8(const LaunchArgs& a, const void* q, const __half* q_scal
                         uint32_t n_kv, uint32_t m, float scale)
 {
     const Int8Params prm{(const uint32_t*)step, (__half*)out, a.status, q_scales, m, n_kv, scale, q, k, v};
-    CUtensorMap tq, tk, tv;
-    if (int r = encode_rows(a, &tq, q, m, n_kv * G, 1, G, ROWS / G)) return r;
-    if (int r = encode_rows(a, &tk, k.data, k.rows, n_kv, 1, 1, TILE_K)) return r;
+    CUtensorMap tv;
     if (int r = encode_rows(a, &tv, v.data, v.rows, n_kv, 2, 1, 64)) return r;
     {
         static std::mutex attr_mutex;
@@ -655,8 +624,8 @@ int launch_prefill_int8(const LaunchArgs& a, const void* q, const __half* q_scal
             if (a.device < 64) attr_set[a.device] = true;
         }
     }
-    const uint32_t q_tiles = (m + ROWS / G - 1) / (ROWS / G);
-    const cudaError_t err = launch_dependent(int8_prefill_kernel, dim3(q_tiles * n_kv), dim3(INT8_THREADS), sizeof(Int8Smem), a.stream, tq, tk, tv, prm);
+    const cudaError_t err = launch_dependent_clusters(int8_prefill_kernel, 2, dim3(2 * (m / PAIR_TOK) * n_kv), dim3(INT8_THREADS), sizeof(Int8Smem), a.stream,
+                                                      tv, prm);
     ++*a.launches;
     return check_cuda(a, err, "attn_prefill_global_flash_sp_iq");
 }

@@ -274,9 +274,9 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
 #pragma unroll
                     for (int kk = 0; kk < 4; kk++)
                         umma_f16_ss(tmem + TMEM_S + (j & 1) * 64, dq + c * (Q_CHUNK >> 4) + 2 * kk, dk + (st * CHUNKS + c) * (K_CHUNK >> 4) + 2 * kk,
-                                    IDESC_QK, (c | kk) ? 1u : 0u);
-                umma_commit(&sm.s_ready[j & 1]);
-                umma_commit(&sm.k_free[st]);
+                                    IDESC_QK, (c | kk) ? 1u : 0u, 1u);
+                umma_commit(&sm.s_ready[j & 1], 1u);
+                umma_commit(&sm.k_free[st], 1u);
             };
             mbar_wait(&sm.q_bar, 0, prm.status, 520, failed);
             for (int j = 0; j < 2 && j < n_tiles; j++) issue_tile(j);
@@ -297,10 +297,10 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
                     const int kk = i >> 1;
-                    umma_f16_ts(tmem + TMEM_O, p + (i & 1) * 32 + kk * 8, dv + (uint64_t)st * (V_TILE >> 4) + 128 * kk, IDESC_PV, (j > 0 || i > 0) ? 1u : 0u);
+                    umma_f16_ts(tmem + TMEM_O, p + (i & 1) * 32 + kk * 8, dv + (uint64_t)st * (V_TILE >> 4) + 128 * kk, IDESC_PV, (j > 0 || i > 0) ? 1u : 0u, 1u);
                 }
-                umma_commit(&sm.pv_done[j & 1]);
-                umma_commit(&sm.v_free[st]);
+                umma_commit(&sm.pv_done[j & 1], 1u);
+                umma_commit(&sm.v_free[st], 1u);
                 if (j + 2 < n_tiles) issue_tile(j + 2);
             }
         }

@@ -76,26 +76,26 @@ __global__ void __launch_bounds__(64, 2) mma_probe_kernel(uint32_t n_mma, unsign
         for (uint32_t i = 0; i < n_mma; i += 16) {
             if (SHAPE != 2) {
 #pragma unroll
-                for (int kk = 0; kk < 4; kk++) umma_f16_ss(tmem, da[0] + 2 * kk, db[0] + 2 * kk, ID_SS, kk ? 1u : 0u);
+                for (int kk = 0; kk < 4; kk++) umma_f16_ss(tmem, da[0] + 2 * kk, db[0] + 2 * kk, ID_SS, kk ? 1u : 0u, 1u);
 #pragma unroll
-                for (int kk = 0; kk < 4; kk++) umma_f16_ss(tmem, da[1] + 2 * kk, db[1] + 2 * kk, ID_SS, 1u);
+                for (int kk = 0; kk < 4; kk++) umma_f16_ss(tmem, da[1] + 2 * kk, db[1] + 2 * kk, ID_SS, 1u, 1u);
             }
             if (SHAPE >= 2) {
 #pragma unroll
-                for (int kk = 0; kk < 8; kk++) umma_f16_ts(tmem + 128, tmem + kk * 8, dv + 128 * kk, ID_PV, kk ? 1u : 0u);
+                for (int kk = 0; kk < 8; kk++) umma_f16_ts(tmem + 128, tmem + kk * 8, dv + 128 * kk, ID_PV, kk ? 1u : 0u, 1u);
             }
             if (SHAPE < 2) {
 #pragma unroll
-                for (int kk = 0; kk < 4; kk++) umma_f16_ss(tmem, da[0] + 2 * kk, db[0] + 2 * kk, ID_SS, kk ? 1u : 0u);
+                for (int kk = 0; kk < 4; kk++) umma_f16_ss(tmem, da[0] + 2 * kk, db[0] + 2 * kk, ID_SS, kk ? 1u : 0u, 1u);
 #pragma unroll
-                for (int kk = 0; kk < 4; kk++) umma_f16_ss(tmem, da[1] + 2 * kk, db[1] + 2 * kk, ID_SS, 1u);
+                for (int kk = 0; kk < 4; kk++) umma_f16_ss(tmem, da[1] + 2 * kk, db[1] + 2 * kk, ID_SS, 1u, 1u);
             }
             if (SHAPE == 2) {
 #pragma unroll
-                for (int kk = 0; kk < 8; kk++) umma_f16_ts(tmem + 128, tmem + kk * 8, dv + 128 * kk, ID_PV, kk ? 1u : 0u);
+                for (int kk = 0; kk < 8; kk++) umma_f16_ts(tmem + 128, tmem + kk * 8, dv + 128 * kk, ID_PV, kk ? 1u : 0u, 1u);
             }
         }
-        umma_commit(&done_bar);
+        umma_commit(&done_bar, 1u);
         const long long t_issued = clock64();
         mbar_wait(&done_bar, 0, status, 901, failed);
         const long long t1 = clock64();

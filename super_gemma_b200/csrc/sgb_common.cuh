@@ -136,30 +136,44 @@ __device__ __forceinline__ void tc_fence_after_sync() { asm volatile("tcgen05.fe
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// D[tmem] (+)= A[smem] * B[smem], f16 inputs, f32 accumulate; issued by ONE thread.
+// MMAs and commits are issued by ONE thread, but the whole warp runs the issuing loop, with `one` set in the elected lane: the
+// operands of tcgen05.mma are uniform registers, which the compiler computes in only where the code around them is uniform.  Moved there
+// from a single thread's registers they cost that thread about 100 cycles an instruction, more than the tensor pipe needs for
+// most: the int8 prefill took 521 us, in uniform code 346.
+__device__ __forceinline__ uint32_t elect_one()
+{
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(e));
+    return e;
+}
+// A value that is the same in all lanes, as one that the compiler knows to be.
+template <typename T>
+__device__ __forceinline__ T warp_uniform(T v) { return __shfl_sync(0xffffffffu, v, 0); }
+// D[tmem] (+)= A[smem] * B[smem], f16 inputs, f32 accumulate.
 __device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                            uint32_t accumulate)
+                                            uint32_t accumulate, uint32_t one)
 {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(one)
         : "memory");
 }
 // Same with the A operand in tensor memory: lane = row, each 32-bit column holds two consecutive
 // f16 elements of K (so a K = 16 step spans 8 columns).
-__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
+__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate, uint32_t one)
 {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(one)
         : "memory");
 }
-// Arrive on an mbarrier once all tcgen05.mma issued so far by this thread have completed.
-__device__ __forceinline__ void umma_commit(uint64_t* bar)
+// Arrive on an mbarrier once all tcgen05.mma issued so far by the elected thread have completed.
+__device__ __forceinline__ void umma_commit(uint64_t* bar, uint32_t one)
 {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+    asm volatile("{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n"
+                 ::"r"(smem_u32(bar)), "r"(one)
                  : "memory");
 }
 

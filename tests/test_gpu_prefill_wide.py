@@ -257,3 +257,13 @@ def test_global_int8_infinite_scale_of_a_key(ctx):
     assert_close(got[:13], clean[:13], ATOL, 2 * RTOL, "queries before it")
     assert np.array_equal(got[:, :16].view(np.uint32), clean[:, :16].view(np.uint32))
     assert np.array_equal(got[:, 24:].view(np.uint32), clean[:, 24:].view(np.uint32))
+
+
+@pytest.mark.parametrize("m,q0,factor", [(16, 104, 1), (16, 112, 1), (16, 120, 1), (32, 120, 2.0**-12), (32, 1000, 2.0**13), (16, 200, 2.0**15)])
+def test_global_int8_pairs_of_ctas(ctx, m, q0, factor):
+    """The two CTAs of a pair end in different tiles (their queries lie on both sides of a multiple of 128), and keys whose scales are subnormal in
+    f16, large, or so large that a quant times its scale overflows f16: those rows are computed again."""
+    q, k, v = _normal(m + q0, m, 32, 512), _normal(q0, q0 + m, 4, 512) * np.float32(factor), _normal(q0 + 2, q0 + m, 4, 512)
+    scale = 0.044194174 / factor
+    got, qd, kd = _iq(ctx, q, k, v, q0, m, scale=scale)
+    assert_close(got, O.attention_f64(qd, kd, v, m, q0, 32, 4, 512, scale), ATOL, RTOL, f"m={m} q0={q0} factor={factor}")
