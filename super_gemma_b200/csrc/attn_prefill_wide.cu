@@ -13,8 +13,9 @@
 // maximum is in l but too small for lo.  The tensor pipe's truncation (2e-9 of the output per key, 2e-6 at 1024 keys) is left in: the error
 // against 64 bits is f16's own, 2.069e-4, as on the streaming kernel.
 // Roles: warps 0-7 softmax, one MMA thread, one K and one V loader; mbarriers only.
-// Measured: 256 queries, 16 kv heads, ring + chunk: 795 us on the streaming kernel, 22.7 here; bound by the chain score -> softmax
-// -> P V of eight tiles plus set-up and merge (3000 cycles a tile, of which the MMAs need 1800).
+// Measured: 256 queries, 16 kv heads, ring + chunk: 795 us on the streaming kernel, 22.7 with one thread running the MMA loop, 20.7 with a
+// warp (sgb_common.cuh); bound by the chain score -> softmax -> P V of eight tiles plus set-up and merge (the MMAs need 1800
+// cycles a tile).
 //
 // What a tile reads beyond a query's own keys must not matter: scores are masked by selection, V rows that hold no key are
 // zeroed.  A V row that is visible to some query of the tile and not finite is visible to all of them as 0 * Inf, so rows that are
@@ -113,7 +114,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
     constexpr int TOK = ROWS / G, CE = 64;  // tokens; elements of a 128-byte chunk
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     WideSmem& sm = *reinterpret_cast<WideSmem*>(smem_raw);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
     const uint32_t rank = blockIdx.x % prm.n_cta, unit = blockIdx.x / prm.n_cta;
     const bool split = prm.n_cta == 2;  // the CTAs of a cluster share the keys
     const bool aligned = (smem_u32(smem_raw) & 1023u) == 0u;  // the swizzled tiles need it; never seen, but never assumed
@@ -257,7 +258,9 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
         }
     } else if (warp == MMA_W) {
         // ======================= MMA issue =======================
-        if (lane == 0) {
+        {
+            const uint32_t one = elect_one(), tm = warp_uniform(tmem);
+            const int tiles = warp_uniform(n_tiles);
             constexpr uint32_t IDESC_QK = umma_idesc_f16(ROWS, TILE_K, 0, 0);
             constexpr uint32_t IDESC_PV = umma_idesc_f16(ROWS, HD, 0, 1);
             const uint64_t dq = umma_desc_sw128(smem_u32(sm.q[0]), 16, 1024), dk = umma_desc_sw128(smem_u32(sm.k[0][0]), 16, 1024);
@@ -266,42 +269,42 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1)
             // Q K^T of tile j, into S buffer j % 2 (free: P V of tile j - 2 was issued before)
             auto issue_tile = [&](int j) {
                 const int st = j % STAGES;
-                mbar_wait(&sm.k_full[st], (j / STAGES) & 1, prm.status, 522, failed);
+                mbar_wait_warp(&sm.k_full[st], (j / STAGES) & 1, prm.status, 522, failed);
                 if (failed) return;
                 tc_fence_after_sync();
 #pragma unroll
                 for (int c = 0; c < CHUNKS; c++)
 #pragma unroll
                     for (int kk = 0; kk < 4; kk++)
-                        umma_f16_ss(tmem + TMEM_S + (j & 1) * 64, dq + c * (Q_CHUNK >> 4) + 2 * kk, dk + (st * CHUNKS + c) * (K_CHUNK >> 4) + 2 * kk,
-                                    IDESC_QK, (c | kk) ? 1u : 0u, 1u);
-                umma_commit(&sm.s_ready[j & 1], 1u);
-                umma_commit(&sm.k_free[st], 1u);
+                        umma_f16_ss(tm + TMEM_S + (j & 1) * 64, dq + c * (Q_CHUNK >> 4) + 2 * kk, dk + (st * CHUNKS + c) * (K_CHUNK >> 4) + 2 * kk,
+                                    IDESC_QK, (c | kk) ? 1u : 0u, one);
+                umma_commit(&sm.s_ready[j & 1], one);
+                umma_commit(&sm.k_free[st], one);
             };
-            mbar_wait(&sm.q_bar, 0, prm.status, 520, failed);
-            for (int j = 0; j < 2 && j < n_tiles; j++) issue_tile(j);
-            for (int j = 0; j < n_tiles && !failed; ++j) {
+            mbar_wait_warp(&sm.q_bar, 0, prm.status, 520, failed);
+            for (int j = 0; j < 2 && j < tiles; j++) issue_tile(j);
+            for (int j = 0; j < tiles && !failed; ++j) {
                 const WideTile t = tile_at(j);
-                const bool tail = t.pos0 + TILE_K - 1 > valid_end(t);
+                const bool tail = warp_uniform((int)(t.pos0 + TILE_K - 1 > valid_end(t))) != 0;
                 const int st = j % STAGES;
-                mbar_wait(&sm.v_full[st], (j / STAGES) & 1, prm.status, 523, failed);
+                mbar_wait_warp(&sm.v_full[st], (j / STAGES) & 1, prm.status, 523, failed);
                 if (tail) {
-                    mbar_wait(&sm.v_ok[st], (ok_phase >> st) & 1, prm.status, 524, failed);
+                    mbar_wait_warp(&sm.v_ok[st], (ok_phase >> st) & 1, prm.status, 524, failed);
                     ok_phase ^= 1u << st;
                 }
-                mbar_wait(&sm.p_ready[j & 1], (j >> 1) & 1, prm.status, 525, failed);
+                mbar_wait_warp(&sm.p_ready[j & 1], (j >> 1) & 1, prm.status, 525, failed);
                 if (failed) break;
                 tc_fence_after_sync();
                 // O += P V in eight instructions (hi and lo of four 16-key steps)
-                const uint32_t p = tmem + TMEM_S + (j & 1) * 64;
+                const uint32_t p = tm + TMEM_S + (j & 1) * 64;
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
                     const int kk = i >> 1;
-                    umma_f16_ts(tmem + TMEM_O, p + (i & 1) * 32 + kk * 8, dv + (uint64_t)st * (V_TILE >> 4) + 128 * kk, IDESC_PV, (j > 0 || i > 0) ? 1u : 0u, 1u);
+                    umma_f16_ts(tm + TMEM_O, p + (i & 1) * 32 + kk * 8, dv + (uint64_t)st * (V_TILE >> 4) + 128 * kk, IDESC_PV, (j > 0 || i > 0) ? 1u : 0u, one);
                 }
-                umma_commit(&sm.pv_done[j & 1], 1u);
-                umma_commit(&sm.v_free[st], 1u);
-                if (j + 2 < n_tiles) issue_tile(j + 2);
+                umma_commit(&sm.pv_done[j & 1], one);
+                umma_commit(&sm.v_free[st], one);
+                if (j + 2 < tiles) issue_tile(j + 2);
             }
         }
     } else {
