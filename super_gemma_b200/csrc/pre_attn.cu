@@ -294,13 +294,13 @@ __device__ __forceinline__ void quant_2x8(const uint32_t (&x)[8], __half (&scale
 // A lane has the octet of dims 8 o .. and the one 64 dims further on that it turns with, so the rotation stays in the lane; it
 // keeps its octets for all of its rows, so the token's cos/sin values and the page lookup are read once and stay in
 // registers.  Bound by issued instructions: 16 lanes a row, which exchanged partners by shuffle and converted what they got,
-// took 40.5 us for 4096 tokens of q, k and v with 16 kv heads, this form 33.0 (120 MB: 18.4 at the copy bandwidth).  What the launcher
+// took 40.5 us for 4096 tokens of q, k and v with 16 kv heads, this form 30.9 (120 MB: 18.4 at the copy bandwidth).  What the launcher
 // chooses is at append_shape.
-constexpr int APPEND_THREADS = 128, APPEND_BLOCKS = 6;
+constexpr int APPEND_THREADS = 128, APPEND_BLOCKS = 8;
 constexpr int ROW_LANES = 8;
-constexpr int MOST_SLOTS = 16;  // groups per token and grid row
+constexpr int MOST_SLOTS = 32;  // groups per token and grid row
 constexpr int ROWS_EACH = 4;   // rows of a group where a launch has more than it takes to fill the GPU
-constexpr int ROWS_AHEAD = 2;  // whose loads are under way at a time
+constexpr int ROWS_AHEAD = 1;  // whose loads are under way at a time: registers for eight blocks an SM are worth more
 
 template <bool PLUS_ONE>
 __global__ void __launch_bounds__(APPEND_THREADS, APPEND_BLOCKS)
@@ -440,13 +440,15 @@ struct AppendShape {
     dim3 grid;
     uint32_t slot_bits;
 };
-// Slots and blocks.  Few rows: one per group, which takes least time for one; beyond, ROWS_EACH of them, which takes least
-// instructions per row, and few rows a token (few kv heads) put several tokens into a block.  us in a recorded chain, 1 row | 4 rows: 16 kv
-// heads with q, 64 tokens 2.7 | 4.3, 150 tokens 3.5 | 4.6, 290 tokens 4.8 | 4.8, 600 tokens 7.6 | 7.0, 4096 tokens 44 | 31.6; 4 kv
-// heads, 1000 tokens 5.2 | 4.7, 8192 tokens 22.3 | 15.2.
+// Slots and blocks.  Few rows: one per group, which takes least time for one; beyond, two, then ROWS_EACH of them, which takes least
+// instructions per row, and few rows a token (few kv heads) put several tokens into a block.  us in a recorded chain, 1 row | 2 | 4: 16 kv
+// heads with q, 64 tokens 2.6 | 3.2 | 4.6, 290 tokens 4.1 | 4.1 | 5.1, 600 tokens 7.4 | 6.9 | 8.4, 1024 tokens 10.5 | 9.3 | 8.9, 4096 tokens
+// 37 | 32 | 30; 4 kv heads, 1000 tokens 4.2 | 3.9 | 5.0, 2000 tokens 6.9 | 5.7 | 6.0, 8192 tokens 19.3 | 15.3 | 14.4.  Six blocks an SM and two
+// rows' loads under way took 31.6 for 4096 tokens, five and four 32.6.
 inline AppendShape append_shape(const LaunchArgs& a, size_t tokens, uint32_t rows)
 {
-    const uint32_t per_thread = tokens * rows <= (size_t)96 * a.sm_count ? 1 : ROWS_EACH;
+    const size_t per_sm = (tokens * rows + a.sm_count - 1) / a.sm_count;
+    const uint32_t per_thread = per_sm <= 64 ? 1 : per_sm <= 384 ? 2 : ROWS_EACH;
     uint32_t bits = 0;
     while ((1u << bits) < MOST_SLOTS && (per_thread << bits) < rows) bits++;
     const size_t groups = tokens << bits;  // < 2^29: at most 2^26 rows of q and of k
