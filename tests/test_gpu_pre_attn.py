@@ -231,7 +231,7 @@ def test_one_launch_qkv_of_a_long_chunk(ctx, tokens, n_kv):
         assert np.array_equal(x.read(), y.read()) and np.any(x.read() != 0)
 
 
-@pytest.mark.parametrize("tokens", [2, 4001])  # a row per group; four, sixteen tokens to a block and the last one short of them
+@pytest.mark.parametrize("tokens", [2, 4001, 15001])  # one, two and four rows per group, with blocks of several tokens and the last one short of them
 @pytest.mark.parametrize("rot", [0, 32, 128])
 def test_fused_kv_append_of_values_that_are_not_finite(ctx, rot, tokens):
     """Weights that make infinities and NaN of some dims: blocks that hold one quantise value by value, with a maximum over what is a number,
