@@ -69,19 +69,10 @@ __device__ __forceinline__ float row_inv_rms(const float (&x)[32])
     return rsqrtf(ss / (float)(BPR * 32) + RMS_EPS);
 }
 
-// y = f16(x * inv * weight) for this thread's block; PLUS_ONE: weight = 1 + w (rmsnorm.wgsl:52-58); w == nullptr: 1.
-template <bool PLUS_ONE>
-__device__ __forceinline__ void apply_norm(float (&x)[32], float inv, const float* w)
-{
-#pragma unroll
-    for (int i = 0; i < 32; i++) {
-        float weight = 1.0f;
-        if (w != nullptr) weight = PLUS_ONE ? 1.0f + ld_global(w + i) : ld_global(w + i);
-        x[i] = round_f16(x[i] * inv * weight);
-    }
-}
-
-// rmsnorm_<ROW_LEN>[_plus1]: x f16[rows x ROW_LEN], w f32[ROW_LEN], y f16.  grid [rows].
+// rmsnorm_<ROW_LEN>[_plus1]: x f16[rows x ROW_LEN], w f32[ROW_LEN], y f16.  grid [rows].  y = f16(x * inv * weight), weight = 1 + w with
+// PLUS_ONE (rmsnorm.wgsl:52-58).  A few rows are one memory latency: the weights are asked for together with the values, 16 bytes at a
+// time where the caller's array allows it (one by one and behind the sum of squares, 32 rows of 512 took 4.0 us in a recorded
+// chain).
 template <int BPR, bool PLUS_ONE>
 __global__ void __launch_bounds__(PRE_THREADS) rmsnorm_kernel(const __half* x, const float* w,
                                                               __half* __restrict__ y, size_t n_blocks)
@@ -90,16 +81,31 @@ __global__ void __launch_bounds__(PRE_THREADS) rmsnorm_kernel(const __half* x, c
     pdl_launch_dependents();
     const size_t blk = (size_t)blockIdx.x * PRE_THREADS + threadIdx.x;
     const bool live = blk < n_blocks;  // whole rows only, and BPR divides 32: a row never straddles a warp
-    float v[32];
+    float v[32], wv[32];
     if (live) {
         load_f16x32(x + blk * 32, v);
+        const float* wp = w + (blk % BPR) * 32;
+        if ((reinterpret_cast<uintptr_t>(w) & 15) == 0) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const float4 f = ld_global(reinterpret_cast<const float4*>(wp) + i);
+                wv[4 * i] = f.x;
+                wv[4 * i + 1] = f.y;
+                wv[4 * i + 2] = f.z;
+                wv[4 * i + 3] = f.w;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 32; i++) wv[i] = ld_global(wp + i);
+        }
     } else {
 #pragma unroll
         for (int i = 0; i < 32; i++) v[i] = 0.0f;
     }
     const float inv = row_inv_rms<BPR>(v);
     if (!live) return;
-    apply_norm<PLUS_ONE>(v, inv, w + (blk % BPR) * 32);
+#pragma unroll
+    for (int i = 0; i < 32; i++) v[i] = v[i] * inv * (PLUS_ONE ? 1.0f + wv[i] : wv[i]);
     uint4 out[4];
     pack_f16x32(v, out);
     uint4* o = reinterpret_cast<uint4*>(y + blk * 32);
