@@ -17,14 +17,16 @@
 // maximum is in l but too small for lo.
 // The tensor pipe truncates an accumulator each time it adds to it: in one accumulator, outputs shrank by 2e-9 of themselves per
 // key (1.7e-5 at 8192 keys, 6.7e-5 at 33280, where the error against 64 bits was 2.22e-4 instead of f16's own 2.08e-4).  From the
-// fifth tile on the softmax threads therefore settle one of the two dim blocks of O in every other tile: the block, plus what was
-// settled of it before, added in f32 with rounding, splits into its upper 16 bits, which they keep in this CTA's share of the
+// fifth tile on one of the two dim blocks of O is therefore settled in every other tile: the block, plus what was
+// settled of it before, added in f32 with rounding, splits into its upper 16 bits, which stay in this CTA's share of the
 // output, and the exact rest, from which the tensor pipe goes on; what it adds to stays as small as the sum of a few tiles.
-// The block comes first in the products before it is settled, so the tensor pipe is at the other meanwhile.
+// The block comes first in the products before it is settled, so the tensor pipe is at the other meanwhile, and the warps that make
+// the keys do it, which have time (the softmax threads, whose chain the tile's time is, took 1500 cycles a tile for it).
 // Roles: warps 0-7 softmax (a row in four threads), 8-11 K, one MMA warp (the even CTA's issues for both), one V loader; mbarriers only.
-// Measured, 256 queries at 7936 + 256 keys: 13500 us on the streaming kernel, 529 in the transposed form, 346 here (floor 82).  A tile takes
-// 9000 cycles, of which the MMAs need 4900; the softmax threads wait for scores 1700, read and scale them 3100, settle 1500
-// and turn them into P 1700.
+// Measured, 256 queries at 7936 + 256 keys with the appends and the quantisation of q: 13500 us on the streaming kernel, 529 in the
+// transposed form, 345 here (floor 82).  The MMAs need 4900 cycles of a tile's 8500; the rest is the chain of the softmax threads: a
+// hand-over of scores has to be read before the buffer takes the one after the next, eight times a tile.  Products issued one or
+// two units earlier among the scores: 352 and 372 us for 346.
 //
 // What a tile reads beyond a query's own keys must not matter: scores are masked by selection, V rows that hold no key are
 // zeroed.  A V row that is visible to some query of the tile and not finite is visible to all of them as 0 * Inf, so rows that are
@@ -60,7 +62,8 @@ constexpr int GROUPS = 8;                      // S hand-overs per tile, two sca
 constexpr uint32_t S_COLS = 128;               // columns of one hand-over
 constexpr uint32_t TMEM_O = 0, TMEM_S = 256, TMEM_COLS = 512;
 static_assert(TMEM_S + 2 * S_COLS <= TMEM_COLS, "O and two S buffers fit");
-constexpr int SETTLE_AT = 5;                   // the hand-over whose scores the tensor pipe computes behind the first block's products
+constexpr int SETTLE_FROM = 4;                 // the first tile in which a dim block is settled; one in every other tile from there on
+constexpr int SETTLE_CHUNK = 4;                // of K, even: the settling comes behind this one and the next
 constexpr float EXP_BIAS = 7.0f, GROW_T = 8.0f;
 
 struct Int8Smem {
@@ -70,7 +73,8 @@ struct Int8Smem {
     uint8_t v[NV][V_UNIT];
     float qs[HD / 32][ROWS];      // scales of Q, [block][row]
     float red[4][ROWS];
-    uint64_t k_full[NK], k_free[NK], v_full[NV], v_free[NV], v_here[NV], v_ok[NV], s_ready[2], s_free[2], p_ready, first_done, pv_done;
+    uint64_t k_full[NK], k_free[NK], v_full[NV], v_free[NV], v_here[NV], v_ok[NV], s_ready[2], s_free[2], p_ready, first_done, pv_done,
+        settle_here, settle_ok;
     uint32_t tmem_base, abort;
     uint32_t redo[ROWS / 32];  // rows that are not finite, a bit each
 };
@@ -101,6 +105,13 @@ __device__ __forceinline__ uint4 as_uint4(const __half2 (&h)[4])
 {
     const uint32_t* w = reinterpret_cast<const uint32_t*>(h);
     return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// Keeps what uses a load's registers behind the wait for it.
+__device__ __forceinline__ void loaded(uint32_t (&r)[32])
+{
+    asm volatile("" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]),
+                      "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31]));
 }
 
 // The rows that are not finite by the streaming statement, a warp per pair of heads.
@@ -162,6 +173,8 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
         }
         mbar_init(&sm.p_ready, 2 * SOFT_WARPS);
         mbar_init(&sm.first_done, 1);
+        mbar_init(&sm.settle_here, K_WARPS);
+        mbar_init(&sm.settle_ok, 2 * K_WARPS);
         mbar_init(&sm.pv_done, 1);
         sm.abort = 0;
         sm.redo[0] = sm.redo[1] = 0;
@@ -196,6 +209,43 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
     // V unit u of tile j: 64 keys (half u & 1) of this CTA's 128 of the 256 dims of block dim_block(j, u); the blocks take turns in
     // coming first, so that the first can be settled while the tensor pipe is at the other
     auto dim_block = [](int j, int u) { return ((u >> 1) + (j >> 1)) & 1; };
+
+    // The settled part of O as 16-bit halves, in this CTA's own share of the output (64 rows x 512 dims x 2 bytes), which nobody reads
+    // before the end: 8 values c of step h (16 of a row's dims) of softmax thread t at [2 * h + c][t].
+    auto settled_at = [&](int t, int h, int c) {
+        const int e = 2 * h + c;
+        return reinterpret_cast<uint4*>(prm.out + ((size_t)(m0 + e / 2) * (prm.n_kv * G) + kvh * G) * HD) + (e & 1) * SOFT_THREADS + t;
+    };
+    auto fetch_settled = [&](int t, int h, uint4 (&u)[2]) {
+        u[0] = *settled_at(t, h, 0);
+        u[1] = *settled_at(t, h, 1);
+    };
+    auto add_settled = [&](const uint4 (&u)[2], uint32_t (&o)[16]) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const uint32_t w = reinterpret_cast<const uint32_t*>(u)[i];
+            o[2 * i] = __float_as_uint(__fadd_rn(__uint_as_float(o[2 * i]), __uint_as_float(w << 16)));
+            o[2 * i + 1] = __float_as_uint(__fadd_rn(__uint_as_float(o[2 * i + 1]), __uint_as_float(w & 0xFFFF0000u)));
+        }
+    };
+    auto settle = [&](int t, int h, uint32_t (&o)[16]) {  // o: whole values, left as the rest
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            uint32_t w[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                uint32_t &a = o[8 * c + 2 * k], &b = o[8 * c + 2 * k + 1];
+                w[k] = __byte_perm(a, b, 0x7632);
+                a = __float_as_uint(__uint_as_float(a) - __uint_as_float(a & 0xFFFF0000u));
+                b = __float_as_uint(__uint_as_float(b) - __uint_as_float(b & 0xFFFF0000u));
+            }
+            *settled_at(t, h, c) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+    };
+    // dim blocks that have a settled part once tile `it` has had its turn
+    auto settled_by = [&](int it) { return it < SETTLE_FROM ? 0u : it < SETTLE_FROM + 2 ? 1u << dim_block(SETTLE_FROM - 1, 0) : 3u; };
+    auto settles = [](int it) { return it >= SETTLE_FROM && (it & 1) == 0; };
+    auto settle_phase = [](int it) { return ((it - SETTLE_FROM) >> 1) & 1; };
 
     if (warp >= SOFT_WARPS && warp < MMA_W) {
         // ======================= K: quants times scales as f16 hi + lo, 64 dims of this CTA's 64 keys at a time =======================
@@ -253,6 +303,43 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
             if (failed) break;
             convert(n + 1, odd);
             fetch(n + 3, odd);
+            const int it = n >> 3;
+            if ((n & 7) == SETTLE_CHUNK && settles(it) && !failed) {
+                // The products of the last tile's first block are done, or soon; the tensor pipe is at the other's and this tile's scores
+                // meanwhile.  These warps have the time, and the 64 lanes and their twins that the softmax threads' parts are named by.
+                const int db = dim_block(it - 1, 0), quarter = warp & 3;
+                const uint32_t block = tmem + ((uint32_t)(quarter * 32) << 16) + TMEM_O + db * 128;
+                const bool before = ((settled_by(it - 1) >> db) & 1) != 0;
+#pragma unroll 1
+                for (int half = 0; half < 2; half++) {
+                    const int owner = half * 128 + quarter * 32 + lane;
+                    uint4 u[4][2] = {};
+                    if (before)
+#pragma unroll
+                        for (int h = 0; h < 4; h++) fetch_settled(owner, 4 * db + h, u[h]);
+                    if (half == 0) {
+                        mbar_wait_warp(&sm.first_done, (it - 1) & 1, prm.status, 535, failed);
+                        tc_fence_after_sync();
+                    }
+#pragma unroll
+                    for (int h = 0; h < 4; h++) {
+                        uint32_t o[16];
+                        tmem_ld_32x32b_x16(block + 64 * half + 16 * h, o);
+                        tc_wait_ld();
+                        add_settled(u[h], o);
+                        settle(owner, 4 * db + h, o);
+                        tmem_st_32x32b_x16(block + 64 * half + 16 * h, o);
+                    }
+                }
+                tc_wait_st();
+                tc_fence_before_sync();
+                __threadfence_block();  // the parts are read by the softmax threads
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(&sm.settle_here);
+                    mbar_arrive_pair(at_leader(&sm.settle_ok));
+                }
+            }
         }
     } else if (warp == V_W) {
         // ======================= V loads in units of 64 keys x 128 dims =======================
@@ -348,6 +435,7 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
                 mbar_wait_warp(&sm.p_ready, j & 1, prm.status, 525, failed);
                 if (failed) break;
                 for (int i = 0; i < 8; i++) {
+                    if (i == 4 && settles(j)) mbar_wait_warp(&sm.settle_ok, settle_phase(j), prm.status, 526, failed);  // the other block has been settled
                     issue_pv(j, i >> 1, i & 1, tail);
                     if (i == 3) umma2_commit(&sm.first_done, one);
                     if (i == 7) umma2_commit(&sm.pv_done, one);
@@ -370,86 +458,41 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
         for (int b = 0; b < 16; b++) odd |= !(fabsf(sm.qs[b][row]) <= 65504.0f);
         float m_ref = NEG_SENTINEL;
         float2 l2[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
-        // The settled part of this thread's O as 16-bit halves, in this CTA's own share of the output (64 rows x 512 dims x 2 bytes),
-        // which nobody reads before the end.  A step takes 16 of the 64 values of a block; 8 values c of step h at [2 * h + c][thread].
-        uint32_t settled = 0;  // a bit per block
-        auto settled_at = [&](int h, int c) {
-            const int e = 2 * h + c;
-            return reinterpret_cast<uint4*>(prm.out + ((size_t)(m0 + e / 2) * (prm.n_kv * G) + kvh * G) * HD) + (e & 1) * SOFT_THREADS + tid;
-        };
         auto o_at = [&](int h) { return lane_addr + TMEM_O + (h >> 2) * 128 + 64 * half + 16 * (h & 3); };
-        auto fetch_settled = [&](int h, uint4 (&u)[2]) {
-            u[0] = *settled_at(h, 0);
-            u[1] = *settled_at(h, 1);
-        };
-        auto add_settled = [&](const uint4 (&u)[2], uint32_t (&o)[16]) {
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const uint32_t w = reinterpret_cast<const uint32_t*>(u)[i];
-                o[2 * i] = __float_as_uint(__fadd_rn(__uint_as_float(o[2 * i]), __uint_as_float(w << 16)));
-                o[2 * i + 1] = __float_as_uint(__fadd_rn(__uint_as_float(o[2 * i + 1]), __uint_as_float(w & 0xFFFF0000u)));
-            }
-        };
-        auto settle = [&](int h, uint32_t (&o)[16]) {  // o: whole values, left as the rest
-#pragma unroll
-            for (int c = 0; c < 2; c++) {
-                uint32_t w[4];
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    uint32_t &a = o[8 * c + 2 * k], &b = o[8 * c + 2 * k + 1];
-                    w[k] = __byte_perm(a, b, 0x7632);
-                    a = __float_as_uint(__uint_as_float(a) - __uint_as_float(a & 0xFFFF0000u));
-                    b = __float_as_uint(__uint_as_float(b) - __uint_as_float(b & 0xFFFF0000u));
-                }
-                *settled_at(h, c) = make_uint4(w[0], w[1], w[2], w[3]);
-            }
-        };
-
         for (int it = 0; it < n_tiles; ++it) {
             float2 s[16];
 #pragma unroll
             for (int i = 0; i < 16; i++) s[i] = make_float2(0.0f, 0.0f);
-#pragma unroll
-            for (int g = 0; g < GROUPS; g++) {
+            // Block by block: the sums of the next are on their way out of tensor memory while one's are scaled by the row's scale.
+            uint32_t r[2][32];
+            auto ready = [&](int g) {
                 mbar_wait(&sm.s_ready[g & 1], ((it * GROUPS + g) >> 1) & 1, prm.status, 531, failed);
                 tc_fence_after_sync();
-                // a block's sums times the row's scale; the second block's are on their way meanwhile
-                auto add = [&](const uint32_t (&r)[32], int block) {
-                    const float q = sm.qs[block][row];
+            };
+            auto at = [&](int n) { return lane_addr + TMEM_S + ((n >> 1) & 1) * S_COLS + (n & 1) * 64 + 32 * half; };
+            ready(0);
+            tmem_ld_32x32b_x32(at(0), r[0]);
+            tc_wait_ld();
+            loaded(r[0]);
 #pragma unroll
-                    for (int i = 0; i < 16; i++)
-                        s[i] = __ffma2_rn(make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), make_float2(q, q), s[i]);
-                };
-                uint32_t r0[32], r1[32];
-                tmem_ld_32x32b_x32(lane_addr + TMEM_S + (g & 1) * S_COLS + 32 * half, r0);
-                tmem_ld_32x32b_x32(lane_addr + TMEM_S + (g & 1) * S_COLS + 64 + 32 * half, r1);
-                tc_wait_ld();
-                tc_fence_before_sync();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_pair(s_free[g & 1]);  // one arrival per warp: they serialise on the barrier's word
-                add(r0, 2 * g);
-                add(r1, 2 * g + 1);
-                if (g == SETTLE_AT && it >= 4 && (it & 1) == 0) {
-                    // the last tile's products of its first block are done, or soon; the tensor pipe goes on with the other's meanwhile
-                    const int db = dim_block(it - 1, 0);
-                    mbar_wait(&sm.first_done, (it - 1) & 1, prm.status, 535, failed);
-                    tc_fence_after_sync();
-                    // every load is under way before the first is used
-                    uint4 u[4][2] = {};
-                    if ((settled >> db) & 1)
+            for (int n = 0; n < 2 * GROUPS; n++) {
+                const int g = n >> 1;
+                if (n & 1) {
+                    if (g + 1 < GROUPS) ready(g + 1);
+                }
+                if (n + 1 < 2 * GROUPS) tmem_ld_32x32b_x32(at(n + 1), r[(n + 1) & 1]);
+                const float q = sm.qs[n][row];
 #pragma unroll
-                        for (int h = 0; h < 4; h++) fetch_settled(4 * db + h, u[h]);
-#pragma unroll
-                    for (int h = 0; h < 4; h++) {
-                        uint32_t o[16];
-                        tmem_ld_32x32b_x16(o_at(4 * db + h), o);
-                        tc_wait_ld();
-                        add_settled(u[h], o);
-                        settle(4 * db + h, o);
-                        tmem_st_32x32b_x16(o_at(4 * db + h), o);
-                    }
-                    tc_wait_st();
-                    settled |= 1u << db;
+                for (int i = 0; i < 16; i++)
+                    s[i] = __ffma2_rn(make_float2(__uint_as_float(r[n & 1][2 * i]), __uint_as_float(r[n & 1][2 * i + 1])), make_float2(q, q), s[i]);
+                if (n + 1 < 2 * GROUPS) {
+                    tc_wait_ld();
+                    loaded(r[(n + 1) & 1]);
+                }
+                if ((n & 1) == 0) {  // both blocks of the hand-over are in registers
+                    tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_pair(s_free[g & 1]);  // one arrival per warp: they serialise on the barrier's word
                 }
             }
 
@@ -481,22 +524,24 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
                 for (int i = 0; i < 2; i++) l2[i] = __fmul2_rn(l2[i], make_float2(corr, corr));
                 if (it > 0) {
                     mbar_wait(&sm.pv_done, (it - 1) & 1, prm.status, 532, failed);
+                    if (settles(it)) mbar_wait(&sm.settle_here, settle_phase(it), prm.status, 536, failed);
                     tc_fence_after_sync();
 #pragma unroll 1
                     for (int h = 0; h < 8; h++) {
-                        const bool in_parts = (settled >> (h >> 2)) & 1;
+                        const bool in_parts = (settled_by(it) >> (h >> 2)) & 1;
                         uint32_t o[16];
                         uint4 u[2];
                         tmem_ld_32x32b_x16(o_at(h), o);
-                        if (in_parts) fetch_settled(h, u);
+                        if (in_parts) fetch_settled(tid, h, u);
                         tc_wait_ld();
                         if (in_parts) add_settled(u, o);
 #pragma unroll
                         for (int i = 0; i < 16; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * corr);
-                        if (in_parts) settle(h, o);
+                        if (in_parts) settle(tid, h, o);
                         tmem_st_32x32b_x16(o_at(h), o);
                     }
                     tc_wait_st();
+                    __threadfence_block();  // the parts are read by the warps that settle
                 }
             }
             // P = 2^(s * scale2 - m + 7) as f16 hi + lo; l from the unrounded values
@@ -536,14 +581,17 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
         const float inv = 1.0f / ((sm.red[0][row] + sm.red[1][row]) + (sm.red[2][row] + sm.red[3][row]));
         mbar_wait(&sm.pv_done, (n_tiles - 1) & 1, prm.status, 534, failed);
         tc_fence_after_sync();
+        const uint32_t settled = settled_by(n_tiles - 1);
         if (settled != 0) {  // whole again before the first result is written over a settled part
+            const int last = (n_tiles - 1) & ~1;  // the last tile with a settling
+            mbar_wait(&sm.settle_here, settle_phase(last), prm.status, 537, failed);
 #pragma unroll 1
             for (int h = 0; h < 8; h++) {
                 if (((settled >> (h >> 2)) & 1) == 0) continue;
                 uint32_t o[16];
                 uint4 u[2];
                 tmem_ld_32x32b_x16(o_at(h), o);
-                fetch_settled(h, u);
+                fetch_settled(tid, h, u);
                 tc_wait_ld();
                 add_settled(u, o);
                 tmem_st_32x32b_x16(o_at(h), o);
