@@ -548,8 +548,8 @@ int run_flash(const LaunchArgs& a, const BufView& q, const BufView& k0, const Bu
     const size_t rows = (size_t)m_tokens * n_q;
     int pieces = TWO_SRC ? 1 : choose_pieces((size_t)q_tiles * n_kv, 2 * a.sm_count, k_rows);
     // Many keys per CTA and several CTAs per SM one after the other: the kernel with 128-key tiles and one CTA per SM, which takes
-    // 5 % less time per key and 3 tiles' time more per CTA (131072 keys, two pieces, with the dequantisation: 8520 us here, 8211 there; 8192 queries over themselves
-    // 593 and 623).  The pieces are those of this kernel, so that no sum in the tensor pipe gets longer.
+    // 5 % less time per key and 3 tiles' time more per CTA (131072 keys, two pieces, with the dequantisation: 8543 us here, 8211 there; 8192 queries over themselves
+    // 593 and 627).  The pieces are those of this kernel, so that no sum in the tensor pipe gets longer.
     bool long_tiles = !TWO_SRC && window == 0 && k_rows / pieces >= 16384 && (size_t)q_tiles * n_kv * pieces >= (size_t)4 * a.sm_count;
     if (const char* e = getenv("SGB_FLASH_LONG")) long_tiles = !TWO_SRC && window == 0 && e[0] == '1';  // tuning and test aid
     const uint32_t box_rows = long_tiles ? LONG_BLOCK_N : BLOCK_N;

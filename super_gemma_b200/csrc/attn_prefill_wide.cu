@@ -12,7 +12,7 @@
 // carries +7, so that lo stays clear of f16's subnormals (the factor cancels in O / l); a p below 2^-32 of its row's reference
 // maximum is in l but too small for lo.  The tensor pipe's truncation (2e-9 of the output per key, 2e-6 at 1024 keys) is left in: the error
 // against 64 bits is f16's own, 2.069e-4, as on the streaming kernel.
-// Roles: warps 0-7 softmax, one MMA thread, one K and one V loader; mbarriers only.
+// Roles: warps 0-7 softmax, one MMA warp, one K and one V loader; mbarriers only.
 // Measured: 256 queries, 16 kv heads, ring + chunk: 795 us on the streaming kernel, 22.7 with one thread running the MMA loop, 20.7 with a
 // warp (sgb_common.cuh); bound by the chain score -> softmax -> P V of eight tiles plus set-up and merge (the MMAs need 1800
 // cycles a tile).
