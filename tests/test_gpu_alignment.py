@@ -124,3 +124,16 @@ def test_global_int8_operands_on_their_own_alignment(ctx, which):
     ctx.dispatch_blocking(ctx.load_kernel("attn_prefill_global_flash_sp_iq"), bind(*bufs, out, _step(ctx, q0=q0)), 512**-0.5, [32, 1, 1])
     want = O.attention_f64(qd.reshape(q.shape), kd.reshape(k.shape), v.astype(np.float32), m, q0, 32, 4, 512, 512**-0.5)
     assert_close(O.f16_bits_to_f32(out.read()).reshape(m, 32, 512), want, 5e-5, 2.0**-11)
+
+
+@pytest.mark.parametrize("name,n", [("rmsnorm_256", 256), ("rmsnorm_512_plus1", 512)])
+def test_rmsnorm_weights_on_their_own_alignment(ctx, name, n):
+    """Weights on 4 bytes come one by one, on 16 four at a time: the same bits, also past the first block of rows."""
+    rows = 40
+    x, w = normal_f16(7, rows, n), np.random.default_rng(8).standard_normal(n, dtype=np.float32)
+    got = []
+    for by in (0, 4):
+        y = ctx.new_buffer(rows * n, np.uint16)
+        ctx.dispatch_blocking(ctx.load_kernel(name), bind(ctx.buffer_from_iter(x), _moved(ctx, w, by), y), None, [rows, 1, 1])
+        got.append(y.read())
+    assert np.array_equal(*got) and np.any(got[0] != 0)
