@@ -39,9 +39,9 @@ SCALE = 1.0 / math.sqrt(D)
 SEED = 0x5605
 
 
-# dram__bytes_read.sum + dram__bytes_write.sum of one flash launch, from an ncu capture of this
+# dram__bytes_read.sum + dram__bytes_write.sum of one flash_prefill_kernel launch, from an ncu capture of this
 # script (summarised under profiles/), keyed by (m, ctx, n_gpus).  Other shapes: not captured.
-FLASH_DRAM_BYTES = {(4096, 131072, 1): 1540000000 + 131430000}
+FLASH_DRAM_BYTES = {(4096, 131072, 1): 1358588672 + 123469312}
 
 
 def peaks():
@@ -852,7 +852,7 @@ def main():
             "warmup": args.warmup, "ms_per_step": head["ms_per_step"], "higher_is_better": True, "scaling": "strong",
             "vs_baseline": None, "dtype": "f16 x f16 -> f32 (Q8_0 K/V dequantised to f16)", "data": "synthetic",
             "config": workload_config(args, world),
-            "roofline": {"bound": "tensor", "kernel": "flash_long_kernel, flash_prefill_kernel (attn_prefill_flash_f16_d128)", "achieved": achieved,
+            "roofline": {"bound": "tensor", "kernel": "flash_prefill_kernel (attn_prefill_flash_f16_d128)", "achieved": achieved,
                          "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                          "peak_kind": f"{pk['kind']} bf16 {'sustained' if long_run else 'burst'}",
                          "traffic": FLASH_DRAM_BYTES.get((args.m, args.ctx, world)),

@@ -26,7 +26,6 @@
 #include <mutex>
 #include <utility>
 
-#include "attn_flash.cuh"
 #include "sgb_common.cuh"
 #include "sgb_kernels.h"
 
@@ -76,6 +75,19 @@ struct FlashSmem {
 static_assert(sizeof(FlashSmem) == 6 * 2 * HALF_TILE + 128, "tiles + barriers, no padding");
 static_assert(2 * (sizeof(FlashSmem) + 1024) <= 228 * 1024, "two CTAs per SM");
 
+struct FlashParams {
+    const uint32_t* step;
+    float* out;
+    float* part_acc;     // pieces > 1: [row][piece][128] unnormalised O
+    float* part_ml;      // pieces > 1: [row][piece][2] = running max (base-2 exponent units), sum
+    uint32_t* status;
+    uint32_t m_tokens;   // query tokens in the chunk
+    uint32_t n_kv;
+    uint32_t window;     // 0 = none
+    uint32_t ring;       // TWO_SRC: ring slots
+    float scale;
+    uint32_t head_group; // kv heads whose query tiles are interleaved in launch order (divides n_kv)
+};
 
 // One 64-key tile: where it comes from and which absolute positions its rows hold.
 struct Tile {
@@ -543,20 +555,10 @@ int run_flash(const LaunchArgs& a, const BufView& q, const BufView& k0, const Bu
     if (q.bytes < (size_t)m_tokens * n_q * HD * 2) return fail_validation(a, "flash prefill: q buffer too small");
     if (out.bytes < (size_t)m_tokens * n_q * HD * 4) return fail_validation(a, "flash prefill: out buffer too small");
     if (step.bytes < 16) return fail_validation(a, "flash prefill: the step buffer holds 4 x u32");
-    const size_t k_rows = k0.bytes / ((size_t)n_kv * HD * 2);
-    const uint32_t q_tiles = (m_tokens + BLOCK_TOK - 1) / BLOCK_TOK;
-    const size_t rows = (size_t)m_tokens * n_q;
-    int pieces = TWO_SRC ? 1 : choose_pieces((size_t)q_tiles * n_kv, 2 * a.sm_count, k_rows);
-    // Many keys per CTA and several CTAs per SM one after the other: the kernel with 128-key tiles and one CTA per SM, which takes
-    // 5 % less time per key and 3 tiles' time more per CTA (131072 keys, two pieces, with the dequantisation: 8543 us here, 8211 there; 8192 queries over themselves
-    // 593 and 627).  The pieces are those of this kernel, so that no sum in the tensor pipe gets longer.
-    bool long_tiles = !TWO_SRC && window == 0 && k_rows / pieces >= 16384 && (size_t)q_tiles * n_kv * pieces >= (size_t)4 * a.sm_count;
-    if (const char* e = getenv("SGB_FLASH_LONG")) long_tiles = !TWO_SRC && window == 0 && e[0] == '1';  // tuning and test aid
-    const uint32_t box_rows = long_tiles ? LONG_BLOCK_N : BLOCK_N;
     CUtensorMap tq, tk0, tv0, tk1, tv1;
     if (int r = encode_qkv_map(a, &tq, BufView{q.ptr, (size_t)m_tokens * n_q * HD * 2}, n_q, G, BLOCK_TOK, "q")) return r;
-    if (int r = encode_qkv_map(a, &tk0, k0, n_kv, 1, box_rows, "k")) return r;
-    if (int r = encode_qkv_map(a, &tv0, v0, n_kv, 1, box_rows, "v")) return r;
+    if (int r = encode_qkv_map(a, &tk0, k0, n_kv, 1, BLOCK_N, "k")) return r;
+    if (int r = encode_qkv_map(a, &tv0, v0, n_kv, 1, BLOCK_N, "v")) return r;
     if (TWO_SRC) {
         if (k0.bytes < (size_t)ring * n_kv * HD * 2 || v0.bytes < (size_t)ring * n_kv * HD * 2)
             return fail_validation(a, "flash prefill: ring buffers smaller than the ring");
@@ -580,6 +582,10 @@ int run_flash(const LaunchArgs& a, const BufView& q, const BufView& k0, const Bu
             attr_set[TWO_SRC][a.device] = true;
         }
     }
+    const size_t k_rows = k0.bytes / ((size_t)n_kv * HD * 2);
+    const uint32_t q_tiles = (m_tokens + BLOCK_TOK - 1) / BLOCK_TOK;
+    const size_t rows = (size_t)m_tokens * n_q;
+    int pieces = TWO_SRC ? 1 : choose_pieces((size_t)q_tiles * n_kv, 2 * a.sm_count, k_rows);
     float* part_acc = nullptr;
     float* part_ml = nullptr;
     if (pieces > 1) {
@@ -625,8 +631,7 @@ int run_flash(const LaunchArgs& a, const BufView& q, const BufView& k0, const Bu
     }
     FlashParams prm{(const uint32_t*)step.ptr, (float*)out.ptr, part_acc, part_ml, a.status, m_tokens, n_kv, window, ring, scale, head_group};
     const dim3 grid(q_tiles * n_kv, 1, pieces);
-    const cudaError_t e = long_tiles ? launch_flash_long(a, tq, tk0, tv0, prm, q_tiles * n_kv, pieces)
-                                     : launch_dependent(flash_prefill_kernel<TWO_SRC>, grid, dim3(FLASH_THREADS), smem, a.stream, tq, tk0, tv0, tk1, tv1, prm);
+    const cudaError_t e = launch_dependent(flash_prefill_kernel<TWO_SRC>, grid, dim3(FLASH_THREADS), smem, a.stream, tq, tk0, tv0, tk1, tv1, prm);
     ++*a.launches;
     if (int r = check_cuda(a, e, "attn_prefill_flash")) return r;
     if (pieces > 1) {

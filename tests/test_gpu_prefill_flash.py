@@ -1,6 +1,6 @@
-"""The head_dim-128 flash prefill kernels where their tiles can go wrong: one to four tiles of 64 and of 128 keys, ends on both sides of a tile,
-windows that begin inside one, the ring's wrap, pieces of the key range, maxima that rise in every tile (which the long kernel's two
-softmax groups pass on to each other), and values that are not finite.  Which kernel a call takes rests on its size; here it is forced.
+"""The head_dim-128 flash prefill kernel where its tiles can go wrong: one to seven tiles of 64 keys, ends on both sides of a tile,
+windows that begin inside one, the ring's wrap, pieces of the key range, maxima that rise from tile to tile, values that are not
+finite, and key buffers that are longer than the keys.
 Against the f64 oracle at the head_dim-128 tolerance (P is f16: 2^-11 of the largest |v|)."""
 import numpy as np
 import pytest
@@ -54,14 +54,13 @@ def test_windows(ctx, m, q0, window):
     assert_close(_linear(ctx, q, k, v, m, q0, window), _want(q, k, v, m, q0, window), what=f"m={m} q0={q0} window={window}")
 
 
-@pytest.mark.parametrize("long,pieces", [(0, 1), (1, 1), (1, 3)])
+@pytest.mark.parametrize("pieces", [1, 3])
 @pytest.mark.parametrize("m,q0", EDGES)
-def test_tiles(ctx, monkeypatch, m, q0, long, pieces):
-    monkeypatch.setenv("SGB_FLASH_LONG", str(long))
+def test_tiles(ctx, monkeypatch, m, q0, pieces):
     monkeypatch.setenv("SGB_FLASH_PIECES", str(pieces))
     q, k, v = _case(m + 3 * q0, m, q0)
     got = _linear(ctx, q, k, v, m, q0, 0)
-    assert_close(got, _want(q, k, v, m, q0, 0), what=f"m={m} q0={q0} long={long} pieces={pieces}")
+    assert_close(got, _want(q, k, v, m, q0, 0), what=f"m={m} q0={q0} pieces={pieces}")
     assert np.array_equal(got.view(np.uint32), _linear(ctx, q, k, v, m, q0, 0).view(np.uint32))
 
 
@@ -80,11 +79,9 @@ def test_ring_and_chunk(ctx, q0, m):
     assert_close(out.read().reshape(m, NKV * G, D), _want(q, k, v, m, q0 - base, 1024), what=f"ring q0={q0} m={m}")
 
 
-@pytest.mark.parametrize("long", [0, 1])
 @pytest.mark.parametrize("m,q0", [(64, 100), (64, 300), (70, 900)])
-def test_maxima_that_rise_in_every_tile(ctx, monkeypatch, m, q0, long):
-    """Scores grow along the keys by far more than 2^8 a tile: every tile raises the maximum, rescales O and both groups' sums."""
-    monkeypatch.setenv("SGB_FLASH_LONG", str(long))
+def test_maxima_that_rise_in_every_tile(ctx, m, q0):
+    """Scores grow along the keys by far more than 2^8 a tile: every tile raises the maximum, rescales O and the sum."""
     q, k, v = _case(7, m, q0)
     q = np.repeat(q[:, ::G], G, axis=1)
     k = (k.astype(np.float32) + np.arange(q0 + m)[:, None, None] * 0.02 * q.astype(np.float32).mean(0)[::G][None]).astype(np.float16)
@@ -92,9 +89,8 @@ def test_maxima_that_rise_in_every_tile(ctx, monkeypatch, m, q0, long):
 
 
 @pytest.mark.parametrize("value", [np.inf, np.nan])
-def test_values_that_are_not_finite_stay_with_the_blocks_that_see_them(ctx, monkeypatch, value):
-    """The long kernel: V rows of a tile that no query of a 64-token block sees leave its bits alone."""
-    monkeypatch.setenv("SGB_FLASH_LONG", "1")
+def test_values_that_are_not_finite_stay_with_the_blocks_that_see_them(ctx, value):
+    """V rows of a tile that no query of a 64-token block sees leave its bits alone."""
     m, q0, at = 256, 130, 250  # the row of position 250 is seen by queries 120 and later
     q, k, v = _case(11, m, q0)
     clean = _linear(ctx, q, k, v, m, q0, 0)
@@ -104,3 +100,18 @@ def test_values_that_are_not_finite_stay_with_the_blocks_that_see_them(ctx, monk
     assert np.array_equal(got[:64].view(np.uint32), clean[:64].view(np.uint32))
     assert np.array_equal(got[:, :G].view(np.uint32), clean[:, :G].view(np.uint32))  # the other kv head
     assert not np.any(np.isfinite(got[120:, G:, 5]))
+
+
+def test_rows_behind_the_keys_do_not_change_the_bits(ctx, monkeypatch):
+    """A program keeps one K and one V of its longest context: what they could hold says nothing about the keys of a call, so for the same
+    pieces a call's kernel and with it its bits must not rest on that."""
+    monkeypatch.setenv("SGB_FLASH_PIECES", "1")
+    m, n_kv = 2368, 16
+    q, k, v = normal_f16(21, m, n_kv * G, D), normal_f16(22, m, n_kv, D), normal_f16(23, m, n_kv, D)
+    up, got = ctx.buffer_from_iter, []
+    for rows in (m, 16384):
+        kv = [up(np.concatenate([x, np.zeros((rows - m, n_kv, D), np.float16)])) for x in (k, v)]
+        out = ctx.new_buffer(m * n_kv * G * D, np.float32)
+        ctx.dispatch_blocking(ctx.load_kernel("attn_prefill_flash_f16_d128"), bind(up(q), *kv, out, _step(ctx, 0)), (SCALE, 0), [n_kv, m, 1])
+        got.append(out.read())
+    assert np.array_equal(got[0].view(np.uint32), got[1].view(np.uint32))
