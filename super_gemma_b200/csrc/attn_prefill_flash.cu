@@ -381,11 +381,11 @@ __global__ void __launch_bounds__(FLASH_THREADS, 2) flash_prefill_kernel(const _
                     tc_wait_st();
                 }
             }
-            // Rows of the V tile that hold no key of this problem (past the last query's position, or past the end
-            // of the history source) are zeroed before P V reads them: their P is 0, but 0 times a stale Inf or NaN
-            // in a caller's over-allocated buffer would not be.  Only the last tile of a source can have such rows.
+            // Rows of the V tile that no query of this CTA sees (past its last query's position, or past the end
+            // of the history source) are zeroed before P V reads them: their P is 0, but 0 times an Inf or NaN of a later
+            // token, or in what a caller's over-allocated buffer holds, would not be.  Only the last tile of a source can have such rows.
             {
-                const int64_t hi_valid = min(t.hi, q0 + (int64_t)prm.m_tokens - 1);
+                const int64_t hi_valid = min(t.hi, last_qpos);
                 if (t.pos0 + BLOCK_N - 1 > hi_valid) {  // uniform over the CTA
                     mbar_wait(&sm.full_v[b], (it / KV_STAGES) & 1, prm.status, 409, failed);
                     if (r < BLOCK_N && t.pos0 + r > hi_valid) {
