@@ -132,12 +132,12 @@ __global__ void __launch_bounds__(FLASH_THREADS, 2) flash_prefill_kernel(const _
         sm.abort = 0;
         mbar_fence_init();
     }
+    pdl_wait();  // the step words, q, K and V come from earlier kernels of the stream
+    pdl_launch_dependents();
     if (warp == 0) {
         tmem_alloc(&sm.tmem_base, TMEM_COLS);
         tmem_relinquish();
     }
-    pdl_wait();  // the step words, q, K and V come from earlier kernels of the stream
-    pdl_launch_dependents();
     // Launch order (blockIdx.x, then pieces): groups of `head_group` kv heads one after the other; inside a group the latest
     // query tile (the one with the most keys) of every head first, then the one before it, and so on.  The CTAs that run
     // together then read the K/V of one group, which the launcher sizes to stay in L2, and within the group the short

@@ -118,6 +118,8 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* m, uin
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // ---- tcgen05 / TMEM ------------------------------------------------------------------------------
+// Waits without a limit until the SM has that many columns left, so it stands behind pdl_wait(): a CTA that held columns while
+// it waited for its predecessor could hold those that a CTA of the predecessor still has to get.
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t ncols)
 {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(ncols)

@@ -50,3 +50,17 @@ def test_a_failed_launch_is_reported_by_its_own_message():
     s = _source("sgb_runtime.cu")
     body = s[s.index("e->fn(a)"):]
     assert body.index("record_after(") < body.index("set_error(r,") < body.index("return recorded")
+
+
+def test_tensor_memory_is_taken_behind_the_wait_for_the_kernel_before():
+    """tcgen05.alloc waits without a limit.  A CTA that holds columns while it waits for its predecessor's end, beside a CTA of the
+    predecessor that has yet to allocate, would wait for ever."""
+    found = 0
+    for n in sorted(os.listdir(CSRC)):
+        if not n.endswith(".cu"):
+            continue
+        for kernel in re.split(r"__global__", _source(n))[1:]:
+            if re.search(r"\btmem_alloc(_pair)?\(", kernel) and "pdl_wait()" in kernel:
+                assert kernel.index("pdl_wait()") < re.search(r"\btmem_alloc(_pair)?\(", kernel).start(), n
+                found += 1
+    assert found >= 3
