@@ -7,7 +7,7 @@
 //   O[64 rows x 512 dims] += P V     V as the MN-major B operand straight from its [key][dim] tile, 256 dims an instruction
 // of which each CTA loads half the keys of K and half the dims of V.
 // Scores: Q's quants are exact as f16.  A key's quants times their f16 scale are whole multiples of the scale's last place, 19 bits, which
-// f16 hi + lo hold exactly; four warps make them from the cache's bytes.  A block's sum so lacks only the scale of Q, which is the
+// f16 hi + lo hold exactly (for scales above 511, whose quants overflow, in a second pass that splits otherwise); four warps make them from the cache's bytes.  A block's sum so lacks only the scale of Q, which is the
 // row's, and the softmax threads have nothing left to do for it but one multiply-add.  (Whole-number sums of int8 MMAs, scaled by
 // both scales in the softmax threads: they then read 16 x 128 scales a tile through shared memory, which the MMAs read their
 // operands from; 364 us.  The transposed form before it, keys and dims as M, took V as the MN-major A operand, 160 cycles
@@ -66,6 +66,11 @@ constexpr int SETTLE_FROM = 4;                 // the first tile in which a dim 
 constexpr int SETTLE_CHUNK = 4;                // of K, even: the settling comes behind this one and the next
 constexpr float EXP_BIAS = 7.0f, GROW_T = 8.0f;
 
+struct Int8Barriers {
+    uint64_t k_full[NK], k_free[NK], v_full[NV], v_free[NV], v_here[NV], v_ok[NV], s_ready[2], s_free[2], p_ready, first_done, pv_done,
+        settle_here, settle_ok;
+};
+
 struct Int8Smem {
     uint8_t q[HD / 64][Q_CHUNK];  // quants
     uint8_t k[NK][2][K_CHUNK];    // quants times scales: hi, lo
@@ -73,9 +78,9 @@ struct Int8Smem {
     uint8_t v[NV][V_UNIT];
     float qs[HD / 32][ROWS];      // scales of Q, [block][row]
     float red[4][ROWS];
-    uint64_t k_full[NK], k_free[NK], v_full[NV], v_free[NV], v_here[NV], v_ok[NV], s_ready[2], s_free[2], p_ready, first_done, pv_done,
-        settle_here, settle_ok;
+    Int8Barriers bars[2];         // of a pass each
     uint32_t tmem_base, abort;
+    uint32_t gone, large, odd;  // of the pair: a wait ran out; a scale that takes quants beyond f16; a row that is not finite
     uint32_t redo[ROWS / 32];  // rows that are not finite, a bit each
 };
 static_assert(sizeof(Int8Smem) <= 227 * 1024, "one CTA per SM");
@@ -91,14 +96,15 @@ struct Int8Params {
     KvOperand k0, v0;
 };
 
-// Eight signed bytes as f16 pairs, exactly: 0x6400 | (q + 128) is the f16 of q + 1152.
+// Eight signed bytes as f16 pairs, exactly: 0x6400 | (q + 128) is the f16 of q + 1152, 0x4400 | (q + 128) that of q / 256 + 4.5.
+template <bool IN_256THS = false>
 __device__ __forceinline__ void whole_f16x8(uint2 q, __half2 (&out)[4])
 {
     const uint32_t x[2] = {q.x ^ 0x80808080u, q.y ^ 0x80808080u};
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const uint32_t u = __byte_perm(x[i >> 1], 0x64646464u, (i & 1) ? 0x4342 : 0x4140);
-        out[i] = __hsub2(*reinterpret_cast<const __half2*>(&u), __float2half2_rn(1152.0f));
+        const uint32_t u = __byte_perm(x[i >> 1], IN_256THS ? 0x44444444u : 0x64646464u, (i & 1) ? 0x4342 : 0x4140);
+        out[i] = __hsub2(*reinterpret_cast<const __half2*>(&u), __float2half2_rn(IN_256THS ? 4.5f : 1152.0f));
     }
 }
 __device__ __forceinline__ uint4 as_uint4(const __half2 (&h)[4])
@@ -126,19 +132,15 @@ __device__ __noinline__ void stream_rows(const Int8Params& prm, const Int8Smem& 
     }
 }
 
-__global__ void __launch_bounds__(INT8_THREADS, 1)
-    int8_prefill_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ Int8Params prm)
+// All roles of a CTA over its tiles.  WIDE takes keys whose scales times quants are beyond f16 as well (see the key warps), for two
+// instructions more per pair of values of K, which the tile's time is: as the only pass it took 327 us instead of 317 (256 queries at
+// 7936 + 256 keys), 1337 instead of 1235 (64 queries, 32768 keys).
+template <bool WIDE>
+__device__ __forceinline__ void int8_pass(const CUtensorMap& tm_v, const Int8Params& prm, Int8Smem& sm)
 {
-    extern __shared__ __align__(1024) uint8_t smem_raw[];
-    Int8Smem& sm = *reinterpret_cast<Int8Smem*>(smem_raw);
-    if ((smem_u32(smem_raw) & 1023u) != 0u) {  // the swizzled tiles need it; never seen, but never assumed (the same in both CTAs)
-        if (threadIdx.x == 0) report_error(prm.status, DEV_ERR_BOUNDS, 500, smem_u32(smem_raw), 0);
-        return;
-    }
     const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
     const uint32_t rank = pair_rank();  // 0 issues the pair's MMAs
-    pdl_wait();  // the step words, q, K and V come from earlier kernels of the stream
-    pdl_launch_dependents();
+    Int8Barriers& bar = sm.bars[WIDE];
     const uint32_t pair = blockIdx.x / 2;
     const int kvh = pair % prm.n_kv;
     const uint32_t n_qt = prm.m_tokens / PAIR_TOK;
@@ -149,40 +151,13 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
     const int64_t rows0 = (int64_t)min(prm.k0.rows, prm.v0.rows);
     int64_t end = last_qpos;  // positions that hold a visible key end here
     if (end >= rows0) {
-        if (tid == 0) report_error(prm.status, DEV_ERR_BOUNDS, 211, (uint32_t)rows0, (uint32_t)rows0);
+        if (!WIDE && tid == 0) report_error(prm.status, DEV_ERR_BOUNDS, 211, (uint32_t)rows0, (uint32_t)rows0);
         end = rows0 - 1;
     }
     const int n_tiles = (int)(end / TILE_K + 1);
     // rows of a tile that hold a key of this problem end here; V rows behind it are zeroed
     const int64_t valid_end = min(rows0 - 1, q0 + (int64_t)prm.m_tokens - 1);
 
-    if (tid == 0) {
-        for (int i = 0; i < NK; i++) {
-            mbar_init(&sm.k_full[i], 2 * K_WARPS);
-            mbar_init(&sm.k_free[i], 1);
-        }
-        for (int i = 0; i < NV; i++) {
-            mbar_init(&sm.v_full[i], 1);
-            mbar_init(&sm.v_free[i], 1);
-            mbar_init(&sm.v_here[i], 1);
-            mbar_init(&sm.v_ok[i], 2);
-        }
-        for (int i = 0; i < 2; i++) {
-            mbar_init(&sm.s_ready[i], 1);
-            mbar_init(&sm.s_free[i], 2 * SOFT_WARPS);
-        }
-        mbar_init(&sm.p_ready, 2 * SOFT_WARPS);
-        mbar_init(&sm.first_done, 1);
-        mbar_init(&sm.settle_here, K_WARPS);
-        mbar_init(&sm.settle_ok, 2 * K_WARPS);
-        mbar_init(&sm.pv_done, 1);
-        sm.abort = 0;
-        sm.redo[0] = sm.redo[1] = 0;
-        mbar_fence_init();
-    }
-    if (warp == 0) {
-        tmem_alloc_pair(&sm.tmem_base, TMEM_COLS);
-    }
     // this CTA's query rows: quants as f16, which holds them exactly, K-major in 128-byte rows; scales in f32
     for (int i = tid; i < ROWS * (HD / 16); i += INT8_THREADS) {
         const int r = i / (HD / 16), c = i % (HD / 16);
@@ -197,7 +172,7 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
     for (int i = tid; i < ROWS * (HD / 32); i += INT8_THREADS) {
         const int r = i / (HD / 32), b = i % (HD / 32);
         const size_t at = (size_t)(m0 + r / G) * (prm.n_kv * G) + kvh * G + r % G;
-        sm.qs[b][r] = __half2float(ld_global(prm.q_scales + at * (HD / 32) + b));
+        sm.qs[b][r] = (WIDE ? 256.0f : 1.0f) * __half2float(ld_global(prm.q_scales + at * (HD / 32) + b));
     }
     fence_proxy_async_smem();  // read by the tensor pipe
     tc_fence_before_sync();
@@ -251,7 +226,10 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
         // ======================= K: quants times scales as f16 hi + lo, 64 dims of this CTA's 64 keys at a time =======================
         // A thread has a key's 32-value block: hi = f16(s * q), lo = s * q - hi, which f16 holds exactly (s * q is a multiple of s's last
         // place, and hi misses it by 64 of those at most).  What overflows f16, or has a scale that is not finite, makes
-        // infinities of both signs, so NaN scores, and its rows are computed again.
+        // infinities of both signs, so NaN scores, and its rows are computed again: by the WIDE pass where the scale is a number.
+        // WIDE: hi = f16(s * q / 256), at most 2^15, and lo = s * q - 256 * hi, exact as well (where hi is subnormal, 256 * hi misses s * q by up to
+        // 2^-17); the MMA that adds the first hi takes the sum of the lo by its 256th.  256 * hi is beyond f16 for a large s and a 256th of
+        // a small one's last place is no f16, so lo comes in either order.
         const int t = tid - 32 * SOFT_WARPS, key = t >> 1, half = t & 1;
         const int64_t key_rows = rows0 - (int)rank * 64 - key;  // tiles that start before this hold the key
         const size_t row_q = (size_t)prm.n_kv * HD, row_s = (size_t)prm.n_kv * (HD / 32);
@@ -274,17 +252,20 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
         };
         auto convert = [&](int n, const Block& b) {
             const int st = n % NK;
-            if (n >= NK && !mbar_wait_warp(&sm.k_free[st], (n / NK - 1) & 1, prm.status, 511, failed)) return;
+            if (n >= NK && !mbar_wait_warp(&bar.k_free[st], (n / NK - 1) & 1, prm.status, 511, failed)) return;
             const __half2 s2 = __half2half2(b.s);
+            const bool upper = !(__habs(b.s) < __float2half_rn(64.0f));
+            const __half2 f256 = __float2half2_rn(256.0f), f1 = __float2half2_rn(1.0f);
+            const __half2 s_lo = upper ? s2 : __hmul2(s2, f256), less = __hneg2(upper ? f1 : f256), times = upper ? f256 : f1;  // WIDE
             const uint2* q = reinterpret_cast<const uint2*>(b.q);
 #pragma unroll
             for (int c = 0; c < 4; c++) {
                 __half2 whole[4], hi[4], lo[4];
-                whole_f16x8(q[c], whole);
+                whole_f16x8<WIDE>(q[c], whole);
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
                     hi[i] = __hmul2(s2, whole[i]);
-                    lo[i] = __hfma2(s2, whole[i], __hneg2(hi[i]));
+                    lo[i] = WIDE ? __hmul2(__hfma2(s_lo, whole[i], __hmul2(hi[i], less)), times) : __hfma2(s2, whole[i], __hneg2(hi[i]));
                 }
                 const uint32_t off = key * 128 + (((4 * half + c) ^ (key & 7)) << 4);
                 *reinterpret_cast<uint4*>(sm.k[st][0] + off) = as_uint4(hi);
@@ -292,7 +273,7 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
             }
             fence_proxy_async_smem();
             __syncwarp();
-            if (lane == 0) mbar_arrive_pair(at_leader(&sm.k_full[st]));
+            if (lane == 0) mbar_arrive_pair(at_leader(&bar.k_full[st]));
         };
         Block even, odd;  // two chunks' loads under way
         fetch(0, even);
@@ -321,7 +302,7 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
 #pragma unroll
                         for (int h = 0; h < 4; h++) fetch_settled(owner, 4 * db + h, u[h]);
                     if (half == 0) {
-                        mbar_wait_warp(&sm.first_done, (it - 1) & 1, prm.status, 535, failed);
+                        mbar_wait_warp(&bar.first_done, (it - 1) & 1, prm.status, 535, failed);
                         tc_fence_after_sync();
                     }
 #pragma unroll
@@ -339,8 +320,8 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
                 __threadfence_block();  // the parts are read by the softmax threads
                 __syncwarp();
                 if (lane == 0) {
-                    mbar_arrive(&sm.settle_here);
-                    mbar_arrive_pair(at_leader(&sm.settle_ok));
+                    mbar_arrive(&bar.settle_here);
+                    mbar_arrive_pair(at_leader(&bar.settle_ok));
                 }
             }
         }
@@ -352,23 +333,23 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
             const bool tail = pos0 + TILE_K - 1 > valid_end;  // the last tile at most: v_here and v_ok of a slot have one phase.  The MMA warp computes the same
             for (int u = 0; u < 4; u++, n++) {
                 const int st = n % NV;
-                if (n >= NV && !mbar_wait_warp(&sm.v_free[st], (n / NV - 1) & 1, prm.status, 512, failed, 50)) break;
+                if (n >= NV && !mbar_wait_warp(&bar.v_free[st], (n / NV - 1) & 1, prm.status, 512, failed, 50)) break;
                 const int kh = u & 1, dim = dim_block(j, u) * 256 + (int)rank * 128;
                 if (!tail) {
                     if (lane == 0) {
-                        if (rank == 0) mbar_arrive_expect_tx(&sm.v_full[st], 2 * V_UNIT);
-                        tma_load_3d_pair(sm.v[st], &tm_v, at_leader(&sm.v_full[st]), dim, kvh, (int)pos0 + kh * 64);
-                        tma_load_3d_pair(sm.v[st] + V_UNIT / 2, &tm_v, at_leader(&sm.v_full[st]), dim + 64, kvh, (int)pos0 + kh * 64);
+                        if (rank == 0) mbar_arrive_expect_tx(&bar.v_full[st], 2 * V_UNIT);
+                        tma_load_3d_pair(sm.v[st], &tm_v, at_leader(&bar.v_full[st]), dim, kvh, (int)pos0 + kh * 64);
+                        tma_load_3d_pair(sm.v[st] + V_UNIT / 2, &tm_v, at_leader(&bar.v_full[st]), dim + 64, kvh, (int)pos0 + kh * 64);
                     }
                     continue;
                 }
                 if (lane == 0) {
-                    mbar_arrive_expect_tx(&sm.v_here[st], V_UNIT);
-                    tma_load_3d(sm.v[st], &tm_v, &sm.v_here[st], dim, kvh, (int)pos0 + kh * 64);
-                    tma_load_3d(sm.v[st] + V_UNIT / 2, &tm_v, &sm.v_here[st], dim + 64, kvh, (int)pos0 + kh * 64);
+                    mbar_arrive_expect_tx(&bar.v_here[st], V_UNIT);
+                    tma_load_3d(sm.v[st], &tm_v, &bar.v_here[st], dim, kvh, (int)pos0 + kh * 64);
+                    tma_load_3d(sm.v[st] + V_UNIT / 2, &tm_v, &bar.v_here[st], dim + 64, kvh, (int)pos0 + kh * 64);
                 }
                 __syncwarp();
-                if (!mbar_wait_warp(&sm.v_here[st], 0, prm.status, 513, failed)) break;
+                if (!mbar_wait_warp(&bar.v_here[st], 0, prm.status, 513, failed)) break;
                 for (int r = lane; r < 64; r += 32) {
                     if (pos0 + kh * 64 + r <= valid_end) continue;
 #pragma unroll
@@ -380,7 +361,7 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
                 }
                 fence_proxy_async_smem();  // generic-proxy writes, read next by the tensor pipe
                 __syncwarp();
-                if (lane == 0) mbar_arrive_pair(at_leader(&sm.v_ok[st]));
+                if (lane == 0) mbar_arrive_pair(at_leader(&bar.v_ok[st]));
             }
         }
     } else if (warp == MMA_W) {
@@ -396,10 +377,10 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
             // S of (tile j, group g) into buffer n & 1, n = j * GROUPS + g
             auto issue_qk = [&](int j, int g) {
                 const int n = j * GROUPS + g;
-                if (n >= 2) mbar_wait_warp(&sm.s_free[n & 1], ((n - 2) >> 1) & 1, prm.status, 521, failed);
+                if (n >= 2) mbar_wait_warp(&bar.s_free[n & 1], ((n - 2) >> 1) & 1, prm.status, 521, failed);
                 const uint32_t d = tm + TMEM_S + (n & 1) * S_COLS;
                 const int st = n % NK;
-                mbar_wait_warp(&sm.k_full[st], (n / NK) & 1, prm.status, 522, failed);
+                mbar_wait_warp(&bar.k_full[st], (n / NK) & 1, prm.status, 522, failed);
                 if (failed) return;
                 tc_fence_after_sync();
 #pragma unroll
@@ -407,19 +388,23 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
 #pragma unroll
                     for (int i = 0; i < 4; i++) {  // lo, then hi
                         const uint32_t off = 2 * (2 * e + (i & 1)), hl = 1 - (i >> 1);
-                        umma2_f16_ss(d + e * 64, dq + g * (Q_CHUNK >> 4) + off, dk + (2 * st + hl) * (K_CHUNK >> 4) + off, IDESC_QK, i ? 1u : 0u, one);
+                        const uint64_t qd = dq + g * (Q_CHUNK >> 4) + off, kd = dk + (2 * st + hl) * (K_CHUNK >> 4) + off;
+                        if (WIDE && i == 2)
+                            umma2_f16_ss<8>(d + e * 64, qd, kd, IDESC_QK, 1u, one);
+                        else
+                            umma2_f16_ss(d + e * 64, qd, kd, IDESC_QK, i ? 1u : 0u, one);
                     }
-                umma2_commit(&sm.k_free[st], one);
-                umma2_commit(&sm.s_ready[n & 1], one);
+                umma2_commit(&bar.k_free[st], one);
+                umma2_commit(&bar.s_ready[n & 1], one);
             };
             // O += P V for one unit of tile j, the upper or lower halves of P
             auto issue_pv = [&](int j, int u, int half, bool tail) {
                 const int n = 4 * j + u, st = n % NV, kh = u & 1;
                 if (half == 0) {
                     if (tail)
-                        mbar_wait_warp(&sm.v_ok[st], 0, prm.status, 524, failed);
+                        mbar_wait_warp(&bar.v_ok[st], 0, prm.status, 524, failed);
                     else
-                        mbar_wait_warp(&sm.v_full[st], (n / NV) & 1, prm.status, 523, failed);
+                        mbar_wait_warp(&bar.v_full[st], (n / NV) & 1, prm.status, 523, failed);
                 }
                 if (failed) return;
                 tc_fence_after_sync();
@@ -427,7 +412,7 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
                 const uint32_t d = tm + TMEM_O + dim_block(j, u) * 128;
 #pragma unroll
                 for (int kk = 0; kk < 4; kk++) umma2_f16_ss(d, p + 2 * kk, v + 128 * kk, IDESC_PV, (j > 0 || kh || half || kk) ? 1u : 0u, one);
-                if (half) umma2_commit(&sm.v_free[st], one);
+                if (half) umma2_commit(&bar.v_free[st], one);
             };
             for (int g = 0; g < GROUPS; g++) issue_qk(0, g);
             for (int j = 0; j < tiles && !failed; ++j) {
@@ -435,13 +420,13 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
                 // the next tile's scores go ahead of this tile's products, and between them
                 int g = 0;
                 for (; more && g < 2; g++) issue_qk(j + 1, g);
-                mbar_wait_warp(&sm.p_ready, j & 1, prm.status, 525, failed);
+                mbar_wait_warp(&bar.p_ready, j & 1, prm.status, 525, failed);
                 if (failed) break;
                 for (int i = 0; i < 8; i++) {
-                    if (i == 4 && settles(j)) mbar_wait_warp(&sm.settle_ok, settle_phase(j), prm.status, 526, failed);  // the other block has been settled
+                    if (i == 4 && settles(j)) mbar_wait_warp(&bar.settle_ok, settle_phase(j), prm.status, 526, failed);  // the other block has been settled
                     issue_pv(j, i >> 1, i & 1, tail);
-                    if (i == 3) umma2_commit(&sm.first_done, one);
-                    if (i == 7) umma2_commit(&sm.pv_done, one);
+                    if (i == 3) umma2_commit(&bar.first_done, one);
+                    if (i == 7) umma2_commit(&bar.pv_done, one);
                     if (more && g < GROUPS) issue_qk(j + 1, g++);
                 }
             }
@@ -452,13 +437,13 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
         const int quarter = warp & 3, half = warp >> 2, tl = quarter * 32 + lane, row = tl & 63, kh = tl >> 6;
         const int key0 = 64 * kh + 32 * half;  // of the tile
         const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
-        const uint32_t s_free[2] = {at_leader(&sm.s_free[0]), at_leader(&sm.s_free[1])}, p_ready = at_leader(&sm.p_ready);
+        const uint32_t s_free[2] = {at_leader(&bar.s_free[0]), at_leader(&bar.s_free[1])}, p_ready = at_leader(&bar.p_ready);
         const int64_t last_key = min(first_qpos + row / G, rows0 - 1) - key0;  // minus the tile's first: the last of this thread's keys that the row sees
         const float scale2 = prm.scale * 1.4426950408889634f;  // > 0 (checked on the host)
         const size_t out_row = ((size_t)(m0 + row / G) * (prm.n_kv * G) + kvh * G + row % G) * HD;
         bool odd = false;  // a scale or a result that is not finite
 #pragma unroll
-        for (int b = 0; b < 16; b++) odd |= !(fabsf(sm.qs[b][row]) <= 65504.0f);
+        for (int b = 0; b < 16; b++) odd |= !(fabsf(sm.qs[b][row]) <= 256.0f * 65504.0f);
         float m_ref = NEG_SENTINEL;
         float2 l2[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
         auto o_at = [&](int h) { return lane_addr + TMEM_O + (h >> 2) * 128 + 64 * half + 16 * (h & 3); };
@@ -469,7 +454,7 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
             // Block by block: the sums of the next are on their way out of tensor memory while one's are scaled by the row's scale.
             uint32_t r[2][32];
             auto ready = [&](int g) {
-                mbar_wait(&sm.s_ready[g & 1], ((it * GROUPS + g) >> 1) & 1, prm.status, 531, failed);
+                mbar_wait(&bar.s_ready[g & 1], ((it * GROUPS + g) >> 1) & 1, prm.status, 531, failed);
                 tc_fence_after_sync();
             };
             auto at = [&](int n) { return lane_addr + TMEM_S + ((n >> 1) & 1) * S_COLS + (n & 1) * 64 + 32 * half; };
@@ -526,8 +511,8 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
 #pragma unroll
                 for (int i = 0; i < 2; i++) l2[i] = __fmul2_rn(l2[i], make_float2(corr, corr));
                 if (it > 0) {
-                    mbar_wait(&sm.pv_done, (it - 1) & 1, prm.status, 532, failed);
-                    if (settles(it)) mbar_wait(&sm.settle_here, settle_phase(it), prm.status, 536, failed);
+                    mbar_wait(&bar.pv_done, (it - 1) & 1, prm.status, 532, failed);
+                    if (settles(it)) mbar_wait(&bar.settle_here, settle_phase(it), prm.status, 536, failed);
                     tc_fence_after_sync();
 #pragma unroll 1
                     for (int h = 0; h < 8; h++) {
@@ -561,7 +546,7 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
                     lo[i] = pack_half2(p.x - h.x, p.y - h.y);
                 }
             }
-            if (it > 0) mbar_wait(&sm.pv_done, (it - 1) & 1, prm.status, 533, failed);  // P of the last tile has been read
+            if (it > 0) mbar_wait(&bar.pv_done, (it - 1) & 1, prm.status, 533, failed);  // P of the last tile has been read
             {
                 uint8_t* to = sm.p[0] + kh * P_HALF + row * 128;
 #pragma unroll
@@ -582,12 +567,12 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
         sm.red[2 * kh + half][row] = (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y);
         named_barrier_sync(2, SOFT_THREADS);
         const float inv = 1.0f / ((sm.red[0][row] + sm.red[1][row]) + (sm.red[2][row] + sm.red[3][row]));
-        mbar_wait(&sm.pv_done, (n_tiles - 1) & 1, prm.status, 534, failed);
+        mbar_wait(&bar.pv_done, (n_tiles - 1) & 1, prm.status, 534, failed);
         tc_fence_after_sync();
         const uint32_t settled = settled_by(n_tiles - 1);
         if (settled != 0) {  // whole again before the first result is written over a settled part
             const int last = (n_tiles - 1) & ~1;  // the last tile with a settling
-            mbar_wait(&sm.settle_here, settle_phase(last), prm.status, 537, failed);
+            mbar_wait(&bar.settle_here, settle_phase(last), prm.status, 537, failed);
 #pragma unroll 1
             for (int h = 0; h < 8; h++) {
                 if (((settled >> (h >> 2)) & 1) == 0) continue;
@@ -617,11 +602,17 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
             to[0] = make_uint4(w[0], w[1], w[2], w[3]);
             to[1] = make_uint4(w[4], w[5], w[6], w[7]);
         }
-        if (odd) atomicOr(&sm.redo[row / 32], 1u << (row % 32));
+        if (odd) {
+            atomicOr(&sm.redo[row / 32], 1u << (row % 32));
+            if (!WIDE) store_both(&sm.odd, 1);
+        }
     }
     // A wait that ran out leaves copies and MMAs of this CTA in flight that nobody will wait for: give them a bounded
     // time to land before the shared and tensor memory they target is handed to the next CTA.
-    if (failed) sm.abort = 1;
+    if (failed) {
+        sm.abort = 1;
+        store_both(&sm.gone, 1);
+    }
     tc_fence_before_sync();
     __syncthreads();
     if (*(volatile uint32_t*)&sm.abort != 0u) {
@@ -629,7 +620,75 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
         __syncthreads();
     }
     pair_sync();  // the pair's MMAs and arrivals reach into both CTAs
-    if (warp == 0) tmem_dealloc_pair(tmem, TMEM_COLS);
+}
+
+// Keys that overflowed made NaN of every row that sees them: where a pair has such rows and such keys, all of it again, with the other split.
+// (Looked for afterwards: one maximum per scale in the key warps cost 0.7 %.  Not inlined, for the registers of the pass that
+// every call takes.)
+__device__ __noinline__ void again_if_large(const CUtensorMap& tm_v, const Int8Params& prm, Int8Smem& sm, uint32_t pair_m0, int kvh)
+{
+    constexpr int BLOCKS = HD / 32, STEP = INT8_THREADS / BLOCKS;  // scales of a key; keys of a CTA at a time
+    const int64_t keys = min((int64_t)min(prm.k0.rows, prm.v0.rows), (int64_t)prm.step[STEP_Q0] + pair_m0 + PAIR_TOK);
+    bool large = false;
+    for (int64_t key = threadIdx.x / BLOCKS + pair_rank() * STEP; key < keys; key += 2 * STEP) {
+        const float s = fabsf(__half2float(ld_global(prm.k0.scales + ((size_t)key * prm.n_kv + kvh) * BLOCKS + threadIdx.x % BLOCKS)));
+        large |= s >= 65504.0f / 128.0f && s <= 65504.0f;
+    }
+    if (large) store_both(&sm.large, 1);
+    pair_sync();
+    if (*(volatile uint32_t*)&sm.large == 0u) return;
+    if (threadIdx.x == 0) sm.redo[0] = sm.redo[1] = 0;
+    int8_pass<true>(tm_v, prm, sm);
+}
+
+__global__ void __launch_bounds__(INT8_THREADS, 1)
+    int8_prefill_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ Int8Params prm)
+{
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    Int8Smem& sm = *reinterpret_cast<Int8Smem*>(smem_raw);
+    if ((smem_u32(smem_raw) & 1023u) != 0u) {  // the swizzled tiles need it; never seen, but never assumed (the same in both CTAs)
+        if (threadIdx.x == 0) report_error(prm.status, DEV_ERR_BOUNDS, 500, smem_u32(smem_raw), 0);
+        return;
+    }
+    const int tid = threadIdx.x, warp = warp_uniform(tid >> 5);
+    pdl_wait();  // the step words, q, K and V come from earlier kernels of the stream
+    pdl_launch_dependents();
+    if (tid < 2) {
+        Int8Barriers& bar = sm.bars[tid];
+        for (int i = 0; i < NK; i++) {
+            mbar_init(&bar.k_full[i], 2 * K_WARPS);
+            mbar_init(&bar.k_free[i], 1);
+        }
+        for (int i = 0; i < NV; i++) {
+            mbar_init(&bar.v_full[i], 1);
+            mbar_init(&bar.v_free[i], 1);
+            mbar_init(&bar.v_here[i], 1);
+            mbar_init(&bar.v_ok[i], 2);
+        }
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&bar.s_ready[i], 1);
+            mbar_init(&bar.s_free[i], 2 * SOFT_WARPS);
+        }
+        mbar_init(&bar.p_ready, 2 * SOFT_WARPS);
+        mbar_init(&bar.first_done, 1);
+        mbar_init(&bar.settle_here, K_WARPS);
+        mbar_init(&bar.settle_ok, 2 * K_WARPS);
+        mbar_init(&bar.pv_done, 1);
+        mbar_fence_init();
+    }
+    if (tid == 0) {
+        sm.abort = sm.gone = sm.large = sm.odd = 0;
+        sm.redo[0] = sm.redo[1] = 0;
+    }
+    if (warp == 0) {
+        tmem_alloc_pair(&sm.tmem_base, TMEM_COLS);
+    }
+    int8_pass<false>(tm_v, prm, sm);
+    const int kvh = (blockIdx.x / 2) % prm.n_kv;
+    const uint32_t pair_m0 = (prm.m_tokens / PAIR_TOK - 1 - blockIdx.x / 2 / prm.n_kv) * PAIR_TOK, m0 = pair_m0 + pair_rank() * (ROWS / G);
+    const volatile uint32_t &gone = sm.gone, &odd = sm.odd;  // a pair agrees: stored in both CTAs ahead of the cluster barrier
+    if (odd != 0u && gone == 0u) again_if_large(tm_v, prm, sm, pair_m0, kvh);
+    if (warp == 0) tmem_dealloc_pair(sm.tmem_base, TMEM_COLS);
     if ((*(volatile uint32_t*)&sm.redo[0] | *(volatile uint32_t*)&sm.redo[1]) != 0) stream_rows(prm, sm, m0, kvh);
 }
 

@@ -33,6 +33,15 @@ __device__ __forceinline__ void mbar_arrive_pair(uint32_t addr)
 {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
 }
+// A word of both CTAs' shared memory, there for all behind the next pair_sync().
+__device__ __forceinline__ void store_both(uint32_t* p, uint32_t v)
+{
+    asm volatile(
+        "{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, 0;\n\tst.shared::cluster.u32 [a], %1;\n\t"
+        "mapa.shared::cluster.u32 a, %0, 1;\n\tst.shared::cluster.u32 [a], %1;\n\t}"
+        ::"r"(smem_u32(p)), "r"(v)
+        : "memory");
+}
 // A copy into this CTA that reports to a barrier of the even CTA.
 __device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* m, uint32_t bar_addr, int c0, int c1, int c2)
 {
@@ -51,13 +60,23 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
 {
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
+// D = A B, + D * 2^-DOWN with `accumulate`.
+template <int DOWN = 0>
 __device__ __forceinline__ void umma2_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate, uint32_t one)
 {
-    asm volatile(
-        "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
-        "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(one)
-        : "memory");
+    static_assert(DOWN >= 0 && DOWN <= 15, "scale-input-d");
+    if constexpr (DOWN != 0)
+        asm volatile(
+            "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
+            "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p, %6;\n\t}\n"
+            ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(one), "n"(DOWN)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
+            "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+            ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(one)
+            : "memory");
 }
 // Arrive on the barrier of both CTAs once all MMAs issued so far by this thread have completed.
 __device__ __forceinline__ void umma2_commit(uint64_t* bar, uint32_t one)

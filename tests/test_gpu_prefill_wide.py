@@ -262,8 +262,19 @@ def test_global_int8_infinite_scale_of_a_key(ctx):
 @pytest.mark.parametrize("m,q0,factor", [(16, 104, 1), (16, 112, 1), (16, 120, 1), (32, 120, 2.0**-12), (32, 1000, 2.0**13), (16, 200, 2.0**15)])
 def test_global_int8_pairs_of_ctas(ctx, m, q0, factor):
     """The two CTAs of a pair end in different tiles (their queries lie on both sides of a multiple of 128), and keys whose scales are subnormal in
-    f16, large, or so large that a quant times its scale overflows f16: those rows are computed again."""
+    f16, large, or so large that a quant times its scale is beyond f16."""
     q, k, v = _normal(m + q0, m, 32, 512), _normal(q0, q0 + m, 4, 512) * np.float32(factor), _normal(q0 + 2, q0 + m, 4, 512)
     scale = 0.044194174 / factor
     got, qd, kd = _iq(ctx, q, k, v, q0, m, scale=scale)
     assert_close(got, O.attention_f64(qd, kd, v, m, q0, 32, 4, 512, scale), ATOL, RTOL, f"m={m} q0={q0} factor={factor}")
+
+
+@pytest.mark.parametrize("power,q0", [(-7, 300), (9, 300), (14, 300), (15, 1100), (20, 300)])
+def test_global_int8_keys_of_any_scale_stay_on_the_tensor_cores(ctx, power, q0):
+    """A power of two on the keys' scales that the softmax scale takes back changes no bit, also where quants times scales are beyond f16
+    (from 2^14 on): no row is left to the streaming statement, whose bits are others."""
+    m = 32
+    q, k, v = _normal(71, m, 32, 512), _normal(72, q0 + m, 4, 512), _normal(73, q0 + m, 4, 512)
+    clean, _, _ = _iq(ctx, q, k, v, q0, m, scale=2.0**-4)
+    got, _, _ = _iq(ctx, q, k * np.float32(2.0**power), v, q0, m, scale=2.0 ** (-4 - power))
+    assert np.array_equal(got.view(np.uint32), clean.view(np.uint32))
