@@ -68,7 +68,7 @@ constexpr float EXP_BIAS = 7.0f, GROW_T = 8.0f;
 
 struct Int8Barriers {
     uint64_t k_full[NK], k_free[NK], v_full[NV], v_free[NV], v_here[NV], v_ok[NV], s_ready[2], s_free[2], p_ready, first_done, pv_done,
-        settle_here, settle_ok;
+        parts_here, settle_here, settle_ok;
 };
 
 struct Int8Smem {
@@ -220,7 +220,10 @@ __device__ __forceinline__ void int8_pass(const CUtensorMap& tm_v, const Int8Par
     // dim blocks that have a settled part once tile `it` has had its turn
     auto settled_by = [&](int it) { return it < SETTLE_FROM ? 0u : it < SETTLE_FROM + 2 ? 1u << dim_block(SETTLE_FROM - 1, 0) : 3u; };
     auto settles = [](int it) { return it >= SETTLE_FROM && (it & 1) == 0; };
-    auto settle_phase = [](int it) { return ((it - SETTLE_FROM) >> 1) & 1; };
+    auto settle_phase = [](int it) { return ((it - SETTLE_FROM) >> 1) & 1; };  // of the last settling up to tile `it`
+    // A CTA's settled parts change hands twice: the softmax threads, who rescale them where a tile raises a maximum, leave them to the key warps
+    // with parts_here ahead of a settling, and get them back with settle_here.  Both are barriers of the CTA itself: the parts lie in
+    // global memory, for which the pair's own hand-overs (pair.cuh) do not stand.
 
     if (warp >= SOFT_WARPS && warp < MMA_W) {
         // ======================= K: quants times scales as f16 hi + lo, 64 dims of this CTA's 64 keys at a time =======================
@@ -291,13 +294,14 @@ __device__ __forceinline__ void int8_pass(const CUtensorMap& tm_v, const Int8Par
                 const int db = dim_block(it - 1, 0), quarter = warp & 3;
                 const uint32_t block = tmem + ((uint32_t)(quarter * 32) << 16) + TMEM_O + db * 128;
                 const bool before = ((settled_by(it - 1) >> db) & 1) != 0;
+                // One phase per settling, and the next one's needs chunks of K that these warps convert behind this wait.  It does not hold
+                // them up: the buffer of the chunk just converted came free behind the last tile's p_ready.
+                static_assert(SETTLE_CHUNK + 1 - NK >= 2, "chunks from the third on are multiplied behind the last tile's p_ready");
+                mbar_wait_warp(&bar.parts_here, settle_phase(it), prm.status, 538, failed);
 #pragma unroll 1
                 for (int half = 0; half < 2; half++) {
                     const int owner = half * 128 + quarter * 32 + lane;
-                    // Settled parts last change where a tile raises a maximum, ahead of its p_ready; the buffer of the chunk just converted came
-                    // free behind the last tile's.  (Behind the wait below they cost 355 us for 345.)
-                    static_assert(SETTLE_CHUNK + 1 - NK >= 2, "chunks from the third on are multiplied behind the last tile's p_ready");
-                    uint4 u[4][2] = {};
+                    uint4 u[4][2] = {};  // asked for ahead of the wait below (behind it they cost 355 us for 345)
                     if (before)
 #pragma unroll
                         for (int h = 0; h < 4; h++) fetch_settled(owner, 4 * db + h, u[h]);
@@ -512,7 +516,8 @@ __device__ __forceinline__ void int8_pass(const CUtensorMap& tm_v, const Int8Par
                 for (int i = 0; i < 2; i++) l2[i] = __fmul2_rn(l2[i], make_float2(corr, corr));
                 if (it > 0) {
                     mbar_wait(&bar.pv_done, (it - 1) & 1, prm.status, 532, failed);
-                    if (settles(it)) mbar_wait(&bar.settle_here, settle_phase(it), prm.status, 536, failed);
+                    // whoever settled last, in this tile or in the one before; pv_done says that the settling ahead of it is over
+                    if (it >= SETTLE_FROM) mbar_wait(&bar.settle_here, settle_phase(it), prm.status, 536, failed);
                     tc_fence_after_sync();
 #pragma unroll 1
                     for (int h = 0; h < 8; h++) {
@@ -559,7 +564,10 @@ __device__ __forceinline__ void int8_pass(const CUtensorMap& tm_v, const Int8Par
             fence_proxy_async_smem();
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive_pair(p_ready);
+            if (lane == 0) {
+                mbar_arrive_pair(p_ready);
+                if (settles(it + 1)) mbar_arrive(&bar.parts_here);
+            }
         }
 
         // ---- epilogue -----------------------------------------------
@@ -571,8 +579,7 @@ __device__ __forceinline__ void int8_pass(const CUtensorMap& tm_v, const Int8Par
         tc_fence_after_sync();
         const uint32_t settled = settled_by(n_tiles - 1);
         if (settled != 0) {  // whole again before the first result is written over a settled part
-            const int last = (n_tiles - 1) & ~1;  // the last tile with a settling
-            mbar_wait(&bar.settle_here, settle_phase(last), prm.status, 537, failed);
+            mbar_wait(&bar.settle_here, settle_phase(n_tiles - 1), prm.status, 537, failed);
 #pragma unroll 1
             for (int h = 0; h < 8; h++) {
                 if (((settled >> (h >> 2)) & 1) == 0) continue;
@@ -671,6 +678,7 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
         }
         mbar_init(&bar.p_ready, 2 * SOFT_WARPS);
         mbar_init(&bar.first_done, 1);
+        mbar_init(&bar.parts_here, SOFT_WARPS);
         mbar_init(&bar.settle_here, K_WARPS);
         mbar_init(&bar.settle_ok, 2 * K_WARPS);
         mbar_init(&bar.pv_done, 1);

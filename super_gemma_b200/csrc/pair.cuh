@@ -26,9 +26,9 @@ __device__ __forceinline__ void pair_sync()
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // Arrive on a barrier of the even CTA.  (With fences of cluster scope on both sides of every hand-over the int8 prefill took 705 us,
-// without 451.)  What is handed over lies in tensor memory or in this CTA's own shared memory and is read by this
+// without 451.)  It is for what lies in tensor memory or in this CTA's own shared memory and is read by this
 // SM's half of the MMA that the barrier's waiter issues, after fence.proxy.async or tcgen05.fence on this side: neither side needs a
-// fence of cluster scope.
+// fence of cluster scope.  Global memory is not handed over this way.
 __device__ __forceinline__ void mbar_arrive_pair(uint32_t addr)
 {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");

@@ -64,3 +64,17 @@ def test_tensor_memory_is_taken_behind_the_wait_for_the_kernel_before():
                 assert kernel.index("pdl_wait()") < re.search(r"\btmem_alloc(_pair)?\(", kernel).start(), n
                 found += 1
     assert found >= 3
+
+
+def test_settled_parts_change_hands_over_barriers_of_the_cta():
+    """The settled parts of O lie in global memory and go back and forth between two roles of one CTA.  Arrivals on the even CTA's barriers
+    order only what the tensor pipe reads, so neither side may rest on them: each waits for a barrier that the other arrives on."""
+    s = _source("attn_prefill_int8.cu")
+    keys = s[s.index("warp >= SOFT_WARPS && warp < MMA_W"):s.index("warp == V_W")]
+    softmax = s[s.rindex("} else {", 0, s.index("const int key0")):]
+    assert 0 < keys.index("mbar_wait_warp(&bar.parts_here") < keys.index("fetch_settled(") < keys.index("__threadfence_block()") < keys.index("mbar_arrive(&bar.settle_here)")
+    assert "mbar_arrive(&bar.parts_here)" in softmax
+    raised = softmax[softmax.index("if (raise)"):]
+    wait = re.search(r"if \((.*)\) mbar_wait\(&bar.settle_here", raised)
+    assert wait.group(1) == "it >= SETTLE_FROM" and wait.start() < raised.index("fetch_settled(") < raised.index("__threadfence_block()")
+    assert raised.index("__threadfence_block()") < raised.index("mbar_arrive(&bar.parts_here)")
