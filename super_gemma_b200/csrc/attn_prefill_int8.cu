@@ -716,10 +716,10 @@ int encode_rows(const LaunchArgs& a, CUtensorMap* tm, const void* base, uint64_t
 // What the tensor-core kernel takes: a positive softmax scale (the row maximum is taken before it), operands whose rows the
 // copies can address (16-byte aligned bases, K and V with at least one row, row indexes within an int), an output that can be
 // settled into (16-byte accesses, whole query tiles).  What else the launcher accepts stays on the streaming kernel: quants on 4
-// bytes, scales and output on 2.
+// bytes, an output on 2.  Scales are read one by one.
 bool prefill_int8_takes(const KvOperand& k, const KvOperand& v, const void* q, const void* out, uint32_t m, float scale)
 {
-    if (!(scale > 0.0f) || !(scale < 1e30f) || !aligned16(q) || !aligned16(k.scales) || !aligned16(out) || m % PAIR_TOK != 0) return false;
+    if (!(scale > 0.0f) || !(scale < 1e30f) || !aligned16(q) || !aligned16(out) || m % PAIR_TOK != 0) return false;
     for (const KvOperand* o : {&k, &v})
         if (o->rows == 0 || o->rows >= (1u << 30) || !aligned16(o->data)) return false;
     return true;

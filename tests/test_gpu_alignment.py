@@ -112,7 +112,7 @@ def test_decode_d128_rows_on_eight_bytes(ctx):
 
 @pytest.mark.parametrize("which", range(6))
 def test_global_int8_operands_on_their_own_alignment(ctx, which):
-    """Quants on 4 bytes, scales and output on 2, one at a time: no tile copies, the streaming kernel."""
+    """Quants on 4 bytes, scales and output on 2, one at a time: the streaming kernel, but for the scales, which the tensor-core kernel reads one by one."""
     m, q0 = 16, 100
     q, k, v = normal_f16(4, m, 32, 512).astype(np.float32), normal_f16(5, q0 + m, 4, 512).astype(np.float32), normal_f16(6, q0 + m, 4, 512)
     qs, qq, qd = O.q8_quant_div(q.ravel())
@@ -124,6 +124,21 @@ def test_global_int8_operands_on_their_own_alignment(ctx, which):
     ctx.dispatch_blocking(ctx.load_kernel("attn_prefill_global_flash_sp_iq"), bind(*bufs, out, _step(ctx, q0=q0)), 512**-0.5, [32, 1, 1])
     want = O.attention_f64(qd.reshape(q.shape), kd.reshape(k.shape), v.astype(np.float32), m, q0, 32, 4, 512, 512**-0.5)
     assert_close(O.f16_bits_to_f32(out.read()).reshape(m, 32, 512), want, 5e-5, 2.0**-11)
+
+
+@pytest.mark.parametrize("by", [2, 4, 8])
+def test_global_int8_scales_of_k_on_two_bytes_keep_the_kernel(ctx, by):
+    """... and so give the bits that scales on 16 bytes give (the streaming kernel's are others)."""
+    m, q0 = 16, 300
+    q, k, v = normal_f16(14, m, 32, 512).astype(np.float32), normal_f16(15, q0 + m, 4, 512).astype(np.float32), normal_f16(16, q0 + m, 4, 512)
+    (qs, qq, _), (ks, kq, _) = O.q8_quant_div(q.ravel()), O.q8_quant_div(k.ravel())
+    got = []
+    for b in (0, by):
+        out = ctx.new_buffer(m * 32 * 512, np.uint16)
+        bufs = [_moved(ctx, x, y) for x, y in zip((qq, qs, kq, ks, v), (0, 0, 0, b, 0))]
+        ctx.dispatch_blocking(ctx.load_kernel("attn_prefill_global_flash_sp_iq"), bind(*bufs, out, _step(ctx, q0=q0)), 512**-0.5, [32, 1, 1])
+        got.append(out.read())
+    assert np.array_equal(*got)
 
 
 @pytest.mark.parametrize("name,n", [("rmsnorm_256", 256), ("rmsnorm_512_plus1", 512)])
