@@ -306,7 +306,6 @@ constexpr int APPEND_THREADS = 128, APPEND_BLOCKS = 8;
 constexpr int ROW_LANES = 8;
 constexpr int MOST_SLOTS = 32;  // groups per token and grid row
 constexpr int ROWS_EACH = 4;   // rows of a group where a launch has more than it takes to fill the GPU
-constexpr int ROWS_AHEAD = 1;  // whose loads are under way at a time: registers for eight blocks an SM are worth more
 
 template <bool PLUS_ONE>
 __global__ void __launch_bounds__(APPEND_THREADS, APPEND_BLOCKS)
@@ -430,16 +429,8 @@ __global__ void __launch_bounds__(APPEND_THREADS, APPEND_BLOCKS)
         }
     };
     const uint32_t stride = gridDim.y << slot_bits;
-    for (uint32_t base = blockIdx.y << slot_bits; base < rows; base += ROWS_AHEAD * stride) {
-        Octets u[ROWS_AHEAD];
-#pragma unroll
-        for (int k = 0; k < ROWS_AHEAD; k++) u[k] = octets(base + k * stride + slot);
-#pragma unroll
-        for (int k = 0; k < ROWS_AHEAD; k++) {
-            if (base + k * stride >= rows) break;  // uniform over the block
-            work(base + k * stride, u[k]);
-        }
-    }
+    // one row's loads under way at a time: registers for eight blocks an SM are worth more (append_shape)
+    for (uint32_t base = blockIdx.y << slot_bits; base < rows; base += stride) work(base, octets(base + slot));
 }
 
 struct AppendShape {
