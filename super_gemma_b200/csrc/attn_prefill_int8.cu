@@ -702,13 +702,13 @@ __global__ void __launch_bounds__(INT8_THREADS, 1)
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// [row][head][512] tensor of `elem`-byte values, boxes of 128 bytes x box_heads x box_rows.
-int encode_rows(const LaunchArgs& a, CUtensorMap* tm, const void* base, uint64_t rows, uint64_t heads, int elem, uint32_t box_heads, uint32_t box_rows)
+// V as [row][head][512] f16, boxes of 64 dims x one head x 64 rows.
+int encode_v(const LaunchArgs& a, CUtensorMap* tm, const KvOperand& v, uint64_t heads)
 {
-    const uint64_t dims[3] = {HD, heads, rows};
-    const uint64_t strides[2] = {(uint64_t)HD * elem, heads * HD * elem};
-    const uint32_t box[3] = {128u / elem, box_heads, box_rows};
-    return encode_tensor_map(a, tm, elem == 2, 3, const_cast<void*>(base), dims, strides, box, 3);
+    const uint64_t dims[3] = {HD, heads, v.rows};
+    const uint64_t strides[2] = {HD * 2, heads * HD * 2};
+    const uint32_t box[3] = {64, 1, 64};
+    return encode_tensor_map(a, tm, 1, 3, const_cast<void*>(v.data), dims, strides, box, 3);
 }
 
 }  // namespace
@@ -730,7 +730,7 @@ int launch_prefill_int8(const LaunchArgs& a, const void* q, const __half* q_scal
 {
     const Int8Params prm{(const uint32_t*)step, (__half*)out, a.status, q_scales, m, n_kv, scale, q, k, v};
     CUtensorMap tv;
-    if (int r = encode_rows(a, &tv, v.data, v.rows, n_kv, 2, 1, 64)) return r;
+    if (int r = encode_v(a, &tv, v, n_kv)) return r;
     {
         static std::mutex attr_mutex;
         static bool attr_set[64] = {};
