@@ -79,13 +79,22 @@ def test_ring_and_chunk(ctx, q0, m):
     assert_close(out.read().reshape(m, NKV * G, D), _want(q, k, v, m, q0 - base, 1024), what=f"ring q0={q0} m={m}")
 
 
+@pytest.mark.parametrize("pieces", [1, 3])
 @pytest.mark.parametrize("m,q0", [(64, 100), (64, 300), (70, 900)])
-def test_maxima_that_rise_in_every_tile(ctx, m, q0):
-    """Scores grow along the keys by far more than 2^8 a tile: every tile raises the maximum, rescales O and the sum."""
+def test_maxima_that_rise_in_every_tile(ctx, monkeypatch, m, q0, pieces):
+    """Keys along the queries' common direction, longer with every position: each tile's maximum is more than 2^8 above the one before, so every
+    tile of every row raises it and rescales O and the sum."""
+    monkeypatch.setenv("SGB_FLASH_PIECES", str(pieces))
     q, k, v = _case(7, m, q0)
-    q = np.repeat(q[:, ::G], G, axis=1)
-    k = (k.astype(np.float32) + np.arange(q0 + m)[:, None, None] * 0.02 * q.astype(np.float32).mean(0)[::G][None]).astype(np.float16)
-    assert_close(_linear(ctx, q, k, v, m, q0, 0, scale=1.0), _want(q, k, v, m, q0, 0, 1.0), what=f"rising m={m} q0={q0}")
+    along = normal_f16(8, NKV, D).astype(np.float32)
+    q = (0.05 * q.astype(np.float32) + np.repeat(along, G, axis=0)[None]).astype(np.float16)
+    k = (0.05 * k.astype(np.float32) + 0.16 / D * np.arange(q0 + m)[:, None, None] * along[None]).astype(np.float16)
+    for h in range(NKV * G):  # the premise, in bits
+        s = q[:, h].astype(np.float64) @ k[:, h // G].astype(np.float64).T * np.log2(np.e)
+        for t in range(m):
+            full = (q0 + t + 1) // 64
+            assert np.all(np.diff(s[t, : 64 * full].reshape(full, 64).max(1)) > 8)
+    assert_close(_linear(ctx, q, k, v, m, q0, 0, scale=1.0), _want(q, k, v, m, q0, 0, 1.0), what=f"rising m={m} q0={q0} pieces={pieces}")
 
 
 @pytest.mark.parametrize("value", [np.inf, np.nan])
