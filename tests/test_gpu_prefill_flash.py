@@ -1,6 +1,7 @@
 """The head_dim-128 flash prefill kernel where its tiles can go wrong: one to seven tiles of 64 keys, ends on both sides of a tile,
 windows that begin inside one, the ring's wrap, pieces of the key range, maxima that rise from tile to tile, values that are not
-finite, and key buffers that are longer than the keys.
+finite, and key buffers that are longer than the keys.  SGB_FLASH_LONG, which some of the tests set, chose a second kernel with 128-key
+tiles that is no longer there: nothing reads it, and what they ask holds for the one kernel.
 Against the f64 oracle at the head_dim-128 tolerance (P is f16: 2^-11 of the largest |v|)."""
 import numpy as np
 import pytest
@@ -54,13 +55,14 @@ def test_windows(ctx, m, q0, window):
     assert_close(_linear(ctx, q, k, v, m, q0, window), _want(q, k, v, m, q0, window), what=f"m={m} q0={q0} window={window}")
 
 
-@pytest.mark.parametrize("pieces", [1, 3])
+@pytest.mark.parametrize("long,pieces", [(0, 1), (1, 1), (1, 3)])
 @pytest.mark.parametrize("m,q0", EDGES)
-def test_tiles(ctx, monkeypatch, m, q0, pieces):
+def test_tiles(ctx, monkeypatch, m, q0, long, pieces):
+    monkeypatch.setenv("SGB_FLASH_LONG", str(long))
     monkeypatch.setenv("SGB_FLASH_PIECES", str(pieces))
     q, k, v = _case(m + 3 * q0, m, q0)
     got = _linear(ctx, q, k, v, m, q0, 0)
-    assert_close(got, _want(q, k, v, m, q0, 0), what=f"m={m} q0={q0} pieces={pieces}")
+    assert_close(got, _want(q, k, v, m, q0, 0), what=f"m={m} q0={q0} long={long} pieces={pieces}")
     assert np.array_equal(got.view(np.uint32), _linear(ctx, q, k, v, m, q0, 0).view(np.uint32))
 
 
@@ -79,9 +81,35 @@ def test_ring_and_chunk(ctx, q0, m):
     assert_close(out.read().reshape(m, NKV * G, D), _want(q, k, v, m, q0 - base, 1024), what=f"ring q0={q0} m={m}")
 
 
+@pytest.mark.parametrize("long", [0, 1])
+@pytest.mark.parametrize("m,q0", [(64, 100), (64, 300), (70, 900)])
+def test_maxima_that_rise_in_every_tile(ctx, monkeypatch, m, q0, long):
+    """Scores grow along the keys by far more than 2^8 a tile: every tile raises the maximum, rescales O and both groups' sums."""
+    monkeypatch.setenv("SGB_FLASH_LONG", str(long))
+    q, k, v = _case(7, m, q0)
+    q = np.repeat(q[:, ::G], G, axis=1)
+    k = (k.astype(np.float32) + np.arange(q0 + m)[:, None, None] * 0.02 * q.astype(np.float32).mean(0)[::G][None]).astype(np.float16)
+    assert_close(_linear(ctx, q, k, v, m, q0, 0, scale=1.0), _want(q, k, v, m, q0, 0, 1.0), what=f"rising m={m} q0={q0}")
+
+
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+def test_values_that_are_not_finite_stay_with_the_blocks_that_see_them(ctx, monkeypatch, value):
+    """The long kernel: V rows of a tile that no query of a 64-token block sees leave its bits alone."""
+    monkeypatch.setenv("SGB_FLASH_LONG", "1")
+    m, q0, at = 256, 130, 250  # the row of position 250 is seen by queries 120 and later
+    q, k, v = _case(11, m, q0)
+    clean = _linear(ctx, q, k, v, m, q0, 0)
+    v2 = v.copy()
+    v2[at, 1, 5] = value
+    got = _linear(ctx, q, k, v2, m, q0, 0)
+    assert np.array_equal(got[:64].view(np.uint32), clean[:64].view(np.uint32))
+    assert np.array_equal(got[:, :G].view(np.uint32), clean[:, :G].view(np.uint32))  # the other kv head
+    assert not np.any(np.isfinite(got[120:, G:, 5]))
+
+
 @pytest.mark.parametrize("pieces", [1, 3])
 @pytest.mark.parametrize("m,q0", [(64, 100), (64, 300), (70, 900)])
-def test_maxima_that_rise_in_every_tile(ctx, monkeypatch, m, q0, pieces):
+def test_maxima_more_than_the_threshold_above_the_last_tiles(ctx, monkeypatch, m, q0, pieces):
     """Keys along the queries' common direction, longer with every position: each tile's maximum is more than 2^8 above the one before, so every
     tile of every row raises it and rescales O and the sum."""
     monkeypatch.setenv("SGB_FLASH_PIECES", str(pieces))
@@ -95,20 +123,6 @@ def test_maxima_that_rise_in_every_tile(ctx, monkeypatch, m, q0, pieces):
             full = (q0 + t + 1) // 64
             assert np.all(np.diff(s[t, : 64 * full].reshape(full, 64).max(1)) > 8)
     assert_close(_linear(ctx, q, k, v, m, q0, 0, scale=1.0), _want(q, k, v, m, q0, 0, 1.0), what=f"rising m={m} q0={q0} pieces={pieces}")
-
-
-@pytest.mark.parametrize("value", [np.inf, np.nan])
-def test_values_that_are_not_finite_stay_with_the_blocks_that_see_them(ctx, value):
-    """V rows of a tile that no query of a 64-token block sees leave its bits alone."""
-    m, q0, at = 256, 130, 250  # the row of position 250 is seen by queries 120 and later
-    q, k, v = _case(11, m, q0)
-    clean = _linear(ctx, q, k, v, m, q0, 0)
-    v2 = v.copy()
-    v2[at, 1, 5] = value
-    got = _linear(ctx, q, k, v2, m, q0, 0)
-    assert np.array_equal(got[:64].view(np.uint32), clean[:64].view(np.uint32))
-    assert np.array_equal(got[:, :G].view(np.uint32), clean[:, :G].view(np.uint32))  # the other kv head
-    assert not np.any(np.isfinite(got[120:, G:, 5]))
 
 
 def test_rows_behind_the_keys_do_not_change_the_bits(ctx, monkeypatch):
