@@ -70,10 +70,10 @@ __device__ __forceinline__ float row_inv_rms(const float (&x)[32])
 }
 
 // rmsnorm_<ROW_LEN>[_plus1]: x f16[rows x ROW_LEN], w f32[ROW_LEN], y f16.  grid [rows].  y = f16(x * inv * weight), weight = 1 + w with
-// PLUS_ONE (rmsnorm.wgsl:52-58).  A few rows are one memory latency: the weights are asked for together with the values, 16 bytes at a
-// time where the caller's array allows it (one by one and behind the sum of squares, 32 rows of 512 took 4.0 us in a recorded
-// chain).
-template <int BPR, bool PLUS_ONE>
+// PLUS_ONE (rmsnorm.wgsl:52-58).  A few rows are one memory latency: the weights are asked for together with the values (AHEAD), 16 bytes
+// at a time where the caller's array allows it (one by one and behind the sum of squares, 32 rows of 512 took 4.0 us in a recorded
+// chain, with AHEAD 2.6).  That takes 75 registers, three blocks an SM; without AHEAD it is 47, five.  rmsnorm_ahead() chooses.
+template <int BPR, bool PLUS_ONE, bool AHEAD>
 __global__ void __launch_bounds__(PRE_THREADS) rmsnorm_kernel(const __half* x, const float* w,
                                                               __half* __restrict__ y, size_t n_blocks)
 {
@@ -81,22 +81,24 @@ __global__ void __launch_bounds__(PRE_THREADS) rmsnorm_kernel(const __half* x, c
     pdl_launch_dependents();
     const size_t blk = (size_t)blockIdx.x * PRE_THREADS + threadIdx.x;
     const bool live = blk < n_blocks;  // whole rows only, and BPR divides 32: a row never straddles a warp
+    const float* wp = w + (blk % BPR) * 32;
     float v[32], wv[32];
     if (live) {
         load_f16x32(x + blk * 32, v);
-        const float* wp = w + (blk % BPR) * 32;
-        if ((reinterpret_cast<uintptr_t>(w) & 15) == 0) {
+        if constexpr (AHEAD) {
+            if ((reinterpret_cast<uintptr_t>(w) & 15) == 0) {
 #pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const float4 f = ld_global(reinterpret_cast<const float4*>(wp) + i);
-                wv[4 * i] = f.x;
-                wv[4 * i + 1] = f.y;
-                wv[4 * i + 2] = f.z;
-                wv[4 * i + 3] = f.w;
+                for (int i = 0; i < 8; i++) {
+                    const float4 f = ld_global(reinterpret_cast<const float4*>(wp) + i);
+                    wv[4 * i] = f.x;
+                    wv[4 * i + 1] = f.y;
+                    wv[4 * i + 2] = f.z;
+                    wv[4 * i + 3] = f.w;
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 32; i++) wv[i] = ld_global(wp + i);
             }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 32; i++) wv[i] = ld_global(wp + i);
         }
     } else {
 #pragma unroll
@@ -105,7 +107,10 @@ __global__ void __launch_bounds__(PRE_THREADS) rmsnorm_kernel(const __half* x, c
     const float inv = row_inv_rms<BPR>(v);
     if (!live) return;
 #pragma unroll
-    for (int i = 0; i < 32; i++) v[i] = v[i] * inv * (PLUS_ONE ? 1.0f + wv[i] : wv[i]);
+    for (int i = 0; i < 32; i++) {
+        const float weight = AHEAD ? wv[i] : ld_global(wp + i);
+        v[i] = v[i] * inv * (PLUS_ONE ? 1.0f + weight : weight);
+    }
     uint4 out[4];
     pack_f16x32(v, out);
     uint4* o = reinterpret_cast<uint4*>(y + blk * 32);
@@ -453,6 +458,18 @@ inline AppendShape append_shape(const LaunchArgs& a, size_t tokens, uint32_t row
     return {dim3((uint32_t)((groups * ROW_LANES + APPEND_THREADS - 1) / APPEND_THREADS), per_thread == 1 ? min(1024u, per_token) : 1), bits};
 }
 
+// Whether rmsnorm asks for its weights ahead: rows of 512 whose weights lie on 16 bytes always, others but where the measurements say
+// otherwise, us in a recorded chain of launches, ahead | not.  Up to 3 blocks for 2 SMs a launch and the one behind it stand side by side: rows of 256, 32
+// of them 2.6 | 3.1, 6000 4.6 | 4.7.  Up to 2 an SM they do so only with five blocks an SM: 8192 6.3 | 4.8; rows of 512 with weights on 4 bytes, 4096
+// 9.8 | 6.9.  Up to 8: 10000 6.3 | 6.5, 16384 8.0 | 11.7, 32768 14.7 | 15.7.  Beyond, what counts is the bytes under way: 65536 27.5 | 26.6; of 512, on 4
+// bytes, 82.8 | 81.4.  (Rows of 512 on 16 bytes: 4096 6.3 | 7.0, 16384 15.3 | 23.0, 65536 53.5 | 81.7.)
+inline bool rmsnorm_ahead(const LaunchArgs& a, uint32_t grid, int row_len, const void* w)
+{
+    if (row_len == 512 && (reinterpret_cast<uintptr_t>(w) & 15) == 0) return true;
+    const uint64_t halves = 2 * (uint64_t)grid, sms = a.sm_count;
+    return halves <= 3 * sms || (halves > 4 * sms && halves <= 16 * sms);
+}
+
 inline uint32_t grid_for(size_t n) { return (uint32_t)((n + PRE_THREADS - 1) / PRE_THREADS); }
 
 struct PushNormRope {
@@ -477,7 +494,8 @@ int launch_rmsnorm(const LaunchArgs& a)
     const size_t n_blocks = a.b[0].bytes / 64;
     if (n_blocks == 0) return 0;
     if (int r = need_aligned(a, {16, 4, 16})) return r;
-    const cudaError_t e = launch_dependent(rmsnorm_kernel<ROW_LEN / 32, PLUS_ONE != 0>, dim3(grid_for(n_blocks)), dim3(PRE_THREADS), 0, a.stream, (const __half*)a.b[0].ptr, (const float*)a.b[1].ptr, (__half*)a.b[2].ptr, n_blocks);
+    const auto kernel = rmsnorm_ahead(a, grid_for(n_blocks), ROW_LEN, a.b[1].ptr) ? rmsnorm_kernel<ROW_LEN / 32, PLUS_ONE != 0, true> : rmsnorm_kernel<ROW_LEN / 32, PLUS_ONE != 0, false>;
+    const cudaError_t e = launch_dependent(kernel, dim3(grid_for(n_blocks)), dim3(PRE_THREADS), 0, a.stream, (const __half*)a.b[0].ptr, (const float*)a.b[1].ptr, (__half*)a.b[2].ptr, n_blocks);
     ++*a.launches;
     return check_cuda(a, e, "rmsnorm");
 }

@@ -152,3 +152,25 @@ def test_rmsnorm_weights_on_their_own_alignment(ctx, name, n):
         ctx.dispatch_blocking(ctx.load_kernel(name), bind(ctx.buffer_from_iter(x), _moved(ctx, w, by), y), None, [rows, 1, 1])
         got.append(y.read())
     assert np.array_equal(*got) and np.any(got[0] != 0)
+
+
+@pytest.mark.parametrize("name,n,by", [("rmsnorm_256", 256, 0), ("rmsnorm_256_plus1", 256, 4), ("rmsnorm_512", 512, 4), ("rmsnorm_512_plus1", 512, 0)])
+def test_rmsnorm_of_many_rows_gives_the_bits_of_few(ctx, name, n, by):
+    """Weights asked for ahead or behind the sum of squares, by the size of the launch: 3 / 2, 2 and 8 blocks an SM and one row more, and the
+    same rows two thousand at a time."""
+    import torch
+
+    sms, per_block = torch.cuda.get_device_properties(0).multi_processor_count, 256 * 32 // n
+    w = _moved(ctx, np.random.default_rng(n).standard_normal(n, dtype=np.float32), by)
+    kernel = ctx.load_kernel(name)
+    x = normal_f16(n, 8 * sms * per_block + 1, n)
+
+    def run(rows):
+        y = ctx.new_buffer(rows.size, np.uint16)
+        ctx.dispatch_blocking(kernel, bind(ctx.buffer_from_iter(rows), w, y), None, [len(rows), 1, 1])
+        return y.read().reshape(rows.shape)
+
+    few = np.concatenate([run(x[i:i + 2000]) for i in range(0, len(x), 2000)])
+    for blocks in (3 * sms // 2, 2 * sms, 8 * sms):
+        for rows in (blocks * per_block, blocks * per_block + 1):
+            assert np.array_equal(run(x[:rows]), few[:rows]), (blocks, rows)
