@@ -312,8 +312,8 @@ constexpr int ROW_LANES = 8;
 constexpr int MOST_SLOTS = 32;  // groups per token and grid row
 constexpr int ROWS_EACH = 4;   // rows of a group where a launch has more than it takes to fill the GPU
 
-template <bool PLUS_ONE>
-__global__ void __launch_bounds__(APPEND_THREADS, APPEND_BLOCKS)
+template <bool PLUS_ONE, bool AHEAD>
+__global__ void __launch_bounds__(APPEND_THREADS, AHEAD ? APPEND_BLOCKS / 2 : APPEND_BLOCKS)
     kv_norm_rope_append_kernel(const __half* q_raw, const float* q_w, __half* __restrict__ q_out,
                                uint32_t n_q, const __half* k_raw, const __half* v_raw, const float* k_w,
                                const float2* cos_sin, __half* __restrict__ k_scales, int8_t* __restrict__ k_quants,
@@ -373,6 +373,14 @@ __global__ void __launch_bounds__(APPEND_THREADS, APPEND_BLOCKS)
         const bool live = r < rows, is_q = r < n_q, is_v = r >= n_q + n_kv;
         const uint32_t head = is_q ? r : is_v ? r - n_q - n_kv : r - n_q;
         uint32_t own[8] = {u.lo.x, u.lo.y, u.lo.z, u.lo.w, u.hi.x, u.hi.y, u.hi.z, u.hi.w};
+        float4 wt[4];
+        if constexpr (AHEAD) {
+            if (live && !is_v) {
+                const float4* w = reinterpret_cast<const float4*>((is_q ? q_w : k_w) + 8 * o);
+#pragma unroll
+                for (int j = 0; j < 4; j++) wt[j] = ld_global(w + (j >> 1) * 16 + (j & 1));
+            }
+        }
         float ss[2] = {0.0f, 0.0f};
         float2 v[8];
 #pragma unroll
@@ -394,7 +402,7 @@ __global__ void __launch_bounds__(APPEND_THREADS, APPEND_BLOCKS)
             const float4* w = reinterpret_cast<const float4*>((is_q ? q_w : k_w) + 8 * o);
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const float4 f = ld_global(w + (j >> 1) * 16 + (j & 1));
+                const float4 f = AHEAD ? wt[j] : ld_global(w + (j >> 1) * 16 + (j & 1));
                 const float2 one = make_float2(1.0f, 1.0f), w0 = make_float2(f.x, f.y), w1 = make_float2(f.z, f.w);
                 v[2 * j] = mul2_rn(v[2 * j], PLUS_ONE ? add2_rn(one, w0) : w0);
                 v[2 * j + 1] = mul2_rn(v[2 * j + 1], PLUS_ONE ? add2_rn(one, w1) : w1);
@@ -441,12 +449,16 @@ __global__ void __launch_bounds__(APPEND_THREADS, APPEND_BLOCKS)
 struct AppendShape {
     dim3 grid;
     uint32_t slot_bits;
+    bool ahead;  // weights asked for together with the values
 };
 // Slots and blocks.  Few rows: one per group, which takes least time for one; beyond, two, then ROWS_EACH of them, which takes least
 // instructions per row, and few rows a token (few kv heads) put several tokens into a block.  us in a recorded chain, 1 row | 2 | 4: 16 kv
 // heads with q, 64 tokens 2.6 | 3.2 | 4.6, 290 tokens 4.1 | 4.1 | 5.1, 600 tokens 7.4 | 6.9 | 8.4, 1024 tokens 10.5 | 9.3 | 8.9, 4096 tokens
 // 37 | 32 | 30; 4 kv heads, 1000 tokens 4.2 | 3.9 | 5.0, 2000 tokens 6.9 | 5.7 | 6.0, 8192 tokens 19.3 | 15.3 | 14.4.  Six blocks an SM and two
 // rows' loads under way took 31.6 for 4096 tokens, five and four 32.6.
+// Up to 48 rows an SM a launch is one memory latency, and it and the one behind it stand side by side on the GPU (three blocks each, of the six that
+// 78 registers leave): the weights are asked for together with the values.  One token of 16 kv heads 1.87 us, with weights 1 + w 2.03; behind the
+// sum of squares 2.00 and 2.11.  128 tokens of 16 kv heads, 56 rows an SM: 3.38 | 2.76 with eight blocks and the weights behind the sum.
 inline AppendShape append_shape(const LaunchArgs& a, size_t tokens, uint32_t rows)
 {
     const size_t per_sm = (tokens * rows + a.sm_count - 1) / a.sm_count;
@@ -455,7 +467,13 @@ inline AppendShape append_shape(const LaunchArgs& a, size_t tokens, uint32_t row
     while ((1u << bits) < MOST_SLOTS && (per_thread << bits) < rows) bits++;
     const size_t groups = tokens << bits;  // < 2^29: at most 2^26 rows of q and of k
     const uint32_t per_token = (rows + (1u << bits) - 1) >> bits;
-    return {dim3((uint32_t)((groups * ROW_LANES + APPEND_THREADS - 1) / APPEND_THREADS), per_thread == 1 ? min(1024u, per_token) : 1), bits};
+    return {dim3((uint32_t)((groups * ROW_LANES + APPEND_THREADS - 1) / APPEND_THREADS), per_thread == 1 ? min(1024u, per_token) : 1), bits, per_sm <= 48};
+}
+
+inline auto append_kernel(bool plus_one, bool ahead)
+{
+    return plus_one ? (ahead ? kv_norm_rope_append_kernel<true, true> : kv_norm_rope_append_kernel<true, false>)
+                    : (ahead ? kv_norm_rope_append_kernel<false, true> : kv_norm_rope_append_kernel<false, false>);
 }
 
 // Whether rmsnorm asks for its weights ahead: rows of 512 whose weights lie on 16 bytes always, others but where the measurements say
@@ -562,8 +580,8 @@ int launch_kv_norm_rope_append_paged_q8_d128(const LaunchArgs& a)
     if (kv_rows == 0) return 0;
     if (kv_rows >= (1u << 26)) return fail_validation(a, "kv_norm_rope_append_paged_q8_d128: at most 2^26 (token, head) rows per launch");
     if (int r = need_aligned(a, {16, 16, 16, 16, 2, 8, 2, 8, 4, 4})) return r;
-    auto kern = p.plus_one ? kv_norm_rope_append_kernel<true> : kv_norm_rope_append_kernel<false>;
     const AppendShape shape = append_shape(a, tokens, 2 * (p.row_len / 128));
+    const auto kern = append_kernel(p.plus_one != 0, shape.ahead);
     const cudaError_t e = launch_dependent(kern, shape.grid, dim3(APPEND_THREADS), 0, a.stream,
         nullptr, nullptr, nullptr, 0u,
         (const __half*)a.b[0].ptr, (const __half*)a.b[1].ptr, (const float*)a.b[2].ptr, (const float2*)a.b[3].ptr, (__half*)a.b[4].ptr,
@@ -599,8 +617,8 @@ int launch_qkv_norm_rope_append_paged_q8_d128(const LaunchArgs& a)
     if (kv_rows >= (1u << 26) || q_rows >= (1u << 26))
         return fail_validation(a, "qkv_norm_rope_append_paged_q8_d128: at most 2^26 (token, head) rows of q and of k per launch");
     if (int r = need_aligned(a, {16, 16, 16, 16, 16, 16, 16, 2, 8, 2, 8, 4, 4})) return r;
-    auto kern = p.plus_one ? kv_norm_rope_append_kernel<true> : kv_norm_rope_append_kernel<false>;
     const AppendShape shape = append_shape(a, tokens, p.n_q_heads + 2 * (p.row_len / 128));
+    const auto kern = append_kernel(p.plus_one != 0, shape.ahead);
     const cudaError_t e = launch_dependent(kern, shape.grid, dim3(APPEND_THREADS), 0, a.stream,
         (const __half*)a.b[0].ptr, (const float*)a.b[1].ptr, (__half*)a.b[2].ptr, p.n_q_heads, (const __half*)kv[0].ptr,
         (const __half*)kv[1].ptr, (const float*)kv[2].ptr, (const float2*)kv[3].ptr, (__half*)kv[4].ptr, (int8_t*)kv[5].ptr,

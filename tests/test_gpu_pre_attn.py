@@ -261,3 +261,31 @@ def test_fused_kv_append_of_values_that_are_not_finite(ctx, rot, tokens):
     ctx.dispatch_blocking(app, bind(v16, b[2], b[3], table, step), (row, page), app.groups_for(tokens * row // 32))
     for x, y in zip(a, b):
         assert np.array_equal(x.read(), y.read())
+
+
+@pytest.mark.parametrize("tokens", [1, 444, 445])  # 16 rows each: up to 48 rows an SM, on 148 SMs, weights are asked for ahead
+@pytest.mark.parametrize("plus_one", [0, 1])
+def test_one_launch_qkv_on_both_sides_of_weights_asked_for_ahead(ctx, tokens, plus_one):
+    """Against the unfused pieces, and weights 1 + w against the same weights with the 1 added on the host, bit for bit."""
+    import super_gemma_b200 as sg
+
+    if not plus_one:
+        return test_one_launch_qkv_of_a_long_chunk(ctx, tokens, 4)
+    n_kv, page, rot = 4, 64, 128
+    pages = -(-tokens // page)
+    row, rows = n_kv * 128, pages * page
+    rng = np.random.default_rng(tokens)
+    up, mk = ctx.buffer_from_iter, lambda dt, n: ctx.new_buffer(n, dt)
+    qr, kr, vr = (up(rng.standard_normal(tokens * h * 128, dtype=np.float32).astype(np.float16)) for h in (2 * n_kv, n_kv, n_kv))
+    q_w, k_w = rng.standard_normal(128, dtype=np.float32), rng.standard_normal(128, dtype=np.float32)
+    csb, table, step = up(O.cos_sin_table(O.inv_freqs(rot, 1e6), 0, tokens)), up(np.arange(pages, dtype=np.uint32)), ctx.new_step_buffer()
+    sg.StepState(pos=0).write_to(step)
+    got = []
+    for flag in (1, 0):
+        w = [up(x if flag else np.float32(1) + x) for x in (q_w, k_w)]
+        out = [mk(np.uint16, tokens * 2 * row), mk(np.uint16, rows * row // 32), mk(np.int8, rows * row), mk(np.uint16, rows * row // 32), mk(np.int8, rows * row)]
+        ctx.dispatch_blocking(ctx.load_kernel("qkv_norm_rope_append_paged_q8_d128"), bind(qr, w[0], out[0], kr, vr, w[1], csb, *out[1:], table, step),
+                              (2 * n_kv, row, page, rot, flag), [1, 1, 1])
+        got.append([x.read() for x in out])
+    for x, y in zip(*got):
+        assert np.array_equal(x, y) and np.any(x != 0)
