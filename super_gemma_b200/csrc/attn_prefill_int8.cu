@@ -8,7 +8,8 @@
 // of which each CTA loads half the keys of K and half the dims of V.
 // Scores: Q's quants are exact as f16.  A key's quants times their f16 scale are whole multiples of the scale's last place, 19 bits, which
 // f16 hi + lo hold exactly (for scales above 511, whose quants overflow, in a second pass that splits otherwise); four warps make them from the cache's bytes.  A block's sum so lacks only the scale of Q, which is the
-// row's, and the softmax threads have nothing left to do for it but one multiply-add.  (Whole-number sums of int8 MMAs, scaled by
+// row's, and the softmax threads have nothing left to do for it but one multiply-add.  The pipe adds the block's 64 products up in f32 and
+// truncates, where a sum of int8 products is a whole number; the error against 64 bits is f16's own in both forms.  (Whole-number sums of int8 MMAs, scaled by
 // both scales in the softmax threads: they then read 16 x 128 scales a tile through shared memory, which the MMAs read their
 // operands from; 364 us.  The transposed form before it, keys and dims as M, took V as the MN-major A operand, 160 cycles
 // an instruction where 48 would do, and converted every sum with an instruction of a sixteenth of the rate: 529 us.)
